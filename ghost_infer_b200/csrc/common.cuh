@@ -23,6 +23,13 @@ bool pdl_enabled();                                // programmatic dependent lau
 int fail(int code, const char* fmt, ...);          // records the message for gi_last_error(), returns code
 int check_launch(const char* what);                // cudaGetLastError() -> GI_OK or a recorded failure
 
+// The order of a 32-bit product's sums (see gemm_f32.cu): SUM_SEGMENTS stretches of sum_segment(K) numbers, the last ones
+// shorter or empty.  A multiple of 32, so that every kernel's tile of K ends where a stretch does.
+constexpr int SUM_SEGMENTS = 32;
+inline int sum_segment(int K) { return ((K + SUM_SEGMENTS - 1) / SUM_SEGMENTS + 31) / 32 * 32; }
+bool gemm_f32_takes(const void* A, const void* W, int N, int K, long lda, long ldw);
+int gemm_f32(float* out, bool accum, const float* A, const float* W, int M, int N, int K, long lda, long ldw, long ldo, cudaStream_t s);
+
 // First statements of a kernel that may be launched with programmatic stream serialization: let the next
 // kernel in the stream begin its own set-up, then wait until everything before this kernel has completed and
 // is visible.  Both are no-ops for a plain launch.  Nothing a predecessor writes may be touched before this.

@@ -14,17 +14,17 @@ constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 template <typename TA, typename TW, typename TO, int MODE>
 __global__ void __launch_bounds__(256)
 gemm_tile_kernel(void* __restrict__ out_, const TA* __restrict__ A, const TW* __restrict__ W, int M, int N, int K,
-                 long lda, long ldw, long ldo) {
+                 long lda, long ldw, long ldo, int seg) {
   __shared__ float As[BK][BM + 4];
   __shared__ float Ws[BK][BN + 4];
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int tx = tid % 16, ty = tid / 16;  // thread owns rows ty*4..+4, cols tx*4..+4
-  float acc[TM][TN];
+  float acc[2][TM][TN], sum[TM][TN];  // even k, odd k; finished stretches
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[1][i][j] = sum[i][j] = 0.f;
 
   for (int k0 = 0; k0 < K; k0 += BK) {
     // 64 rows x 16 k per operand = 1024 elements, 4 per thread; consecutive threads walk k (contiguous)
@@ -52,9 +52,18 @@ gemm_tile_kernel(void* __restrict__ out_, const TA* __restrict__ A, const TW* __
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+        for (int j = 0; j < TN; ++j) acc[kk & 1][i][j] = fmaf(a[i], w[j], acc[kk & 1][i][j]);
     }
     __syncthreads();
+    if ((k0 + BK) % seg == 0 || k0 + BK >= K) {  // a stretch ends
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          sum[i][j] = __fadd_rn(sum[i][j], __fadd_rn(acc[0][i][j], acc[1][i][j]));
+          acc[0][i][j] = acc[1][i][j] = 0.f;
+        }
+    }
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -66,9 +75,9 @@ gemm_tile_kernel(void* __restrict__ out_, const TA* __restrict__ A, const TW* __
       if (n >= N) continue;
       if (MODE == GI_GEMM_ACCUM_F32) {
         float* o = (float*)out_ + (size_t)m * ldo + n;
-        *o = *o + acc[i][j];
+        *o = *o + sum[i][j];
       } else {
-        gi::stf((TO*)out_ + (size_t)m * ldo + n, acc[i][j]);
+        gi::stf((TO*)out_ + (size_t)m * ldo + n, sum[i][j]);
       }
     }
   }
@@ -77,13 +86,14 @@ gemm_tile_kernel(void* __restrict__ out_, const TA* __restrict__ A, const TW* __
 template <typename TA, typename TW>
 int launch(void* out, int out_dtype, int mode, const void* A, const void* W, int M, int N, int K, long lda, long ldw,
            long ldo, cudaStream_t s) {
+  const int seg = gi::sum_segment(K);
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (mode == GI_GEMM_ACCUM_F32) {
-    gemm_tile_kernel<TA, TW, float, GI_GEMM_ACCUM_F32><<<grid, 256, 0, s>>>(out, (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldo);
+    gemm_tile_kernel<TA, TW, float, GI_GEMM_ACCUM_F32><<<grid, 256, 0, s>>>(out, (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldo, seg);
   } else if (out_dtype == GI_F32) {
-    gemm_tile_kernel<TA, TW, float, GI_GEMM_STORE><<<grid, 256, 0, s>>>(out, (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldo);
+    gemm_tile_kernel<TA, TW, float, GI_GEMM_STORE><<<grid, 256, 0, s>>>(out, (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldo, seg);
   } else {
-    gemm_tile_kernel<TA, TW, __nv_bfloat16, GI_GEMM_STORE><<<grid, 256, 0, s>>>(out, (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldo);
+    gemm_tile_kernel<TA, TW, __nv_bfloat16, GI_GEMM_STORE><<<grid, 256, 0, s>>>(out, (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldo, seg);
   }
   return gi::check_launch("gemm_generic");
 }
@@ -98,6 +108,8 @@ extern "C" int gi_gemm_generic(void* out, int out_dtype, int mode, const void* A
   if (mode == GI_GEMM_ACCUM_F32 && out_dtype != GI_F32) return gi::fail(GI_ERR_ARG, "gemm: accumulation needs a float output");
   if ((N + BN - 1) / BN > 2147483647 || (M + BM - 1) / BM > 65535)
     return gi::fail(GI_ERR_UNSUPPORTED, "gemm: %d rows are more than one launch takes (%d)", M, 65535 * BM);
+  if (a_dtype == GI_F32 && w_dtype == GI_F32 && out_dtype == GI_F32 && gi::gemm_f32_takes(A, W, N, K, lda, ldw))
+    return gi::gemm_f32((float*)out, mode == GI_GEMM_ACCUM_F32, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldo, (cudaStream_t)stream);
   GI_DISPATCH_DTYPE(a_dtype, TA, GI_DISPATCH_DTYPE(w_dtype, TW,
       return (launch<TA, TW>(out, out_dtype, mode, A, W, M, N, K, lda, ldw, ldo, (cudaStream_t)stream))));
   return GI_OK;

@@ -1104,3 +1104,35 @@ def test_prompt_attention_with_one_row_warp_far_behind_the_others(hd, slow_warp)
                 torch.testing.assert_close(out.double(), ref, rtol=2e-2, atol=2e-2)
         finally:
             ops.attn_prefill_t5_pairing(1)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 16, 32), (1, 2055, 4), (2, 17, 36), (3, 130, 1028), (4, 2048, 2048), (5, 33, 512), (8, 1000, 3076),
+                                   (9, 31, 1024), (16, 48, 2080), (17, 129, 96), (33, 16400, 64), (49, 100, 320), (65, 2047, 1100),
+                                   (300, 384, 2048)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_float32_products_share_one_order_of_additions(m, n, k, accumulate):
+    """The kernels of few and of many rows and the general one (which takes rows that start off a 16-byte boundary) give
+    the same bits; |error| <= (terms in a chain + chains + 2) * 2^-24 * sum |a w|, the bound of any summation."""
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(m * 7 + n + k)
+    a = torch.randn((m, k), generator=gen, device=DEV)
+    w = torch.randn((n, k), generator=gen, device=DEV)
+    start = torch.randn((m, n), generator=gen, device=DEV)
+
+    def product(a, w):
+        if not accumulate:
+            return ops.gemm_generic(a, w)
+        out = start.clone()
+        return ops.gemm_generic(a, w, out=out, accumulate=True)
+
+    got = product(a, w)
+    odd = torch.empty((n, k + 1), device=DEV)
+    odd[:, :k] = w
+    assert torch.equal(got, product(a, odd[:, :k]))                      # general kernel
+    assert torch.equal(got[:1], ops.gemm_generic(a[:1], w, out=start[:1].clone(), accumulate=True) if accumulate else ops.gemm_generic(a[:1], w))
+    many = ops.gemm_generic(a.repeat((600 + m - 1) // m, 1), w)          # enough rows for the tiled kernel
+    assert accumulate or torch.equal(got, many[:m])
+    chain = ((k + 31) // 32 + 31) // 32 * 16
+    exact = a.double() @ w.double().T + (start.double() if accumulate else 0)
+    bound = (a.double().abs() @ w.double().abs().T + start.double().abs()) * (chain + 32 + 3) * 2.0 ** -24
+    assert ((got.double() - exact).abs() <= bound).all()
