@@ -81,6 +81,7 @@ def _bind():
         "gi_kv_store": [P, I, L, P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, P],
         "gi_mamba2_conv": [P, P, I, L, P, P, I, P, L, I, P, P, I, I, I, I, I, I, P],
         "gi_mamba2_conv_update": [P, I, L, P, L, I, P, P, I, I, I, I, I, P],
+        "gi_mamba2_chunks": [P, P, P, L, P, P, P, P, L, I, P, P, I, I, I, I, I, P],
         "gi_mamba2_scan": [P, P, P, I, L, P, P, P, I, P, L, I, P, P, I, I, I, I, I, P],
         "gi_mamba2_gate_norm": [P, I, P, P, I, L, P, I, I, I, I, F, P],
         "gi_moe_route": [P, P, P, P, I, L, P, P, I, I, I, I, I, P],
@@ -1497,6 +1498,17 @@ def mamba2_conv(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, 
     return out
 
 
+# tokens of a step's longest sequence from which the recurrence goes 64 tokens at a time
+MAMBA2_CHUNKS_FROM = 24
+
+
+def mamba2_chunks_ok(xbc: torch.Tensor, dt_bias: torch.Tensor, head_dim: int, n_state: int) -> bool:
+    """16-bit rows read 16 bytes at a time, a state that fits the warps of a block; the 32-bit path keeps the walk, whose
+    bits do not depend on how a prompt is cut."""
+    return (xbc.dtype == torch.bfloat16 and dt_bias.dtype == torch.float32 and head_dim % 8 == 0 and n_state % 8 == 0
+            and n_state <= 128 and xbc.data_ptr() % 16 == 0)
+
+
 def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
                 state: torch.Tensor, step, heads: int, head_dim: int, n_state: int, groups: int, taps: int) -> torch.Tensor:
     """The recurrence over the step's tokens from and into `state`; float32 [tokens, heads * head_dim]."""
@@ -1514,6 +1526,12 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_bias: torch.Tensor, a_
         if t.numel() != heads or t.dtype != dt_bias.dtype or not t.is_contiguous():
             raise KernelError(f"the recurrence's per-head constants must be {heads} values of one type")
     y = torch.empty((proj.shape[0], inner), dtype=torch.float32, device=proj.device)
+    if mamba2_chunks_ok(xbc, dt_bias, head_dim, n_state) and step.max_q_len >= MAMBA2_CHUNKS_FROM:
+        _check(lib, lib.gi_mamba2_chunks(y.data_ptr(), xbc.data_ptr(), proj.data_ptr(), _rows(proj, "projected rows"), dt_bias.data_ptr(),
+                                         a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), state.stride(0), state.shape[0],
+                                         _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"), step.n_seqs, heads,
+                                         head_dim, n_state, groups, _stream()))
+        return y
     _check(lib, lib.gi_mamba2_scan(y.data_ptr(), xbc.data_ptr(), proj.data_ptr(), _dt(proj, "projected rows"),
                                    _rows(proj, "projected rows"), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
                                    _dt(dt_bias, "per-head constants"), state.data_ptr(), state.stride(0), state.shape[0],

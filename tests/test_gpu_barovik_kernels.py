@@ -297,3 +297,47 @@ def test_experts_expert_by_expert_on_tensor_cores():
     got = ops.moe_experts_by_expert(ops.moe_gather_rows(h, perm, top), gu, down, offsets.cpu().tolist())
     ops.check_status()
     assert (got - want).abs().max().item() < 0.02 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("sizes", [(64, 64, 128, 8, [2048]), (12, 40, 96, 4, [500, 1, 63]), (4, 24, 16, 2, [63, 65, 128, 17]), (2, 8, 40, 1, [130, 2]),
+                                   (3, 72, 72, 3, [64]), (2, 32, 8, 1, [24])])
+@pytest.mark.parametrize("rate", [(-1.0, -0.5), (-6.0, -2.0), (3.0, 1.0)])
+def test_recurrence_by_chunks_errs_no_more_than_the_walk(sizes, rate):
+    """Against 64 bits.  A sum of n terms in 32 bits errs by a few 2^-24 of the terms' size; the walk adds up one rounding per
+    token while a state is kept (thousands of tokens at the slow rates), so twice its error plus 2^-22 is the bound."""
+    heads, P, N, G, lens = sizes
+    g = torch.Generator(device=DEV).manual_seed(heads + N)
+    inner, ch, T = heads * P, heads * P + 2 * G * N, sum(lens)
+    xbc = torch.nn.functional.silu(torch.randn(T, ch, generator=g, device=DEV)).bfloat16()
+    proj = torch.randn(T, 2 * inner + 2 * G * N + heads, generator=g, device=DEV).bfloat16()
+    dt_bias, a_log, d_skip = (0.5 * torch.randn(heads, generator=g, device=DEV) + m for m in (*rate, 1.0))
+    before = torch.randn(len(lens) + 2, heads * N * P + 3 * ch, generator=g, device=DEV)
+    step = step_of(lens, [0] * len(lens), [n + 1 for n in range(len(lens))])
+    assert ops.mamba2_chunks_ok(xbc, dt_bias, P, N) and step.max_q_len >= ops.MAMBA2_CHUNKS_FROM
+    chunks = before.clone()
+    y = ops.mamba2_scan(xbc, proj, dt_bias, a_log, d_skip, chunks, step, heads, P, N, G, 4)
+    walk, y_walk = before.clone(), torch.empty_like(y)
+    lib = ops._bind()
+    assert lib.gi_mamba2_scan(y_walk.data_ptr(), xbc.data_ptr(), proj.data_ptr(), 1, proj.stride(0), dt_bias.data_ptr(), a_log.data_ptr(),
+                              d_skip.data_ptr(), 0, walk.data_ptr(), walk.stride(0), walk.shape[0], step.cu_seqlens.data_ptr(),
+                              step.seq_slots.data_ptr(), len(lens), heads, P, N, G, torch.cuda.current_stream().cuda_stream) == 0
+    x = xbc.double()
+    dt = torch.nn.functional.softplus(proj[:, 2 * inner + 2 * G * N:].double() + dt_bias.double())
+    keep = torch.exp(-torch.exp(a_log.double()) * dt)
+    X = x[:, :inner].view(T, heads, P)
+    B, C = (x[:, a:a + G * N].view(T, G, N).repeat_interleave(heads // G, 1) for a in (inner, inner + G * N))
+    want, state, at = torch.empty_like(X), before.double(), 0
+    for s, n in enumerate(lens):
+        S = state[s + 1, :heads * N * P].view(heads, P, N)
+        for t in range(at, at + n):
+            S.mul_(keep[t][:, None, None]).add_((dt[t][:, None] * X[t])[:, :, None] * B[t][:, None, :])
+            want[t] = (S * C[t][:, None, :]).sum(-1) + d_skip.double()[:, None] * X[t]
+        at += n
+    want = want.view(T, inner)
+
+    def err(a, b):
+        return ((a.double() - b).norm() / b.norm()).item()
+
+    assert err(y, want) <= 2 * err(y_walk, want) + 2.0 ** -22
+    assert err(chunks, state) <= 2 * err(walk, state) + 2.0 ** -22
+    assert torch.equal(chunks[:, heads * N * P:], before[:, heads * N * P:]) and torch.equal(chunks[0], before[0]) and torch.equal(chunks[-1], before[-1])
