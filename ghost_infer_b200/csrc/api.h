@@ -242,6 +242,17 @@ int gi_latent_prepare(void* cq, const void* in, int dtype, long ld, const void* 
 // [heads][r + dr]).
 int gi_latent_query_rot(void* qa, long ldqa, const void* q, long ldq, int dtype, const float* table, int rot, int n_tokens,
                         int n_heads, int dn, int dr, int r, void* stream);
+// A latent cache's rows (16-bit) of every sequence's positions that this step's tokens see, from a page boundary on, one below
+// the other; `max_rows`: of the longest.
+int gi_latent_gather(void* out, const void* cache, const int* block_table, int max_pages, const int* cu_seqlens, const int* seq_slots,
+                     const int* seq_pos0, int n_seqs, int max_rows, int hd, int window, void* stream);
+// Prompt attention over keys and values formed per head from those rows (see attention_prefill_t5.cu): q [heads][dim + rot],
+// k [heads][dim], r [rot] shared by the heads, v [heads][vdim], all 16-bit; dim 64 or 128, rot a multiple of 16 up to 64, vdim a
+// multiple of 8 up to 128.  sinks float[heads] or null; gate [tokens][heads] or null: a head's result times its sigmoid.
+int gi_attn_prefill_t5_rows(void* out, long ldo, const void* q, long ldq, long q_rows, const void* k, long ldk, const void* v,
+                            long ldv, const void* r, long ldr, long kv_rows, const int* cu_seqlens, const int* seq_slots,
+                            const int* seq_pos0, int n_seqs, int max_q_len, int n_heads, int dim, int rot, int vdim,
+                            float scale, int window, const float* sinks, const void* gate, long ldg, void* stream);
 // out[t, h * ohs + n] = sum_k a[t, h * ahs + k] * w[h * whs + n * ldw + k * kstride], n < N, k < K, for every head h; out has
 // a's type.  tensor_cores: bfloat16 operands with kstride 1 take `mma.sync`.
 int gi_bmm_heads(void* out, long ldo, long ohs, const void* a, long lda, long ahs, int dtype, const void* w, int w_dtype,

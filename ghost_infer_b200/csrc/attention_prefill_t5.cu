@@ -16,8 +16,17 @@
 // one full round and a ragged one.  Longer prompts keep one tile per block, longest first (measured: paired blocks
 // are 10% slower at 8,192 tokens, where the many rounds even out by themselves).
 // Every wait has an iteration limit and reports through a status word.
+//
+// The same kernel serves a latent cache's prompt steps over keys and values that were formed per head from the latents
+// (ROWS): keys are [rows of every head's unrotated numbers | one rotated part shared by all heads], values rows of their
+// own width, a sequence's positions one below the other instead of in pages.  Queries and keys are then up to 192 numbers
+// wide beside values of up to 128; at 192 and 128 the values get one stage, so that two blocks still fit an SM.
+// B200, 2,048 tokens, 16 heads of 128 + 64 and values of 128, forming the rows included: 86 us; the carried form
+// (attention_latent.cu, 576 and 512 numbers per head, query and key) with its two products per head 593 us.
 #include <cuda.h>
 #include <math.h>
+
+#include <type_traits>
 
 #include "api.h"
 #include "common.cuh"
@@ -75,27 +84,39 @@ __device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo_byt
          ((uint64_t)2 << 61);
 }
 
-template <int HD>
+// What the ROWS form needs beside the rest: the shared part's rows, the numbers of a head's key outside and inside it, of a
+// head's value, and gates (a head's result times the sigmoid of its gate; null: none).
+struct RowsArgs {
+  CUtensorMap map_r;
+  int dim, rot, vdim;
+  const __nv_bfloat16* gate;
+  long ldg;
+};
+struct NoRows {};
+
+// HALVES, V_HALVES: 64-number parts of a head's queries and keys, and of its values (and output); V_STAGES: stages of values
+template <int HALVES, int V_HALVES, int V_STAGES, bool ROWS>
 __global__ void __launch_bounds__(THREADS, 2)
 attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                       const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out, long ldo,
+                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ std::conditional_t<ROWS, RowsArgs, NoRows> rows,
+                       __nv_bfloat16* __restrict__ out, long ldo,
                        const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_seqlens,
                        const int* __restrict__ seq_slots, const int* __restrict__ seq_pos0, int n_heads, int n_kv, float scale,
                        int window, int q_tiles, int paired, float softcap, const float* __restrict__ sinks, int chunk, int keep_first) {
-  constexpr int HALVES = HD / 64;
-  constexpr uint32_t Q_BYTES = HALVES * Q_HALF, KV_BYTES = HALVES * KV_HALF;
+  constexpr uint32_t Q_BYTES = HALVES * Q_HALF, K_BYTES = HALVES * KV_HALF, V_BYTES = V_HALVES * KV_HALF;
+  constexpr int KSTEPS = HALVES * 4, VD = V_HALVES * 64;   // steps of 16 numbers of a key; columns of the accumulator
   // instruction descriptors: float accumulator, bfloat16 operands, M 128; S = Q K^T has N 64 and both operands K-major,
-  // O = P V has N 128 and B (V) MN-major (bit 16)
+  // O = P V has N VD and B (V) MN-major (bit 16)
   constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BKV >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
-  constexpr uint32_t IDESC_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
+  constexpr uint32_t IDESC_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(VD >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
   // Two blocks must fit one SM (2 x 113 KB at head size 128), which leaves no room for alignment slack: the tiles need 1024-byte
   // alignment, the dynamic shared memory of a kernel without static shared memory starts on such a boundary, and
   // the block checks that before it does anything.
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* q_s = smem;                              // [halves][128 rows][64 dims]
   unsigned char* k_s = q_s + Q_BYTES;                     // [2 stages][halves][64 keys][64 dims]
-  unsigned char* v_s = k_s + 2 * KV_BYTES;                // the same
-  uint64_t* bars = (uint64_t*)(v_s + 2 * KV_BYTES);       // q_full, k_full[2], v_full[2], kv_empty[2], s_full[2], p_full[2], o_full
+  unsigned char* v_s = k_s + 2 * K_BYTES;                 // [stages] of the same
+  uint64_t* bars = (uint64_t*)(v_s + V_STAGES * V_BYTES);       // q_full, k_full[2], v_full[2], kv_empty[2], s_full[2], p_full[2], o_full
   uint32_t* tmem_slot = (uint32_t*)(bars + 12);
 
   // Blocks start in the order x, y, z: heads fastest (the heads of a group read the same keys and values at the
@@ -112,7 +133,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     return;
   }
   const int slot = seq_slots[b], pos0 = seq_pos0[b];
-  const int kvh = h / (n_heads / n_kv);
+  const int kvh = ROWS ? h : h / (n_heads / n_kv);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   const uint32_t bar0 = smem_u32(bars);
@@ -152,6 +173,18 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const uint32_t tmem_s = tmem, tmem_o = tmem + 128;
   gi::pdl_prologue();      // set-up overlapped the previous kernel's end; its results are visible from here on
 
+  // ROWS: a sequence's rows begin at position 64 * (first of them that any of its tokens sees / 64); sequences follow each other
+  int row0_seq = 0, first_row = 0;
+  if constexpr (ROWS) {
+    if (warp >= 4) {
+      for (int i = 0; i <= b; ++i) {
+        const int p = seq_pos0[i];
+        first_row = window > 0 ? max(0, p - window + 1) / BKV * BKV : 0;
+        if (i < b) row0_seq += p + cu_seqlens[i + 1] - cu_seqlens[i] - first_row;
+      }
+    }
+  }
+
   bool first_pass = true;
   for (int pass = 0; pass < 2; ++pass) {
   const int q_tile = pass == 0 ? tile_a : tile_b;
@@ -182,6 +215,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   // the one chain's waits while the other chain was ready.
   auto row_of = [&](int tile) {        // where a tile's keys and values lie: the page comes from the sequence's page table
     const int kt = tile < kept_tiles ? tile * BKV : kt_begin + (tile - kept_tiles) * BKV;
+    if constexpr (ROWS) return row0_seq + kt - first_row;
     const int page = block_table[(size_t)slot * max_pages + kt / PAGE_TOKENS];
     return (page * n_kv + kvh) * PAGE_TOKENS;
   };
@@ -190,23 +224,34 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       bool ok = true;
       auto load_k = [&](int tile) {
         const int s = tile & 1, row0 = row_of(tile);
-        mbar_expect_tx(k_full0 + 8 * s, KV_BYTES);
+        mbar_expect_tx(k_full0 + 8 * s, K_BYTES);
 #pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf) tma_load_2d(smem_u32(k_s + s * KV_BYTES + hf * KV_HALF), &map_k, hf * 64, row0, k_full0 + 8 * s);
+        for (int hf = 0; hf < HALVES; ++hf) {
+          const uint32_t dst = smem_u32(k_s + s * K_BYTES + hf * KV_HALF);
+          if constexpr (ROWS) {                            // the last part is the one all heads share
+            if (hf == HALVES - 1) tma_load_2d(dst, &rows.map_r, 0, row0, k_full0 + 8 * s);
+            else tma_load_2d(dst, &map_k, h * rows.dim + hf * 64, row0, k_full0 + 8 * s);
+          } else {
+            tma_load_2d(dst, &map_k, hf * 64, row0, k_full0 + 8 * s);
+          }
+        }
       };
+      int q_width = HALVES * 64, k_steps = KSTEPS;
+      // (what the last 64 columns of queries hold past a head's own numbers is the next head's, and no step reads it)
+      if constexpr (ROWS) q_width = rows.dim + rows.rot, k_steps = q_width / 16;
       mbar_expect_tx(q_full, Q_BYTES);
 #pragma unroll
-      for (int hf = 0; hf < HALVES; ++hf) tma_load_2d(smem_u32(q_s + hf * Q_HALF), &map_q, h * HD + hf * 64, tok0 + q0, q_full);
+      for (int hf = 0; hf < HALVES; ++hf) tma_load_2d(smem_u32(q_s + hf * Q_HALF), &map_q, h * q_width + hf * 64, tok0 + q0, q_full);
       load_k(0);
       if (n_tiles > 1) load_k(1);
       ok = mbar_wait(q_full, 0, 1, &g_attn_status);
       // the operands' descriptors do not change from tile to tile (but for the stage): made once
-      uint64_t dq[HD / 16], dk[2][HD / 16];
+      uint64_t dq[KSTEPS], dk[2][KSTEPS];
 #pragma unroll
-      for (int ks = 0; ks < HD / 16; ++ks) {
+      for (int ks = 0; ks < KSTEPS; ++ks) {
         dq[ks] = smem_desc(smem_u32(q_s) + (ks / 4) * Q_HALF + (ks % 4) * 32);
         dk[0][ks] = smem_desc(smem_u32(k_s) + (ks / 4) * KV_HALF + (ks % 4) * 32);
-        dk[1][ks] = smem_desc(smem_u32(k_s) + KV_BYTES + (ks / 4) * KV_HALF + (ks % 4) * 32);
+        dk[1][ks] = smem_desc(smem_u32(k_s) + K_BYTES + (ks / 4) * KV_HALF + (ks % 4) * 32);
       }
       for (int j = 0; j < n_tiles && ok; ++j) {
         const int s = j & 1;
@@ -217,7 +262,8 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < HD / 16; ++ks) tc_mma(tmem_s + (uint32_t)(s * 64), dq[ks], s ? dk[1][ks] : dk[0][ks], IDESC_S, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < KSTEPS; ++ks)
+          if (!ROWS || ks < k_steps) tc_mma(tmem_s + (uint32_t)(s * 64), dq[ks], s ? dk[1][ks] : dk[0][ks], IDESC_S, ks > 0 ? 1u : 0u);
         tc_commit(s_full0 + 8 * s);
         // keys two tiles ahead go into this tile's stage as soon as its scores are complete: a whole tile's softmax
         // before they are wanted
@@ -232,39 +278,41 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (lane == 0) {
       bool ok = true;
       auto load_v = [&](int tile) {
-        const int s = tile & 1, row0 = row_of(tile);
-        mbar_expect_tx(v_full0 + 8 * s, KV_BYTES);
+        const int s = tile & (V_STAGES - 1), row0 = row_of(tile);
+        int col = 0;
+        if constexpr (ROWS) col = h * rows.vdim;           // (past a head's own values: columns of the output that nobody reads)
+        mbar_expect_tx(v_full0 + 8 * s, V_BYTES);
 #pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf) tma_load_2d(smem_u32(v_s + s * KV_BYTES + hf * KV_HALF), &map_v, hf * 64, row0, v_full0 + 8 * s);
+        for (int hf = 0; hf < V_HALVES; ++hf) tma_load_2d(smem_u32(v_s + s * V_BYTES + hf * KV_HALF), &map_v, col + hf * 64, row0, v_full0 + 8 * s);
       };
       load_v(0);
-      if (n_tiles > 1) load_v(1);
+      if (V_STAGES > 1 && n_tiles > 1) load_v(1);
       uint64_t dv[2][BKV / 16];
 #pragma unroll
       for (int kk = 0; kk < BKV / 16; ++kk) {
         dv[0][kk] = smem_desc_mn(smem_u32(v_s) + kk * 2048, KV_HALF);
-        dv[1][kk] = smem_desc_mn(smem_u32(v_s) + KV_BYTES + kk * 2048, KV_HALF);
+        dv[1][kk] = smem_desc_mn(smem_u32(v_s) + (V_STAGES - 1) * V_BYTES + kk * 2048, KV_HALF);
       }
       for (int j = 0; j < n_tiles && ok; ++j) {
         const int s = j & 1;
         // O += P V once the probabilities are staged (which also says: O has been rescaled) and the values are here
         ok = mbar_wait(p_full0 + 8 * s, (uint32_t)((j >> 1) & 1), 2, &g_attn_status);
-        if (ok) ok = mbar_wait(v_full0 + 8 * s, (uint32_t)((j >> 1) & 1), 2, &g_attn_status);
+        if (ok) ok = mbar_wait(v_full0 + 8 * (j & (V_STAGES - 1)), (uint32_t)((j / V_STAGES) & 1), 2, &g_attn_status);
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < BKV / 16; ++kk)      // 16 keys of the probabilities = 8 columns of the tile's score buffer
-          tc_mma_a_tmem(tmem_o, tmem_s + (uint32_t)(s * 64 + kk * 8), s ? dv[1][kk] : dv[0][kk], IDESC_O, (j > 0 || kk > 0) ? 1u : 0u);
+          tc_mma_a_tmem(tmem_o, tmem_s + (uint32_t)(s * 64 + kk * 8), V_STAGES > 1 && s ? dv[1][kk] : dv[0][kk], IDESC_O, (j > 0 || kk > 0) ? 1u : 0u);
         // `o_full` first: the barrier asked last by the row warps (the stage's, at the end of the tile loop) is then the
         // one whose arrival is issued last, and no arrival can still be on its way when the barriers are made anew
         // for the block's second query tile
         tc_commit(o_full);
         tc_commit(kv_empty0 + 8 * s);
-        // values two tiles ahead go into this tile's stage once this product no longer reads it
-        if (j + 2 < n_tiles) {
+        // values two tiles (with one stage: one tile) ahead go into this tile's stage once this product no longer reads it
+        if (j + V_STAGES < n_tiles) {
           ok = mbar_wait(kv_empty0 + 8 * s, (uint32_t)((j >> 1) & 1), 1, &g_attn_status);
           if (!ok) break;
-          load_v(j + 2);
+          load_v(j + V_STAGES);
         }
       }
     }
@@ -356,7 +404,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (!ok) break;
         tc_fence_after();
 #pragma unroll 1
-        for (int c = 0; c < HD / 32; ++c) {
+        for (int c = 0; c < VD / 32; ++c) {
           uint32_t orow[32];
           tc_ld32(tmem_o + lane_base + c * 32, orow);
           tc_wait_ld();
@@ -374,11 +422,11 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int lo = max(0, t_first - kt), hi = min(BKV, p_last + 1 - kt);
       const int lo_kept = min(lo, max(0, kept - kt));      // of the rows before every window, the first lo_kept are kept first positions: seen
       if (lo > lo_kept || hi < BKV) {
-        ok = mbar_wait(v_full0 + 8 * s, (uint32_t)((j >> 1) & 1), 3, &g_attn_status);
+        ok = mbar_wait(v_full0 + 8 * (j & (V_STAGES - 1)), (uint32_t)((j / V_STAGES) & 1), 3, &g_attn_status);
         if (!ok) break;
-        unsigned char* vt = v_s + s * KV_BYTES;
-        for (int idx = threadIdx.x; idx < BKV * (HD / 8); idx += 128) {
-          const int r = idx / (HD / 8), cidx = idx % (HD / 8);   // key row, 16-byte chunk of the row (its halves lie apart)
+        unsigned char* vt = v_s + (j & (V_STAGES - 1)) * V_BYTES;
+        for (int idx = threadIdx.x; idx < BKV * (VD / 8); idx += 128) {
+          const int r = idx / (VD / 8), cidx = idx % (VD / 8);   // key row, 16-byte chunk of the row (its halves lie apart)
           if ((r < lo && r >= lo_kept) || r >= hi) *reinterpret_cast<uint4*>(vt + (cidx / 8) * KV_HALF + r * 128 + (cidx % 8) * 16) = make_uint4(0, 0, 0, 0);
         }
       }
@@ -407,10 +455,15 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         a_sink = (m_run == -INFINITY) ? 0.f : ex2(m_run - m_f);
         l_run = l_run * a_sink + ex2(sk - m_f);
       }
-      const float inv = l_run > 0.f ? a_sink / l_run : 0.f;
-      __nv_bfloat16* orow_g = out + (size_t)(tok0 + q0 + row) * ldo + (size_t)h * HD;
+      float inv = l_run > 0.f ? a_sink / l_run : 0.f;
+      int width = VD;
+      if constexpr (ROWS) {
+        width = rows.vdim;
+        if (rows.gate != nullptr && row < rows_here) inv /= 1.0f + expf(-gi::ldf(rows.gate + (size_t)(tok0 + q0 + row) * rows.ldg + h));
+      }
+      __nv_bfloat16* orow_g = out + (size_t)(tok0 + q0 + row) * ldo + (size_t)h * width;
 #pragma unroll 1
-      for (int c = 0; c < HD / 32; ++c) {
+      for (int c = 0; c < VD / 32; ++c) {
         uint32_t orow[32];
         tc_ld32(tmem_o + lane_base + c * 32, orow);
         tc_wait_ld();
@@ -423,7 +476,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
               __nv_bfloat162 v2 = __floats2bfloat162_rn(__uint_as_float(orow[e + 2 * u]) * inv, __uint_as_float(orow[e + 2 * u + 1]) * inv);
               pkd[u] = *reinterpret_cast<uint32_t*>(&v2);
             }
-            *reinterpret_cast<uint4*>(orow_g + c * 32 + e) = make_uint4(pkd[0], pkd[1], pkd[2], pkd[3]);
+            if (!ROWS || c * 32 + e < width) *reinterpret_cast<uint4*>(orow_g + c * 32 + e) = make_uint4(pkd[0], pkd[1], pkd[2], pkd[3]);
           }
         }
         __syncwarp();
@@ -442,19 +495,20 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   }
 }
 
-template <int HD>
-int launch_t5(dim3 grid, cudaStream_t stream, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, __nv_bfloat16* out,
-              long ldo, const int* block_table, int max_pages, const int* cu_seqlens, const int* seq_slots, const int* seq_pos0,
+template <int HALVES, int V_HALVES, int V_STAGES, bool ROWS>
+int launch_t5(dim3 grid, cudaStream_t stream, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+              const std::conditional_t<ROWS, RowsArgs, NoRows>& rows, __nv_bfloat16* out, long ldo, const int* block_table, int max_pages, const int* cu_seqlens, const int* seq_slots, const int* seq_pos0,
               int n_heads, int n_kv, float scale, int window, int q_tiles, int paired, float softcap, const float* sinks, int chunk, int keep_first) {
-  constexpr size_t smem = (HD / 64) * (Q_HALF + 4 * KV_HALF) + 12 * 8 + 16;
+  constexpr size_t smem = HALVES * (Q_HALF + 2 * KV_HALF) + V_STAGES * V_HALVES * KV_HALF + 12 * 8 + 16;
+  auto kern = attn_prefill_t5_kernel<HALVES, V_HALVES, V_STAGES, ROWS>;
   static bool configured[gi::MAX_DEVICES_SEEN] = {false};
   int dev;
   if (gi::unconfigured_here(configured, &dev)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_t5_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return gi::fail(GI_ERR_CUDA, "attention prefill (tcgen05): %s", cudaGetErrorString(e));
     if (dev >= 0) configured[dev] = true;
   }
-  return gi::check(gi::launch(attn_prefill_t5_kernel<HD>, grid, dim3(THREADS), smem, stream, mq, mk, mv, out, ldo, block_table, max_pages,
+  return gi::check(gi::launch(kern, grid, dim3(THREADS), smem, stream, mq, mk, mv, rows, out, ldo, block_table, max_pages,
                               cu_seqlens, seq_slots, seq_pos0, n_heads, n_kv, scale, window, q_tiles, paired, softcap, sinks, chunk, keep_first),
                    "attention prefill (tcgen05)");
 }
@@ -517,10 +571,44 @@ extern "C" int gi_attn_prefill_t5_ex2(void* out, long ldo, const void* q, long l
   const int paired = (g_pairing != 0 && q_tiles > 1 && (g_pairing == 2 || paired_blocks <= 2L * (sms > 0 ? sms : 148))) ? 1 : 0;
   dim3 grid(n_heads, n_seqs, paired ? (q_tiles + 1) / 2 : q_tiles);
   if (hd == 128)
-    return launch_t5<128>(grid, (cudaStream_t)stream, mq, mk, mv, (__nv_bfloat16*)out, ldo, block_table, max_pages, cu_seqlens, seq_slots,
+    return launch_t5<2, 2, 2, false>(grid, (cudaStream_t)stream, mq, mk, mv, NoRows{}, (__nv_bfloat16*)out, ldo, block_table, max_pages, cu_seqlens, seq_slots,
                           seq_pos0, n_heads, n_kv, scale, window, q_tiles, paired, softcap, sinks, chunk, keep_first);
-  return launch_t5<64>(grid, (cudaStream_t)stream, mq, mk, mv, (__nv_bfloat16*)out, ldo, block_table, max_pages, cu_seqlens, seq_slots,
+  return launch_t5<1, 1, 2, false>(grid, (cudaStream_t)stream, mq, mk, mv, NoRows{}, (__nv_bfloat16*)out, ldo, block_table, max_pages, cu_seqlens, seq_slots,
                        seq_pos0, n_heads, n_kv, scale, window, q_tiles, paired, softcap, sinks, chunk, keep_first);
+}
+
+extern "C" int gi_attn_prefill_t5_rows(void* out, long ldo, const void* q, long ldq, long q_rows, const void* k, long ldk, const void* v,
+                                       long ldv, const void* r, long ldr, long kv_rows, const int* cu_seqlens, const int* seq_slots,
+                                       const int* seq_pos0, int n_seqs, int max_q_len, int n_heads, int dim, int rot, int vdim,
+                                       float scale, int window, const float* sinks, const void* gate, long ldg, void* stream) {
+  if (n_seqs <= 0 || max_q_len <= 0) return GI_OK;
+  if (n_heads <= 0 || window < 0 || kv_rows <= 0) return gi::fail(GI_ERR_ARG, "attention over rows: %d heads, window %d, %ld rows", n_heads, window, kv_rows);
+  if ((dim != 64 && dim != 128) || rot <= 0 || rot > 64 || rot % 16 != 0 || vdim <= 0 || vdim > 128 || vdim % 8 != 0)
+    return gi::fail(GI_ERR_UNSUPPORTED, "attention over rows: keys of %d + %d numbers, values of %d", dim, rot, vdim);
+  if ((ldq | ldk | ldv | ldr | ldo) % 8 != 0 || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)r | (uintptr_t)out) & 15))
+    return gi::fail(GI_ERR_UNSUPPORTED, "attention over rows: rows must be 16-byte aligned");
+  if (n_seqs > 65535 || (max_q_len + BQ - 1) / BQ > 65535) return gi::fail(GI_ERR_UNSUPPORTED, "attention: more than 65535 sequences or query tiles in one launch");
+  if (kv_rows > 0x7fffffffL || q_rows > 0x7fffffffL) return gi::fail(GI_ERR_UNSUPPORTED, "attention over rows: more than 2^31 - 1 rows");
+  CUtensorMap mq, mk, mv;
+  RowsArgs rows = {};
+  int rc = gi::tensor_map_2d_ex(&mq, q, q_rows, (long)n_heads * (dim + rot), ldq, GI_BF16, 64, BQ);
+  if (rc == GI_OK) rc = gi::tensor_map_2d_ex(&mk, k, kv_rows, (long)n_heads * dim, ldk, GI_BF16, 64, BKV);
+  if (rc == GI_OK) rc = gi::tensor_map_2d_ex(&mv, v, kv_rows, (long)n_heads * vdim, ldv, GI_BF16, 64, BKV);
+  if (rc == GI_OK) rc = gi::tensor_map_2d_ex(&rows.map_r, r, kv_rows, rot, ldr, GI_BF16, 64, BKV);
+  if (rc != GI_OK) return rc;
+  rows.dim = dim, rows.rot = rot, rows.vdim = vdim, rows.gate = (const __nv_bfloat16*)gate, rows.ldg = ldg;
+  const int q_tiles = (max_q_len + BQ - 1) / BQ;
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long paired_blocks = (long)n_heads * n_seqs * ((q_tiles + 1) / 2);
+  const int paired = (g_pairing != 0 && q_tiles > 1 && (g_pairing == 2 || paired_blocks <= 2L * (sms > 0 ? sms : 148))) ? 1 : 0;
+  const dim3 grid(n_heads, n_seqs, paired ? (q_tiles + 1) / 2 : q_tiles);
+#define GI_ROWS(H, VH, VS) launch_t5<H, VH, VS, true>(grid, (cudaStream_t)stream, mq, mk, mv, rows, (__nv_bfloat16*)out, ldo, nullptr, 0, cu_seqlens, \
+                                                      seq_slots, seq_pos0, n_heads, n_heads, scale, window, q_tiles, paired, 0.f, sinks, 0, 0)
+  if (dim == 128) return vdim > 64 ? GI_ROWS(3, 2, 1) : GI_ROWS(3, 1, 2);
+  return vdim > 64 ? GI_ROWS(2, 2, 2) : GI_ROWS(2, 1, 2);
+#undef GI_ROWS
 }
 
 // Query tiles two to a block: 0 never, 1 where the launch then is one round of blocks (default), 2 always; for

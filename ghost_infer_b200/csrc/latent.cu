@@ -303,6 +303,30 @@ latent_query_rot_kernel(LatentQueries<T> lq, const float2* table, int half, int 
   turn_queries(lq, blockIdx.x, table, half, dr, r);
 }
 
+// ---- a sequence's cached rows out of their pages, one below the other ------------------------------------------------
+// grid (tiles of 64 positions, sequences): tile i of sequence b is the page that holds positions first + 64 i .. + 63, with
+// first = 64 * (the first position that any of the sequence's tokens sees / 64); sequences follow each other without gaps.
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(uint4* __restrict__ out, const uint4* cache, const int* __restrict__ block_table, int max_pages,
+                     const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slots, const int* __restrict__ seq_pos0, int words, int window) {
+  gi::pdl_prologue();
+  const int b = blockIdx.y;
+  int first = 0, end = 0;
+  size_t row0 = 0;
+  for (int i = 0; i <= b; ++i) {
+    const int p = seq_pos0[i];
+    end = p + cu_seqlens[i + 1] - cu_seqlens[i];
+    first = window > 0 ? max(0, p - window + 1) / PAGE_TOKENS * PAGE_TOKENS : 0;
+    if (i < b) row0 += end - first;
+  }
+  const int at = first + (int)blockIdx.x * PAGE_TOKENS, slot = seq_slots[b];
+  if (at >= end || slot < 0) return;
+  const uint4* src = cache + (size_t)block_table[(size_t)slot * max_pages + at / PAGE_TOKENS] * PAGE_TOKENS * words;
+  uint4* dst = out + (row0 + at - first) * words;
+  const int n = min(PAGE_TOKENS, end - at) * words;
+  for (int i = threadIdx.x; i < n; i += 256) dst[i] = src[i];
+}
+
 // ---- one small product per head, CUDA cores ------------------------------------------------------------------------
 // out[t, h * ohs + n] = sum_k a[t, h * ahs + k] * W[h * whs + n * ldw + k * kstride]; every output is summed by one thread
 // in k order, so a row's result does not depend on the step's other rows.
@@ -617,6 +641,17 @@ extern "C" int gi_latent_query_rot(void* qa, long ldqa, const void* q, long ldq,
       e = gi::launch(latent_query_rot_kernel<T>, dim3(n_tokens), dim3(256), 0, (cudaStream_t)stream,
                      LatentQueries<T>{(T*)qa, ldqa, (const T*)q, ldq, n_heads, dn}, (const float2*)table, rot / 2, dr, r));
   return gi::check(e, "latent queries");
+}
+
+extern "C" int gi_latent_gather(void* out, const void* cache, const int* block_table, int max_pages, const int* cu_seqlens,
+                                const int* seq_slots, const int* seq_pos0, int n_seqs, int max_rows, int hd, int window, void* stream) {
+  if (n_seqs <= 0 || max_rows <= 0) return GI_OK;
+  if (hd <= 0 || hd % 8 != 0 || window < 0 || (((uintptr_t)out | (uintptr_t)cache) & 15))
+    return gi::fail(GI_ERR_UNSUPPORTED, "latent rows: rows of %d 16-bit numbers must be a multiple of 8 wide and aligned", hd);
+  if (n_seqs > 65535) return gi::fail(GI_ERR_UNSUPPORTED, "latent rows: more than 65535 sequences in one launch");
+  return gi::check(gi::launch(latent_gather_kernel, dim3((max_rows + PAGE_TOKENS - 1) / PAGE_TOKENS, n_seqs), dim3(256), 0, (cudaStream_t)stream,
+                              (uint4*)out, (const uint4*)cache, block_table, max_pages, cu_seqlens, seq_slots, seq_pos0, hd / 8, window),
+                   "latent rows");
 }
 
 extern "C" int gi_bmm_heads(void* out, long ldo, long ohs, const void* a, long lda, long ahs, int dtype, const void* w, int w_dtype,

@@ -62,6 +62,8 @@ def _bind():
         "gi_attn_prefill_t5": [P, L, P, L, L, P, P, L, P, I, P, P, P, I, I, I, I, I, F, I, P],
         "gi_attn_prefill_t5_status": [P],
         "gi_attn_prefill_t5_ex": [P, L, P, L, L, P, P, L, P, I, P, P, P, I, I, I, I, I, F, I, F, P, I, P],
+        "gi_latent_gather": [P, P, P, I, P, P, P, I, I, I, I, P],
+        "gi_attn_prefill_t5_rows": [P, L, P, L, L, P, L, P, L, P, L, L, P, P, P, I, I, I, I, I, I, F, I, P, P, L, P],
         "gi_attn_prefill_t5_ex2": [P, L, P, L, L, L, P, P, L, P, I, P, P, P, I, I, I, I, I, F, I, F, P, I, I, P],
         "gi_attn_prefill_tc_ex2": [P, L, P, L, P, P, P, I, P, P, P, I, I, I, I, I, F, I, I, F, P, I, I, P],
         "gi_attn_decode_tc": [P, L, P, P, P, L, P, P, P, I, P, P, I, I, I, I, F, I, I, P],
@@ -1990,6 +1992,76 @@ def attention_latent(qa: torch.Tensor, memory, step, n_heads: int, rank: int, ro
         _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"), _i32(step.seq_pos0, "start positions"), step.n_seqs,
         step.max_q_len, n_heads, 1, hd, float(scale), window, rank, 0.0, sp, 0, hd, 0, _stream()))
     return out if gate is None else head_gate_rows(out, gate, n_heads, rank)
+
+
+LATENT_EXPAND_BYTES = 1 << 30      # of keys and values per head that a prompt step may form at a time
+
+
+def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, rank: int, window: Optional[int], dtype: torch.dtype) -> int:
+    """How many cached rows a prompt step should turn into keys and values per head (`attention_latent_expanded`), or 0: carry
+    its queries onto the latents instead (`attention_latent`).
+
+    Carried, a head spends 2 rank + rot_dim multiply-adds on a query and key; expanded, dim + rot_dim + v_dim, and rank (dim +
+    v_dim) more on every visible position once.  Measured multiply-adds per microsecond: the carried kernel 74e6 (a block's
+    tile of 64 keys 8.3 us at 1,088 of them, which is what few tokens behind a long prefix wait for), the products that carry
+    queries and results 32e6, the attention over rows 200e6 (2 us a tile), the product that forms the rows 400e6; 15 us for the
+    launches more.  16 heads, rank 512: 64 fresh tokens are carried; 16 tokens behind 3,000 take 98 us expanded, 418 carried.
+    Only prompt steps have the host's lists of lengths; sizes are those the tcgen05 kernel takes."""
+    if (step.is_decode or dtype != torch.bfloat16 or not TUNE["attn_latent_tc"] or dim not in (64, 128) or not 0 < rot_dim <= 64
+            or rot_dim % 16 or not 0 < v_dim <= 128 or v_dim % 8 or rank % 8):
+        return 0
+    pos0, lens = getattr(step, "_host_pos0", None), getattr(step, "_host_q_lens", None)
+    if not pos0 or not lens or len(pos0) != step.n_seqs or len(lens) != step.n_seqs:
+        return 0
+    rows = pairs = tokens = tiles = 0
+    span = int(window) if window else 1 << 62
+    for p, n in zip(pos0, lens):
+        rows += p + n - max(0, p - span + 1) // 64 * 64
+        whole = max(0, min(n, span - p))                 # tokens that see everything before them
+        pairs += whole * p + whole * (whole + 1) // 2 + (n - whole) * (0 if whole == n else span)
+        tokens += n
+        tiles = max(tiles, (min(p + n, span) + 63) // 64)
+    if rows * n_heads * (dim + v_dim) * 2 > LATENT_EXPAND_BYTES:
+        return 0
+    work = 2 * rank + rot_dim
+    carried = max(n_heads * pairs * work / 74e6, tiles * work * 7.6e-3) + n_heads * tokens * rank * (dim + v_dim) / 32e6
+    expanded = max(n_heads * pairs * (dim + rot_dim + v_dim) / 200e6, tiles * 2.0) + n_heads * rows * rank * (dim + v_dim) / 400e6 + 15.0
+    return rows if expanded < carried else 0
+
+
+def attention_latent_expanded(q: torch.Tensor, memory, step, w_uk_uv: torch.Tensor, rows: int, n_heads: int, dim: int, rot_dim: int,
+                              v_dim: int, rank: int, scale: float, window: Optional[int] = None, sinks: Optional[torch.Tensor] = None,
+                              gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """A prompt step's latent attention with keys and values formed per head: the visible positions' rows [latent (rank) | rotary
+    key part (rot_dim)] leave their pages, one product with `w_uk_uv` [heads * dim + heads * v_dim (+ padding), rank] gives every
+    head's unrotated keys and values, and the tcgen05 kernel reads those beside the shared rotary part.  `q` [tokens, heads *
+    (dim + rot_dim)] with its rotated parts turned, `rows` from `latent_expand_rows`; returns [tokens, heads * v_dim].  `window`,
+    `sinks`, `gate`: as `attention_latent`'s."""
+    hd = rank + rot_dim
+    if memory.k is None or memory.k.dtype != q.dtype or tuple(memory.k.shape[1:]) != (1, 64, hd) or not memory.k.is_contiguous():
+        raise KernelError(f"the latent cache must be contiguous [pages, 1, 64, {hd}] of the queries' type")
+    if q.shape[1] != n_heads * (dim + rot_dim) or w_uk_uv.shape[0] < n_heads * (dim + v_dim) or w_uk_uv.shape[1] != rank:
+        raise KernelError("latent attention: rows of the wrong sizes")
+    if gate is not None and (gate.dtype != q.dtype or tuple(gate.shape) != (q.shape[0], n_heads) or not gate.is_cuda):
+        raise KernelError(f"the heads' gates must be [{q.shape[0]}, {n_heads}] rows of the queries' type")
+    lib = _bind()
+    _cuda(q, "queries")
+    bt, window = memory.block_table, int(window or 0)
+    latents = torch.empty((rows, hd), dtype=q.dtype, device=q.device)
+    longest = min(step.max_kv_len, window + step.max_q_len + 63) if window else step.max_kv_len
+    _check(lib, lib.gi_latent_gather(latents.data_ptr(), memory.k.data_ptr(), _i32(bt, "block table"), bt.shape[1],
+                                     _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"), _i32(step.seq_pos0, "start positions"),
+                                     step.n_seqs, int(longest), hd, window, _stream()))
+    kv = linear(latents[:, :rank], w_uk_uv, out_dtype=q.dtype)
+    out = torch.empty((q.shape[0], n_heads * v_dim), dtype=q.dtype, device=q.device)
+    v, r = kv[:, n_heads * dim:], latents[:, rank:]
+    _check(lib, lib.gi_attn_prefill_t5_rows(
+        out.data_ptr(), _rows(out, "attention output"), q.data_ptr(), _rows(q, "queries"), q.shape[0], kv.data_ptr(), _rows(kv, "keys"),
+        v.data_ptr(), _rows(kv, "values"), r.data_ptr(), hd, rows, _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"),
+        _i32(step.seq_pos0, "start positions"), step.n_seqs, step.max_q_len, n_heads, dim, rot_dim, v_dim, float(scale), window,
+        _sinks_ptr(sinks, n_heads), gate.data_ptr() if gate is not None else None, _rows(gate, "gate rows") if gate is not None else 0,
+        _stream()))
+    return out
 
 
 def head_gate_rows(a: torch.Tensor, gate: torch.Tensor, n_heads: int, width: int) -> torch.Tensor:

@@ -112,6 +112,8 @@ class LatentAttention(Mixer):
         # per head: W_uk,h^T as [rank, dim] (rows of the carried query), W_uv,h as [v_dim, rank]
         self.w_uk_t = place("uk").view(H, self.dim, self.rank).transpose(1, 2).contiguous()
         self.w_uv = place("uv").view(H, self.v_dim, self.rank).contiguous()
+        # the same matrices stacked, for prompt steps that form keys and values per head
+        self.w_uk_uv = stack_rows([place("uk"), self.w_uv.view(H * self.v_dim, self.rank)]) if rt.dtype == torch.bfloat16 else None
         qn, cn = place("dq_norm") if self.q_rank else None, place("dkv_norm")
         if qn is not None and qn.dtype != cn.dtype:
             qn, cn = qn.to(torch.float32), cn.to(torch.float32)
@@ -123,6 +125,12 @@ class LatentAttention(Mixer):
         H, T, dt = self.n_heads, h.shape[0], self.rt.dtype
         with ops.bucket("qkv matmul"):
             down = linear(h, self.w_down, out_dtype=dt)
+        rows = 0
+        if self.w_uk_uv is not None and self.w_uk_uv.dtype == dt and memory.k is not None and down.dtype == dt:
+            rows = ops.latent_expand_rows(step, H, self.dim, self.rot_dim, self.v_dim, self.rank, self.window, dt)
+        if rows:
+            return self._forward_expanded(h, residual, step, memory, down, rows)
+        with ops.bucket("qkv matmul"):
             qa = torch.empty((T, H * (self.rank + self.rot_dim)), dtype=dt, device=h.device)
         with ops.bucket("rope+cache"):
             table = self.position.table(step) if self.position is not None else None
@@ -155,6 +163,32 @@ class LatentAttention(Mixer):
         with ops.bucket("out matmul"):
             att = torch.empty((T, H * self.v_dim), dtype=dt, device=h.device)
             ops.bmm_heads(att, self.v_dim, lat, self.rank, self.w_uv, self.v_dim, self.rank)
+            if self.out_gate == "sigmoid":
+                att = ops.gate_mul(att, linear(h, self.w_g, out_dtype=dt), "sigmoid")
+            linear(att, self.w_o, out=residual, accumulate=True)
+
+    def _forward_expanded(self, h, residual, step, memory, down, rows) -> None:
+        """A prompt step whose attention reads keys and values per head (see `ops.latent_expand_rows`)."""
+        H, dt = self.n_heads, self.rt.dtype
+        own = self.q_rank + self.rank + self.rot_dim
+        with ops.bucket("rope+cache"):
+            table = self.position.table(step) if self.position is not None else None
+            cq = ops.latent_prepare(down if self.q_rank else down[:, :own], self.w_q_norm, self.w_c_norm, self.eps, table, self.rot,
+                                    step.positions, step.token_slots, memory, self.q_rank, self.rank, self.rot_dim)
+        with ops.bucket("qkv matmul"):
+            q = linear(cq, self.w_uq, out_dtype=dt) if self.q_rank else down[:, own:own + H * (self.dim + self.rot_dim)]
+        if self.rot:
+            with ops.bucket("rope+cache"):
+                ops.latent_query_rot(q, q, table, self.rot, H, self.dim, self.rot_dim, self.dim)      # in place
+        gate = None
+        if self.out_gate == "head_sigmoid":
+            with ops.bucket("out matmul"):
+                at = own + H * (self.dim + self.rot_dim)
+                gate = linear(h, self.w_g, out_dtype=dt) if self.w_g is not None else down[:, at:at + H]
+        with ops.bucket("attention"):
+            att = ops.attention_latent_expanded(q, memory, step, self.w_uk_uv, rows, H, self.dim, self.rot_dim, self.v_dim, self.rank,
+                                                self.scale, window=self.window, sinks=self.sinks, gate=gate)
+        with ops.bucket("out matmul"):
             if self.out_gate == "sigmoid":
                 att = ops.gate_mul(att, linear(h, self.w_g, out_dtype=dt), "sigmoid")
             linear(att, self.w_o, out=residual, accumulate=True)

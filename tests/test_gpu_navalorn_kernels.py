@@ -346,3 +346,42 @@ def test_ungated_experts_stretch_by_stretch():
         lo, hi = offs[e], offs[e + 1]
         hid = (torch.relu(rows[lo:hi].double() @ w_up[e].double().T) ** 2).to(torch.bfloat16).double()
         torch.testing.assert_close(got[lo:hi].double(), hid @ w_down[e].double().T, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("sizes", [(16, 128, 64, 128, 512), (3, 128, 16, 48, 128), (4, 64, 32, 40, 256), (2, 64, 64, 128, 64), (5, 64, 48, 64, 256)])
+@pytest.mark.parametrize("seqs,window", [([(0, 300)], None), ([(70, 130), (0, 1), (5, 64), (64, 129)], None), ([(0, 513), (900, 64)], 100), ([(63, 65)], 64)])
+def test_prompt_attention_with_keys_and_values_per_head(sizes, seqs, window):
+    """Rows formed per head against the formula in 64 bits: what is rounded to 8 bits (keys, values, probabilities, result) errs
+    by 2^-9 each, so a relative distance of 2^-8 holds for any of the sizes; pages that belong to nobody hold no numbers."""
+    H, dim, rot, vd, rank = sizes
+    g = torch.Generator(device=DEV).manual_seed(dim + vd + len(seqs))
+    rnd = lambda *s, k=1.0: (torch.randn(*s, generator=g, device=DEV) * k).to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(np.asarray(v), dtype=torch.int32, device=DEV)
+    order = list(np.random.default_rng(1).permutation(np.arange(1, 60)))
+    table = np.zeros((len(seqs) + 1, max((p + n + 63) // 64 for p, n in seqs)), dtype=np.int32)
+    cache = torch.full((60, 1, 64, rank + rot), float("nan"), device=DEV, dtype=torch.bfloat16)
+    latents = [rnd(p + n, rank + rot) for p, n in seqs]
+    for b, rows in enumerate(latents):
+        for j in range((len(rows) + 63) // 64):
+            table[b + 1, j] = order.pop()
+            cache[int(table[b + 1, j]), 0, :len(rows[64 * j:64 * j + 64])] = rows[64 * j:64 * j + 64]
+    lens, pos0 = [n for _, n in seqs], [p for p, _ in seqs]
+    cu = np.concatenate([[0], np.cumsum(lens)])
+    step = SimpleNamespace(n_seqs=len(seqs), max_q_len=max(lens), max_kv_len=max(p + n for p, n in seqs), cu_seqlens=i32(cu),
+                           seq_slots=i32(np.arange(1, len(seqs) + 1)), seq_pos0=i32(pos0))
+    uk, uv, q = rnd(H * dim, rank, k=rank ** -0.5), rnd(H * vd, rank, k=rank ** -0.5), rnd(cu[-1], H * (dim + rot))
+    sinks, gate = torch.randn(H, generator=g, device=DEV), rnd(cu[-1], H)
+    span = window or 1 << 40
+    total = sum(p + n - max(0, p - span + 1) // 64 * 64 for p, n in seqs)
+    got = ops.attention_latent_expanded(q, SimpleNamespace(k=cache, block_table=i32(table)), step, torch.cat([uk, uv]), total, H, dim, rot, vd,
+                                        rank, (dim + rot) ** -0.5, window=window, sinks=sinks, gate=gate)
+    assert ops.attn_prefill_t5_status() == 0
+    for b, (p, n) in enumerate(seqs):
+        c, kr = latents[b][:, :rank].double(), latents[b][:, rank:].double()
+        k = torch.cat([(c @ uk.double().T).view(-1, H, dim), kr[:, None].expand(-1, H, rot)], -1)
+        s = torch.einsum("qhd,khd->hqk", q[cu[b]:cu[b + 1]].double().view(n, H, dim + rot), k) * (dim + rot) ** -0.5
+        i, j = torch.arange(p, p + n, device=DEV)[:, None], torch.arange(p + n, device=DEV)[None]
+        s.masked_fill_((j > i) | (i - j >= span), -float("inf"))
+        w = torch.softmax(torch.cat([s, sinks.double()[:, None, None].expand(H, n, 1)], -1), -1)[..., :-1]
+        want = torch.einsum("hqk,khd->qhd", w, (c @ uv.double().T).view(-1, H, vd)) * torch.sigmoid(gate[cu[b]:cu[b + 1]].double())[:, :, None]
+        assert (got[cu[b]:cu[b + 1]].double() - want.reshape(n, -1)).norm() <= 2.0 ** -8 * want.norm()
