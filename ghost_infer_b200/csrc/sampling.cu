@@ -11,7 +11,13 @@
 // a 256-bin histogram of weights for the keys that share the prefix found so far, a scan of the bins
 // picks the next byte.  Weights are 41-bit fixed point and summed as integers, so the result does not
 // depend on the order in which threads add.  Equal logits are ordered by token id (lower first), with
-// a second descent over the ids.  One block per row.
+// a second descent over the ids.
+//
+// A row belongs to a cluster of blocks where there are fewer rows than the GPU holds blocks: each block sweeps its part of the
+// row, and what the sweeps find (the highest logit, the counts or weights of the bins, the few logits of a wanted bin) meets
+// in the first block's shared memory, where the pick is made.  One block per row was bound by what one SM reads: three
+// sweeps over 513 KB a row on 64 of 148 SMs.  64 rows of 128,256 logits, top_k 40, top_p 0.9: 22 us (44 us with a
+// block per row); one row: 17 us (27 us).  Sums are integers and lists are sorted, so the cut changes no pick.
 //
 // The usual case, a top_k of at most 2048, takes a shorter way to the same pick: one sweep counts the keys by their
 // distance below the highest key (4096 bins of 2^16 key steps: the seven upper bits of the mantissa, 32 octaves),
@@ -19,6 +25,10 @@
 // a few more) into shared memory, where they are sorted (key descending, token id ascending) and the cut and the
 // draw are made over at most top_k entries with the same fixed-point weights and the same rules.  Some twenty
 // sweeps over the row, with an exponential per logit in half of them, become two sweeps and top_k exponentials.
+// Where top_k is at most an eighth of the row's threads, the highest logits of the threads' own shares are counted in the
+// place of all: top_k of those lie at or above the bin that is found, so at least top_k keys do, and few more; the counting
+// sweep falls away.  A list of up to 256 is put in order by counting who stands before whom, and the picks are one warp's.
+#include <cooperative_groups.h>
 #include <math.h>
 #include <stddef.h>
 
@@ -29,7 +39,7 @@ namespace {
 
 typedef unsigned long long u64;
 
-constexpr int THREADS = 1024;
+constexpr int THREADS = 512;        // two blocks per SM
 constexpr float FIXED_ONE = 1099511627776.0f;  // 2^40
 
 __device__ __forceinline__ unsigned order_key(float v) {
@@ -163,16 +173,21 @@ __device__ u64 block_sum_u64(Shared& sh, u64 v) {
   return sh.total;
 }
 
-// The first place j < count (count <= 2 * blockDim.x) at which base + item(0) + ... + item(j) reaches `target`, found by
-// the whole block: every thread takes two neighbouring items, a scan over the threads gives each the sum before its
-// pair.  Returns the place (-1: the sum never gets there), `before_out` = base + the items before it, `total_out` =
+// The first place j < count (count <= 4 * blockDim.x) at which base + item(0) + ... + item(j) reaches `target`, found by
+// the whole block: every thread takes four neighbouring items, a scan over the threads gives each the sum before its
+// own.  Returns the place (-1: the sum never gets there), `before_out` = base + the items before it, `total_out` =
 // the sum of all items.  Sums are integers: no order of additions can change them.
 template <typename F>
 __device__ int first_reaching(Shared& sh, int count, u64 base, u64 target, F item, u64& before_out, u64& total_out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int j0 = 2 * tid;
-  const u64 a = j0 < count ? item(j0) : 0, b = j0 + 1 < count ? item(j0 + 1) : 0;
-  u64 incl = a + b;
+  const int j0 = 4 * tid;
+  u64 own[4], sum = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    own[k] = j0 + k < count ? item(j0 + k) : 0;
+    sum += own[k];
+  }
+  u64 incl = sum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const u64 up = __shfl_up_sync(0xffffffffu, incl, o);
@@ -192,14 +207,20 @@ __device__ int first_reaching(Shared& sh, int count, u64 base, u64 target, F ite
     sh.red64[lane] = t;                               // inclusive over the warps
   }
   __syncthreads();
-  const u64 mine_before = base + (warp > 0 ? sh.red64[warp - 1] : 0) + (incl - a - b);
+  u64 before = base + (warp > 0 ? sh.red64[warp - 1] : 0) + (incl - sum), at_found = 0;
   int found = 0x7fffffff;
-  if (j0 < count && mine_before + a >= target) found = j0;
-  else if (j0 + 1 < count && mine_before + a + b >= target) found = j0 + 1;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (found == 0x7fffffff && j0 + k < count && before + own[k] >= target) {
+      found = j0 + k;
+      at_found = before;
+    }
+    before += own[k];
+  }
   if (found != 0x7fffffff) atomicMin(&sh.first_bin, found);
   __syncthreads();
   const int first = sh.first_bin;
-  if (found != 0x7fffffff && first == found) sh.before = (found == j0) ? mine_before : mine_before + a;
+  if (found != 0x7fffffff && first == found) sh.before = at_found;
   __syncthreads();
   before_out = sh.before;
   total_out = sh.red64[(blockDim.x >> 5) - 1];
@@ -208,22 +229,74 @@ __device__ int first_reaching(Shared& sh, int count, u64 base, u64 target, F ite
   return result;
 }
 
-__global__ void __launch_bounds__(THREADS)
+// The same by one warp over `w` in shared memory, count <= 256: eight neighbouring items a lane.
+__device__ __forceinline__ int warp_first_reaching(const u64* w, int count, u64 target, u64& before_out, u64& total_out) {
+  const int lane = threadIdx.x & 31;
+  u64 own[8], sum = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    own[k] = 8 * lane + k < count ? w[8 * lane + k] : 0;
+    sum += own[k];
+  }
+  u64 incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u64 up = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += up;
+  }
+  total_out = __shfl_sync(0xffffffffu, incl, 31);
+  u64 before = incl - sum, at_found = 0;
+  int found = -1;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (found < 0 && 8 * lane + k < count && before + own[k] >= target) {
+      found = 8 * lane + k;
+      at_found = before;
+    }
+    before += own[k];
+  }
+  const unsigned who = __ballot_sync(0xffffffffu, found >= 0);
+  if (who == 0) return -1;
+  const int src = __ffs(who) - 1;
+  before_out = __shfl_sync(0xffffffffu, at_found, src);
+  return __shfl_sync(0xffffffffu, found, src);
+}
+
+// The largest of 1, 2, 4, 8 blocks a row whose blocks all fit the GPU at once and have 4,096 logits or more.  (Two blocks per SM,
+// an eighth left out, since a cluster stays inside one group of SMs: 37 rows in clusters of 8 would fill the places exactly
+// and took 36 us, where 64 rows in clusters of 4 take 22.)
+int blocks_per_row(int rows, int n, int sms) {
+  int c = 1;
+  while (c < 8 && 16L * c * rows <= 14L * sms && n / (2 * c) >= 4096) c *= 2;
+  return c;
+}
+
+__global__ void __launch_bounds__(THREADS, 2)
 sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, int n, float temperature, int top_k,
               float top_p, u64* __restrict__ rng_state, const int* __restrict__ state_index) {
   __shared__ Shared sh;
   gi::pdl_prologue();
-  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int blocks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int r = blockIdx.x / blocks, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float* row = logits + (size_t)r * ld;
+  // this block's part of the row; `first` is the shared memory of the row's first block
+  const int share = ((n + blocks - 1) / blocks + 3) / 4 * 4, lo = min(n, rank * share), hi = min(n, lo + share);
+  Shared& first = *cluster.map_shared_rank(&sh, 0);
+  auto meet = [&] {
+    if (blocks > 1) cluster.sync();
+    else __syncthreads();
+  };
 
   // ---- highest logit, first index on ties
-  float bv = -INFINITY;
+  float bv = -INFINITY;                                        // (a thread's own: it starts the count of a top_k below)
   int bi = 0x7fffffff;
   if ((((uintptr_t)row) & 15) == 0) {
     // four logits per load, four loads in flight: a thread's candidates still come in increasing index order
-    const int n4 = n / 4;
+    const int n4 = hi / 4;                                    // (`lo` is a multiple of 4)
     const float4* row4 = reinterpret_cast<const float4*>(row);
-    for (int i0 = tid; i0 < n4; i0 += 4 * blockDim.x) {
+    for (int i0 = lo / 4 + tid; i0 < n4; i0 += 4 * blockDim.x) {
       float4 v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -239,12 +312,12 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
         if (v[u].w > bv) { bv = v[u].w; bi = base + 3; }
       }
     }
-    for (int i = 4 * n4 + tid; i < n; i += blockDim.x) {
+    for (int i = max(lo, 4 * n4) + tid; i < hi; i += blockDim.x) {
       const float v = row[i];
       if (v > bv) { bv = v; bi = i; }
     }
   } else {
-    for (int i = tid; i < n; i += blockDim.x) {
+    for (int i = lo + tid; i < hi; i += blockDim.x) {
       const float v = row[i];
       if (v > bv) {  // strictly greater keeps the first; NaN never enters
         bv = v;
@@ -252,6 +325,7 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
       }
     }
   }
+  const float thread_max = bv;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
@@ -280,18 +354,33 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
     }
     if (lane == 0) {
       sh.bestv = bv;
-      sh.besti = bi == 0x7fffffff ? 0 : bi;
+      sh.besti = bi;
     }
   }
-  __syncthreads();
-  const float lmax = sh.bestv;
+  meet();
+  // (parts follow each other in the row: a later one's equal logit is not the first)
+  float lmax = sh.bestv;
+  int best = sh.besti;
+  if (blocks > 1) {
+    lmax = first.bestv;
+    best = first.besti;
+    for (int k = 1; k < blocks; ++k) {
+      const Shared& part = *cluster.map_shared_rank(&sh, k);
+      if (part.besti != 0x7fffffff && (best == 0x7fffffff || part.bestv > lmax)) {
+        lmax = part.bestv;
+        best = part.besti;
+      }
+    }
+  }
+  if (best == 0x7fffffff) best = 0;
   if (!(temperature > 0.f) || rng_state == nullptr) {
-    if (tid == 0) out[r] = sh.besti;
+    meet();                                                    // nobody leaves while its memory is being read
+    if (rank == 0 && tid == 0) out[r] = best;
     return;
   }
 
   // ---- one draw from this row's xorshift64* stream
-  if (tid == 0) {
+  if (rank == 0 && tid == 0) {
     const int si = state_index ? state_index[r] : r;
     u64 s = rng_state[si];
     if (s == 0) s = 1;
@@ -309,57 +398,115 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
     __syncthreads();
     // (eight loads in flight per thread: one at a time, a sweep waits for the L2 cache 125 times in a row)
     const unsigned top_key = order_key(lmax);
-    for (int i0 = 0; i0 < n; i0 += 8 * blockDim.x) {
-      float v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = i0 + u * blockDim.x + tid;
-        v[u] = i < n ? row[i] : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = i0 + u * blockDim.x + tid;
-        const unsigned below = (top_key - order_key(v[u])) >> 16;       // a NaN's key is 0: far below
-        if (i < n && below < FAST_BINS) atomicAdd(&sh.bins[below], 1u);
-      }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      // from the highest key's bin downwards until top_k keys are covered (or the bins end: then the long way)
-      unsigned covered = 0;
-      int b = 0;
-      for (; b < FAST_BINS; ++b) {
-        covered += sh.bins[b];
-        if (covered >= (unsigned)top_k) break;
-      }
-      sh.first_bin = b;
-      sh.n_list = b < FAST_BINS ? (int)covered : FAST_CAP + 1;
-    }
-    __syncthreads();
-    const int total_c = sh.n_list;
-    const unsigned last_bin = (unsigned)sh.first_bin;
-    __syncthreads();
-    if (total_c <= FAST_CAP) {
-      if (tid == 0) sh.n_list = 0;
-      __syncthreads();
-      for (int i0 = 0; i0 < n; i0 += 8 * blockDim.x) {
+    const bool by_threads = 8 * top_k <= blocks * THREADS;
+    // (few rows: the threads' maxima; if they lead to a list that overflows, all keys are counted after all)
+    for (int counting = by_threads ? 0 : 1; counting < 2; ++counting) {
+    if (counting == 0) {
+      const unsigned below = (top_key - order_key(thread_max)) >> 16;
+      if (thread_max > -INFINITY && below < FAST_BINS) atomicAdd(&sh.bins[below], 1u);
+    } else {
+      for (int i0 = lo; i0 < hi; i0 += 8 * blockDim.x) {
         float v[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int i = i0 + u * blockDim.x + tid;
-          v[u] = i < n ? row[i] : 0.f;
+          v[u] = i < hi ? row[i] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int i = i0 + u * blockDim.x + tid;
+          const unsigned below = (top_key - order_key(v[u])) >> 16;     // a NaN's key is 0: far below
+          if (i < hi && below < FAST_BINS) atomicAdd(&sh.bins[below], 1u);
+        }
+      }
+    }
+    meet();
+    if (rank == 0) {
+      // from the highest key's bin downwards until top_k keys are covered (or the bins end: then the long way)
+      if (blocks > 1) {
+        for (int b = tid; b < FAST_BINS; b += blockDim.x) {
+          unsigned t = sh.bins[b];
+          for (int k = 1; k < blocks; ++k) t += cluster.map_shared_rank(&sh, k)->bins[b];
+          sh.bins[b] = t;
+        }
+        __syncthreads();
+      }
+      u64 above = 0, all = 0;
+      const int pair = first_reaching(sh, FAST_BINS / 2, 0, (u64)top_k, [&](int j) { return (u64)sh.bins[2 * j] + sh.bins[2 * j + 1]; }, above, all);
+      if (tid == 0) {
+        const u64 covered = pair < 0 ? 0 : above + sh.bins[2 * pair];
+        const bool half = covered >= (u64)top_k;
+        sh.first_bin = half ? 2 * pair : 2 * pair + 1;
+        const u64 list = half || pair < 0 ? covered : covered + sh.bins[2 * pair + 1];
+        sh.besti = pair < 0 || list > (u64)FAST_CAP ? FAST_CAP + 1 : (int)list;      // how many were counted down to there
+      }
+    }
+    meet();
+    const int counted = first.besti;
+    const unsigned last_bin = (unsigned)first.first_bin;
+    if (counted <= FAST_CAP) {
+      for (int i0 = lo; i0 < hi; i0 += 8 * blockDim.x) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int i = i0 + u * blockDim.x + tid;
+          v[u] = i < hi ? row[i] : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int i = i0 + u * blockDim.x + tid;
           const unsigned key = order_key(v[u]);
-          if (i < n && ((top_key - key) >> 16) <= last_bin) {
-            const int at = atomicAdd(&sh.n_list, 1);
-            sh.list[at] = ((u64)key << 32) | (u64)(~(unsigned)i);
+          if (i < hi && ((top_key - key) >> 16) <= last_bin) {
+            const int at = atomicAdd(&first.n_list, 1);
+            if (at < FAST_CAP) first.list[at] = ((u64)key << 32) | (u64)(~(unsigned)i);
           }
         }
       }
-      __syncthreads();
+      meet();
+      const int total_c = first.n_list;
+      if (total_c > FAST_CAP) {                                // (only where the threads' maxima were counted)
+        meet();                                                // everybody has read the length
+        for (int b = tid; b < FAST_BINS; b += blockDim.x) sh.bins[b] = 0;
+        if (tid == 0) sh.n_list = 0;
+        __syncthreads();
+        continue;
+      }
+      if (blocks > 1) {
+        meet();
+        if (rank != 0) return;
+      }
+      if (total_c <= 256) {
+        // in order by rank: no two entries are alike
+        u64* sorted = reinterpret_cast<u64*>(sh.bins);
+        const int k = top_k < total_c ? top_k : total_c;
+        if (tid < total_c) {
+          const u64 mine = sh.list[tid];
+          int place = 0;
+          for (int i = 0; i < total_c; ++i) place += sh.list[i] > mine ? 1 : 0;
+          sorted[place] = mine;
+          sh.hist[place] = fixed_weight(key_value((unsigned)(mine >> 32)), lmax, temperature);
+        }
+        __syncthreads();
+        if (warp != 0) return;
+        u64 upto = 0, mass = 0, unused = 0;
+        warp_first_reaching(sh.hist, k, ~(u64)0, upto, mass);                        // (only the total is wanted here)
+        int kept = k;
+        if (top_p < 1.0f && mass > 0) {
+          u64 target = (u64)ceil((double)top_p * (double)mass);
+          target = target < 1 ? 1 : (target > mass ? mass : target);
+          const int j = warp_first_reaching(sh.hist, k, target, upto, unused);
+          if (j >= 0) {
+            kept = j + 1;
+            mass = upto + sh.hist[j];
+          }
+        }
+        u64 target = (u64)ceil((double)sh.u * (double)mass);
+        target = target < 1 ? 1 : (target > mass ? mass : target);
+        int pick = warp_first_reaching(sh.hist, kept, target, upto, unused);
+        if (pick < 0) pick = kept - 1;
+        if (lane == 0) out[r] = mass > 0 ? (int)(~(unsigned)(sorted[pick] & 0xffffffffu)) : best;
+        return;
+      }
       // bitonic sort, descending, over the next power of two (the padding, zeros, sorts to the end)
       int m = 1;
       while (m < total_c) m <<= 1;
@@ -398,9 +545,14 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
       target = target < 1 ? 1 : (target > mass ? mass : target);
       int pick = first_reaching(sh, kept, 0, target, weight_at, upto, unused);
       if (pick < 0) pick = kept - 1;
-      if (tid == 0) out[r] = mass > 0 ? (int)(~(unsigned)(sh.list[pick] & 0xffffffffu)) : sh.besti;
+      if (tid == 0) out[r] = mass > 0 ? (int)(~(unsigned)(sh.list[pick] & 0xffffffffu)) : best;
       return;
     }
+    meet();                                                    // nobody leaves while its memory is being read, or clears it
+    for (int b = tid; b < FAST_BINS; b += blockDim.x) sh.bins[b] = 0;
+    __syncthreads();
+    }  // counting
+    if (rank != 0) return;
   }
 
   // ---- the short way without a top_k: every logit is a candidate.  Weights are summed by the logits' distance below
@@ -420,12 +572,12 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
     for (int b = tid; b < 2 * WBINS; b += blockDim.x) sh.bins[b] = 0;
     __syncthreads();
     u64 rest_mine = 0;
-    for (int i0 = 0; i0 < n; i0 += 8 * blockDim.x) {
+    for (int i0 = lo; i0 < hi; i0 += 8 * blockDim.x) {
       float v[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int i = i0 + u * blockDim.x + tid;
-        v[u] = i < n ? row[i] : __int_as_float(0x7fc00000);        // past the row: not a number, weight 0
+        v[u] = i < hi ? row[i] : __int_as_float(0x7fc00000);        // past the row: not a number, weight 0
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
@@ -442,30 +594,72 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
         }
       }
     }
-    const u64 rest = block_sum_u64(sh, rest_mine);                  // (synchronises)
-    // gathers bin `b` into the list, sorted; false if it does not fit
-    auto gather_sorted = [&](int b) -> bool {
-      __syncthreads();
-      if (tid == 0) sh.n_list = 0;
-      __syncthreads();
-      for (int i0 = 0; i0 < n; i0 += 8 * blockDim.x) {
+    u64 rest = block_sum_u64(sh, rest_mine);                        // (synchronises)
+    if (blocks > 1) {
+      meet();
+      if (rank == 0) {
+        for (int b = tid; b < WBINS; b += blockDim.x) {
+          u64 t = wb_at(b);
+          for (int k = 1; k < blocks; ++k) {
+            const unsigned* part = cluster.map_shared_rank(&sh, k)->bins;
+            t += ((u64)part[WBINS + b] << 32) | (u64)part[b];
+          }
+          wlo[b] = (unsigned)t;
+          whi[b] = (unsigned)(t >> 32);
+        }
+        for (int k = 1; k < blocks; ++k) rest += cluster.map_shared_rank(&sh, k)->total;
+      }
+    }
+    // every block's part of bin `b` into the first block's list
+    auto gather = [&](int b) {
+      for (int i0 = lo; i0 < hi; i0 += 8 * blockDim.x) {
         float v[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int i = i0 + u * blockDim.x + tid;
-          v[u] = i < n ? row[i] : 0.f;
+          v[u] = i < hi ? row[i] : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int i = i0 + u * blockDim.x + tid;
           const unsigned key = order_key(v[u]);
-          if (i < n && bin_of(v[u]) == b && fixed_weight(v[u], lmax, temperature) > 0) {
-            const int at = atomicAdd(&sh.n_list, 1);
-            if (at < FAST_CAP) sh.list[at] = ((u64)key << 32) | (u64)(~(unsigned)i);
+          if (i < hi && bin_of(v[u]) == b && fixed_weight(v[u], lmax, temperature) > 0) {
+            const int at = atomicAdd(&first.n_list, 1);
+            if (at < FAST_CAP) first.list[at] = ((u64)key << 32) | (u64)(~(unsigned)i);
           }
         }
       }
+    };
+    // The blocks beside the first one gather what it asks for (`besti`: a bin, or -1: no more) until it needs nothing more;
+    // both sides meet twice for a bin and once for the end.
+    if (rank != 0) {
+      for (;;) {
+        meet();
+        const int b = first.besti;
+        if (b < 0) break;
+        gather(b);
+        meet();
+      }
+      meet();
+      return;
+    }
+    auto dismiss = [&] {
+      if (blocks == 1) return;
       __syncthreads();
+      if (tid == 0) sh.besti = -1;
+      meet();
+      meet();                                                  // (they have read it)
+    };
+    // gathers bin `b` into the list, sorted; false if it does not fit
+    auto gather_sorted = [&](int b) -> bool {
+      __syncthreads();
+      if (tid == 0) {
+        sh.n_list = 0;
+        sh.besti = b;
+      }
+      meet();
+      gather(b);
+      meet();
       const int c = sh.n_list;
       if (c > FAST_CAP) return false;
       int m = 1;
@@ -522,11 +716,17 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
         u64 upto = 0;
         int pick = first_reaching(sh, limit, before, target, weight_of, upto, unused);
         if (pick < 0) pick = limit - 1;
-        if (tid == 0) out[r] = pick >= 0 ? (int)(~(unsigned)(sh.list[pick] & 0xffffffffu)) : sh.besti;
+        if (tid == 0) out[r] = pick >= 0 ? (int)(~(unsigned)(sh.list[pick] & 0xffffffffu)) : best;
+        dismiss();
         return;
       }
     }
+    dismiss();
     __syncthreads();
+  }
+  if (top_k > FAST_CAP && top_k < n) {                         // neither short way: the other blocks are still here
+    meet();                                                    // (and their memory has been read)
+    if (rank != 0) return;
   }
 
   const int ishift = index_start_shift(n);
@@ -601,7 +801,7 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
   }
   radix_descend<false>(sh, n, ishift, jj, [&](int i, unsigned& v) { v = (unsigned)i; return order_key(row[i]) == sel && kept(i, sel); },
                        [&](int, unsigned) { return (u64)1; }, val, before, equal);
-  if (tid == 0) out[r] = equal > 0 ? (int)val : sh.besti;
+  if (tid == 0) out[r] = equal > 0 ? (int)val : best;
 }
 
 }  // namespace
@@ -612,6 +812,25 @@ extern "C" int gi_sample(int* out_tokens, const float* logits, long ld, int n_ro
   if (vocab <= 0) return gi::fail(GI_ERR_ARG, "sample: empty vocabulary");
   if (temperature > 0.f && !rng_state) return gi::fail(GI_ERR_ARG, "sample: temperature sampling needs generator states");
   if (top_k < 0) return gi::fail(GI_ERR_ARG, "sample: top_k must not be negative");
-  return gi::check(gi::launch(sample_kernel, dim3(n_rows), dim3(THREADS), 0, (cudaStream_t)stream, out_tokens, logits, ld, vocab,
-                              temperature, top_k, top_p, rng_state, state_index), "sample");
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0, count = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || count <= 0) count = 148;
+    sms = count;
+  }
+  const int blocks = blocks_per_row(n_rows, vocab, sms);
+  if ((long)n_rows * blocks > 2147483647L) return gi::fail(GI_ERR_UNSUPPORTED, "sample: %d rows are more than one launch takes", n_rows);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n_rows * blocks);
+  cfg.blockDim = dim3(THREADS);
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = gi::pdl_enabled() ? 2 : 1;
+  return gi::check(cudaLaunchKernelEx(&cfg, sample_kernel, out_tokens, logits, ld, vocab, temperature, top_k, top_p, rng_state, state_index), "sample");
 }

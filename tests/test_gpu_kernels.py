@@ -1136,3 +1136,28 @@ def test_float32_products_share_one_order_of_additions(m, n, k, accumulate):
     exact = a.double() @ w.double().T + (start.double() if accumulate else 0)
     bound = (a.double().abs() @ w.double().abs().T + start.double().abs()) * (chain + 32 + 3) * 2.0 ** -24
     assert ((got.double() - exact).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("vocab", [4099, 8192, 20001, 70000, 128256])
+@pytest.mark.parametrize("temp,top_k,top_p", [(0.0, 0, 1.0), (0.7, 40, 0.9), (1.3, 1, 1.0), (0.9, 2048, 0.95), (0.8, 2049, 1.0), (1.0, 0, 1.0), (0.5, 0, 0.9)])
+def test_sampler_picks_do_not_depend_on_the_blocks_a_row_gets(vocab, temp, top_k, top_p):
+    """160 rows get a block each; 100, 60, 20 and 1 of them clusters of 1, 2, 4 and 8: the same picks and generator states,
+    with rows of ties, of numbers that are none, of one value, with the highest logit at either end, off 16-byte boundaries."""
+    g = torch.Generator(device=DEV).manual_seed(vocab + top_k)
+    whole = torch.empty((160, vocab + 1), device=DEV).normal_(0.0, 2.5, generator=g)
+    for rows in (whole[:, :vocab], torch.nn.functional.pad(whole[:, :vocab], (0, (-vocab) % 4))[:, :vocab]):
+        rows[1] = 0.25                                       # all alike
+        rows[2] = (rows[2] * 2).round() / 2                  # many ties
+        rows[3, ::3] = float("nan")
+        rows[4] = float("nan")
+        rows[5] = -float("inf")
+        rows[6, :-1] = -float("inf")
+        rows[7, 0] = rows[7, -1] = 99.0                      # the first of two highest
+        rows[8, vocab // 2] = 1e30
+        states = torch.arange(1, 161, dtype=torch.int64, device=DEV) * 7919
+        want_states = states.clone()
+        want = ops.sample(rows, temp, top_k, top_p, want_states)
+        for a, b in ((0, 100), (0, 60), (0, 20), (0, 1), (1, 2), (2, 3), (3, 4), (4, 5), (5, 6), (6, 7), (7, 8), (8, 9), (150, 160)):
+            mine = states[a:b].clone()
+            assert torch.equal(ops.sample(rows[a:b], temp, top_k, top_p, mine), want[a:b]), (a, b)
+            assert torch.equal(mine, want_states[a:b])
