@@ -341,3 +341,36 @@ def test_recurrence_by_chunks_errs_no_more_than_the_walk(sizes, rate):
     assert err(y, want) <= 2 * err(y_walk, want) + 2.0 ** -22
     assert err(chunks, state) <= 2 * err(walk, state) + 2.0 ** -22
     assert torch.equal(chunks[:, heads * N * P:], before[:, heads * N * P:]) and torch.equal(chunks[0], before[0]) and torch.equal(chunks[-1], before[-1])
+
+
+@pytest.mark.parametrize("heads,P,N,G,taps,parts", [(4, 24, 16, 2, 4, 2), (2, 8, 40, 1, 3, 1), (8, 64, 128, 4, 2, 4), (16, 40, 96, 4, 4, 1), (34, 32, 8, 2, 4, 17)])
+def test_convolution_and_gated_norm_in_eights_and_fours(heads, P, N, G, taps, parts):
+    """16-bit rows by the kernels that read 16 bytes at a time, against 64 bits: the convolution to half a unit in the last of 8
+    bits (a number in [1, 2) has units of 2^-7, so at most 2^-8 of the value) beside 2^-20 of its terms for sums in 32 bits, the
+    norm likewise; sequences that begin in the middle and end
+    off the tiles of eight tokens."""
+    g = torch.Generator(device=DEV).manual_seed(heads + taps)
+    inner, ch = heads * P, heads * P + 2 * G * N
+    lens, T = [1, 8, 37, 3], 49
+    proj = torch.randn(T, 2 * inner + 2 * G * N + heads + (-heads) % 8, generator=g, device=DEV).bfloat16()
+    w, bias = (torch.randn(ch, taps, generator=g, device=DEV) * 0.5).bfloat16(), (torch.randn(ch, generator=g, device=DEV) * 0.2).bfloat16()
+    state = torch.randn(6, 5 + (taps - 1) * ch, generator=g, device=DEV)
+    before = state.clone()
+    step = step_of(lens, [0, 4, 9, 2], [1, 4, 0, 2])
+    got = ops.mamba2_conv(proj, w, bias, state, step, inner, ch, taps, 5)
+    at = 0
+    for n, slot in zip(lens, [1, 4, 0, 2]):
+        x = torch.cat([before[slot, 5:].view(taps - 1, ch), proj[at:at + n, inner:inner + ch]]).double()
+        terms = torch.stack([x[j:j + n] * w.double()[:, j] for j in range(taps)])
+        acc = terms.sum(0) + bias.double()
+        want = torch.nn.functional.silu(acc)
+        slack = (terms.abs().sum(0) + bias.double().abs()) * 2.0 ** -20
+        assert ((got[at:at + n].double() - want).abs() <= want.abs() * 2.0 ** -8 + slack).all()
+        assert torch.equal(state[slot, 5:].view(taps - 1, ch), x[n:].float())
+        at += n
+    y = torch.randn(T, inner, generator=g, device=DEV)
+    for nw in (torch.randn(inner, generator=g, device=DEV), torch.randn(inner, generator=g, device=DEV).bfloat16()):
+        out = ops.mamba2_gate_norm(y, proj, nw, parts, 1e-5, torch.bfloat16)
+        v = (y.double() * torch.nn.functional.silu(proj[:, :inner].double())).view(T, parts, -1)
+        v = (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5)).view(T, inner) * nw.double()
+        assert ((out.double() - v).abs() <= v.abs() * (2.0 ** -8 + 2.0 ** -18)).all()

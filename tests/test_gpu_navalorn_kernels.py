@@ -352,7 +352,7 @@ def test_ungated_experts_stretch_by_stretch():
 @pytest.mark.parametrize("seqs,window", [([(0, 300)], None), ([(70, 130), (0, 1), (5, 64), (64, 129)], None), ([(0, 513), (900, 64)], 100), ([(63, 65)], 64)])
 def test_prompt_attention_with_keys_and_values_per_head(sizes, seqs, window):
     """Rows formed per head against the formula in 64 bits: what is rounded to 8 bits (keys, values, probabilities, result) errs
-    by 2^-9 each, so a relative distance of 2^-8 holds for any of the sizes; pages that belong to nobody hold no numbers."""
+    by at most 2^-8 and on average by 2^-9.6 of itself, so a relative distance of 2^-8 holds for any of the sizes; pages that belong to nobody hold no numbers."""
     H, dim, rot, vd, rank = sizes
     g = torch.Generator(device=DEV).manual_seed(dim + vd + len(seqs))
     rnd = lambda *s, k=1.0: (torch.randn(*s, generator=g, device=DEV) * k).to(torch.bfloat16)
