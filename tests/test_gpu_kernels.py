@@ -1161,3 +1161,33 @@ def test_sampler_picks_do_not_depend_on_the_blocks_a_row_gets(vocab, temp, top_k
             mine = states[a:b].clone()
             assert torch.equal(ops.sample(rows[a:b], temp, top_k, top_p, mine), want[a:b]), (a, b)
             assert torch.equal(mine, want_states[a:b])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hd,hdv", [(64, 64), (4, 4), (36, 20), (128, 128), (128, 40), (20, 128)])
+@pytest.mark.parametrize("opts", [dict(), dict(window=40), dict(window=33, keep_first=5), dict(chunk=50)])
+def test_plain_attention_gives_the_same_bits_off_aligned_rows(dtype, hd, hdv, opts):
+    """Prompt and one-token attention four numbers a load, and one at a time (the same cache an element off): the same sums."""
+    g = torch.Generator(device=DEV).manual_seed(hd + hdv)
+    H, G, seqs = 6, 2, [(0, 70), (45, 33), (100, 1)]
+    lens, pos0 = [n for _, n in seqs], [p for p, _ in seqs]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    cu = i32([0, 70, 103, 104])
+    table, slots = i32([[3, 1], [5, 2], [4, 6]]), i32([0, 1, 2])
+    q = torch.randn(104, H * hd, generator=g, device=DEV).to(dtype)
+    sinks = torch.randn(H, generator=g, device=DEV)
+    outs = []
+    for off in (0, 1):
+        g.manual_seed(7)
+        k, v = (torch.empty(7 * G * 64 * d + 1, device=DEV, dtype=dtype)[off:off + 7 * G * 64 * d].view(7, G, 64, d) for d in (hd, hdv))
+        k.copy_(torch.randn(7, G, 64, hd, generator=g, device=DEV))
+        v.copy_(torch.randn(7, G, 64, hdv, generator=g, device=DEV))
+        a = torch.empty(104, H * hdv, device=DEV, dtype=dtype)
+        window = opts.get("window")
+        kw = dict(v_dim=hdv, sinks=sinks, **{n: x for n, x in opts.items() if n != "window"})
+        ops.attn_prefill_generic(q, k, v, table, cu, slots, i32(pos0), 3, 70, H, G, hd, 0.3, window, a, **kw)
+        b = torch.empty(3, H * hdv, device=DEV, dtype=dtype)
+        ops.attn_decode_generic(q[:3], k, v, table, slots, i32([p + n for p, n in seqs]), 3, H, G, hd, 0.3, window, 1, b, **kw)
+        outs.append((a, b))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert bool(torch.isfinite(outs[0][0].float()).all()) and bool(torch.isfinite(outs[0][1].float()).all())
