@@ -19,11 +19,11 @@
 // before took 844 us on average over a decode step's products of a 1B model (a 64-row tile for 4 rows, a fifth of the SMs).
 //
 // many_rows (a prompt): bound by the FFMA pipe (72 TFLOP/s at the maximum clock, 54-63 with three different operands).
-// 32 x 128 tiles, 8 x 4 outputs a thread, operands kept in k order in shared memory (rows padded to 36 numbers) and read
+// Tiles of 32 (to 48) x 128, 8 (to 12) x 4 outputs a thread, operands kept in k order in shared memory (rows padded to 36 numbers) and read
 // 16 bytes at a time, a warp's lanes along the columns so that a row's number is one broadcast; three blocks per SM:
 // small tiles because 600 rows x 2,048 columns are only 80 tiles of 128 x 128.  600 rows: 16,384 x 2,048 956 us (42 TFLOP/s;
-// single multiply-adds in 64 x 64 tiles 1,079 us, the kernel before 2,480 us), 2,048 x 2,048 184 us (three tiles on the
-// fullest SM where 2.05 would do; 245 us and 300 us).
+// single multiply-adds in 64 x 64 tiles 1,079 us, the kernel before 2,480 us), 2,048 x 2,048 142 us in tiles
+// of 36 rows, 184 us in tiles of 32 (three on the fullest SM where 2.05 would do; 245 us and 300 us).
 #include "api.h"
 #include "common.cuh"
 
@@ -158,12 +158,15 @@ few_rows_kernel(float* __restrict__ out, const float* A, const float* W, int M, 
   }
 }
 
-constexpr int BM = 32, BN = 128, BK = 32, TM = 8, TN = 4, KP = BK + 4, MANY_STAGES = 3, MANY_THREADS = 128;
-constexpr size_t MANY_SMEM = sizeof(float) * MANY_STAGES * (BM + BN) * KP;
+constexpr int BN = 128, BK = 32, TN = 4, KP = BK + 4, MANY_STAGES = 3, MANY_THREADS = 128;
+template <int TM>
+constexpr size_t MANY_SMEM = sizeof(float) * MANY_STAGES * (4 * TM + BN) * KP;
 
-template <bool ACCUM>
-__global__ void __launch_bounds__(MANY_THREADS, 3)
+// TM: rows a thread takes, a tile has 4 TM
+template <int TM, bool ACCUM>
+__global__ void __launch_bounds__(MANY_THREADS, TM == 8 ? 3 : 2)
 many_rows_kernel(float* __restrict__ out, const float* A, const float* W, int M, int N, int K, long lda, long ldw, long ldo, int seg) {
+  constexpr int BM = 4 * TM;
   extern __shared__ __align__(16) float smem[];
   const int tid = threadIdx.x, tx = tid % 32, ty = tid / 32;  // thread owns rows ty + 4 i, columns tx + 32 j
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
@@ -176,10 +179,10 @@ many_rows_kernel(float* __restrict__ out, const float* A, const float* W, int M,
       float* st = smem + (size_t)(g % MANY_STAGES) * (BM + BN) * KP + q * 4;
       const int k = g * BK + q * 4;
 #pragma unroll
-      for (int i = 0; i < BM / 16; ++i) {
+      for (int i = 0; i < (BM + 15) / 16; ++i) {
         const int r = r0 + 16 * i;
         const bool ok = k < K && m0 + r < M;
-        cp16(st + r * KP, ok ? A + (size_t)(m0 + r) * lda + k : A, ok);
+        if (r < BM) cp16(st + r * KP, ok ? A + (size_t)(m0 + r) * lda + k : A, ok);
       }
 #pragma unroll
       for (int i = 0; i < BN / 16; ++i) {
@@ -279,25 +282,40 @@ int launch_few(float* out, const float* A, const float* W, int M, int N, int K, 
 }
 
 // Which of the two, by what they measured (us per 2,048 of K): few_rows takes 33 / 52 / 65 for each pass of up to 4 / 8 / 16
-// tokens over 16,384 columns; many_rows 20 and 55 more for every tile the fullest SM works through.  2,048 columns: 48
-// rows 32 against 75, 100 rows 57 against 77; 16,384 columns: 48 rows 186 against 128; 128,256 columns: 16 rows 468
-// against about 400.
-bool many_is_faster(int M, int N) {
-  const double few = (M <= 4 ? 33.0 : M <= 8 ? 52.0 : 65.0 * ((M + 15) / 16)) / 16384.0 * N;
-  const long tiles = (long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  return few > 20.0 + 55.0 * ((tiles + sm_count() - 1) / sm_count());
+// tokens over 16,384 columns; many_rows 20 and 55 more for every tile of 32 rows the fullest SM works through.  2,048
+// columns: 48 rows 32 against 75, 100 rows 57 against 77; 16,384 columns: 48 rows 186 against 128; 128,256 columns: 16 rows
+// 468 against about 400.
+// A tile has 32 rows, or 36, 40 or 48 where that spares the fullest SM a tile: 601 rows x 2,048 columns are 304 tiles of 32
+// rows, three on some SMs (184 us), and 272 of 36, two at most (142 us).
+// The wider tiles leave room for two blocks an SM instead of three and cost 5% more for their rows (16,384 columns: 985 us
+// against 956).
+double few_cost(int M, int N) { return (M <= 4 ? 33.0 : M <= 8 ? 52.0 : 65.0 * ((M + 15) / 16)) / 16384.0 * N; }
+double many_cost(int M, int N, int tm) {
+  const long tiles = (long)((M + 4 * tm - 1) / (4 * tm)) * ((N + BN - 1) / BN);
+  return 20.0 + (tm == 8 ? 55.0 : 7.2 * tm) * (double)((tiles + sm_count() - 1) / sm_count());
+}
+
+template <int TM, bool ACCUM>
+int launch_many(float* out, const float* A, const float* W, int M, int N, int K, long lda, long ldw, long ldo, int seg, cudaStream_t s) {
+  static bool seen[gi::MAX_DEVICES_SEEN];
+  const int rc = allow_smem(many_rows_kernel<TM, ACCUM>, MANY_SMEM<TM>, seen);
+  if (rc != GI_OK) return rc;
+  // row tiles fastest: blocks that run together share a tile of W, the larger operand
+  const dim3 grid((M + 4 * TM - 1) / (4 * TM), (N + BN - 1) / BN);
+  return gi::check(gi::launch(many_rows_kernel<TM, ACCUM>, grid, dim3(MANY_THREADS), MANY_SMEM<TM>, s, out, A, W, M, N, K, lda, ldw, ldo, seg), "gemm_f32");
 }
 
 template <bool ACCUM>
 int launch_product(float* out, const float* A, const float* W, int M, int N, int K, long lda, long ldw, long ldo, cudaStream_t s) {
   const int seg = gi::sum_segment(K);
-  if (many_is_faster(M, N)) {
-    static bool seen[gi::MAX_DEVICES_SEEN];
-    const int rc = allow_smem(many_rows_kernel<ACCUM>, MANY_SMEM, seen);
-    if (rc != GI_OK) return rc;
-    // row tiles fastest: blocks that run together share a tile of W, the larger operand
-    const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
-    return gi::check(gi::launch(many_rows_kernel<ACCUM>, grid, dim3(MANY_THREADS), MANY_SMEM, s, out, A, W, M, N, K, lda, ldw, ldo, seg), "gemm_f32");
+  int tm = 8;
+  for (int t : {9, 10, 12})
+    if (many_cost(M, N, t) < many_cost(M, N, tm)) tm = t;
+  if (few_cost(M, N) > many_cost(M, N, tm)) {
+    if (tm == 8) return launch_many<8, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
+    if (tm == 9) return launch_many<9, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
+    if (tm == 10) return launch_many<10, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
+    return launch_many<12, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
   }
   if (M == 1) return launch_few<1, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
   if (M == 2) return launch_few<2, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
