@@ -8,6 +8,7 @@
 //           Everything here is 32-bit; the tokens of a sequence are walked in order, thirty-two at a time through shared
 //           memory; a warp owns two or four columns p of S, its lanes the rows n, kept in registers across the step.
 //           One token or a thousand, alone or in a batch, take the same arithmetic in the same order: no bit changes.
+//           (Prompt steps in 16-bit rows take chunks of tokens as matrix products instead: mamba2_chunks.cu.)
 //  * gate + norm: y * silu(z), divided by the root mean square of each of `parts` equal parts, times a weight.
 // Per-sequence state: one float row per slot, [S: heads * P * N, a column's N rows side by side (a lane's rows are then
 // neighbours in memory: a one-token step, which is all loading and storing of S, moves whole lines) | last taps - 1 conv

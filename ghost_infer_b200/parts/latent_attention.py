@@ -16,7 +16,8 @@ Only c and the rotated kr are cached: one row [c | kr] per position, shared by a
 as key and as value (`CacheRequest(values_in_keys=True)`).  To attend over such rows a head's unrotated query is carried
 onto the latent, qa_h = W_uk,h^T q_h,unrot (so that qa_h . c = q_h,unrot . k_h), the attention runs with every head
 reading the same rows, its result per head is a weighted sum of latents, and W_uv,h turns that into the head's values (which
-is why one gate per head may as well multiply the sum of latents).
+is why one gate per head may as well multiply the sum of latents).  A 16-bit prompt step of more than a few tokens forms k_h
+and v_h of the visible positions instead and attends over those (`ops.latent_expand_rows` says when).
 Norms, angles, scores and softmax are 32-bit.
 
 Tensor names: prefix + "mix.{dq,dq.norm,uq,dkv,dkv.norm,uk,uv,o}" ("mix.q" in place of the first three without a query latent;
