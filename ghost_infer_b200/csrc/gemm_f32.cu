@@ -311,7 +311,8 @@ int launch_product(float* out, const float* A, const float* W, int M, int N, int
   int tm = 8;
   for (int t : {9, 10, 12})
     if (many_cost(M, N, t) < many_cost(M, N, tm)) tm = t;
-  if (few_cost(M, N) > many_cost(M, N, tm)) {
+  // (few_rows has 16 tokens to a block of the grid's y, which takes 65,535)
+  if (few_cost(M, N) > many_cost(M, N, tm) || M > 16 * 65535) {
     if (tm == 8) return launch_many<8, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
     if (tm == 9) return launch_many<9, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
     if (tm == 10) return launch_many<10, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);

@@ -1994,7 +1994,7 @@ def attention_latent(qa: torch.Tensor, memory, step, n_heads: int, rank: int, ro
     return out if gate is None else head_gate_rows(out, gate, n_heads, rank)
 
 
-LATENT_EXPAND_BYTES = 1 << 30      # of keys and values per head that a prompt step may form at a time
+LATENT_EXPAND_BYTES = 1 << 28      # of keys and values per head that a prompt step may form at a time (32,768 positions of 16 heads of 128 and 128)
 
 
 def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, rank: int, window: Optional[int], dtype: torch.dtype) -> int:
