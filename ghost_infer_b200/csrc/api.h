@@ -253,6 +253,15 @@ int gi_attn_prefill_t5_rows(void* out, long ldo, const void* q, long ldq, long q
                             long ldv, const void* r, long ldr, long kv_rows, const int* cu_seqlens, const int* seq_slots,
                             const int* seq_pos0, int n_seqs, int max_q_len, int n_heads, int dim, int rot, int vdim,
                             float scale, int window, const float* sinks, const void* gate, long ldg, void* stream);
+// A prompt step's latent attention through both and the product between them: the queries' rotated parts turned in place by
+// `table` (the first `rot_numbers` of each, 0: none), the visible latents out of the cache into rows [kv_rows][rank + rot], kv
+// [kv_rows][w_rows] = rows' latents x w_uk_uv^T [heads * dim + heads * vdim (+ padding)][rank], then the attention.
+int gi_latent_attend_expanded(void* out, long ldo, void* q, long ldq, long n_tokens, const float* table, int rot_numbers,
+                              void* rows, void* kv, long kv_rows, const void* w_uk_uv, int w_rows, const void* cache,
+                              const int* block_table, int max_pages, const int* cu_seqlens, const int* seq_slots,
+                              const int* seq_pos0, int n_seqs, int max_q_len, int max_rows, int n_heads, int dim, int rot,
+                              int vdim, int rank, float scale, int window, const float* sinks, const void* gate, long ldg,
+                              int tile_n, void* stream);
 // out[t, h * ohs + n] = sum_k a[t, h * ahs + k] * w[h * whs + n * ldw + k * kstride], n < N, k < K, for every head h; out has
 // a's type.  tensor_cores: bfloat16 operands with kstride 1 take `mma.sync`.
 int gi_bmm_heads(void* out, long ldo, long ohs, const void* a, long lda, long ahs, int dtype, const void* w, int w_dtype,

@@ -654,6 +654,28 @@ extern "C" int gi_latent_gather(void* out, const void* cache, const int* block_t
                    "latent rows");
 }
 
+// Four launches behind one call: in a prompt of a few hundred tokens the host's time per call is what a layer takes.
+extern "C" int gi_latent_attend_expanded(void* out, long ldo, void* q, long ldq, long n_tokens, const float* table, int rot_numbers,
+                                         void* rows, void* kv, long kv_rows, const void* w_uk_uv, int w_rows, const void* cache,
+                                         const int* block_table, int max_pages, const int* cu_seqlens, const int* seq_slots,
+                                         const int* seq_pos0, int n_seqs, int max_q_len, int max_rows, int n_heads, int dim, int rot,
+                                         int vdim, int rank, float scale, int window, const float* sinks, const void* gate, long ldg,
+                                         int tile_n, void* stream) {
+  if (n_tokens <= 0) return GI_OK;
+  if (n_heads <= 0 || rank <= 0 || (long)n_heads * (dim + vdim) > w_rows || kv_rows <= 0 || kv_rows > 0x7fffffffL || n_tokens > 0x7fffffffL)
+    return gi::fail(GI_ERR_ARG, "latent attention: %d heads, rank %d, %d rows of matrices, %ld positions", n_heads, rank, w_rows, kv_rows);
+  const int hd = rank + rot;
+  int rc = GI_OK;
+  if (rot_numbers > 0) rc = gi_latent_query_rot(q, ldq, q, ldq, GI_BF16, table, rot_numbers, (int)n_tokens, n_heads, dim, rot, dim, stream);
+  if (rc == GI_OK) rc = gi_latent_gather(rows, cache, block_table, max_pages, cu_seqlens, seq_slots, seq_pos0, n_seqs, max_rows, hd, window, stream);
+  if (rc == GI_OK) rc = gi_gemm_tc_bf16(kv, GI_SKINNY_STORE_BF16, rows, w_uk_uv, (int)kv_rows, w_rows, rank, hd, rank, w_rows, tile_n, stream);
+  if (rc != GI_OK) return rc;
+  const __nv_bfloat16* k = (const __nv_bfloat16*)kv;
+  return gi_attn_prefill_t5_rows(out, ldo, q, ldq, n_tokens, k, w_rows, k + (size_t)n_heads * dim, w_rows, (const __nv_bfloat16*)rows + rank,
+                                 hd, kv_rows, cu_seqlens, seq_slots, seq_pos0, n_seqs, max_q_len, n_heads, dim, rot, vdim, scale, window,
+                                 sinks, gate, ldg, stream);
+}
+
 extern "C" int gi_bmm_heads(void* out, long ldo, long ohs, const void* a, long lda, long ahs, int dtype, const void* w, int w_dtype,
                             long whs, long ldw, long kstride, int M, int N, int K, int heads, int tensor_cores, void* stream) {
   if (M <= 0 || heads <= 0) return GI_OK;

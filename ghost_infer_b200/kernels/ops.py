@@ -62,8 +62,7 @@ def _bind():
         "gi_attn_prefill_t5": [P, L, P, L, L, P, P, L, P, I, P, P, P, I, I, I, I, I, F, I, P],
         "gi_attn_prefill_t5_status": [P],
         "gi_attn_prefill_t5_ex": [P, L, P, L, L, P, P, L, P, I, P, P, P, I, I, I, I, I, F, I, F, P, I, P],
-        "gi_latent_gather": [P, P, P, I, P, P, P, I, I, I, I, P],
-        "gi_attn_prefill_t5_rows": [P, L, P, L, L, P, L, P, L, P, L, L, P, P, P, I, I, I, I, I, I, F, I, P, P, L, P],
+        "gi_latent_attend_expanded": [P, L, P, L, L, P, I, P, P, L, P, I, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, P, L, I, P],
         "gi_attn_prefill_t5_ex2": [P, L, P, L, L, L, P, P, L, P, I, P, P, P, I, I, I, I, I, F, I, F, P, I, I, P],
         "gi_attn_prefill_tc_ex2": [P, L, P, L, P, P, P, I, P, P, P, I, I, I, I, I, F, I, I, F, P, I, I, P],
         "gi_attn_decode_tc": [P, L, P, P, P, L, P, P, P, I, P, P, I, I, I, I, F, I, I, P],
@@ -2004,8 +2003,8 @@ def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, r
     Carried, a head spends 2 rank + rot_dim multiply-adds on a query and key; expanded, dim + rot_dim + v_dim, and rank (dim +
     v_dim) more on every visible position once.  Measured multiply-adds per microsecond: the carried kernel 74e6 (a block's
     tile of 64 keys 8.3 us at 1,088 of them, which is what few tokens behind a long prefix wait for), the products that carry
-    queries and results 32e6, the attention over rows 200e6 (2 us a tile), the product that forms the rows 400e6; 15 us for the
-    launches more.  16 heads, rank 512: 64 fresh tokens are carried; 16 tokens behind 3,000 take 98 us expanded, 418 carried.
+    queries and results 32e6, the attention over rows 200e6 (2 us a tile), the product that forms the rows 400e6; 40 us
+    for what the host spends more on a few hundred tokens (tensor maps of new buffers).  16 heads, rank 512: 64 fresh tokens are carried; 16 tokens behind 3,000 take 98 us expanded, 418 carried.
     Only prompt steps have the host's lists of lengths; sizes are those the tcgen05 kernel takes."""
     if (step.is_decode or dtype != torch.bfloat16 or not TUNE["attn_latent_tc"] or dim not in (64, 128) or not 0 < rot_dim <= 64
             or rot_dim % 16 or not 0 < v_dim <= 128 or v_dim % 8 or rank % 8):
@@ -2025,17 +2024,17 @@ def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, r
         return 0
     work = 2 * rank + rot_dim
     carried = max(n_heads * pairs * work / 74e6, tiles * work * 7.6e-3) + n_heads * tokens * rank * (dim + v_dim) / 32e6
-    expanded = max(n_heads * pairs * (dim + rot_dim + v_dim) / 200e6, tiles * 2.0) + n_heads * rows * rank * (dim + v_dim) / 400e6 + 15.0
+    expanded = max(n_heads * pairs * (dim + rot_dim + v_dim) / 200e6, tiles * 2.0) + n_heads * rows * rank * (dim + v_dim) / 400e6 + 40.0
     return rows if expanded < carried else 0
 
 
 def attention_latent_expanded(q: torch.Tensor, memory, step, w_uk_uv: torch.Tensor, rows: int, n_heads: int, dim: int, rot_dim: int,
                               v_dim: int, rank: int, scale: float, window: Optional[int] = None, sinks: Optional[torch.Tensor] = None,
-                              gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+                              gate: Optional[torch.Tensor] = None, table: Optional[torch.Tensor] = None, rot: int = 0) -> torch.Tensor:
     """A prompt step's latent attention with keys and values formed per head: the visible positions' rows [latent (rank) | rotary
     key part (rot_dim)] leave their pages, one product with `w_uk_uv` [heads * dim + heads * v_dim (+ padding), rank] gives every
     head's unrotated keys and values, and the tcgen05 kernel reads those beside the shared rotary part.  `q` [tokens, heads *
-    (dim + rot_dim)] with its rotated parts turned, `rows` from `latent_expand_rows`; returns [tokens, heads * v_dim].  `window`,
+    (dim + rot_dim)], the first `rot` numbers of whose rotated parts are turned in place by `table` (0: they are already), `rows` from `latent_expand_rows`; returns [tokens, heads * v_dim].  `window`,
     `sinks`, `gate`: as `attention_latent`'s."""
     hd = rank + rot_dim
     if memory.k is None or memory.k.dtype != q.dtype or tuple(memory.k.shape[1:]) != (1, 64, hd) or not memory.k.is_contiguous():
@@ -2044,23 +2043,24 @@ def attention_latent_expanded(q: torch.Tensor, memory, step, w_uk_uv: torch.Tens
         raise KernelError("latent attention: rows of the wrong sizes")
     if gate is not None and (gate.dtype != q.dtype or tuple(gate.shape) != (q.shape[0], n_heads) or not gate.is_cuda):
         raise KernelError(f"the heads' gates must be [{q.shape[0]}, {n_heads}] rows of the queries' type")
+    if not tc_ok(q, w_uk_uv) or not w_uk_uv.is_contiguous() or w_uk_uv.shape[0] % 8:
+        raise KernelError("latent attention: queries and matrices must be bfloat16 rows on 16-byte boundaries")
+    if rot and (table is None or table.dtype != torch.float32 or tuple(table.shape) != (q.shape[0], rot // 2, 2) or not table.is_contiguous()):
+        raise KernelError(f"the table of angles must be contiguous float32 [{q.shape[0]}, {rot // 2}, 2]")
     lib = _bind()
     _cuda(q, "queries")
-    bt, window = memory.block_table, int(window or 0)
+    bt, window, w_rows = memory.block_table, int(window or 0), w_uk_uv.shape[0]
     latents = torch.empty((rows, hd), dtype=q.dtype, device=q.device)
-    longest = min(step.max_kv_len, window + step.max_q_len + 63) if window else step.max_kv_len
-    _check(lib, lib.gi_latent_gather(latents.data_ptr(), memory.k.data_ptr(), _i32(bt, "block table"), bt.shape[1],
-                                     _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"), _i32(step.seq_pos0, "start positions"),
-                                     step.n_seqs, int(longest), hd, window, _stream()))
-    kv = linear(latents[:, :rank], w_uk_uv, out_dtype=q.dtype)
+    kv = torch.empty((rows, w_rows), dtype=q.dtype, device=q.device)
     out = torch.empty((q.shape[0], n_heads * v_dim), dtype=q.dtype, device=q.device)
-    v, r = kv[:, n_heads * dim:], latents[:, rank:]
-    _check(lib, lib.gi_attn_prefill_t5_rows(
-        out.data_ptr(), _rows(out, "attention output"), q.data_ptr(), _rows(q, "queries"), q.shape[0], kv.data_ptr(), _rows(kv, "keys"),
-        v.data_ptr(), _rows(kv, "values"), r.data_ptr(), hd, rows, _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"),
-        _i32(step.seq_pos0, "start positions"), step.n_seqs, step.max_q_len, n_heads, dim, rot_dim, v_dim, float(scale), window,
-        _sinks_ptr(sinks, n_heads), gate.data_ptr() if gate is not None else None, _rows(gate, "gate rows") if gate is not None else 0,
-        _stream()))
+    longest = min(step.max_kv_len, window + step.max_q_len + 63) if window else step.max_kv_len
+    _check(lib, lib.gi_latent_attend_expanded(
+        out.data_ptr(), n_heads * v_dim, q.data_ptr(), _rows(q, "queries"), q.shape[0], table.data_ptr() if rot else None, int(rot),
+        latents.data_ptr(), kv.data_ptr(), rows, w_uk_uv.data_ptr(), w_rows, memory.k.data_ptr(), _i32(bt, "block table"), bt.shape[1],
+        _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"), _i32(step.seq_pos0, "start positions"), step.n_seqs,
+        step.max_q_len, int(longest), n_heads, dim, rot_dim, v_dim, rank, float(scale), window, _sinks_ptr(sinks, n_heads),
+        gate.data_ptr() if gate is not None else None, _rows(gate, "gate rows") if gate is not None else 0, TC_TILE_N, _stream()),
+        4 if rot else 3)
     return out
 
 

@@ -178,9 +178,6 @@ class LatentAttention(Mixer):
                                     step.positions, step.token_slots, memory, self.q_rank, self.rank, self.rot_dim)
         with ops.bucket("qkv matmul"):
             q = linear(cq, self.w_uq, out_dtype=dt) if self.q_rank else down[:, own:own + H * (self.dim + self.rot_dim)]
-        if self.rot:
-            with ops.bucket("rope+cache"):
-                ops.latent_query_rot(q, q, table, self.rot, H, self.dim, self.rot_dim, self.dim)      # in place
         gate = None
         if self.out_gate == "head_sigmoid":
             with ops.bucket("out matmul"):
@@ -188,7 +185,7 @@ class LatentAttention(Mixer):
                 gate = linear(h, self.w_g, out_dtype=dt) if self.w_g is not None else down[:, at:at + H]
         with ops.bucket("attention"):
             att = ops.attention_latent_expanded(q, memory, step, self.w_uk_uv, rows, H, self.dim, self.rot_dim, self.v_dim, self.rank,
-                                                self.scale, window=self.window, sinks=self.sinks, gate=gate)
+                                                self.scale, window=self.window, sinks=self.sinks, gate=gate, table=table, rot=self.rot)
         with ops.bucket("out matmul"):
             if self.out_gate == "sigmoid":
                 att = ops.gate_mul(att, linear(h, self.w_g, out_dtype=dt), "sigmoid")
