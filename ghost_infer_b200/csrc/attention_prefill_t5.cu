@@ -422,7 +422,12 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int lo = max(0, t_first - kt), hi = min(BKV, p_last + 1 - kt);
       const int lo_kept = min(lo, max(0, kept - kt));      // of the rows before every window, the first lo_kept are kept first positions: seen
       if (lo > lo_kept || hi < BKV) {
-        ok = mbar_wait(v_full0 + 8 * (j & (V_STAGES - 1)), (uint32_t)((j / V_STAGES) & 1), 3, &g_attn_status);
+        // Which phase of `v_full` a parity names is only known once the stage's phase before is complete.  With two stages
+        // that is tile j - 2's, which the scores of tile j waited for; with one it is tile j - 1's, whose values may still be
+        // on their way: the wait would return at once and the zeros go over the rows of tile j - 1.  Its product (the
+        // barrier's phase before is tile j - 3's, known to be done) says that they came and have been read.
+        if (V_STAGES == 1 && j > 0) ok = mbar_wait(kv_empty0 + 8 * ((j - 1) & 1), (uint32_t)(((j - 1) >> 1) & 1), 3, &g_attn_status);
+        if (ok) ok = mbar_wait(v_full0 + 8 * (j & (V_STAGES - 1)), (uint32_t)((j / V_STAGES) & 1), 3, &g_attn_status);
         if (!ok) break;
         unsigned char* vt = v_s + (j & (V_STAGES - 1)) * V_BYTES;
         for (int idx = threadIdx.x; idx < BKV * (VD / 8); idx += 128) {
