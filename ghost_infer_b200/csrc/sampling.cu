@@ -608,6 +608,7 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
           whi[b] = (unsigned)(t >> 32);
         }
         for (int k = 1; k < blocks; ++k) rest += cluster.map_shared_rank(&sh, k)->total;
+        __syncthreads();                                            // every bin is whole before any thread sums its neighbours
       }
     }
     // every block's part of bin `b` into the first block's list

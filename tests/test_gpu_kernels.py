@@ -1163,6 +1163,22 @@ def test_sampler_picks_do_not_depend_on_the_blocks_a_row_gets(vocab, temp, top_k
             assert torch.equal(mine, want_states[a:b])
 
 
+@pytest.mark.parametrize("rows", [1, 16, 32, 60])
+@pytest.mark.parametrize("top_p", [1.0, 0.9])
+def test_sampler_without_top_k_sums_the_blocks_bins_before_it_reads_them(rows, top_p):
+    """Logits whose weights spread over some 700 of the 2,048 bins, 300 draws a row: a bin left out of the total moves the
+    target, and with it nearly every pick.  The answer is that of rows that get a block each."""
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    logits = torch.empty((rows, 50000), device=DEV).normal_(0.0, 2.5, generator=g)
+    alone = logits.repeat((299 + rows) // rows, 1)           # 300 rows and more: no clusters
+    states = torch.arange(1, 1 + rows, dtype=torch.int64, device=DEV) * 6364136223846793005
+    for _ in range(300):
+        want_states = states.repeat(alone.shape[0] // rows)
+        want = ops.sample(alone, 1.0, 0, top_p, want_states)
+        assert torch.equal(ops.sample(logits, 1.0, 0, top_p, states), want[:rows])
+        assert torch.equal(states, want_states[:rows])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("hd,hdv", [(64, 64), (4, 4), (36, 20), (128, 128), (128, 40), (20, 128)])
 @pytest.mark.parametrize("opts", [dict(), dict(window=40), dict(window=33, keep_first=5), dict(chunk=50)])
