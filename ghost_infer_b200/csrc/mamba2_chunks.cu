@@ -12,7 +12,8 @@
 // tensor cores' rounding towards zero does not pile up over chunks.  c is summed in 64 bits: exp(c_i - c_j) of neighbours
 // would lose the digits that c has grown by.  Decays between different 16-token tiles are products of two factors, both
 // at most 1, taken at the first tile's start: 64 + 192 exponentials a chunk instead of 2,016.
-// Rows and columns past N, P and the chunk's end are zeros.
+// Rows and columns past N, P and the chunk's end are zeros.  A chunk that comes to an infinity or a not-a-number is walked
+// token by token after all (`walk_chunk`), so that neither reaches an earlier token.
 // B200, 2,048 tokens, 64 heads of 64, N 128: 172 us, the walk 660 us; 2,556 tokens in three sequences, 64 heads of 40, N 96:
 // 227 and 404 us; 365 in four: 58 and 92 us.  What bounds it now is the chain of a chunk (about 5 us: operands out of shared
 // memory, four products one after the other, two barriers), not the tensor cores' rate.
@@ -36,14 +37,25 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16 (&part)[3]) {
   part[1] = __float2bfloat16_rn(r);
   part[2] = __float2bfloat16_rn(r - __bfloat162float(part[1]));
 }
+__device__ __forceinline__ uint32_t two(__nv_bfloat16 lo, __nv_bfloat16 hi) {
+  return (uint32_t)__bfloat16_as_ushort(lo) | (uint32_t)__bfloat16_as_ushort(hi) << 16;
+}
 __device__ __forceinline__ void split3_pair(float lo, float hi, uint32_t (&out)[3]) {
   __nv_bfloat16 a[3], b[3];
   split3(lo, a);
   split3(hi, b);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) out[i] = (uint32_t)__bfloat16_as_ushort(a[i]) | (uint32_t)__bfloat16_as_ushort(b[i]) << 16;
+  for (int i = 0; i < 3; ++i) out[i] = two(a[i], b[i]);
 }
 
+// the same of a number of the state, which may be beyond what rounds to a finite 16-bit number, or infinite
+__device__ __forceinline__ void split3_state(float v, __nv_bfloat16 (&part)[3]) {
+  part[0] = __float2bfloat16_rn(v);
+  if (__hisinf(part[0])) part[0] = __float2bfloat16_rz(v);
+  const float r = isinf(v) ? 0.f : v - __bfloat162float(part[0]);
+  part[1] = __float2bfloat16_rn(r);
+  part[2] = __float2bfloat16_rn(r - __bfloat162float(part[1]));
+}
 template <int NT>
 struct Layout {
   static constexpr int NP = 16 * NT;                         // rows of S with padding
@@ -55,6 +67,53 @@ struct Layout {
   static constexpr int DT_AT = CUM_AT + 2 * 8 * Q;           // float[2][Q]
   static constexpr int EI_AT = DT_AT + 2 * 4 * Q, EJ_AT = EI_AT + 4 * Q, IN_AT = EJ_AT + 16 * Q, BYTES = IN_AT + 4 * Q;
 };
+
+// A chunk whose products came to something that is no finite number, walked token by token from the state before it: a
+// product over 16 tokens lets an infinity or a not-a-number of one token meet the zero weights of earlier ones, and a split
+// infinity is none any more, where the recurrence carries both forward only.  `y`: the chunk's first token, this block's
+// columns; `cols` of them exist.  The state behind the chunk is left in the next buffer of S, [n][column] in 32 bits.
+// Thread: column tid % 32, every eighth row from tid / 32 on.
+template <int NT>
+__device__ __noinline__ void walk_chunk(unsigned char* smem, int buf, float* y, int inner, int nc, int cols, int N, float A, float D) {
+  using L = Layout<NT>;
+  constexpr int ROWS = L::NP / 8;
+  const int p = threadIdx.x & 31, first = threadIdx.x >> 5;
+  const unsigned char* in = smem + buf * L::BUF;
+  const float* dts = reinterpret_cast<const float*>(smem + L::DT_AT) + buf * Q;
+  float* sums = reinterpret_cast<float*>(smem + L::W_AT);    // [8][32]
+  auto number = [](const unsigned char* at) { return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(at)); };
+  float S[ROWS];
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k) {
+    const unsigned char* at = smem + L::S_AT + 3 * buf * L::S_PART + (first + 8 * k) * XP + 2 * p;
+    S[k] = number(at) + (number(at + L::S_PART) + number(at + 2 * L::S_PART));
+  }
+  for (int t = 0; t < nc; ++t) {
+    const float dt = dts[t], keep = expf(A * dt), x = number(in + L::X_AT + t * XP + 2 * p);
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const int n = first + 8 * k;
+      if (n < N) {
+        S[k] = fmaf(keep, S[k], x * (number(in + L::B_AT + t * L::BP + 2 * n) * dt));
+        sum = fmaf(S[k], number(in + L::C_AT + t * L::BP + 2 * n), sum);
+      }
+    }
+    sums[threadIdx.x] = sum;
+    __syncthreads();
+    if (first == 0 && p < cols) {
+      sum = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) sum += sums[w * 32 + p];
+      y[(size_t)t * inner + p] = fmaf(D, x, sum);
+    }
+    __syncthreads();
+  }
+  float* next = reinterpret_cast<float*>(smem + L::S_AT + 3 * (buf ^ 1) * L::S_PART);
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k) next[(first + 8 * k) * PT + p] = first + 8 * k < N ? S[k] : 0.f;
+  __syncthreads();
+}
 
 // grid (heads, sequences, column tiles of 32)
 template <int NT>
@@ -153,11 +212,12 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
       for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          uint32_t part[3];
-          split3_pair(sacc[k][2 * r], sacc[k][2 * r + 1], part);
+          __nv_bfloat16 lo[3], hi[3];
+          split3_state(sacc[k][2 * r], lo);
+          split3_state(sacc[k][2 * r + 1], hi);
 #pragma unroll
           for (int s = 0; s < 3; ++s)
-            *reinterpret_cast<uint32_t*>(smem + L::S_AT + (3 * buf + s) * L::S_PART + (srow + 8 * r) * XP + (8 * k + lc) * 2) = part[s];
+            *reinterpret_cast<uint32_t*>(smem + L::S_AT + (3 * buf + s) * L::S_PART + (srow + 8 * r) * XP + (8 * k + lc) * 2) = two(lo[s], hi[s]);
         }
     }
   };
@@ -168,12 +228,30 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
   const uint32_t a_row = (uint32_t)((lane & 7) + ((lane >> 3) & 1) * 8), a_col = (uint32_t)(lane >> 4) * 16;   // ldmatrix rows, bytes
   const uint32_t b_row = (uint32_t)((lane & 7) + (lane >> 4) * 8), b_col = (uint32_t)((lane >> 3) & 1) * 16;
 
-  for (int c0 = 0, buf = 0; c0 < qlen; c0 += Q, buf ^= 1) {
+  // the chunk before once more, token by token
+  auto again = [&](int c0, int buf) {
+    walk_chunk<NT>(smem, buf, y + (size_t)(tok0 + c0) * inner + (size_t)h * P + p0, inner, min(Q, qlen - c0), P - p0, N, A, D);
+    const float* next = reinterpret_cast<const float*>(smem + L::S_AT + 3 * (buf ^ 1) * L::S_PART);
+    if (warp < NT) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sacc[k][i] = next[(srow + (i >> 1) * 8) * PT + 8 * k + lc + (i & 1)];
+    }
+    __syncthreads();
+    put_state(buf ^ 1);
+    __syncthreads();
+  };
+  float odd = 0.f;                                           // 0 while what this thread found in a chunk is finite
+  int c0 = 0, buf = 0;
+  for (; c0 < qlen; c0 += Q, buf ^= 1) {
     const int nc = min(Q, qlen - c0);
     const double* cum = cum_s + buf * Q;
     const float* sdt = dt_s + buf * Q;
     gi::cp_async_wait<0>();
-    __syncthreads();                                         // the chunk, its sums and S are in shared memory; the other buffers are free
+    // the chunk, its sums and S are in shared memory; the other buffers are free, once the chunk in them is right
+    if (__syncthreads_or(odd != 0.f)) again(c0 - Q, buf ^ 1);
+    odd = 0.f;
     if (c0 + Q < qlen) load(c0 + Q, buf ^ 1);
     const double last = cum[Q - 1];
     const unsigned char* bx = smem + buf * L::BUF + L::X_AT;
@@ -276,7 +354,10 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) yin[k][i] += main0[k][i] + small[k][i];
+      for (int i = 0; i < 4; ++i) {
+        yin[k][i] += main0[k][i] + small[k][i];
+        odd = fmaf(yin[k][i], 0.f, odd);
+      }
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
@@ -310,7 +391,10 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
 #pragma unroll
       for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sacc[k][i] = fmaf(keep, sacc[k][i], add[k][i] + low[k][i]);
+        for (int i = 0; i < 4; ++i) {
+          sacc[k][i] = fmaf(keep, sacc[k][i], add[k][i] + low[k][i]);
+          odd = fmaf(sacc[k][i], 0.f, odd);
+        }
       put_state(buf ^ 1);
     }
     if (warp == 0 && c0 + Q < qlen) {
@@ -318,6 +402,7 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
       load_dt(c0 + 2 * Q);
     }
   }
+  if (__syncthreads_or(odd != 0.f)) again(c0 - Q, buf ^ 1);
 #pragma unroll
   for (int k = 0; k < 4; ++k)
 #pragma unroll

@@ -343,6 +343,56 @@ def test_recurrence_by_chunks_errs_no_more_than_the_walk(sizes, rate):
     assert torch.equal(chunks[:, heads * N * P:], before[:, heads * N * P:]) and torch.equal(chunks[0], before[0]) and torch.equal(chunks[-1], before[-1])
 
 
+@pytest.mark.parametrize("sizes", [(4, 40, 128, 2), (2, 64, 96, 1), (3, 8, 24, 3)])
+@pytest.mark.parametrize("where", ["x", "x nan", "B", "C", "step", "state", "large state", "two chunks"])
+@pytest.mark.parametrize("at", [0, 5, 70, 129])
+def test_recurrence_by_chunks_keeps_what_is_no_number_where_the_walk_does(sizes, where, at):
+    """One token's input, or one number of the state, is infinite or none: the same outputs and states as the walk's are no finite
+    numbers, none of an earlier token among them, and the others agree (24 bits, sums of up to 128 rows and 130 tokens: 2^-16
+    of the largest beside them)."""
+    heads, P, N, G = sizes
+    g = torch.Generator(device=DEV).manual_seed(N + at)
+    lens, inner, ch, T = [130, 40], heads * P, heads * P + 2 * G * N, 170
+    xbc = torch.randn(T, ch, generator=g, device=DEV).bfloat16()
+    proj = torch.randn(T, 2 * inner + 2 * G * N + heads, generator=g, device=DEV).bfloat16()
+    dt_bias, a_log, d_skip = (0.3 * torch.randn(heads, generator=g, device=DEV) + m for m in (-1.0, -1.5, 1.0))
+    before = torch.randn(4, heads * N * P, generator=g, device=DEV)
+    inf, nan = float("inf"), float("nan")
+    if where == "x":
+        xbc[at, 3] = inf
+    elif where == "x nan":
+        xbc[at, inner - 1] = nan
+    elif where == "B":
+        xbc[at, inner + 7] = -inf
+    elif where == "C":
+        xbc[at, inner + G * N + 5] = nan
+    elif where == "step":
+        proj[at, 2 * inner + 2 * G * N] = inf
+    elif where == "state":
+        before[1, 2 * N + 1] = inf
+    elif where == "large state":
+        before[1, 2 * N + 1] = 3.4e38                         # finite in 32 bits, infinite rounded to 16
+        xbc[:, inner + G * N:] *= 0.125
+    else:
+        xbc[at, 0] = inf
+        xbc[min(at + 30, 129), P - 1] = nan
+    step = step_of(lens, [0, 0], [1, 2])
+    chunks, walk = before.clone(), before.clone()
+    y = ops.mamba2_scan(xbc, proj, dt_bias, a_log, d_skip, chunks, step, heads, P, N, G, 1)
+    y_walk = torch.empty_like(y)
+    lib = ops._bind()
+    assert lib.gi_mamba2_scan(y_walk.data_ptr(), xbc.data_ptr(), proj.data_ptr(), 1, proj.stride(0), dt_bias.data_ptr(), a_log.data_ptr(),
+                              d_skip.data_ptr(), 0, walk.data_ptr(), walk.stride(0), walk.shape[0], step.cu_seqlens.data_ptr(),
+                              step.seq_slots.data_ptr(), 2, heads, P, N, G, torch.cuda.current_stream().cuda_stream) == 0
+    touched = at if where not in ("state", "large state") else 0
+    assert torch.isfinite(y[:touched]).all() and torch.isfinite(y[130:]).all()
+    for got, want in ((y, y_walk), (chunks, walk)):
+        assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+        scale = torch.nan_to_num(want, 0.0, 0.0, 0.0).abs().amax(-1, keepdim=True).clamp_min(1.0)
+        assert (torch.nan_to_num(got - want, 0.0, 0.0, 0.0).abs() <= 2.0 ** -16 * scale).all()
+    assert (where == "large state") == bool(torch.isfinite(y).all())
+
+
 @pytest.mark.parametrize("heads,P,N,G,taps,parts", [(4, 24, 16, 2, 4, 2), (2, 8, 40, 1, 3, 1), (8, 64, 128, 4, 2, 4), (16, 40, 96, 4, 4, 1), (34, 32, 8, 2, 4, 17)])
 def test_convolution_and_gated_norm_in_eights_and_fours(heads, P, N, G, taps, parts):
     """16-bit rows by the kernels that read 16 bytes at a time, against 64 bits: the convolution to half a unit in the last of 8
