@@ -1996,6 +1996,11 @@ def attention_latent(qa: torch.Tensor, memory, step, n_heads: int, rank: int, ro
 LATENT_EXPAND_BYTES = 1 << 28      # of keys and values per head that a prompt step may form at a time (32,768 positions of 16 heads of 128 and 128)
 
 
+def latent_expand_sizes(dim: int, rot_dim: int, v_dim: int, rank: int, dtype: torch.dtype) -> bool:
+    """Whether keys and values of these sizes can be formed per head for a prompt step: those the tcgen05 kernel takes."""
+    return dtype == torch.bfloat16 and dim in (64, 128) and 0 < rot_dim <= 64 and rot_dim % 16 == 0 and 0 < v_dim <= 128 and v_dim % 8 == 0 and rank % 8 == 0
+
+
 def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, rank: int, window: Optional[int], dtype: torch.dtype) -> int:
     """How many cached rows a prompt step should turn into keys and values per head (`attention_latent_expanded`), or 0: carry
     its queries onto the latents instead (`attention_latent`).
@@ -2005,9 +2010,8 @@ def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, r
     tile of 64 keys 8.3 us at 1,088 of them, which is what few tokens behind a long prefix wait for), the products that carry
     queries and results 32e6, the attention over rows 200e6 (2 us a tile), the product that forms the rows 400e6; 40 us
     for what the host spends more on a few hundred tokens (tensor maps of new buffers).  16 heads, rank 512: 64 fresh tokens are carried; 16 tokens behind 3,000 take 98 us expanded, 418 carried.
-    Only prompt steps have the host's lists of lengths; sizes are those the tcgen05 kernel takes."""
-    if (step.is_decode or dtype != torch.bfloat16 or not TUNE["attn_latent_tc"] or dim not in (64, 128) or not 0 < rot_dim <= 64
-            or rot_dim % 16 or not 0 < v_dim <= 128 or v_dim % 8 or rank % 8):
+    Only prompt steps have the host's lists of lengths."""
+    if step.is_decode or not TUNE["attn_latent_tc"] or not latent_expand_sizes(dim, rot_dim, v_dim, rank, dtype):
         return 0
     pos0, lens = getattr(step, "_host_pos0", None), getattr(step, "_host_q_lens", None)
     if not pos0 or not lens or len(pos0) != step.n_seqs or len(lens) != step.n_seqs:

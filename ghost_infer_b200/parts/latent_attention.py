@@ -111,10 +111,14 @@ class LatentAttention(Mixer):
         self.w_o = place("o")
         self.sinks = tensors[n["sink"]].to(device=rt.device, dtype=torch.float32).contiguous() if self.sink else None
         # per head: W_uk,h^T as [rank, dim] (rows of the carried query), W_uv,h as [v_dim, rank]
-        self.w_uk_t = place("uk").view(H, self.dim, self.rank).transpose(1, 2).contiguous()
-        self.w_uv = place("uv").view(H, self.v_dim, self.rank).contiguous()
-        # the same matrices stacked, for prompt steps that form keys and values per head
-        self.w_uk_uv = stack_rows([place("uk"), self.w_uv.view(H * self.v_dim, self.rank)]) if rt.dtype == torch.bfloat16 else None
+        uk, uv = place("uk"), place("uv")
+        self.w_uk_t = uk.view(H, self.dim, self.rank).transpose(1, 2).contiguous()
+        # the same matrices one below the other, where prompt steps may form keys and values per head; W_uv is their lower part
+        self.w_uk_uv = None
+        if uk.dtype == uv.dtype == rt.dtype and ops.latent_expand_sizes(self.dim, self.rot_dim, self.v_dim, self.rank, rt.dtype):
+            self.w_uk_uv = torch.cat([uk, uv], dim=0)
+            uv = self.w_uk_uv[H * self.dim:]
+        self.w_uv = uv.view(H, self.v_dim, self.rank).contiguous()
         qn, cn = place("dq_norm") if self.q_rank else None, place("dkv_norm")
         if qn is not None and qn.dtype != cn.dtype:
             qn, cn = qn.to(torch.float32), cn.to(torch.float32)
@@ -127,7 +131,7 @@ class LatentAttention(Mixer):
         with ops.bucket("qkv matmul"):
             down = linear(h, self.w_down, out_dtype=dt)
         rows = 0
-        if self.w_uk_uv is not None and self.w_uk_uv.dtype == dt and memory.k is not None and down.dtype == dt:
+        if self.w_uk_uv is not None and memory.k is not None and down.dtype == dt:
             rows = ops.latent_expand_rows(step, H, self.dim, self.rot_dim, self.v_dim, self.rank, self.window, dt)
         if rows:
             return self._forward_expanded(h, residual, step, memory, down, rows)

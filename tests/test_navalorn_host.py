@@ -147,3 +147,20 @@ def test_command_line_makes_and_lists_a_model_folder(tmp_path, capsys):
     model = Model.from_config_dict(CFG)
     got = load_model_tensors(str(other), model.weight_manifest(), model.ignorable_tensors())
     assert torch.equal(got["l0.mix.dq"].float(), torch.from_numpy(w["l0.mix.dq"]).float())
+
+
+def test_matrices_are_kept_a_second_time_only_where_a_prompt_step_reads_them():
+    """W_uk and W_uv one below the other serve prompt steps that form keys and values per head; W_uv of the other steps is its
+    lower part.  Sizes that no such step takes, and 32-bit matrices, keep no second copy."""
+    def mixer(dtype="bfloat16", stored=torch.bfloat16, **sizes):
+        cfg = dict(CFG, layers=[{"type": "latent_attention", "mixer": dict(MIX, rot={"base": 5000.0, "dims": 4}, **sizes), "mlp": None}])
+        w = {k: torch.from_numpy(v).to(stored) for k, v in pn.random_weights(cfg, seed=1).items()}
+        return Model.from_config_dict(cfg).bind(w, dtype, "cpu").layers[0].block.mixer, w
+
+    fits = dict(dim=64, rot_dim=16, vdim=24, kv_rank=40)
+    m, w = mixer(**fits)
+    assert torch.equal(m.w_uk_uv, torch.cat([w["l0.mix.uk"], w["l0.mix.uv"]]))
+    assert torch.equal(m.w_uv, w["l0.mix.uv"].view(3, 24, 40)) and m.w_uv.untyped_storage().data_ptr() == m.w_uk_uv.untyped_storage().data_ptr()
+    assert torch.equal(m.w_uk_t, w["l0.mix.uk"].view(3, 64, 40).transpose(1, 2))
+    for other in (dict(dim=72), dict(rot_dim=24), dict(vdim=136), dict(vdim=20), dict(kv_rank=36), dict(dtype="float32"), dict(stored=torch.float32)):
+        assert mixer(**{**fits, **other})[0].w_uk_uv is None, other
