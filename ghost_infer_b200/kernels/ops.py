@@ -2001,6 +2001,29 @@ def latent_expand_sizes(dim: int, rot_dim: int, v_dim: int, rank: int, dtype: to
     return dtype == torch.bfloat16 and dim in (64, 128) and 0 < rot_dim <= 64 and rot_dim % 16 == 0 and 0 < v_dim <= 128 and v_dim % 8 == 0 and rank % 8 == 0
 
 
+def _latent_visible(step, window: Optional[int]):
+    """(cached rows that the step's tokens see, from a page boundary on; pairs of a token and a position it sees; tokens; tiles of 64
+    that the longest span has), None where the host has no lists of lengths.  Worked out once per step and window."""
+    pos0, lens = getattr(step, "_host_pos0", None), getattr(step, "_host_q_lens", None)
+    if not pos0 or not lens or len(pos0) != step.n_seqs or len(lens) != step.n_seqs:
+        return None
+    shared = getattr(step, "shared", None)
+    key = ("latent_visible", window)
+    if shared is not None and key in shared:
+        return shared[key]
+    rows = pairs = tokens = tiles = 0
+    span = int(window) if window else 1 << 62
+    for p, n in zip(pos0, lens):
+        rows += p + n - max(0, p - span + 1) // 64 * 64
+        whole = max(0, min(n, span - p))                 # tokens that see everything before them
+        pairs += whole * p + whole * (whole + 1) // 2 + (n - whole) * (0 if whole == n else span)
+        tokens += n
+        tiles = max(tiles, (min(p + n, span) + 63) // 64)
+    if shared is not None:
+        shared[key] = rows, pairs, tokens, tiles
+    return rows, pairs, tokens, tiles
+
+
 def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, rank: int, window: Optional[int], dtype: torch.dtype) -> int:
     """How many cached rows a prompt step should turn into keys and values per head (`attention_latent_expanded`), or 0: carry
     its queries onto the latents instead (`attention_latent`).
@@ -2013,17 +2036,10 @@ def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, r
     Only prompt steps have the host's lists of lengths."""
     if step.is_decode or not TUNE["attn_latent_tc"] or not latent_expand_sizes(dim, rot_dim, v_dim, rank, dtype):
         return 0
-    pos0, lens = getattr(step, "_host_pos0", None), getattr(step, "_host_q_lens", None)
-    if not pos0 or not lens or len(pos0) != step.n_seqs or len(lens) != step.n_seqs:
+    visible = _latent_visible(step, window)
+    if visible is None:
         return 0
-    rows = pairs = tokens = tiles = 0
-    span = int(window) if window else 1 << 62
-    for p, n in zip(pos0, lens):
-        rows += p + n - max(0, p - span + 1) // 64 * 64
-        whole = max(0, min(n, span - p))                 # tokens that see everything before them
-        pairs += whole * p + whole * (whole + 1) // 2 + (n - whole) * (0 if whole == n else span)
-        tokens += n
-        tiles = max(tiles, (min(p + n, span) + 63) // 64)
+    rows, pairs, tokens, tiles = visible
     if rows * n_heads * (dim + v_dim) * 2 > LATENT_EXPAND_BYTES:
         return 0
     work = 2 * rank + rot_dim

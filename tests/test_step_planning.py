@@ -1,4 +1,8 @@
-"""Host-side planning of a decode step: into how many slices of its context the attention cuts a sequence."""
+"""Host-side planning of a step: into how many slices of its context a decode step's attention cuts a sequence, which form a
+prompt step over a latent cache takes."""
+import random
+from types import SimpleNamespace
+
 import torch
 
 from ghost_infer_b200.kernels import ops
@@ -94,3 +98,47 @@ def test_32_bit_slices_follow_the_sequence_s_own_length():
     # a window bounds the span: at most window + 31 keys from the tile the window starts in, plus that tile's head
     assert plan(3, 5000, 4, 2, 16, window=100, dtype=F32) == (1, 8)
     assert plan(3, 5000, 4, 2, 16, window=300, dtype=F32) == (2, 8)
+
+# ---- prompt steps over a latent cache: which of the two forms, over how many rows ------------------------------------------
+def prompt(pos0, lens, **kw):
+    return SimpleNamespace(**{**dict(is_decode=False, n_seqs=len(lens), _host_pos0=list(pos0), _host_q_lens=list(lens), shared={}), **kw})
+
+
+def test_rows_formed_per_head_are_those_the_kernels_count():
+    """The gathering kernel and the attention lay a sequence's rows from the page of the first position that its first token
+    sees to its last position; the buffers are as large as the host's count, which must be the same."""
+    rng, chosen = random.Random(5), 0
+    for _ in range(400):
+        n = rng.randint(1, 5)
+        pos0, lens = [rng.choice([0, rng.randint(1, 3000)]) for _ in range(n)], [rng.choice([1, rng.randint(1, 1500)]) for _ in range(n)]
+        window = rng.choice([None, 1, 63, 64, 65, 500, rng.randint(1, 4000)])
+        rows = tokens = pairs = tiles = 0
+        for p, q in zip(pos0, lens):
+            seen = [(max(0, i - window + 1) if window else 0, i) for i in range(p, p + q)]
+            rows += p + q - seen[0][0] // 64 * 64
+            pairs += sum(b - a + 1 for a, b in seen)
+            tokens += q
+            tiles = max(tiles, (max(b - a + 1 for a, b in seen) + 63) // 64)
+        step = prompt(pos0, lens)
+        assert ops._latent_visible(step, window) == (rows, pairs, tokens, tiles)
+        assert ops._latent_visible(step, window) == (rows, pairs, tokens, tiles) and len(step.shared) == 1
+        got = ops.latent_expand_rows(step, 16, 128, 64, 128, 512, window, BF)
+        assert got in (0, rows)
+        chosen += got > 0
+    assert 100 < chosen < 400
+
+
+def test_what_keeps_a_prompt_on_the_latents():
+    ask = lambda step, H=16, dim=128, rot=64, vdim=128, rank=512, window=None, dtype=BF: ops.latent_expand_rows(step, H, dim, rot, vdim, rank, window, dtype)
+    step = prompt([0], [2048])
+    assert ask(step) == 2048 and ask(step, dim=64, rot=16, vdim=8) == 2048
+    for sizes in (dict(dim=96), dict(dim=32), dict(rot=0), dict(rot=24), dict(rot=80), dict(vdim=136), dict(vdim=20), dict(rank=508), dict(dtype=F32)):
+        assert ask(step, **sizes) == 0
+        assert not ops.latent_expand_sizes(**{**dict(dim=128, rot_dim=sizes.get("rot", 64), v_dim=sizes.get("vdim", 128), rank=512, dtype=BF), **{k: v for k, v in sizes.items() if k in ("dim", "rank", "dtype")}})
+    assert ask(prompt([0], [2048], is_decode=True)) == 0
+    assert ask(prompt([], [2048], n_seqs=1)) == 0 and ask(prompt([0], [2048], _host_pos0=None)) == 0
+    assert ask(prompt([0], [8])) == 0                                  # a few tokens alone
+    assert ask(prompt([3000], [16])) == 3016                           # and behind a long prefix
+    rows = ops.LATENT_EXPAND_BYTES // (16 * 256 * 2)
+    assert ask(prompt([rows - 500], [500])) == rows and ask(prompt([rows - 499], [500])) == 0
+    assert ask(prompt([rows], [500]), window=1024) == rows + 500 - (rows - 1023) // 64 * 64
