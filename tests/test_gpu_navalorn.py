@@ -489,3 +489,25 @@ def test_trace_replay_program(tmp_path, dtype):
             check(np.fromfile(f, dtype="<f4").reshape(-1, cfg["vocab"]), np.stack(want_rows), dtype, f"step {s['step']}")
         else:
             assert not f.exists()
+
+
+@pytest.mark.parametrize("sizes", [(16, 128, 64, 128, 512, 64, 32), (32, 64, 48, 40, 256, 40, 16)])
+def test_prompts_with_keys_and_values_per_head(monkeypatch, sizes):
+    """Queries out of a latent of their own, of whose rotated parts only some numbers turn; sizes and lengths for which a
+    prompt step forms keys and values per head; a piece behind a prefix, then tokens one by one."""
+    from ghost_infer_b200.kernels import ops
+    *s, turned = sizes
+    cfg = model_cfg(72, 110, [layer(mixer(*s, 0.08, rot_dims=turned, base=700.0, scaling=(6.0, 200, 16.0, 1.0)), dense(56))] * 2)
+    w = pn.random_weights(cfg, seed=turned)
+    tensors = {k: torch.from_numpy(np.asarray(v, dtype=np.float32)).to(torch.bfloat16) for k, v in w.items()}
+    model = gi.Model.from_config_dict(cfg).bind(tensors, "bfloat16", "cuda:0")
+    eng = gi.Engine(model, model.new_cache(max_tokens=64 * 40, max_seq_len=4096, beyond_trained_positions=True))
+    counts, rule = [], ops.latent_expand_rows
+    monkeypatch.setattr(ops, "latent_expand_rows", lambda *a, **kw: counts.append(rule(*a, **kw)) or counts[-1])
+    t = np.random.default_rng(3).integers(0, 110, size=1103).tolist()
+    slot = eng.cache.open_slot()
+    rows = [eng.step([gi.StepEntry(slot, t[a:b], range(b - a))]) for a, b in ((0, 701), (701, 1100))]
+    assert counts == [701, 701, 1100, 1100]
+    run = eng.decoder([slot])
+    rows += [run.forward(tokens=[x]).clone() for x in t[1100:]]
+    check(torch.cat(rows).cpu().numpy(), pn.forward(cfg, w, t), "bfloat16")

@@ -769,3 +769,39 @@ def test_drawn_schedules(name):
         for s in slots:
             eng.cache.close_slot(s)
     assert rows >= 40 and eng.cache.free_pages == eng.cache.n_pages
+
+
+# ---- prompts whose latent layers form keys and values per head ---------------------------------------------------------
+def expanding(monkeypatch):
+    """The row counts that the steps' latent layers are told to form from here on (0: queries are carried onto the latents)."""
+    from ghost_infer_b200.kernels import ops
+    counts, rule = [], ops.latent_expand_rows
+
+    def watched(*a, **kw):
+        counts.append(rule(*a, **kw))
+        return counts[-1]
+
+    monkeypatch.setattr(ops, "latent_expand_rows", watched)
+    return counts
+
+
+@pytest.mark.parametrize("sizes", [(16, 128, 64, 128, 512, 300), (32, 64, 32, 40, 512, 130), (16, 128, 48, 56, 512, None)])
+def test_prompts_with_keys_and_values_per_head(monkeypatch, sizes):
+    """Sizes that the tcgen05 kernel takes, prompts long enough for the rule to choose it: queries and gates as columns of
+    the product that also gives the latents, a window whose first pages have been given back, a second piece behind a prefix,
+    two sequences of unlike lengths in a step, one-token steps on the same cache afterwards."""
+    cfg = model_cfg(64, 120, [layer("L", lat(*sizes, 0.08, base=3000.0), 48)])
+    w = pv.random_weights(cfg, seed=sizes[1] + sizes[3])
+    eng = engine_of(cfg, tensors_of(w), "bfloat16", max_tokens=64 * 60)
+    counts = expanding(monkeypatch)
+    a, b = (np.random.default_rng(s).integers(0, 120, size=n).tolist() for s, n in ((1, 1003), (2, 707)))
+    ref_a, ref_b = Reference(cfg, w, a), Reference(cfg, w, b)
+    sa, sb = eng.cache.open_slot(), eng.cache.open_slot()
+    rows = [eng.step([gi.StepEntry(sa, a[:600], range(600))])]
+    both = eng.step([gi.StepEntry(sa, a[600:1001], range(401)), gi.StepEntry(sb, b[:707], range(707))])
+    assert len(counts) == 2 and min(counts) > 0, counts
+    span = sizes[5] or 1 << 30
+    assert counts[1] == 1001 - max(0, 601 - span) // 64 * 64 + 707
+    rows += [both[:401]] + [eng.decoder([sa]).forward(tokens=[t]).clone() for t in a[1001:]]
+    check(torch.cat(rows).cpu().numpy(), ref_a, "bfloat16", "pieces and tokens")
+    check(both[401:].cpu().numpy(), ref_b, "bfloat16", "the other sequence")
