@@ -12,8 +12,8 @@
 // tensor cores' rounding towards zero does not pile up over chunks.  c is summed in 64 bits: exp(c_i - c_j) of neighbours
 // would lose the digits that c has grown by.  Decays between different 16-token tiles are products of two factors, both
 // at most 1, taken at the first tile's start: 64 + 192 exponentials a chunk instead of 2,016.
-// Rows and columns past N, P and the chunk's end are zeros.  A chunk that comes to an infinity or a not-a-number is walked
-// token by token after all (`walk_chunk`), so that neither reaches an earlier token.
+// Rows and columns past N, P and the chunk's end are zeros.  A block that meets an infinity or a not-a-number walks its
+// tokens one by one after all (`walk_all`), so that neither reaches an earlier token.
 // B200, 2,048 tokens, 64 heads of 64, N 128: 172 us, the walk 660 us; 2,556 tokens in three sequences, 64 heads of 40, N 96:
 // 227 and 404 us; 365 in four: 58 and 92 us.  What bounds it now is the chain of a chunk (about 5 us: operands out of shared
 // memory, four products one after the other, two barriers), not the tensor cores' rate.
@@ -37,25 +37,14 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16 (&part)[3]) {
   part[1] = __float2bfloat16_rn(r);
   part[2] = __float2bfloat16_rn(r - __bfloat162float(part[1]));
 }
-__device__ __forceinline__ uint32_t two(__nv_bfloat16 lo, __nv_bfloat16 hi) {
-  return (uint32_t)__bfloat16_as_ushort(lo) | (uint32_t)__bfloat16_as_ushort(hi) << 16;
-}
 __device__ __forceinline__ void split3_pair(float lo, float hi, uint32_t (&out)[3]) {
   __nv_bfloat16 a[3], b[3];
   split3(lo, a);
   split3(hi, b);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) out[i] = two(a[i], b[i]);
+  for (int i = 0; i < 3; ++i) out[i] = (uint32_t)__bfloat16_as_ushort(a[i]) | (uint32_t)__bfloat16_as_ushort(b[i]) << 16;
 }
 
-// the same of a number of the state, which may be beyond what rounds to a finite 16-bit number, or infinite
-__device__ __forceinline__ void split3_state(float v, __nv_bfloat16 (&part)[3]) {
-  part[0] = __float2bfloat16_rn(v);
-  if (__hisinf(part[0])) part[0] = __float2bfloat16_rz(v);
-  const float r = isinf(v) ? 0.f : v - __bfloat162float(part[0]);
-  part[1] = __float2bfloat16_rn(r);
-  part[2] = __float2bfloat16_rn(r - __bfloat162float(part[1]));
-}
 template <int NT>
 struct Layout {
   static constexpr int NP = 16 * NT;                         // rows of S with padding
@@ -68,51 +57,62 @@ struct Layout {
   static constexpr int EI_AT = DT_AT + 2 * 4 * Q, EJ_AT = EI_AT + 4 * Q, IN_AT = EJ_AT + 16 * Q, BYTES = IN_AT + 4 * Q;
 };
 
-// A chunk whose products came to something that is no finite number, walked token by token from the state before it: a
-// product over 16 tokens lets an infinity or a not-a-number of one token meet the zero weights of earlier ones, and a split
-// infinity is none any more, where the recurrence carries both forward only.  `y`: the chunk's first token, this block's
-// columns; `cols` of them exist.  The state behind the chunk is left in the next buffer of S, [n][column] in 32 bits.
-// Thread: column tid % 32, every eighth row from tid / 32 on.
+// The whole stretch token by token, by a block that met an infinity or a not-a-number: a product over 16 tokens lets one
+// token's meet the zero weights of earlier ones, and a split infinity is none any more, where the recurrence carries both
+// forward only.  The state in memory is still that before the step, and `y` is written again.  `bc`, `x`, `dt_in`: the first
+// token's row of B, of x from this block's first column on (`cols` of them exist), its step size before softplus; C is
+// `c_after` numbers behind B.  Thread: column tid % 32, every eighth row from tid / 32 on.
 template <int NT>
-__device__ __noinline__ void walk_chunk(unsigned char* smem, int buf, float* y, int inner, int nc, int cols, int N, float A, float D) {
+__device__ __noinline__ void walk_all(unsigned char* smem, float* y, int inner, const __nv_bfloat16* bc, const __nv_bfloat16* x, int channels,
+                                      int c_after, const __nv_bfloat16* dt_in, long ld_proj, float* S_cols, int qlen, int cols, int N,
+                                      float A, float D, float bias) {
   using L = Layout<NT>;
   constexpr int ROWS = L::NP / 8;
-  const int p = threadIdx.x & 31, first = threadIdx.x >> 5;
-  const unsigned char* in = smem + buf * L::BUF;
-  const float* dts = reinterpret_cast<const float*>(smem + L::DT_AT) + buf * Q;
-  float* sums = reinterpret_cast<float*>(smem + L::W_AT);    // [8][32]
-  auto number = [](const unsigned char* at) { return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(at)); };
+  const int tid = threadIdx.x, p = tid & 31, first = tid >> 5;
+  float* sB = reinterpret_cast<float*>(smem);                // [32][NP]
+  float* sC = sB + 32 * L::NP;
+  float* sx = sC + 32 * L::NP;                               // [32][PT]
+  float* sdt = sx + 32 * PT;
+  float* sums = sdt + 32;                                    // [8][32]
   float S[ROWS];
 #pragma unroll
-  for (int k = 0; k < ROWS; ++k) {
-    const unsigned char* at = smem + L::S_AT + 3 * buf * L::S_PART + (first + 8 * k) * XP + 2 * p;
-    S[k] = number(at) + (number(at + L::S_PART) + number(at + 2 * L::S_PART));
-  }
-  for (int t = 0; t < nc; ++t) {
-    const float dt = dts[t], keep = expf(A * dt), x = number(in + L::X_AT + t * XP + 2 * p);
-    float sum = 0.f;
+  for (int k = 0; k < ROWS; ++k) S[k] = p < cols && first + 8 * k < N ? S_cols[(size_t)p * N + first + 8 * k] : 0.f;
+  for (int c0 = 0; c0 < qlen; c0 += 32) {
+    const int nc = min(32, qlen - c0);
+    __syncthreads();
+    for (int i = tid; i < nc * N; i += THREADS) {
+      const __nv_bfloat16* at = bc + (size_t)(c0 + i / N) * channels + i % N;
+      sB[i / N * L::NP + i % N] = gi::ldf(at);
+      sC[i / N * L::NP + i % N] = gi::ldf(at + c_after);
+    }
+    for (int i = tid; i < nc * PT; i += THREADS) sx[i] = i % PT < cols ? gi::ldf(x + (size_t)(c0 + i / PT) * channels + i % PT) : 0.f;
+    if (tid < nc) sdt[tid] = softplus_f(gi::ldf(dt_in + (size_t)(c0 + tid) * ld_proj) + bias);
+    __syncthreads();
+    for (int t = 0; t < nc; ++t) {
+      const float dt = sdt[t], keep = expf(A * dt), xv = sx[t * PT + p];
+      float sum = 0.f;
 #pragma unroll
-    for (int k = 0; k < ROWS; ++k) {
-      const int n = first + 8 * k;
-      if (n < N) {
-        S[k] = fmaf(keep, S[k], x * (number(in + L::B_AT + t * L::BP + 2 * n) * dt));
-        sum = fmaf(S[k], number(in + L::C_AT + t * L::BP + 2 * n), sum);
+      for (int k = 0; k < ROWS; ++k) {
+        const int n = first + 8 * k;
+        if (n < N) {
+          S[k] = fmaf(keep, S[k], xv * (sB[t * L::NP + n] * dt));
+          sum = fmaf(S[k], sC[t * L::NP + n], sum);
+        }
       }
-    }
-    sums[threadIdx.x] = sum;
-    __syncthreads();
-    if (first == 0 && p < cols) {
-      sum = 0.f;
+      sums[tid] = sum;
+      __syncthreads();
+      if (first == 0 && p < cols) {
+        sum = 0.f;
 #pragma unroll
-      for (int w = 0; w < 8; ++w) sum += sums[w * 32 + p];
-      y[(size_t)t * inner + p] = fmaf(D, x, sum);
+        for (int w = 0; w < 8; ++w) sum += sums[w * 32 + p];
+        y[(size_t)(c0 + t) * inner + p] = fmaf(D, xv, sum);
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
-  float* next = reinterpret_cast<float*>(smem + L::S_AT + 3 * (buf ^ 1) * L::S_PART);
 #pragma unroll
-  for (int k = 0; k < ROWS; ++k) next[(first + 8 * k) * PT + p] = first + 8 * k < N ? S[k] : 0.f;
-  __syncthreads();
+  for (int k = 0; k < ROWS; ++k)
+    if (p < cols && first + 8 * k < N) S_cols[(size_t)p * N + first + 8 * k] = S[k];
 }
 
 // grid (heads, sequences, column tiles of 32)
@@ -212,15 +212,23 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
       for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          __nv_bfloat16 lo[3], hi[3];
-          split3_state(sacc[k][2 * r], lo);
-          split3_state(sacc[k][2 * r + 1], hi);
+          uint32_t part[3];
+          split3_pair(sacc[k][2 * r], sacc[k][2 * r + 1], part);
 #pragma unroll
           for (int s = 0; s < 3; ++s)
-            *reinterpret_cast<uint32_t*>(smem + L::S_AT + (3 * buf + s) * L::S_PART + (srow + 8 * r) * XP + (8 * k + lc) * 2) = two(lo[s], hi[s]);
+            *reinterpret_cast<uint32_t*>(smem + L::S_AT + (3 * buf + s) * L::S_PART + (srow + 8 * r) * XP + (8 * k + lc) * 2) = part[s];
         }
     }
   };
+  // 0 while all that this thread found is finite, the state also when rounded to 16 bits; not-a-number after that
+  float odd = 0.f;
+  auto check_state = [&] {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) odd = fmaf(sacc[k][i] * 1.0625f, 0.f, odd);
+  };
+  check_state();
   put_state(0);
 
   // this warp's rows and columns of y: of the two warps a scheduler holds one has a late row tile, one an early one
@@ -228,30 +236,15 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
   const uint32_t a_row = (uint32_t)((lane & 7) + ((lane >> 3) & 1) * 8), a_col = (uint32_t)(lane >> 4) * 16;   // ldmatrix rows, bytes
   const uint32_t b_row = (uint32_t)((lane & 7) + (lane >> 4) * 8), b_col = (uint32_t)((lane >> 3) & 1) * 16;
 
-  // the chunk before once more, token by token
-  auto again = [&](int c0, int buf) {
-    walk_chunk<NT>(smem, buf, y + (size_t)(tok0 + c0) * inner + (size_t)h * P + p0, inner, min(Q, qlen - c0), P - p0, N, A, D);
-    const float* next = reinterpret_cast<const float*>(smem + L::S_AT + 3 * (buf ^ 1) * L::S_PART);
-    if (warp < NT) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) sacc[k][i] = next[(srow + (i >> 1) * 8) * PT + 8 * k + lc + (i & 1)];
-    }
-    __syncthreads();
-    put_state(buf ^ 1);
-    __syncthreads();
-  };
-  float odd = 0.f;                                           // 0 while what this thread found in a chunk is finite
-  int c0 = 0, buf = 0;
-  for (; c0 < qlen; c0 += Q, buf ^= 1) {
+  bool walk = false;
+  for (int c0 = 0, buf = 0; c0 < qlen; c0 += Q, buf ^= 1) {
     const int nc = min(Q, qlen - c0);
     const double* cum = cum_s + buf * Q;
     const float* sdt = dt_s + buf * Q;
     gi::cp_async_wait<0>();
-    // the chunk, its sums and S are in shared memory; the other buffers are free, once the chunk in them is right
-    if (__syncthreads_or(odd != 0.f)) again(c0 - Q, buf ^ 1);
-    odd = 0.f;
+    // the chunk, its sums and S are in shared memory; the other buffers are free
+    walk = __syncthreads_or(odd != 0.f);
+    if (walk) break;
     if (c0 + Q < qlen) load(c0 + Q, buf ^ 1);
     const double last = cum[Q - 1];
     const unsigned char* bx = smem + buf * L::BUF + L::X_AT;
@@ -391,10 +384,8 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
 #pragma unroll
       for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          sacc[k][i] = fmaf(keep, sacc[k][i], add[k][i] + low[k][i]);
-          odd = fmaf(sacc[k][i], 0.f, odd);
-        }
+        for (int i = 0; i < 4; ++i) sacc[k][i] = fmaf(keep, sacc[k][i], add[k][i] + low[k][i]);
+      check_state();
       put_state(buf ^ 1);
     }
     if (warp == 0 && c0 + Q < qlen) {
@@ -402,7 +393,12 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
       load_dt(c0 + 2 * Q);
     }
   }
-  if (__syncthreads_or(odd != 0.f)) again(c0 - Q, buf ^ 1);
+  if (walk || __syncthreads_or(odd != 0.f)) {
+    walk_all<NT>(smem, y + (size_t)tok0 * inner + (size_t)h * P + p0, inner, xbc + (size_t)tok0 * channels + inner + (size_t)g * N,
+                 xbc + (size_t)tok0 * channels + (size_t)h * P + p0, channels, groups * N, dt_in + (size_t)tok0 * ld_proj, ld_proj,
+                 S_row + (size_t)p0 * N, qlen, min(PT, P - p0), N, A, D, bias);
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < 4; ++k)
 #pragma unroll
