@@ -6,17 +6,22 @@
 //     S   <- exp(c_last) S   +  sum_j B_j (exp(c_last - c_j) dt_j x_j)^T
 // The walk was bound by its chain: 64 heads x 64 columns of one prompt are 7 warps an SM, each with 2,048 dependent steps.
 // Here a block takes a head's 32 columns of S (128 blocks for 64 heads of 64) and walks the chunks; eight warps form the
-// four products with mma.sync.  B, C and x are 16-bit numbers and enter exactly.  What is 32-bit (S, the weighted x, the
-// decayed scores) enters as three 16-bit parts, 24 bits together, in three products with 32-bit sums, so nothing is held or
-// summed in less than the walk did; a chunk's addition to S is summed apart and joined with one rounding, so that the
-// tensor cores' rounding towards zero does not pile up over chunks.  c is summed in 64 bits: exp(c_i - c_j) of neighbours
-// would lose the digits that c has grown by.  Decays between different 16-token tiles are products of two factors, both
-// at most 1, taken at the first tile's start: 64 + 192 exponentials a chunk instead of 2,016.
+// four products with mma.sync.  B, C and x are 16-bit numbers and enter exactly; what is 32-bit (S, the weighted x, the
+// decayed scores) enters as three 16-bit parts, 24 bits together, in three products.  Sums are 32-bit.  The tensor cores cut
+// off what does not fit into a sum that they add to themselves, so the products that make up most of y (C . B, scores x)
+// leave them 16 numbers at a time and are added with one rounding to nearest, and a chunk's addition to S is summed apart
+// and joined with one rounding.  c is summed in 64 bits: exp(c_i - c_j) of neighbours would lose the digits that c has grown
+// by.  Distance of y from 64 bits, 64 heads of 64, N 128, 512 tokens (the walk's beside it): 0.95e-7 (0.95e-7) where a state
+// lasts a few tokens, 1.2e-7 (39e-7) where it lasts hundreds, 0.88e-7 (0.71e-7) where it is gone at the next token; with sums
+// left to the tensor cores 1.2e-7, 1.2e-7 and 1.1e-7, for 1% less time.
+// Between different 16-token tiles decays are products of two factors, both at most 1, taken at the later tile's start:
+// 64 + 96 exponentials a chunk for 1,536 pairs.  The pairs inside the four diagonal tiles take one each (544, in both halves
+// of the columns), and a token's weight for S is worked out by the four threads that apply it.
 // Rows and columns past N, P and the chunk's end are zeros.  A block that meets an infinity or a not-a-number walks its
 // tokens one by one after all (`walk_all`), so that neither reaches an earlier token.
-// B200, 2,048 tokens, 64 heads of 64, N 128: 172 us, the walk 660 us; 2,556 tokens in three sequences, 64 heads of 40, N 96:
-// 227 and 404 us; 365 in four: 58 and 92 us.  What bounds it now is the chain of a chunk (about 5 us: operands out of shared
-// memory, four products one after the other, two barriers), not the tensor cores' rate.
+// B200, 2,048 tokens, 64 heads of 64, N 128: 175 us, the walk 660 us; 64 heads of 40, N 96: 165 and 536 us.  What bounds it
+// now is the chain of a chunk (about 5 us: operands out of shared memory, four products one after the other, two barriers),
+// not the tensor cores' rate.
 #include <math.h>
 
 #include "api.h"
@@ -43,6 +48,15 @@ __device__ __forceinline__ void split3_pair(float lo, float hi, uint32_t (&out)[
   split3(hi, b);
 #pragma unroll
   for (int i = 0; i < 3; ++i) out[i] = (uint32_t)__bfloat16_as_ushort(a[i]) | (uint32_t)__bfloat16_as_ushort(b[i]) << 16;
+}
+
+// acc + a b, the product over 16 numbers added with one rounding to nearest: the tensor cores cut off what does not fit into a
+// sum that they add to themselves
+__device__ __forceinline__ void add_mma(float (&acc)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  float t[4] = {};
+  gi::mma_16816(t, a, b0, b1);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i] += t[i];
 }
 
 template <int NT>
@@ -274,8 +288,7 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
     __syncthreads();
 
     const uint32_t cb = base + buf * L::BUF;
-    // sums of the main parts in two chains and of the small ones apart: the tensor cores cut every sum they add to
-    float main0[2][4] = {}, main1[2][4] = {}, small[2][4] = {};
+    float main[2][4] = {}, main1[2][4] = {}, small[2][4] = {};
     uint32_t cf[NT][4];
 #pragma unroll
     for (int k = 0; k < NT; ++k) {
@@ -284,7 +297,7 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
       for (int s = 2; s >= 0; --s) {
         uint32_t f[4];
         gi::ldmatrix_x4_trans(f, base + L::S_AT + (3 * buf + s) * L::S_PART + (16 * k + a_row) * XP + ch * 32 + a_col);
-        float (&acc)[2][4] = s > 0 ? small : (k & 1) ? main1 : main0;
+        float (&acc)[2][4] = s > 0 ? small : (k & 1) ? main1 : main;
         gi::mma_16816(acc[0], cf[k], f[0], f[1]);
         gi::mma_16816(acc[1], cf[k], f[2], f[3]);
       }
@@ -297,24 +310,20 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
       for (int k = 0; k < 2; ++k)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          yin[k][i] = ((main0[k][i] + main1[k][i]) + small[k][i]) * (i < 2 ? t0 : t1);
-          main0[k][i] = small[k][i] = 0.f;
+          yin[k][i] = ((main[k][i] + main1[k][i]) + small[k][i]) * (i < 2 ? t0 : t1);
+          main[k][i] = small[k][i] = 0.f;
         }
     }
     const float e0 = ei[i0], e1 = ei[i0 + 8];
     for (int jt = 0; jt <= rt; ++jt) {
-      float m[2][4] = {}, m1[2][4] = {};
+      float m[2][4] = {};
 #pragma unroll
       for (int k = 0; k < NT; ++k) {
         uint32_t f[4];
         gi::ldmatrix_x4(f, cb + L::B_AT + (16 * jt + b_row) * L::BP + k * 32 + b_col);
-        gi::mma_16816((k & 1) ? m1[0] : m[0], cf[k], f[0], f[1]);
-        gi::mma_16816((k & 1) ? m1[1] : m[1], cf[k], f[2], f[3]);
+        add_mma(m[0], cf[k], f[0], f[1]);
+        add_mma(m[1], cf[k], f[2], f[3]);
       }
-#pragma unroll
-      for (int k = 0; k < 2; ++k)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) m[k][i] += m1[k][i];
 #pragma unroll
       for (int k = 0; k < 2; ++k)
 #pragma unroll
@@ -340,15 +349,20 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
 #pragma unroll
       for (int s = 2; s >= 0; --s) {
         const uint32_t af[4] = {a01[s], a23[s], b01[s], b23[s]};
-        gi::mma_16816(s > 0 ? small[0] : main0[0], af, xf[0], xf[1]);
-        gi::mma_16816(s > 0 ? small[1] : main0[1], af, xf[2], xf[3]);
+        if (s > 0) {
+          gi::mma_16816(small[0], af, xf[0], xf[1]);
+          gi::mma_16816(small[1], af, xf[2], xf[3]);
+        } else {
+          add_mma(main[0], af, xf[0], xf[1]);
+          add_mma(main[1], af, xf[2], xf[3]);
+        }
       }
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        yin[k][i] += main0[k][i] + small[k][i];
+        yin[k][i] += main[k][i] + small[k][i];
         odd = fmaf(yin[k][i], 0.f, odd);
       }
 #pragma unroll

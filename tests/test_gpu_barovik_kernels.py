@@ -303,8 +303,10 @@ def test_experts_expert_by_expert_on_tensor_cores():
                                    (3, 72, 72, 3, [64]), (2, 32, 8, 1, [24])])
 @pytest.mark.parametrize("rate", [(-1.0, -0.5), (-6.0, -2.0), (3.0, 1.0)])
 def test_recurrence_by_chunks_errs_no_more_than_the_walk(sizes, rate):
-    """Against 64 bits.  A sum of n terms in 32 bits errs by a few 2^-24 of the terms' size; the walk adds up one rounding per
-    token while a state is kept (thousands of tokens at the slow rates), so twice its error plus 2^-22 is the bound."""
+    """Against 64 bits.  Both forms round each product and sum to 24 bits (2^-24 = 6e-8 of it at most), the walk once per token
+    while a state is kept, so it errs far more at the slow rates; at the fast ones, where a sum has a few terms, the products
+    cut inside 16 numbers where the walk rounds to nearest: 2^-25 of the result apart at most.  y and state are measured at 0.2
+    to 1.25 times and 0.02 to 1.3 times the walk's."""
     heads, P, N, G, lens = sizes
     g = torch.Generator(device=DEV).manual_seed(heads + N)
     inner, ch, T = heads * P, heads * P + 2 * G * N, sum(lens)
@@ -338,8 +340,8 @@ def test_recurrence_by_chunks_errs_no_more_than_the_walk(sizes, rate):
     def err(a, b):
         return ((a.double() - b).norm() / b.norm()).item()
 
-    assert err(y, want) <= 2 * err(y_walk, want) + 2.0 ** -22
-    assert err(chunks, state) <= 2 * err(walk, state) + 2.0 ** -22
+    assert err(y, want) <= err(y_walk, want) + 2.0 ** -25
+    assert err(chunks, state) <= err(walk, state) + 2.0 ** -25
     assert torch.equal(chunks[:, heads * N * P:], before[:, heads * N * P:]) and torch.equal(chunks[0], before[0]) and torch.equal(chunks[-1], before[-1])
 
 
