@@ -324,10 +324,16 @@ int gi_mamba2_scan(float* y, const void* xbc, const void* proj, int dtype, long 
                    const void* a_log, const void* d_skip, int w_dtype, float* state, long state_ld, int state_rows,
                    const int* cu_seqlens, const int* seq_slots, int n_seqs, int heads, int P, int N, int groups,
                    void* stream);
-// The same for 16-bit rows and 32-bit constants, 64 tokens at a time on tensor cores (P and N multiples of 8, N <= 128).
+// The same for the sequences of fewer than `below` tokens in this step; the others are left alone.
+int gi_mamba2_scan_below(float* y, const void* xbc, const void* proj, int dtype, long ld_proj, const void* dt_bias,
+                         const void* a_log, const void* d_skip, int w_dtype, float* state, long state_ld, int state_rows,
+                         const int* cu_seqlens, const int* seq_slots, int n_seqs, int heads, int P, int N, int groups, int below,
+                         void* stream);
+// The same for 16-bit rows and 32-bit constants, 64 tokens at a time on tensor cores (P and N multiples of 8, N <= 128): the
+// sequences of `from` (>= 1) tokens and more; the others are left alone.
 int gi_mamba2_chunks(float* y, const void* xbc, const void* proj, long ld_proj, const float* dt_bias, const float* a_log,
                      const float* d_skip, float* state, long state_ld, int state_rows, const int* cu_seqlens,
-                     const int* seq_slots, int n_seqs, int heads, int P, int N, int groups, void* stream);
+                     const int* seq_slots, int n_seqs, int heads, int P, int N, int groups, int from, void* stream);
 // out[t, :] = groupwise_rmsnorm(y[t, :] * silu(z[t, :])) * w, z the first inner columns of proj; `parts` equal parts,
 // each divided by its own root mean square (eps inside the root).
 int gi_mamba2_gate_norm(void* out, int out_dtype, const float* y, const void* proj, int dtype, long ld_proj,

@@ -8,7 +8,8 @@
 //           Everything here is 32-bit; the tokens of a sequence are walked in order, thirty-two at a time through shared
 //           memory; a warp owns two or four columns p of S, its lanes the rows n, kept in registers across the step.
 //           One token or a thousand, alone or in a batch, take the same arithmetic in the same order: no bit changes.
-//           (Prompt steps in 16-bit rows take chunks of tokens as matrix products instead: mamba2_chunks.cu.)
+//           (In 16-bit rows a sequence's stretch of many tokens goes by chunks as matrix products instead: mamba2_chunks.cu.
+//           Its own length decides, whatever else is in the step.)
 //  * gate + norm: y * silu(z), divided by the root mean square of each of `parts` equal parts, times a weight.
 // Per-sequence state: one float row per slot, [S: heads * P * N, a column's N rows side by side (a lane's rows are then
 // neighbours in memory: a one-token step, which is all loading and storing of S, moves whole lines) | last taps - 1 conv
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(SC_W * 32)
 scan_kernel(float* __restrict__ y, const T* __restrict__ xbc, const T* __restrict__ proj, long ld_proj,
             const TW* __restrict__ dt_bias, const TW* __restrict__ a_log, const TW* __restrict__ d_skip,
             float* __restrict__ state, long state_ld, int state_rows, const int* __restrict__ cu_seqlens,
-            const int* __restrict__ seq_slots, int heads, int P, int N, int groups) {
+            const int* __restrict__ seq_slots, int heads, int P, int N, int groups, int below) {
   constexpr int NP = 32 * NPT;       // rows with padding
   constexpr int SC_COLS = SC_W * SC_CPW, SC_RB = 32 / SC_CPW, SC_CPW_LOG2 = SC_CPW == 2 ? 1 : 2;
   static_assert(SC_CPW == 2 || SC_CPW == 4, "a warp takes 2 or 4 columns");
@@ -179,7 +180,7 @@ scan_kernel(float* __restrict__ y, const T* __restrict__ xbc, const T* __restric
   gi::pdl_prologue();
   const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * SC_COLS;
   const int tok0 = cu_seqlens[b], qlen = cu_seqlens[b + 1] - tok0;
-  if (qlen <= 0) return;
+  if (qlen <= 0 || qlen >= below) return;
   const int slot = seq_slots[b];
   float* S_row = state + (size_t)(slot >= 0 ? slot : state_rows - 1) * state_ld + (size_t)h * N * P;
   const int g = h / (heads / groups);
@@ -346,14 +347,14 @@ gate_norm_warp_kernel(__nv_bfloat16* __restrict__ out, const float* y, const __n
 template <typename T, typename TW, int NPT, int CPW>
 int launch_scan(dim3 grid, size_t smem, cudaStream_t s, float* y, const T* xbc, const T* proj, long ld_proj, const TW* dt_bias,
                 const TW* a_log, const TW* d_skip, float* state, long state_ld, int state_rows, const int* cu, const int* slots,
-                int heads, int P, int N, int groups) {
+                int heads, int P, int N, int groups, int below) {
   auto kern = scan_kernel<T, TW, NPT, CPW>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return gi::fail(GI_ERR_CUDA, "mamba2 scan: %s", cudaGetErrorString(e));
   }
   return gi::check(gi::launch(kern, grid, dim3(SC_W * 32), smem, s, y, xbc, proj, ld_proj, dt_bias, a_log, d_skip, state, state_ld,
-                              state_rows, cu, slots, heads, P, N, groups), "mamba2 scan");
+                              state_rows, cu, slots, heads, P, N, groups, below), "mamba2 scan");
 }
 
 }  // namespace
@@ -406,6 +407,14 @@ extern "C" int gi_mamba2_scan(float* y, const void* xbc, const void* proj, int d
                               const void* a_log, const void* d_skip, int w_dtype, float* state, long state_ld,
                               int state_rows, const int* cu_seqlens, const int* seq_slots, int n_seqs, int heads, int P,
                               int N, int groups, void* stream) {
+  return gi_mamba2_scan_below(y, xbc, proj, dtype, ld_proj, dt_bias, a_log, d_skip, w_dtype, state, state_ld, state_rows, cu_seqlens,
+                              seq_slots, n_seqs, heads, P, N, groups, 2147483647, stream);
+}
+
+extern "C" int gi_mamba2_scan_below(float* y, const void* xbc, const void* proj, int dtype, long ld_proj, const void* dt_bias,
+                                    const void* a_log, const void* d_skip, int w_dtype, float* state, long state_ld,
+                                    int state_rows, const int* cu_seqlens, const int* seq_slots, int n_seqs, int heads, int P,
+                                    int N, int groups, int below, void* stream) {
   if (n_seqs <= 0) return GI_OK;
   if (heads <= 0 || P <= 0 || N <= 0 || groups <= 0 || heads % groups != 0)
     return gi::fail(GI_ERR_ARG, "mamba2 scan: %d heads, %d groups, head size %d, state %d", heads, groups, P, N);
@@ -427,7 +436,7 @@ extern "C" int gi_mamba2_scan(float* y, const void* xbc, const void* proj, int d
   GI_DISPATCH_DTYPE(dtype, T, GI_DISPATCH_DTYPE(w_dtype, TW,                                                           \
       rc = (launch_scan<T, TW, NPT, CPW>(grid, smem, s, y, (const T*)xbc, (const T*)proj, ld_proj, (const TW*)dt_bias, \
                                          (const TW*)a_log, (const TW*)d_skip, state, state_ld, state_rows, cu_seqlens, \
-                                         seq_slots, heads, P, N, groups))))
+                                         seq_slots, heads, P, N, groups, below))))
 #define GI_SCAN_CASE(NPT)                                                                                              \
   case NPT:                                                                                                            \
     if (cpw == 4) GI_SCAN_LAUNCH(NPT, 4);                                                                              \

@@ -1,5 +1,5 @@
 // The Mamba-2 recurrence of a prompt step in 16-bit rows, 64 tokens at a time as matrix products (the "state-space dual"
-// form of Dao and Gu, 2024), beside the token-by-token walk of mamba2.cu, which serves one-token steps and the 32-bit path.
+// form of Dao and Gu, 2024), beside the token-by-token walk of mamba2.cu, which serves short stretches and the 32-bit path.
 //
 // With a_t = -exp(A_log) dt_t and c_t the sum of a over a chunk's tokens up to t, S the state before the chunk:
 //     y_i  = exp(c_i) C_i S  +  sum_{j <= i} (C_i . B_j) exp(c_i - c_j) dt_j x_j  +  D x_i
@@ -19,10 +19,12 @@
 // of the columns), and a token's weight for S is worked out by the four threads that apply it.
 // Rows and columns past N, P and the chunk's end are zeros.  A block that meets an infinity or a not-a-number walks its
 // tokens one by one after all (`walk_all`), so that neither reaches an earlier token.
-// B200, 2,048 tokens, 64 heads of 64, N 128: 175 us, the walk 660 us; 64 heads of 40, N 96: 165 and 536 us.  What bounds it
+// B200, 2,048 tokens, 64 heads of 64, N 128: 176 us, the walk 660 us; 64 heads of 40, N 96: 165 and 536 us.  What bounds it
 // now is the chain of a chunk (about 5 us: operands out of shared memory, four products one after the other, two barriers),
 // not the tensor cores' rate.
 #include <math.h>
+
+#include <type_traits>
 
 #include "api.h"
 #include "common.cuh"
@@ -134,7 +136,7 @@ template <int NT>
 __global__ void __launch_bounds__(THREADS, 1)
 mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv_bfloat16* proj, long ld_proj, const float* dt_bias,
                      const float* a_log, const float* d_skip, float* state, long state_ld, int state_rows, const int* cu_seqlens,
-                     const int* seq_slots, int heads, int P, int N, int groups) {
+                     const int* seq_slots, int heads, int P, int N, int groups, int from) {
   using L = Layout<NT>;
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t base = gi::smem_u32(smem);
@@ -146,7 +148,7 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
   gi::pdl_prologue();
   const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * PT;
   const int tok0 = cu_seqlens[b], qlen = cu_seqlens[b + 1] - tok0;
-  if (qlen <= 0) return;
+  if (qlen < from) return;
   const int slot = seq_slots[b];
   float* S_row = state + (size_t)(slot >= 0 ? slot : state_rows - 1) * state_ld + (size_t)h * N * P;
   const int g = h / (heads / groups);
@@ -250,16 +252,13 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
   const uint32_t a_row = (uint32_t)((lane & 7) + ((lane >> 3) & 1) * 8), a_col = (uint32_t)(lane >> 4) * 16;   // ldmatrix rows, bytes
   const uint32_t b_row = (uint32_t)((lane & 7) + (lane >> 4) * 8), b_col = (uint32_t)((lane >> 3) & 1) * 16;
 
-  bool walk = false;
-  for (int c0 = 0, buf = 0; c0 < qlen; c0 += Q, buf ^= 1) {
-    const int nc = min(Q, qlen - c0);
+  // A chunk.  Only a sequence's last one may have fewer tokens; its late row tiles are then left out (65 tokens of 16 sequences,
+  // 64 heads of 64, N 128: 185 us -> 164), in a copy of its own, since the tests alone cost full chunks 2%.
+  auto chunk = [&](int c0, int buf, auto full) {
+    constexpr bool FULL = decltype(full)::value;
+    const int nc = FULL ? Q : qlen - c0;
     const double* cum = cum_s + buf * Q;
     const float* sdt = dt_s + buf * Q;
-    gi::cp_async_wait<0>();
-    // the chunk, its sums and S are in shared memory; the other buffers are free
-    walk = __syncthreads_or(odd != 0.f);
-    if (walk) break;
-    if (c0 + Q < qlen) load(c0 + Q, buf ^ 1);
     const double last = cum[Q - 1];
     const unsigned char* bx = smem + buf * L::BUF + L::X_AT;
     {
@@ -288,100 +287,103 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
     __syncthreads();
 
     const uint32_t cb = base + buf * L::BUF;
-    float main[2][4] = {}, main1[2][4] = {}, small[2][4] = {};
-    uint32_t cf[NT][4];
+    if (FULL || 16 * rt < nc) {
+      float main[2][4] = {}, main1[2][4] = {}, small[2][4] = {};
+      uint32_t cf[NT][4];
 #pragma unroll
-    for (int k = 0; k < NT; ++k) {
-      gi::ldmatrix_x4(cf[k], cb + L::C_AT + (16 * rt + a_row) * L::BP + k * 32 + a_col);
+      for (int k = 0; k < NT; ++k) {
+        gi::ldmatrix_x4(cf[k], cb + L::C_AT + (16 * rt + a_row) * L::BP + k * 32 + a_col);
 #pragma unroll
-      for (int s = 2; s >= 0; --s) {
-        uint32_t f[4];
-        gi::ldmatrix_x4_trans(f, base + L::S_AT + (3 * buf + s) * L::S_PART + (16 * k + a_row) * XP + ch * 32 + a_col);
-        float (&acc)[2][4] = s > 0 ? small : (k & 1) ? main1 : main;
-        gi::mma_16816(acc[0], cf[k], f[0], f[1]);
-        gi::mma_16816(acc[1], cf[k], f[2], f[3]);
+        for (int s = 2; s >= 0; --s) {
+          uint32_t f[4];
+          gi::ldmatrix_x4_trans(f, base + L::S_AT + (3 * buf + s) * L::S_PART + (16 * k + a_row) * XP + ch * 32 + a_col);
+          float (&acc)[2][4] = s > 0 ? small : (k & 1) ? main1 : main;
+          gi::mma_16816(acc[0], cf[k], f[0], f[1]);
+          gi::mma_16816(acc[1], cf[k], f[2], f[3]);
+        }
       }
-    }
-    const int i0 = 16 * rt + lr;
-    float yin[2][4];                                         // what the state before the chunk gives
-    {
-      const float t0 = e_in[i0], t1 = e_in[i0 + 8];
+      const int i0 = 16 * rt + lr;
+      float yin[2][4];                                         // what the state before the chunk gives
+      {
+        const float t0 = e_in[i0], t1 = e_in[i0 + 8];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            yin[k][i] = ((main[k][i] + main1[k][i]) + small[k][i]) * (i < 2 ? t0 : t1);
+            main[k][i] = small[k][i] = 0.f;
+          }
+      }
+      const float e0 = ei[i0], e1 = ei[i0 + 8];
+      for (int jt = 0; jt <= rt; ++jt) {
+        float m[2][4] = {};
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          uint32_t f[4];
+          gi::ldmatrix_x4(f, cb + L::B_AT + (16 * jt + b_row) * L::BP + k * 32 + b_col);
+          add_mma(m[0], cf[k], f[0], f[1]);
+          add_mma(m[1], cf[k], f[2], f[3]);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int j = 16 * jt + 8 * k + lc + e;
+            if (jt < rt) {
+              const float w = ej[rt * Q + j];
+              m[k][e] *= e0 * w;
+              m[k][2 + e] *= e1 * w;
+            } else {
+              const double cj = cum[j];
+              const float dt = sdt[j];
+              m[k][e] = i0 >= j ? m[k][e] * (expf((float)(cum[i0] - cj)) * dt) : 0.f;
+              m[k][2 + e] = i0 + 8 >= j ? m[k][2 + e] * (expf((float)(cum[i0 + 8] - cj)) * dt) : 0.f;
+            }
+          }
+        uint32_t a01[3], a23[3], b01[3], b23[3], xf[4];
+        split3_pair(m[0][0], m[0][1], a01);
+        split3_pair(m[0][2], m[0][3], a23);
+        split3_pair(m[1][0], m[1][1], b01);
+        split3_pair(m[1][2], m[1][3], b23);
+        gi::ldmatrix_x4_trans(xf, cb + L::X_AT + (16 * jt + a_row) * XP + ch * 32 + a_col);
+#pragma unroll
+        for (int s = 2; s >= 0; --s) {
+          const uint32_t af[4] = {a01[s], a23[s], b01[s], b23[s]};
+          if (s > 0) {
+            gi::mma_16816(small[0], af, xf[0], xf[1]);
+            gi::mma_16816(small[1], af, xf[2], xf[3]);
+          } else {
+            add_mma(main[0], af, xf[0], xf[1]);
+            add_mma(main[1], af, xf[2], xf[3]);
+          }
+        }
+      }
 #pragma unroll
       for (int k = 0; k < 2; ++k)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          yin[k][i] = ((main[k][i] + main1[k][i]) + small[k][i]) * (i < 2 ? t0 : t1);
-          main[k][i] = small[k][i] = 0.f;
+          yin[k][i] += main[k][i] + small[k][i];
+          odd = fmaf(yin[k][i], 0.f, odd);
         }
-    }
-    const float e0 = ei[i0], e1 = ei[i0 + 8];
-    for (int jt = 0; jt <= rt; ++jt) {
-      float m[2][4] = {};
-#pragma unroll
-      for (int k = 0; k < NT; ++k) {
-        uint32_t f[4];
-        gi::ldmatrix_x4(f, cb + L::B_AT + (16 * jt + b_row) * L::BP + k * 32 + b_col);
-        add_mma(m[0], cf[k], f[0], f[1]);
-        add_mma(m[1], cf[k], f[2], f[3]);
-      }
 #pragma unroll
       for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int j = 16 * jt + 8 * k + lc + e;
-          if (jt < rt) {
-            const float w = ej[rt * Q + j];
-            m[k][e] *= e0 * w;
-            m[k][2 + e] *= e1 * w;
-          } else {
-            const double cj = cum[j];
-            const float dt = sdt[j];
-            m[k][e] = i0 >= j ? m[k][e] * (expf((float)(cum[i0] - cj)) * dt) : 0.f;
-            m[k][2 + e] = i0 + 8 >= j ? m[k][2 + e] * (expf((float)(cum[i0 + 8] - cj)) * dt) : 0.f;
+        for (int r = 0; r < 2; ++r) {
+          const int i = i0 + 8 * r, col = ch * 16 + 8 * k + lc;
+          if (i < nc && p0 + col < P) {
+            const uint32_t xv = *reinterpret_cast<const uint32_t*>(bx + i * XP + col * 2);
+            const float2 o = make_float2(fmaf(D, __uint_as_float(xv << 16), yin[k][2 * r]),
+                                         fmaf(D, __uint_as_float(xv & 0xffff0000u), yin[k][2 * r + 1]));
+            *reinterpret_cast<float2*>(y + (size_t)(tok0 + c0 + i) * inner + (size_t)h * P + p0 + col) = o;
           }
         }
-      uint32_t a01[3], a23[3], b01[3], b23[3], xf[4];
-      split3_pair(m[0][0], m[0][1], a01);
-      split3_pair(m[0][2], m[0][3], a23);
-      split3_pair(m[1][0], m[1][1], b01);
-      split3_pair(m[1][2], m[1][3], b23);
-      gi::ldmatrix_x4_trans(xf, cb + L::X_AT + (16 * jt + a_row) * XP + ch * 32 + a_col);
-#pragma unroll
-      for (int s = 2; s >= 0; --s) {
-        const uint32_t af[4] = {a01[s], a23[s], b01[s], b23[s]};
-        if (s > 0) {
-          gi::mma_16816(small[0], af, xf[0], xf[1]);
-          gi::mma_16816(small[1], af, xf[2], xf[3]);
-        } else {
-          add_mma(main[0], af, xf[0], xf[1]);
-          add_mma(main[1], af, xf[2], xf[3]);
-        }
-      }
     }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        yin[k][i] += main[k][i] + small[k][i];
-        odd = fmaf(yin[k][i], 0.f, odd);
-      }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int i = i0 + 8 * r, col = ch * 16 + 8 * k + lc;
-        if (i < nc && p0 + col < P) {
-          const uint32_t xv = *reinterpret_cast<const uint32_t*>(bx + i * XP + col * 2);
-          const float2 o = make_float2(fmaf(D, __uint_as_float(xv << 16), yin[k][2 * r]),
-                                       fmaf(D, __uint_as_float(xv & 0xffff0000u), yin[k][2 * r + 1]));
-          *reinterpret_cast<float2*>(y + (size_t)(tok0 + c0 + i) * inner + (size_t)h * P + p0 + col) = o;
-        }
-      }
 
     if (warp < NT) {
       float add[4][4] = {}, low[4][4] = {};
 #pragma unroll
       for (int k = 0; k < Q / 16; ++k) {
+        if (!FULL && 16 * k >= nc) break;
         uint32_t af[4];
         gi::ldmatrix_x4_trans(af, cb + L::B_AT + (16 * k + b_row) * L::BP + warp * 32 + b_col);
 #pragma unroll
@@ -406,6 +408,16 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
       sum_dt(c0 + Q, buf ^ 1);
       load_dt(c0 + 2 * Q);
     }
+  };
+  bool walk = false;
+  for (int c0 = 0, buf = 0; c0 < qlen; c0 += Q, buf ^= 1) {
+    gi::cp_async_wait<0>();
+    // the chunk, its sums and S are in shared memory; the other buffers are free
+    walk = __syncthreads_or(odd != 0.f);
+    if (walk) break;
+    if (c0 + Q < qlen) load(c0 + Q, buf ^ 1);
+    if (qlen - c0 >= Q) chunk(c0, buf, std::true_type());
+    else chunk(c0, buf, std::false_type());
   }
   if (walk || __syncthreads_or(odd != 0.f)) {
     walk_all<NT>(smem, y + (size_t)tok0 * inner + (size_t)h * P + p0, inner, xbc + (size_t)tok0 * channels + inner + (size_t)g * N,
@@ -424,7 +436,7 @@ mamba2_chunks_kernel(float* __restrict__ y, const __nv_bfloat16* xbc, const __nv
 
 template <int NT>
 int launch_chunks(dim3 grid, cudaStream_t s, float* y, const void* xbc, const void* proj, long ld_proj, const float* dt_bias, const float* a_log,
-           const float* d_skip, float* state, long state_ld, int state_rows, const int* cu, const int* slots, int heads, int P, int N, int groups) {
+           const float* d_skip, float* state, long state_ld, int state_rows, const int* cu, const int* slots, int heads, int P, int N, int groups, int from) {
   static bool seen[gi::MAX_DEVICES_SEEN];
   int dev;
   if (gi::unconfigured_here(seen, &dev)) {
@@ -434,23 +446,23 @@ int launch_chunks(dim3 grid, cudaStream_t s, float* y, const void* xbc, const vo
   }
   return gi::check(gi::launch(mamba2_chunks_kernel<NT>, grid, dim3(THREADS), Layout<NT>::BYTES, s, y, (const __nv_bfloat16*)xbc,
                               (const __nv_bfloat16*)proj, ld_proj, dt_bias, a_log, d_skip, state, state_ld, state_rows, cu, slots, heads, P, N,
-                              groups), "mamba2 chunks");
+                              groups, from), "mamba2 chunks");
 }
 
 }  // namespace
 
 extern "C" int gi_mamba2_chunks(float* y, const void* xbc, const void* proj, long ld_proj, const float* dt_bias, const float* a_log,
                                 const float* d_skip, float* state, long state_ld, int state_rows, const int* cu_seqlens,
-                                const int* seq_slots, int n_seqs, int heads, int P, int N, int groups, void* stream) {
+                                const int* seq_slots, int n_seqs, int heads, int P, int N, int groups, int from, void* stream) {
   if (n_seqs <= 0) return GI_OK;
-  if (heads <= 0 || P <= 0 || N <= 0 || groups <= 0 || heads % groups != 0)
+  if (heads <= 0 || P <= 0 || N <= 0 || groups <= 0 || heads % groups != 0 || from < 1)
     return gi::fail(GI_ERR_ARG, "mamba2 chunks: %d heads, %d groups, head size %d, state %d", heads, groups, P, N);
   if (P % 8 != 0 || N % 8 != 0 || N > 128 || ((uintptr_t)xbc & 15) || ((uintptr_t)y & 7))
     return gi::fail(GI_ERR_UNSUPPORTED, "mamba2 chunks: head size and state must be multiples of 8, the state at most 128, rows aligned");
   if (n_seqs > 65535 || (P + PT - 1) / PT > 65535) return gi::fail(GI_ERR_UNSUPPORTED, "mamba2 chunks: more than one launch takes");
   const dim3 grid(heads, n_seqs, (P + PT - 1) / PT);
   cudaStream_t s = (cudaStream_t)stream;
-#define GI_CHUNKS(NT) launch_chunks<NT>(grid, s, y, xbc, proj, ld_proj, dt_bias, a_log, d_skip, state, state_ld, state_rows, cu_seqlens, seq_slots, heads, P, N, groups)
+#define GI_CHUNKS(NT) launch_chunks<NT>(grid, s, y, xbc, proj, ld_proj, dt_bias, a_log, d_skip, state, state_ld, state_rows, cu_seqlens, seq_slots, heads, P, N, groups, from)
   if (N <= 32) return GI_CHUNKS(2);
   if (N <= 64) return GI_CHUNKS(4);
   if (N <= 96) return GI_CHUNKS(6);

@@ -82,7 +82,8 @@ def _bind():
         "gi_kv_store": [P, I, L, P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, P],
         "gi_mamba2_conv": [P, P, I, L, P, P, I, P, L, I, P, P, I, I, I, I, I, I, P],
         "gi_mamba2_conv_update": [P, I, L, P, L, I, P, P, I, I, I, I, I, P],
-        "gi_mamba2_chunks": [P, P, P, L, P, P, P, P, L, I, P, P, I, I, I, I, I, P],
+        "gi_mamba2_chunks": [P, P, P, L, P, P, P, P, L, I, P, P, I, I, I, I, I, I, P],
+        "gi_mamba2_scan_below": [P, P, P, I, L, P, P, P, I, P, L, I, P, P, I, I, I, I, I, I, P],
         "gi_mamba2_scan": [P, P, P, I, L, P, P, P, I, P, L, I, P, P, I, I, I, I, I, P],
         "gi_mamba2_gate_norm": [P, I, P, P, I, L, P, I, I, I, I, F, P],
         "gi_moe_route": [P, P, P, P, I, L, P, P, I, I, I, I, I, P],
@@ -1499,8 +1500,15 @@ def mamba2_conv(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, 
     return out
 
 
-# tokens of a step's longest sequence from which the recurrence goes 64 tokens at a time
-MAMBA2_CHUNKS_FROM = 24
+def mamba2_chunks_from(n_state: int) -> int:
+    """From how many tokens in a step a sequence's recurrence goes 64 tokens at a time.  A sequence's own length decides, so that
+    its bits do not depend on what shares the step; so the line lies where the chunks gain, or lose little, for any number.  A
+    block of the chunks takes an SM for 7 to 10 us a chunk, and a batch queues for them; the walk's warps share an SM.  Walk
+    and chunks in us, 64 heads of 64, state of 128: one sequence of 32 tokens 14 and 9, of 48 20 and 10; 16 of 48 127 and 110, 64
+    of 40 512 and 446.  64 heads of 40, state of 96: 64 of 48 375 and 400, of 56 437 and 432, of 65 562 and 603, of 72 634
+    and 609.  24 heads of 64, state of 64, which the walk takes in half the time: 16 of 129 77 and 85, of 160 90 and 91, 64 of
+    128 274 and 252."""
+    return 56 if n_state > 64 else 160
 
 
 def mamba2_chunks_ok(xbc: torch.Tensor, dt_bias: torch.Tensor, head_dim: int, n_state: int) -> bool:
@@ -1527,17 +1535,22 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_bias: torch.Tensor, a_
         if t.numel() != heads or t.dtype != dt_bias.dtype or not t.is_contiguous():
             raise KernelError(f"the recurrence's per-head constants must be {heads} values of one type")
     y = torch.empty((proj.shape[0], inner), dtype=torch.float32, device=proj.device)
-    if mamba2_chunks_ok(xbc, dt_bias, head_dim, n_state) and step.max_q_len >= MAMBA2_CHUNKS_FROM:
+    chunks_from = mamba2_chunks_from(n_state)
+    below = 2 ** 31 - 1                  # the walk's sequences: those of fewer tokens
+    if mamba2_chunks_ok(xbc, dt_bias, head_dim, n_state) and step.max_q_len >= chunks_from:
         _check(lib, lib.gi_mamba2_chunks(y.data_ptr(), xbc.data_ptr(), proj.data_ptr(), _rows(proj, "projected rows"), dt_bias.data_ptr(),
                                          a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), state.stride(0), state.shape[0],
                                          _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"), step.n_seqs, heads,
-                                         head_dim, n_state, groups, _stream()))
-        return y
-    _check(lib, lib.gi_mamba2_scan(y.data_ptr(), xbc.data_ptr(), proj.data_ptr(), _dt(proj, "projected rows"),
-                                   _rows(proj, "projected rows"), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
-                                   _dt(dt_bias, "per-head constants"), state.data_ptr(), state.stride(0), state.shape[0],
-                                   _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"), step.n_seqs, heads,
-                                   head_dim, n_state, groups, _stream()))
+                                         head_dim, n_state, groups, chunks_from, _stream()))
+        lens = getattr(step, "_host_q_lens", None)
+        if lens and len(lens) == step.n_seqs and min(lens) >= chunks_from:
+            return y
+        below = chunks_from
+    _check(lib, lib.gi_mamba2_scan_below(y.data_ptr(), xbc.data_ptr(), proj.data_ptr(), _dt(proj, "projected rows"),
+                                         _rows(proj, "projected rows"), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
+                                         _dt(dt_bias, "per-head constants"), state.data_ptr(), state.stride(0), state.shape[0],
+                                         _i32(step.cu_seqlens, "cu_seqlens"), _i32(step.seq_slots, "slots"), step.n_seqs, heads,
+                                         head_dim, n_state, groups, below, _stream()))
     return y
 
 

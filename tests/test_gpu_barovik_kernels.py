@@ -299,8 +299,8 @@ def test_experts_expert_by_expert_on_tensor_cores():
     assert (got - want).abs().max().item() < 0.02 * want.abs().max().item()
 
 
-@pytest.mark.parametrize("sizes", [(64, 64, 128, 8, [2048]), (12, 40, 96, 4, [500, 1, 63]), (4, 24, 16, 2, [63, 65, 128, 17]), (2, 8, 40, 1, [130, 2]),
-                                   (3, 72, 72, 3, [64]), (2, 32, 8, 1, [24])])
+@pytest.mark.parametrize("sizes", [(64, 64, 128, 8, [2048]), (12, 40, 96, 4, [500, 1, 63]), (4, 24, 16, 2, [163, 165, 192, 17]), (2, 8, 40, 1, [230, 2]),
+                                   (3, 72, 72, 3, [64]), (2, 32, 8, 1, [177]), (2, 16, 80, 1, [56, 81])])
 @pytest.mark.parametrize("rate", [(-1.0, -0.5), (-6.0, -2.0), (3.0, 1.0)])
 def test_recurrence_by_chunks_errs_no_more_than_the_walk(sizes, rate):
     """Against 64 bits.  Both forms round each product and sum to 24 bits (2^-24 = 6e-8 of it at most), the walk once per token
@@ -315,7 +315,7 @@ def test_recurrence_by_chunks_errs_no_more_than_the_walk(sizes, rate):
     dt_bias, a_log, d_skip = (0.5 * torch.randn(heads, generator=g, device=DEV) + m for m in (*rate, 1.0))
     before = torch.randn(len(lens) + 2, heads * N * P + 3 * ch, generator=g, device=DEV)
     step = step_of(lens, [0] * len(lens), [n + 1 for n in range(len(lens))])
-    assert ops.mamba2_chunks_ok(xbc, dt_bias, P, N) and step.max_q_len >= ops.MAMBA2_CHUNKS_FROM
+    assert ops.mamba2_chunks_ok(xbc, dt_bias, P, N) and step.max_q_len >= ops.mamba2_chunks_from(N)
     chunks = before.clone()
     y = ops.mamba2_scan(xbc, proj, dt_bias, a_log, d_skip, chunks, step, heads, P, N, G, 4)
     walk, y_walk = before.clone(), torch.empty_like(y)
@@ -345,6 +345,35 @@ def test_recurrence_by_chunks_errs_no_more_than_the_walk(sizes, rate):
     assert torch.equal(chunks[:, heads * N * P:], before[:, heads * N * P:]) and torch.equal(chunks[0], before[0]) and torch.equal(chunks[-1], before[-1])
 
 
+@pytest.mark.parametrize("heads,P,N,G", [(4, 40, 128, 2), (3, 24, 72, 1), (2, 32, 64, 2), (2, 16, 16, 1)])
+@pytest.mark.parametrize("host_lists", [True, False])
+def test_a_recurrences_bits_do_not_depend_on_what_shares_its_step(heads, P, N, G, host_lists):
+    """Sequences just below and above the length from which chunks are taken, tile and chunk borders, single tokens: each alone, and
+    all in one step, give the same bits."""
+    at = ops.mamba2_chunks_from(N)
+    lens = [1, at - 1, at, 3, at + 17, 64 * 3, at + 1, 1]
+    g = torch.Generator(device=DEV).manual_seed(N)
+    inner, ch, T = heads * P, heads * P + 2 * G * N, sum(lens)
+    xbc = torch.randn(T, ch, generator=g, device=DEV).bfloat16()
+    proj = torch.randn(T, 2 * inner + 2 * G * N + heads, generator=g, device=DEV).bfloat16()
+    dt_bias, a_log, d_skip = (0.3 * torch.randn(heads, generator=g, device=DEV) + m for m in (-1.0, -0.5, 1.0))
+    before = torch.randn(len(lens) + 2, heads * N * P, generator=g, device=DEV)
+
+    def run(lens, rows, slots):
+        step, state = step_of(lens, [0] * len(lens), slots), before.clone()
+        if host_lists:
+            step._host_q_lens = lens
+        y = ops.mamba2_scan(xbc[rows].contiguous(), proj[rows].contiguous(), dt_bias, a_log, d_skip, state, step, heads, P, N, G, 1)
+        return y, state
+
+    y, state = run(lens, slice(0, T), list(range(1, len(lens) + 1)))
+    off = 0
+    for i, n in enumerate(lens):
+        alone, own = run([n], slice(off, off + n), [i + 1])
+        assert torch.equal(alone, y[off:off + n]) and torch.equal(own[i + 1], state[i + 1]), (i, n)
+        off += n
+
+
 @pytest.mark.parametrize("sizes", [(4, 40, 128, 2), (2, 64, 96, 1), (3, 8, 24, 3)])
 @pytest.mark.parametrize("where", ["x", "x nan", "B", "C", "step", "state", "large state", "two chunks"])
 @pytest.mark.parametrize("at", [0, 5, 70, 129])
@@ -354,7 +383,7 @@ def test_recurrence_by_chunks_keeps_what_is_no_number_where_the_walk_does(sizes,
     of the largest beside them)."""
     heads, P, N, G = sizes
     g = torch.Generator(device=DEV).manual_seed(N + at)
-    lens, inner, ch, T = [130, 40], heads * P, heads * P + 2 * G * N, 170
+    lens, inner, ch, T = [130 if N > 64 else 170, 40], heads * P, heads * P + 2 * G * N, 170 if N > 64 else 210
     xbc = torch.randn(T, ch, generator=g, device=DEV).bfloat16()
     proj = torch.randn(T, 2 * inner + 2 * G * N + heads, generator=g, device=DEV).bfloat16()
     dt_bias, a_log, d_skip = (0.3 * torch.randn(heads, generator=g, device=DEV) + m for m in (-1.0, -1.5, 1.0))
@@ -387,7 +416,7 @@ def test_recurrence_by_chunks_keeps_what_is_no_number_where_the_walk_does(sizes,
                               d_skip.data_ptr(), 0, walk.data_ptr(), walk.stride(0), walk.shape[0], step.cu_seqlens.data_ptr(),
                               step.seq_slots.data_ptr(), 2, heads, P, N, G, torch.cuda.current_stream().cuda_stream) == 0
     touched = at if where not in ("state", "large state") else 0
-    assert torch.isfinite(y[:touched]).all() and torch.isfinite(y[130:]).all()
+    assert torch.isfinite(y[:touched]).all() and torch.isfinite(y[lens[0]:]).all()
     for got, want in ((y, y_walk), (chunks, walk)):
         assert torch.equal(torch.isfinite(got), torch.isfinite(want))
         scale = torch.nan_to_num(want, 0.0, 0.0, 0.0).abs().amax(-1, keepdim=True).clamp_min(1.0)
