@@ -304,43 +304,55 @@ gate_norm_kernel(TO* __restrict__ out, const float* __restrict__ y, const T* __r
   }
 }
 
-// The same for 16-bit rows and parts of up to 128 VEC numbers in fours: a warp per part keeps its values in registers, so that
-// y and z are read once, 16 and 8 bytes at a time, and silu is worked out once.  grid (tokens, ceil(parts / 8)).
-// 2,048 tokens of 4,096 in 8 parts: 17 us, before 45 us.
-template <typename TW, int VEC>
+// The same for 16-bit rows and parts of up to 1,024 numbers in fours: TPP threads share a part, 4 VEC numbers each, kept in
+// registers, so that y and z are read once, 16 and 8 bytes at a time, and silu is worked out once.  The order of a part's sum
+// follows from its width alone, the same for one token and for many.  A block has 256 threads, fewer where the parts are fewer;
+// grid (tokens, ceil(parts / parts a block)).  Bound by silu's exponential and division where there are many tokens, else by
+// the chain from load to store.  4,096 numbers in 8 parts: one token 2.2 us, 2,048 tokens 14.5 us; the kernel above 2.4 and
+// 40 us, a warp per part with 16 numbers a lane 3.6 and 14.4 us, four numbers a thread 1.8 and 18 us.
+template <typename TW, int TPP, int VEC>
 __global__ void __launch_bounds__(256)
-gate_norm_warp_kernel(__nv_bfloat16* __restrict__ out, const float* y, const __nv_bfloat16* proj, long ld_proj, const TW* __restrict__ w,
-                      int inner, int parts, float eps) {
+gate_norm_vec_kernel(__nv_bfloat16* __restrict__ out, const float* y, const __nv_bfloat16* proj, long ld_proj, const TW* __restrict__ w,
+                     int inner, int parts, float eps) {
+  __shared__ float sums[8];
   gi::pdl_prologue();
-  const int t = blockIdx.x, part = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (part >= parts) return;
-  const int gw = inner / parts, c0 = part * gw;
-  float4 v[VEC];
+  const int t = blockIdx.x, part = blockIdx.y * (blockDim.x / TPP) + threadIdx.x / TPP, lane = threadIdx.x % TPP;
+  const int gw = inner / parts, c0 = part * gw, width = part < parts ? gw : 0;
+  float4 v[VEC], z[VEC];
+#pragma unroll
+  for (int k = 0; k < VEC; ++k) {
+    const int i = 4 * (lane + TPP * k);
+    v[k] = z[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < width) {
+      v[k] = gi::ld4(y + (size_t)t * inner + c0 + i);
+      z[k] = gi::ld4(proj + (size_t)t * ld_proj + c0 + i);
+    }
+  }
   float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < VEC; ++j) {
-    const int i = 4 * (lane + 32 * j);
-    v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < gw) {
-      v[j] = gi::ld4(y + (size_t)t * inner + c0 + i);
-      const float4 z = gi::ld4(proj + (size_t)t * ld_proj + c0 + i);
-      v[j].x *= silu_f(z.x);
-      v[j].y *= silu_f(z.y);
-      v[j].z *= silu_f(z.z);
-      v[j].w *= silu_f(z.w);
-    }
-    ss = fmaf(v[j].x, v[j].x, ss);
-    ss = fmaf(v[j].y, v[j].y, ss);
-    ss = fmaf(v[j].z, v[j].z, ss);
-    ss = fmaf(v[j].w, v[j].w, ss);
+  for (int k = 0; k < VEC; ++k) {
+    if (4 * (lane + TPP * k) >= width) continue;
+    v[k].x *= silu_f(z[k].x);
+    v[k].y *= silu_f(z[k].y);
+    v[k].z *= silu_f(z[k].z);
+    v[k].w *= silu_f(z[k].w);
+    ss = fmaf(v[k].w, v[k].w, fmaf(v[k].z, v[k].z, fmaf(v[k].y, v[k].y, fmaf(v[k].x, v[k].x, ss))));
   }
-  const float inv = 1.0f / sqrtf(gi::warp_sum(ss) / (float)gw + eps);
+  ss = gi::warp_sum(ss);
+  if (TPP > 32) {
+    if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < VEC; ++j) {
-    const int i = 4 * (lane + 32 * j);
-    if (i >= gw) continue;
+    for (int k = 0; k < TPP / 32; ++k) ss += sums[threadIdx.x / TPP * (TPP / 32) + k];
+  }
+  const float inv = 1.0f / sqrtf(ss / (float)gw + eps);
+#pragma unroll
+  for (int k = 0; k < VEC; ++k) {
+    const int i = 4 * (lane + TPP * k);
+    if (i >= width) continue;
     const float4 g = gi::ld4(w + c0 + i);
-    gi::st4(out + (size_t)t * inner + c0 + i, make_float4(v[j].x * inv * g.x, v[j].y * inv * g.y, v[j].z * inv * g.z, v[j].w * inv * g.w));
+    gi::st4(out + (size_t)t * inner + c0 + i, make_float4(v[k].x * inv * g.x, v[k].y * inv * g.y, v[k].z * inv * g.z, v[k].w * inv * g.w));
   }
 }
 
@@ -368,8 +380,12 @@ extern "C" int gi_mamba2_conv(void* xbc_out, const void* proj, int dtype, long l
   if (n_seqs > 65535) return gi::fail(GI_ERR_UNSUPPORTED, "mamba2 conv: more than 65535 sequences in one launch");
   if ((channels + 255) / 256 > 65535) return gi::fail(GI_ERR_UNSUPPORTED, "mamba2 conv: %d channels are more than one launch takes", channels);
   cudaError_t e = cudaSuccess;
-  // (state rows and `s_floats` in eights are not needed: the state is read number by number)
-  if (dtype == GI_BF16 && w_dtype == GI_BF16 && taps >= 2 && taps <= 4 && channels % 8 == 0 && inner % 8 == 0 && ld_proj % 8 == 0 &&
+  // Eight channels of eight tokens a thread leave too few threads where there are few tokens: the line lies at 64 tiles of
+  // eight tokens of 6,144 channels.  Kernel below and this one in us, 6,144 channels: one token 2.1 and 3.9, 64 sequences
+  // of one 4.8 and 8.8, 32 tokens 6.1 and 9.0, 256 13.4 and 13.1, 512 22 and 14; 3,328 channels: 512 tokens 13.4 and 13.8, 1,024
+  // 24 and 15.  (State rows and `s_floats` in eights are not needed: the state is read number by number.)
+  const long tiles = (long)((max_q_len + 7) / 8) * n_seqs;
+  if (max_q_len >= 8 && tiles * channels >= 64L * 6144 && dtype == GI_BF16 && w_dtype == GI_BF16 && taps >= 2 && taps <= 4 && channels % 8 == 0 && inner % 8 == 0 && ld_proj % 8 == 0 &&
       (((uintptr_t)xbc_out | (uintptr_t)proj | (uintptr_t)conv_b) & 15) == 0) {
     const dim3 grid((max_q_len + 7) / 8, n_seqs, (channels / 8 + 127) / 128);
 #define GI_CONV8(TAPS)                                                                                                              \
@@ -466,12 +482,17 @@ extern "C" int gi_mamba2_gate_norm(void* out, int out_dtype, const float* y, con
   const int gw = inner / parts;
   if (dtype == GI_BF16 && out_dtype == GI_BF16 && gw % 4 == 0 && gw <= 1024 && ld_proj % 4 == 0 && ((uintptr_t)y & 15) == 0 &&
       (((uintptr_t)proj | (uintptr_t)out) & 7) == 0 && ((uintptr_t)w & (w_dtype == GI_F32 ? 15 : 7)) == 0) {
-    const dim3 grid(n_tokens, (parts + 7) / 8);
-    GI_DISPATCH_DTYPE(w_dtype, TW,
-        e = gw <= 512 ? gi::launch(gate_norm_warp_kernel<TW, 4>, grid, dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)out, y,
-                                   (const __nv_bfloat16*)proj, ld_proj, (const TW*)w, inner, parts, eps)
-                      : gi::launch(gate_norm_warp_kernel<TW, 8>, grid, dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)out, y,
-                                   (const __nv_bfloat16*)proj, ld_proj, (const TW*)w, inner, parts, eps));
+    const int tpp = gw <= 256 ? 32 : gw <= 512 ? 64 : 128, here = parts < 256 / tpp ? parts : 256 / tpp;
+    const dim3 grid(n_tokens, (parts + here - 1) / here);
+#define GI_NORM(TPP, VEC)                                                                                                        \
+  GI_DISPATCH_DTYPE(w_dtype, TW,                                                                                                 \
+      e = gi::launch(gate_norm_vec_kernel<TW, TPP, VEC>, grid, dim3(here * tpp), 0, (cudaStream_t)stream, (__nv_bfloat16*)out, y, \
+                     (const __nv_bfloat16*)proj, ld_proj, (const TW*)w, inner, parts, eps))
+    if (gw <= 128) GI_NORM(32, 1);
+    else if (tpp == 32) GI_NORM(32, 2);
+    else if (tpp == 64) GI_NORM(64, 2);
+    else GI_NORM(128, 2);
+#undef GI_NORM
     return gi::check(e, "mamba2 norm");
   }
   dim3 grid(n_tokens, parts);

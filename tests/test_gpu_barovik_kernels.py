@@ -424,15 +424,18 @@ def test_recurrence_by_chunks_keeps_what_is_no_number_where_the_walk_does(sizes,
     assert (where == "large state") == bool(torch.isfinite(y).all())
 
 
-@pytest.mark.parametrize("heads,P,N,G,taps,parts", [(4, 24, 16, 2, 4, 2), (2, 8, 40, 1, 3, 1), (8, 64, 128, 4, 2, 4), (16, 40, 96, 4, 4, 1), (34, 32, 8, 2, 4, 17)])
+@pytest.mark.parametrize("heads,P,N,G,taps,parts", [(4, 24, 16, 2, 4, 2), (2, 8, 40, 1, 3, 1), (8, 64, 128, 4, 2, 4), (16, 40, 96, 4, 4, 1), (34, 32, 8, 2, 4, 17),
+                                                    (64, 64, 128, 8, 4, 8), (64, 64, 128, 8, 3, 4), (64, 64, 128, 8, 2, 16), (65, 64, 120, 8, 4, 13)])
 def test_convolution_and_gated_norm_in_eights_and_fours(heads, P, N, G, taps, parts):
     """16-bit rows by the kernels that read 16 bytes at a time, against 64 bits: the convolution to half a unit in the last of 8
     bits (a number in [1, 2) has units of 2^-7, so at most 2^-8 of the value) beside 2^-20 of its terms for sums in 32 bits, the
     norm likewise; sequences that begin in the middle and end
-    off the tiles of eight tokens."""
+    off the tiles of eight tokens; 6,144 channels and the many tokens that take the convolution by eights, alone the plain one,
+    with the same bits."""
     g = torch.Generator(device=DEV).manual_seed(heads + taps)
     inner, ch = heads * P, heads * P + 2 * G * N
-    lens, T = [1, 8, 37, 3], 49
+    lens = [1, 8, 133 if ch >= 6144 else 37, 3]
+    T = sum(lens)
     proj = torch.randn(T, 2 * inner + 2 * G * N + heads + (-heads) % 8, generator=g, device=DEV).bfloat16()
     w, bias = (torch.randn(ch, taps, generator=g, device=DEV) * 0.5).bfloat16(), (torch.randn(ch, generator=g, device=DEV) * 0.2).bfloat16()
     state = torch.randn(6, 5 + (taps - 1) * ch, generator=g, device=DEV)
@@ -448,6 +451,9 @@ def test_convolution_and_gated_norm_in_eights_and_fours(heads, P, N, G, taps, pa
         slack = (terms.abs().sum(0) + bias.double().abs()) * 2.0 ** -20
         assert ((got[at:at + n].double() - want).abs() <= want.abs() * 2.0 ** -8 + slack).all()
         assert torch.equal(state[slot, 5:].view(taps - 1, ch), x[n:].float())
+        own = before.clone()
+        alone = ops.mamba2_conv(proj[at:at + n].contiguous(), w, bias, own, step_of([n], [0], [slot]), inner, ch, taps, 5)
+        assert torch.equal(alone, got[at:at + n]) and torch.equal(own[slot], state[slot])
         at += n
     y = torch.randn(T, inner, generator=g, device=DEV)
     for nw in (torch.randn(inner, generator=g, device=DEV), torch.randn(inner, generator=g, device=DEV).bfloat16()):
@@ -455,3 +461,4 @@ def test_convolution_and_gated_norm_in_eights_and_fours(heads, P, N, G, taps, pa
         v = (y.double() * torch.nn.functional.silu(proj[:, :inner].double())).view(T, parts, -1)
         v = (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5)).view(T, inner) * nw.double()
         assert ((out.double() - v).abs() <= v.abs() * (2.0 ** -8 + 2.0 ** -18)).all()
+        assert torch.equal(ops.mamba2_gate_norm(y[7:8], proj[7:8], nw, parts, 1e-5, torch.bfloat16), out[7:8])
