@@ -16,8 +16,9 @@
 // A row belongs to a cluster of blocks where there are fewer rows than the GPU holds blocks: each block sweeps its part of the
 // row, and what the sweeps find (the highest logit, the counts or weights of the bins, the few logits of a wanted bin) meets
 // in the first block's shared memory, where the pick is made.  One block per row was bound by what one SM reads: three
-// sweeps over 513 KB a row on 64 of 148 SMs.  64 rows of 128,256 logits, top_k 40, top_p 0.9: 22 us (44 us with a
-// block per row); one row: 17 us (27 us).  Sums are integers and lists are sorted, so the cut changes no pick.
+// sweeps over 513 KB a row on 64 of 148 SMs.  64 rows of 128,256 logits, top_k 40, top_p 0.9: 19 us (22 us with a
+// block per row); one row: 16 us (22 us).  Sums are integers and lists are sorted, so the cut changes no pick.  What neither short way
+// settles goes to the first block alone, whose 1,024 threads take 0.8 ms for a top_k of 4,096 (with 512 threads 1.3 ms).
 //
 // The usual case, a top_k of at most 2048, takes a shorter way to the same pick: one sweep counts the keys by their
 // distance below the highest key (4096 bins of 2^16 key steps: the seven upper bits of the mantissa, 32 octaves),
@@ -39,7 +40,6 @@ namespace {
 
 typedef unsigned long long u64;
 
-constexpr int THREADS = 512;        // two blocks per SM
 constexpr float FIXED_ONE = 1099511627776.0f;  // 2^40
 
 __device__ __forceinline__ unsigned order_key(float v) {
@@ -262,30 +262,44 @@ __device__ __forceinline__ int warp_first_reaching(const u64* w, int count, u64 
   return __shfl_sync(0xffffffffu, found, src);
 }
 
-// The largest of 1, 2, 4, 8 blocks a row whose blocks all fit the GPU at once and have 4,096 logits or more.  (Two blocks per SM,
-// an eighth left out, since a cluster stays inside one group of SMs: 37 rows in clusters of 8 would fill the places exactly
-// and took 36 us, where 64 rows in clusters of 4 take 22.)
-int blocks_per_row(int rows, int n, int sms) {
+// How a launch is cut: threads a block and blocks a row.  A cluster stays inside one group of SMs, which does not hold as many
+// clusters of 8 as it has SMs / 8: with a block of 1,024 threads per SM, 14 rows and more of 8 blocks, and 33 and more of 4,
+// wait for each other (16 rows of 128,256 logits without a top_k: 46 us in clusters of 8, 31 in clusters of 4).  64 rows of 2
+// blocks take 46 us, of one 67; 100 rows of one 68.  Two sweeps of a short row take less than the blocks' meetings where a small
+// top_k ends the work (32,000 logits, top_k 40: 10.0 us, in clusters 13.3; without a top_k 23 and 18), and greedy sweeps but
+// once (4.0 us, in clusters 4.6; one row of 128,256 6.5 and 5.7).  More rows than SMs share them two by two where rows are
+// short (200 rows of 32,000, top_k 40: 15.2 us, with 1,024 threads 22; of 128,256 54 and 46).
+struct Cut {
+  int threads, blocks;
+};
+Cut cut_of(int rows, int n, int top_k, bool greedy, int sms) {
+  const bool short_rows = n < 65536;
+  if (rows > sms && short_rows) return {512, 1};
+  if (short_rows && (greedy || (top_k > 0 && top_k <= 128))) return {1024, 1};
+  if (greedy) return {1024, 32L * rows <= 7L * sms ? 4 : 1};
   int c = 1;
-  while (c < 8 && 16L * c * rows <= 14L * sms && n / (2 * c) >= 4096) c *= 2;
-  return c;
+  while (c < 8 && 16L * c * rows <= (c == 4 ? 6L : 7L) * sms && n / (2 * c) >= 6144) c *= 2;
+  return {1024, c};
 }
 
-__global__ void __launch_bounds__(THREADS, 2)
+// GREEDY: no draw follows.  CLUSTER: a row has several blocks; without, `blocks` is 1 at compile time (64 registers, and no meeting
+// that is more than a barrier).
+template <int THREADS, bool GREEDY, bool CLUSTER>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, int n, float temperature, int top_k,
               float top_p, u64* __restrict__ rng_state, const int* __restrict__ state_index) {
-  __shared__ Shared sh;
+  __shared__ __align__(16) Shared sh;
   gi::pdl_prologue();
   namespace cg = cooperative_groups;
   const cg::cluster_group cluster = cg::this_cluster();
-  const int blocks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int blocks = CLUSTER ? (int)cluster.num_blocks() : 1, rank = CLUSTER ? (int)cluster.block_rank() : 0;
   const int r = blockIdx.x / blocks, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float* row = logits + (size_t)r * ld;
   // this block's part of the row; `first` is the shared memory of the row's first block
   const int share = ((n + blocks - 1) / blocks + 3) / 4 * 4, lo = min(n, rank * share), hi = min(n, lo + share);
-  Shared& first = *cluster.map_shared_rank(&sh, 0);
+  Shared& first = CLUSTER ? *cluster.map_shared_rank(&sh, 0) : sh;
   auto meet = [&] {
-    if (blocks > 1) cluster.sync();
+    if (CLUSTER) cluster.sync();
     else __syncthreads();
   };
 
@@ -373,7 +387,7 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
     }
   }
   if (best == 0x7fffffff) best = 0;
-  if (!(temperature > 0.f) || rng_state == nullptr) {
+  if (GREEDY) {
     meet();                                                    // nobody leaves while its memory is being read
     if (rank == 0 && tid == 0) out[r] = best;
     return;
@@ -431,14 +445,32 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long ld, 
         }
         __syncthreads();
       }
-      u64 above = 0, all = 0;
-      const int pair = first_reaching(sh, FAST_BINS / 2, 0, (u64)top_k, [&](int j) { return (u64)sh.bins[2 * j] + sh.bins[2 * j + 1]; }, above, all);
-      if (tid == 0) {
-        const u64 covered = pair < 0 ? 0 : above + sh.bins[2 * pair];
-        const bool half = covered >= (u64)top_k;
-        sh.first_bin = half ? 2 * pair : 2 * pair + 1;
-        const u64 list = half || pair < 0 ? covered : covered + sh.bins[2 * pair + 1];
-        sh.besti = pair < 0 || list > (u64)FAST_CAP ? FAST_CAP + 1 : (int)list;      // how many were counted down to there
+      if (warp == 0) {
+        bool found = false;
+        u64 covered = 0;
+        for (int b0 = 0; b0 < FAST_BINS && !found; b0 += 128) {              // four bins a lane
+          const uint4 own = *reinterpret_cast<const uint4*>(sh.bins + b0 + 4 * lane);
+          const u64 mine = (u64)own.x + own.y + own.z + own.w;
+          u64 upto = mine;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const u64 up = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += up;
+          }
+          upto += covered;
+          const unsigned who = __ballot_sync(0xffffffffu, upto >= (u64)top_k);
+          found = who != 0;
+          if (found && lane == __ffs(who) - 1) {
+            const unsigned bins[4] = {own.x, own.y, own.z, own.w};
+            int k = 0;
+            upto -= mine;
+            while ((upto += bins[k]) < (u64)top_k) ++k;
+            sh.first_bin = b0 + 4 * lane + k;
+            sh.besti = upto > (u64)FAST_CAP ? FAST_CAP + 1 : (int)upto;      // how many were counted down to there
+          }
+          covered = __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (!found && lane == 0) sh.besti = FAST_CAP + 1;
       }
     }
     meet();
@@ -819,19 +851,27 @@ extern "C" int gi_sample(int* out_tokens, const float* logits, long ld, int n_ro
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || count <= 0) count = 148;
     sms = count;
   }
-  const int blocks = blocks_per_row(n_rows, vocab, sms);
-  if ((long)n_rows * blocks > 2147483647L) return gi::fail(GI_ERR_UNSUPPORTED, "sample: %d rows are more than one launch takes", n_rows);
+  const bool greedy = !(temperature > 0.f);
+  const Cut cut = cut_of(n_rows, vocab, top_k < vocab ? top_k : 0, greedy, sms);
+  if ((long)n_rows * cut.blocks > 2147483647L) return gi::fail(GI_ERR_UNSUPPORTED, "sample: %d rows are more than one launch takes", n_rows);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(n_rows * blocks);
-  cfg.blockDim = dim3(THREADS);
+  cfg.gridDim = dim3(n_rows * cut.blocks);
+  cfg.blockDim = dim3(cut.threads);
   cfg.stream = (cudaStream_t)stream;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = blocks;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = gi::pdl_enabled() ? 2 : 1;
-  return gi::check(cudaLaunchKernelEx(&cfg, sample_kernel, out_tokens, logits, ld, vocab, temperature, top_k, top_p, rng_state, state_index), "sample");
+  if (gi::pdl_enabled()) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cut.blocks > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cut.blocks;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  auto kern = cut.blocks > 1       ? (greedy ? sample_kernel<1024, true, true> : sample_kernel<1024, false, true>)
+              : cut.threads == 512 ? (greedy ? sample_kernel<512, true, false> : sample_kernel<512, false, false>)
+                                   : (greedy ? sample_kernel<1024, true, false> : sample_kernel<1024, false, false>);
+  return gi::check(cudaLaunchKernelEx(&cfg, kern, out_tokens, logits, ld, vocab, temperature, top_k, top_p, rng_state, state_index), "sample");
 }

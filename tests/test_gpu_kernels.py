@@ -1139,10 +1139,12 @@ def test_float32_products_share_one_order_of_additions(m, n, k, accumulate):
 
 
 @pytest.mark.parametrize("vocab", [4099, 8192, 20001, 70000, 128256])
-@pytest.mark.parametrize("temp,top_k,top_p", [(0.0, 0, 1.0), (0.7, 40, 0.9), (1.3, 1, 1.0), (0.9, 2048, 0.95), (0.8, 2049, 1.0), (1.0, 0, 1.0), (0.5, 0, 0.9)])
+@pytest.mark.parametrize("temp,top_k,top_p", [(0.0, 0, 1.0), (0.7, 40, 0.9), (1.3, 1, 1.0), (0.9, 300, 0.95), (0.9, 2048, 0.95), (0.8, 2049, 1.0), (1.0, 0, 1.0), (0.5, 0, 0.9)])
 def test_sampler_picks_do_not_depend_on_the_blocks_a_row_gets(vocab, temp, top_k, top_p):
-    """160 rows get a block each; 100, 60, 20 and 1 of them clusters of 1, 2, 4 and 8: the same picks and generator states,
-    with rows of ties, of numbers that are none, of one value, with the highest logit at either end, off 16-byte boundaries."""
+    """160 rows get a block each, of 512 threads where rows are short; fewer get blocks of 1,024, in clusters of 1, 2, 4 and 8 for
+    100, 60, 20 and 1 of them (no more than a row has 6,144 logits for, and none for a greedy pick or a small top_k of a short row): the
+    same picks and generator states, with rows of ties, of numbers that are none, of one value, with the highest logit at
+    either end, off 16-byte boundaries."""
     g = torch.Generator(device=DEV).manual_seed(vocab + top_k)
     whole = torch.empty((160, vocab + 1), device=DEV).normal_(0.0, 2.5, generator=g)
     for rows in (whole[:, :vocab], torch.nn.functional.pad(whole[:, :vocab], (0, (-vocab) % 4))[:, :vocab]):
@@ -1170,7 +1172,7 @@ def test_sampler_without_top_k_sums_the_blocks_bins_before_it_reads_them(rows, t
     target, and with it nearly every pick.  The answer is that of rows that get a block each."""
     g = torch.Generator(device=DEV).manual_seed(rows)
     logits = torch.empty((rows, 50000), device=DEV).normal_(0.0, 2.5, generator=g)
-    alone = logits.repeat((299 + rows) // rows, 1)           # 300 rows and more: no clusters
+    alone = logits.repeat((299 + rows) // rows, 1)           # 300 rows and more: a block each
     states = torch.arange(1, 1 + rows, dtype=torch.int64, device=DEV) * 6364136223846793005
     for _ in range(300):
         want_states = states.repeat(alone.shape[0] // rows)
