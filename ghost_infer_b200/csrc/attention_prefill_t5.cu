@@ -569,11 +569,8 @@ extern "C" int gi_attn_prefill_t5_ex2(void* out, long ldo, const void* q, long l
   if (rc != GI_OK) return rc;
   const int q_tiles = (max_q_len + BQ - 1) / BQ;
   // two query tiles per block where that makes the launch a single round of blocks (two blocks per SM)
-  int sms = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long paired_blocks = (long)n_heads * n_seqs * ((q_tiles + 1) / 2);
-  const int paired = (g_pairing != 0 && q_tiles > 1 && (g_pairing == 2 || paired_blocks <= 2L * (sms > 0 ? sms : 148))) ? 1 : 0;
+  const int paired = (g_pairing != 0 && q_tiles > 1 && (g_pairing == 2 || paired_blocks <= 2L * gi::sm_count())) ? 1 : 0;
   dim3 grid(n_heads, n_seqs, paired ? (q_tiles + 1) / 2 : q_tiles);
   if (hd == 128)
     return launch_t5<2, 2, 2, false>(grid, (cudaStream_t)stream, mq, mk, mv, NoRows{}, (__nv_bfloat16*)out, ldo, block_table, max_pages, cu_seqlens, seq_slots,
@@ -603,11 +600,8 @@ extern "C" int gi_attn_prefill_t5_rows(void* out, long ldo, const void* q, long 
   if (rc != GI_OK) return rc;
   rows.dim = dim, rows.rot = rot, rows.vdim = vdim, rows.gate = (const __nv_bfloat16*)gate, rows.ldg = ldg;
   const int q_tiles = (max_q_len + BQ - 1) / BQ;
-  int sms = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long paired_blocks = (long)n_heads * n_seqs * ((q_tiles + 1) / 2);
-  const int paired = (g_pairing != 0 && q_tiles > 1 && (g_pairing == 2 || paired_blocks <= 2L * (sms > 0 ? sms : 148))) ? 1 : 0;
+  const int paired = (g_pairing != 0 && q_tiles > 1 && (g_pairing == 2 || paired_blocks <= 2L * gi::sm_count())) ? 1 : 0;
   const dim3 grid(n_heads, n_seqs, paired ? (q_tiles + 1) / 2 : q_tiles);
 #define GI_ROWS(H, VH, VS) launch_t5<H, VH, VS, true>(grid, (cudaStream_t)stream, mq, mk, mv, rows, (__nv_bfloat16*)out, ldo, nullptr, 0, cu_seqlens, \
                                                       seq_slots, seq_pos0, n_heads, n_heads, scale, window, q_tiles, paired, 0.f, sinks, 0, 0)

@@ -22,6 +22,7 @@ namespace gi {
 bool pdl_enabled();                                // programmatic dependent launch switched on (gi_set_pdl)
 int fail(int code, const char* fmt, ...);          // records the message for gi_last_error(), returns code
 int check_launch(const char* what);                // cudaGetLastError() -> GI_OK or a recorded failure
+int sm_count();                                    // of the current device, asked once per device (148 if it does not say)
 
 // The order of a 32-bit product's sums (see gemm_f32.cu): SUM_SEGMENTS stretches of sum_segment(K) numbers, the last ones
 // shorter or empty.  A multiple of 32, so that every kernel's tile of K ends where a stretch does.

@@ -3,6 +3,8 @@
 #include <stdarg.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "api.h"
 #include "common.cuh"
 
@@ -24,6 +26,16 @@ int check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(GI_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   return GI_OK;
+}
+int sm_count() {
+  static std::atomic<int> counts[MAX_DEVICES_SEEN];
+  int dev = -1, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 148;
+  if (dev < MAX_DEVICES_SEEN) n = counts[dev].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  if (dev < MAX_DEVICES_SEEN) counts[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 }  // namespace gi
 

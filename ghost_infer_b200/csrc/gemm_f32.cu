@@ -261,22 +261,12 @@ int allow_smem(Kern kern, size_t bytes, bool (&seen)[gi::MAX_DEVICES_SEEN]) {
   return GI_OK;
 }
 
-int sm_count() {
-  static int counts[gi::MAX_DEVICES_SEEN];
-  int dev = -1, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 148;
-  if (dev < gi::MAX_DEVICES_SEEN && counts[dev] > 0) return counts[dev];
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  if (dev < gi::MAX_DEVICES_SEEN) counts[dev] = n;
-  return n;
-}
-
 template <int MT, bool ACCUM>
 int launch_few(float* out, const float* A, const float* W, int M, int N, int K, long lda, long ldw, long ldo, int seg, cudaStream_t s) {
   static bool seen[gi::MAX_DEVICES_SEEN];
   const int rc = allow_smem(few_rows_kernel<MT, ACCUM>, FEW_SMEM<MT>, seen);
   if (rc != GI_OK) return rc;
-  const int tiles = (N + ROWS - 1) / ROWS, blocks = sm_count();
+  const int tiles = (N + ROWS - 1) / ROWS, blocks = gi::sm_count();
   const dim3 grid(tiles < blocks ? tiles : blocks, (M + MT - 1) / MT);
   return gi::check(gi::launch(few_rows_kernel<MT, ACCUM>, grid, dim3(FEW_THREADS), FEW_SMEM<MT>, s, out, A, W, M, N, K, lda, ldw, ldo, seg), "gemm_f32");
 }
@@ -292,7 +282,7 @@ int launch_few(float* out, const float* A, const float* W, int M, int N, int K, 
 double few_cost(int M, int N) { return (M <= 4 ? 33.0 : M <= 8 ? 52.0 : 65.0 * ((M + 15) / 16)) / 16384.0 * N; }
 double many_cost(int M, int N, int tm) {
   const long tiles = (long)((M + 4 * tm - 1) / (4 * tm)) * ((N + BN - 1) / BN);
-  return 20.0 + (tm == 8 ? 55.0 : 7.2 * tm) * (double)((tiles + sm_count() - 1) / sm_count());
+  return 20.0 + (tm == 8 ? 55.0 : 7.2 * tm) * (double)((tiles + gi::sm_count() - 1) / gi::sm_count());
 }
 
 template <int TM, bool ACCUM>

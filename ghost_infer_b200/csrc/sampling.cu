@@ -845,14 +845,8 @@ extern "C" int gi_sample(int* out_tokens, const float* logits, long ld, int n_ro
   if (vocab <= 0) return gi::fail(GI_ERR_ARG, "sample: empty vocabulary");
   if (temperature > 0.f && !rng_state) return gi::fail(GI_ERR_ARG, "sample: temperature sampling needs generator states");
   if (top_k < 0) return gi::fail(GI_ERR_ARG, "sample: top_k must not be negative");
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0, count = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || count <= 0) count = 148;
-    sms = count;
-  }
   const bool greedy = !(temperature > 0.f);
-  const Cut cut = cut_of(n_rows, vocab, top_k < vocab ? top_k : 0, greedy, sms);
+  const Cut cut = cut_of(n_rows, vocab, top_k < vocab ? top_k : 0, greedy, gi::sm_count());
   if ((long)n_rows * cut.blocks > 2147483647L) return gi::fail(GI_ERR_UNSUPPORTED, "sample: %d rows are more than one launch takes", n_rows);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_rows * cut.blocks);
