@@ -23,7 +23,8 @@
 // 16 bytes at a time, a warp's lanes along the columns so that a row's number is one broadcast; three blocks per SM:
 // small tiles because 600 rows x 2,048 columns are only 80 tiles of 128 x 128.  600 rows: 16,384 x 2,048 956 us (42 TFLOP/s;
 // single multiply-adds in 64 x 64 tiles 1,079 us, the kernel before 2,480 us), 2,048 x 2,048 142 us in tiles
-// of 36 rows, 184 us in tiles of 32 (three on the fullest SM where 2.05 would do; 245 us and 300 us).
+// of 36 rows, 184 us in tiles of 32 (three on the fullest SM where 2.05 would do; single multiply-adds in 64 x 64 tiles 245 us,
+// the kernel before 300 us).
 #include "api.h"
 #include "common.cuh"
 
@@ -271,18 +272,24 @@ int launch_few(float* out, const float* A, const float* W, int M, int N, int K, 
   return gi::check(gi::launch(few_rows_kernel<MT, ACCUM>, grid, dim3(FEW_THREADS), FEW_SMEM<MT>, s, out, A, W, M, N, K, lda, ldw, ldo, seg), "gemm_f32");
 }
 
-// Which of the two, by what they measured (us per 2,048 of K): few_rows takes 33 / 52 / 65 for each pass of up to 4 / 8 / 16
-// tokens over 16,384 columns; many_rows 20 and 55 more for every tile of 32 rows the fullest SM works through.  2,048
-// columns: 48 rows 32 against 75, 100 rows 57 against 77; 16,384 columns: 48 rows 186 against 128; 128,256 columns: 16 rows
-// 468 against about 400.
+// Which of the two, by a model of what they measure (us), fitted to 1,134 sizes of 1 to 600 rows, 64 to 32,000 columns and K of 32
+// to 8,192; the faster of the two is missed by 0.1% on average, by 12% at most.  An SM of few_rows takes 4.8 / 7.9 / 9.4 a 16-row
+// tile of W and pass of up to 4 / 8 / 16 tokens and 2,048 of K, and works through all 32 stretches however short they are;
+// one of many_rows 63.5 for a round of 32-row tiles and 2,048 of K (its tiles share the FFMA pipe), 17.5 once.  2,048 columns:
+// 48 rows 32 against 75, 100 rows 57 against 77; 16,384 columns: 48 rows 186 against 128; 128,256 columns: 16 rows 468 against
+// about 400; K of 64, 4,096 columns: 64 rows 31 against 5.
 // A tile has 32 rows, or 36, 40 or 48 where that spares the fullest SM a tile: 601 rows x 2,048 columns are 304 tiles of 32
 // rows, three on some SMs (184 us), and 272 of 36, two at most (142 us).
 // The wider tiles leave room for two blocks an SM instead of three and cost 5% more for their rows (16,384 columns: 985 us
 // against 956).
-double few_cost(int M, int N) { return (M <= 4 ? 33.0 : M <= 8 ? 52.0 : 65.0 * ((M + 15) / 16)) / 16384.0 * N; }
-double many_cost(int M, int N, int tm) {
-  const long tiles = (long)((M + 4 * tm - 1) / (4 * tm)) * ((N + BN - 1) / BN);
-  return 20.0 + (tm == 8 ? 55.0 : 7.2 * tm) * (double)((tiles + gi::sm_count() - 1) / gi::sm_count());
+double few_cost(int M, int N, int seg) {
+  const int mt = M <= 4 ? M : M <= 8 ? 8 : 16, sms = gi::sm_count();
+  const long tiles = (N + ROWS - 1) / ROWS, blocks = tiles < sms ? tiles : sms, passes = (M + mt - 1) / mt;
+  return 4.1 + (M <= 4 ? 4.8 : M <= 8 ? 7.9 : 9.4) * (SUM_SEGMENTS * seg / 2048.0) * (double)((tiles + blocks - 1) / blocks) * (double)((blocks * passes + sms - 1) / sms);
+}
+double many_cost(int M, int N, int K, int tm) {
+  const long tiles = (long)((M + 4 * tm - 1) / (4 * tm)) * ((N + BN - 1) / BN), sms = gi::sm_count();
+  return 5.0 + (17.5 + (tm == 8 ? 63.5 : 8.3 * tm) * (double)((tiles + sms - 1) / sms)) * (K / 2048.0);
 }
 
 template <int TM, bool ACCUM>
@@ -300,9 +307,9 @@ int launch_product(float* out, const float* A, const float* W, int M, int N, int
   const int seg = gi::sum_segment(K);
   int tm = 8;
   for (int t : {9, 10, 12})
-    if (many_cost(M, N, t) < many_cost(M, N, tm)) tm = t;
+    if (many_cost(M, N, K, t) < many_cost(M, N, K, tm)) tm = t;
   // (few_rows has 16 tokens to a block of the grid's y, which takes 65,535)
-  if (few_cost(M, N) > many_cost(M, N, tm) || M > 16 * 65535) {
+  if (few_cost(M, N, seg) > many_cost(M, N, K, tm) || M > 16 * 65535) {
     if (tm == 8) return launch_many<8, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
     if (tm == 9) return launch_many<9, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
     if (tm == 10) return launch_many<10, ACCUM>(out, A, W, M, N, K, lda, ldw, ldo, seg, s);
