@@ -1,58 +1,70 @@
-// Plain matrix product on CUDA cores with 32-bit accumulation: out[M,N] (op)= A[M,K] * W[N,K]^T.
+// Plain matrix product on CUDA cores with 32-bit accumulation: out[M,N] (op)= A[M,K] * W[N,K]^T, for any types, sizes and strides.
 //
-// This is the kernel of the true 32-bit path (no tensor cores, no reduced-precision mode), and the
-// reference beside every faster product.  Each output element is summed by one thread walking k in
-// increasing order, so a row's result does not depend on what else is in the batch.  Weights are
+// The true 32-bit path's rows that start on 16-byte boundaries go to gemm_f32.cu; this kernel takes the rest (odd K, rows off such
+// boundaries, mixed and 16-bit types) and is the reference beside every faster product.  It has that file's order of
+// additions, which follows from K alone: the same bits whichever kernel ran, whatever else is in the batch.  Weights are
 // row-major [out, in] without bias, as the reference keeps them (src/model.rs:1019, src/quant.rs:73-78).
+//
+// Bound by the FFMA pipe where there are many rows, else by the chain over K (load, barrier, multiply).  Operands lie in k order
+// in shared memory, rows padded to 20 numbers (eight lanes' 16-byte reads fall into different banks), so that a packed
+// multiply-add takes the even and the odd k of two operands at once; two blocks an SM, whose 124 registers let loads and products
+// overlap.  32-bit rows off 16-byte boundaries: 300 x 8,192 x 2,047 527 us, 2,000 x 2,048 x 8,191 3.18 ms, one row x 2,048 x
+// 2,047 120 us; single multiply-adds, even and odd k in accumulators of their own, 820 us, 4.74 ms and 189 us; one running
+// sum over K 696 us, 3.10 ms and 192 us.
 #include "api.h"
 #include "common.cuh"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4, PITCH = BK + 4;
+
+// (lo, hi) of acc += the products of the halves, each rounded once, as fmaf would
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float join2(uint64_t v) { return __fadd_rn(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32))); }
 
 template <typename TA, typename TW, typename TO, int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 gemm_tile_kernel(void* __restrict__ out_, const TA* __restrict__ A, const TW* __restrict__ W, int M, int N, int K,
                  long lda, long ldw, long ldo, int seg) {
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Ws[BK][BN + 4];
+  __shared__ __align__(16) float As[BM * PITCH];
+  __shared__ __align__(16) float Ws[BN * PITCH];
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int tx = tid % 16, ty = tid / 16;  // thread owns rows ty*4..+4, cols tx*4..+4
-  float acc[2][TM][TN], sum[TM][TN];  // even k, odd k; finished stretches
+  const int tx = tid % 16, ty = tid / 16;  // thread owns rows ty + 16 i, columns tx + 16 j
+  uint64_t acc[TM][TN];                    // (even k, odd k)
+  float sum[TM][TN];                       // finished stretches
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[1][i][j] = sum[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0, sum[i][j] = 0.f;
 
   for (int k0 = 0; k0 < K; k0 += BK) {
     // 64 rows x 16 k per operand = 1024 elements, 4 per thread; consecutive threads walk k (contiguous)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int idx = tid + e * 256;
-      const int r = idx / BK, kk = idx % BK;
-      const int k = k0 + kk;
-      float a = 0.f, w = 0.f;
-      if (k < K) {
-        if (m0 + r < M) a = gi::ldf(A + (size_t)(m0 + r) * lda + k);
-        if (n0 + r < N) w = gi::ldf(W + (size_t)(n0 + r) * ldw + k);
-      }
-      As[kk][r] = a;
-      Ws[kk][r] = w;
+    for (int it = 0; it < 4; ++it) {
+      const int r = (tid >> 4) + 16 * it, k = tid & 15;
+      float av = 0.f, wv = 0.f;
+      if (m0 + r < M && k0 + k < K) av = gi::ldf(A + (size_t)(m0 + r) * lda + k0 + k);
+      if (n0 + r < N && k0 + k < K) wv = gi::ldf(W + (size_t)(n0 + r) * ldw + k0 + k);
+      As[r * PITCH + k] = av;
+      Ws[r * PITCH + k] = wv;
     }
     __syncthreads();
 #pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[TM], w[TN];
+    for (int k = 0; k < BK; k += 4) {
+      ulonglong2 w[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
+      for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(Ws + (tx + 16 * j) * PITCH + k);
 #pragma unroll
-      for (int j = 0; j < TN; ++j) w[j] = Ws[kk][tx * TN + j];
+      for (int i = 0; i < TM; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(As + (ty + 16 * i) * PITCH + k);
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+        for (int j = 0; j < TN; ++j) fma2(acc[i][j], a.x, w[j].x);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[kk & 1][i][j] = fmaf(a[i], w[j], acc[kk & 1][i][j]);
+        for (int j = 0; j < TN; ++j) fma2(acc[i][j], a.y, w[j].y);
+      }
     }
     __syncthreads();
     if ((k0 + BK) % seg == 0 || k0 + BK >= K) {  // a stretch ends
@@ -60,18 +72,18 @@ gemm_tile_kernel(void* __restrict__ out_, const TA* __restrict__ A, const TW* __
       for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-          sum[i][j] = __fadd_rn(sum[i][j], __fadd_rn(acc[0][i][j], acc[1][i][j]));
-          acc[0][i][j] = acc[1][i][j] = 0.f;
+          sum[i][j] = __fadd_rn(sum[i][j], join2(acc[i][j]));
+          acc[i][j] = 0;
         }
     }
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
-    const int m = m0 + ty * TM + i;
+    const int m = m0 + ty + 16 * i;
     if (m >= M) continue;
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      const int n = n0 + tx * TN + j;
+      const int n = n0 + tx + 16 * j;
       if (n >= N) continue;
       if (MODE == GI_GEMM_ACCUM_F32) {
         float* o = (float*)out_ + (size_t)m * ldo + n;
