@@ -2016,14 +2016,10 @@ def latent_expand_sizes(dim: int, rot_dim: int, v_dim: int, rank: int, dtype: to
 
 def _latent_visible(step, window: Optional[int]):
     """(cached rows that the step's tokens see, from a page boundary on; pairs of a token and a position it sees; tokens; tiles of 64
-    that the longest span has), None where the host has no lists of lengths.  Worked out once per step and window."""
+    that the longest span has), None where the host has no lists of lengths."""
     pos0, lens = getattr(step, "_host_pos0", None), getattr(step, "_host_q_lens", None)
     if not pos0 or not lens or len(pos0) != step.n_seqs or len(lens) != step.n_seqs:
         return None
-    shared = getattr(step, "shared", None)
-    key = ("latent_visible", window)
-    if shared is not None and key in shared:
-        return shared[key]
     rows = pairs = tokens = tiles = 0
     span = int(window) if window else 1 << 62
     for p, n in zip(pos0, lens):
@@ -2032,14 +2028,12 @@ def _latent_visible(step, window: Optional[int]):
         pairs += whole * p + whole * (whole + 1) // 2 + (n - whole) * (0 if whole == n else span)
         tokens += n
         tiles = max(tiles, (min(p + n, span) + 63) // 64)
-    if shared is not None:
-        shared[key] = rows, pairs, tokens, tiles
     return rows, pairs, tokens, tiles
 
 
 def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, rank: int, window: Optional[int], dtype: torch.dtype) -> int:
     """How many cached rows a prompt step should turn into keys and values per head (`attention_latent_expanded`), or 0: carry
-    its queries onto the latents instead (`attention_latent`).
+    its queries onto the latents instead (`attention_latent`).  Worked out once per step for layers of the same sizes.
 
     Carried, a head spends 2 rank + rot_dim multiply-adds on a query and key; expanded, dim + rot_dim + v_dim, and rank (dim +
     v_dim) more on every visible position once.  Measured multiply-adds per microsecond: the carried kernel 74e6 (a block's
@@ -2047,18 +2041,22 @@ def latent_expand_rows(step, n_heads: int, dim: int, rot_dim: int, v_dim: int, r
     queries and results 32e6, the attention over rows 200e6 (2 us a tile), the product that forms the rows 400e6; 40 us
     for what the host spends more on a few hundred tokens (tensor maps of new buffers).  16 heads, rank 512: 64 fresh tokens are carried; 16 tokens behind 3,000 take 98 us expanded, 418 carried.
     Only prompt steps have the host's lists of lengths."""
-    if step.is_decode or not TUNE["attn_latent_tc"] or not latent_expand_sizes(dim, rot_dim, v_dim, rank, dtype):
+    if step.is_decode:
         return 0
-    visible = _latent_visible(step, window)
-    if visible is None:
-        return 0
-    rows, pairs, tokens, tiles = visible
-    if rows * n_heads * (dim + v_dim) * 2 > LATENT_EXPAND_BYTES:
-        return 0
-    work = 2 * rank + rot_dim
-    carried = max(n_heads * pairs * work / 74e6, tiles * work * 7.6e-3) + n_heads * tokens * rank * (dim + v_dim) / 32e6
-    expanded = max(n_heads * pairs * (dim + rot_dim + v_dim) / 200e6, tiles * 2.0) + n_heads * rows * rank * (dim + v_dim) / 400e6 + 40.0
-    return rows if expanded < carried else 0
+    shared, key = getattr(step, "shared", None), ("latent_expand", n_heads, dim, rot_dim, v_dim, rank, window, dtype, TUNE["attn_latent_tc"])
+    if shared is not None and key in shared:
+        return shared[key]
+    found = 0
+    visible = _latent_visible(step, window) if TUNE["attn_latent_tc"] and latent_expand_sizes(dim, rot_dim, v_dim, rank, dtype) else None
+    if visible is not None and visible[0] * n_heads * (dim + v_dim) * 2 <= LATENT_EXPAND_BYTES:
+        rows, pairs, tokens, tiles = visible
+        work = 2 * rank + rot_dim
+        carried = max(n_heads * pairs * work / 74e6, tiles * work * 7.6e-3) + n_heads * tokens * rank * (dim + v_dim) / 32e6
+        expanded = max(n_heads * pairs * (dim + rot_dim + v_dim) / 200e6, tiles * 2.0) + n_heads * rows * rank * (dim + v_dim) / 400e6 + 40.0
+        found = rows if expanded < carried else 0
+    if shared is not None:
+        shared[key] = found
+    return found
 
 
 def attention_latent_expanded(q: torch.Tensor, memory, step, w_uk_uv: torch.Tensor, rows: int, n_heads: int, dim: int, rot_dim: int,

@@ -121,9 +121,9 @@ def test_rows_formed_per_head_are_those_the_kernels_count():
             tiles = max(tiles, (max(b - a + 1 for a, b in seen) + 63) // 64)
         step = prompt(pos0, lens)
         assert ops._latent_visible(step, window) == (rows, pairs, tokens, tiles)
-        assert ops._latent_visible(step, window) == (rows, pairs, tokens, tiles) and len(step.shared) == 1
         got = ops.latent_expand_rows(step, 16, 128, 64, 128, 512, window, BF)
-        assert got in (0, rows)
+        assert got in (0, rows) and list(step.shared.values()) == [got]
+        assert ops.latent_expand_rows(step, 16, 128, 64, 128, 512, window, BF) == got and len(step.shared) == 1
         chosen += got > 0
     assert 100 < chosen < 400
 
