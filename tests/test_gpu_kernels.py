@@ -1108,7 +1108,7 @@ def test_prompt_attention_with_one_row_warp_far_behind_the_others(hd, slow_warp)
 
 @pytest.mark.parametrize("m,n,k", [(1, 16, 32), (1, 2055, 4), (2, 17, 36), (3, 130, 1028), (4, 2048, 2048), (5, 33, 512), (8, 1000, 3076),
                                    (9, 31, 1024), (16, 48, 2080), (17, 129, 96), (33, 16400, 64), (49, 100, 320), (65, 2047, 1100),
-                                   (300, 384, 2048)])
+                                   (300, 384, 2048), (16, 20000, 128), (64, 4096, 64), (100, 2048, 32)])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_float32_products_share_one_order_of_additions(m, n, k, accumulate):
     """The kernels of few and of many rows and the general one (which takes rows that start off a 16-byte boundary) give
