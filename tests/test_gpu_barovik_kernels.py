@@ -300,7 +300,7 @@ def test_experts_expert_by_expert_on_tensor_cores():
 
 
 @pytest.mark.parametrize("sizes", [(64, 64, 128, 8, [2048]), (12, 40, 96, 4, [500, 1, 63]), (4, 24, 16, 2, [163, 165, 192, 17]), (2, 8, 40, 1, [230, 2]),
-                                   (3, 72, 72, 3, [64]), (2, 32, 8, 1, [177]), (2, 16, 80, 1, [56, 81])])
+                                   (3, 72, 72, 3, [64]), (2, 32, 8, 1, [177]), (2, 16, 80, 1, [56, 81]), (2, 40, 128, 1, [65, 80, 129, 112])])
 @pytest.mark.parametrize("rate", [(-1.0, -0.5), (-6.0, -2.0), (3.0, 1.0)])
 def test_recurrence_by_chunks_errs_no_more_than_the_walk(sizes, rate):
     """Against 64 bits.  Both forms round each product and sum to 24 bits (2^-24 = 6e-8 of it at most), the walk once per token
