@@ -111,6 +111,13 @@ int gi_silu_mul(void* out, const void* gate_up, int dtype, int n_rows, int f, in
 int gi_gemm_generic(void* out, int out_dtype, int mode, const void* A, int a_dtype, const void* W, int w_dtype, int M,
                     int N, int K, long lda, long ldw, long ldo, void* stream);
 
+// The float products of larger matrices on tensor cores (gemm_f32_split.cu): bytes of scratch they need, or -1 where
+// gi_gemm_generic takes the matrix.  The scratch starts on a 16-byte boundary and is used until the launched kernels end.
+long gi_gemm_f32_split_scratch(int M, int N, int K);
+int gi_gemm_f32_split(float* out, int mode, const float* A, const float* W, int M, int N, int K, long lda, long ldw, long ldo,
+                      void* scratch, long scratch_bytes, void* stream);
+int gi_gemm_f32_split_status(int* status);
+
 // mode of gi_gemm_skinny_bf16
 #define GI_SKINNY_STORE_BF16 0
 #define GI_SKINNY_STORE_F32 1

@@ -48,6 +48,9 @@ def _bind():
         "gi_silu_mul": [P, P, I, I, I, I, P],
         "gi_gemm_skinny_bf16": [P, I, P, P, I, I, I, L, L, L, P],
         "gi_gemm_generic": [P, I, I, P, I, P, I, I, I, I, L, L, L, P],
+        "gi_gemm_f32_split": [P, I, P, P, I, I, I, L, L, L, P, L, P],
+        "gi_gemm_f32_split_status": [P],
+        "gi_gemm_f32_split_scratch": [I, I, I],
         "gi_rope_table": [P, P, P, I, I, P],
         "gi_rope_cache_write": [P, I, L, P, P, P, P, I, P, P, I, I, I, I, I, I, I, P],
         "gi_rope_cache_write_settle": [P, I, L, P, P, P, P, I, P, P, I, I, I, I, I, I, I, SettleT, P],
@@ -157,6 +160,7 @@ def _bind():
         fn.argtypes = argtypes
         fn.restype = c_int
     lib.gi_gemm_stream_scratch_floats.restype = c_long
+    lib.gi_gemm_f32_split_scratch.restype = c_long
     if os.environ.get("GHOST_INFER_PDL") in ("0", "1"):         # the process-wide default of set_pdl
         lib.gi_set_pdl(int(os.environ["GHOST_INFER_PDL"]))
     _bound = lib
@@ -508,7 +512,8 @@ def silu_mul(gate_up: torch.Tensor, out: Optional[torch.Tensor] = None, interlea
 
 def gemm_generic(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None,
                  out_dtype: Optional[torch.dtype] = None, accumulate: bool = False) -> torch.Tensor:
-    """out[M, N] (+)= a[M, K] @ w[N, K]^T with 32-bit accumulation on CUDA cores."""
+    """out[M, N] (+)= a[M, K] @ w[N, K]^T with 32-bit accumulation: in float32 the matrices of 1,024 rows and columns or more
+    on tensor cores (every number in two 16-bit parts), the rest on CUDA cores."""
     lib = _bind()
     _cuda(a, "activations")
     _cuda(w, "weights")
@@ -525,6 +530,13 @@ def gemm_generic(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor
     if out.shape != (m, n):
         raise KernelError(f"matrix product: output is {tuple(out.shape)}, wanted {(m, n)}")
     mode = GEMM_ACCUM_F32 if accumulate else GEMM_STORE
+    if a.dtype == w.dtype == out.dtype == torch.float32:
+        need = lib.gi_gemm_f32_split_scratch(m, n, k)
+        if need >= 0:                        # a larger matrix: on the tensor cores, whatever the rows
+            scratch = torch.empty((need,), dtype=torch.uint8, device=a.device) if need > 0 else None
+            _check(lib, lib.gi_gemm_f32_split(out.data_ptr(), mode, a.data_ptr(), w.data_ptr(), m, n, k, lda, ldw, ldo,
+                                              scratch.data_ptr() if scratch is not None else None, need, _stream()), 2 if need > 0 else 1)
+            return out
     _check(lib, lib.gi_gemm_generic(out.data_ptr(), _dt(out, "output"), mode, a.data_ptr(), _dt(a, "activations"),
                                     w.data_ptr(), _dt(w, "weights"), m, n, k, lda, ldw, ldo, _stream()))
     return out
@@ -824,13 +836,21 @@ def gemm_tc_status() -> int:
     return status.value
 
 
+def gemm_f32_split_status() -> int:
+    """0 if every wait inside the 32-bit product on tensor cores was met since the last call; synchronises the device."""
+    lib = _bind()
+    status = ctypes.c_int(0)
+    _check(lib, lib.gi_gemm_f32_split_status(ctypes.byref(status)), 0)
+    return status.value
+
+
 def check_status() -> None:
     """Raises if any bounded wait inside the tensor-core kernels ran out since the last call (the kernel then left
     through its normal exit with its work undone: the results of that launch are not to be trusted).  Reads and
     clears the kernels' status words; synchronises the device."""
     bad = []
     for name, fn in (("prompt product", gemm_tc_status), ("decode product", gemm_stream_status),
-                     ("prompt attention", attn_prefill_t5_status)):
+                     ("prompt attention", attn_prefill_t5_status), ("32-bit product", gemm_f32_split_status)):
         code = fn()
         if code:
             bad.append(f"{name} (wait {code})")

@@ -1138,6 +1138,45 @@ def test_float32_products_share_one_order_of_additions(m, n, k, accumulate):
     assert ((got.double() - exact).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 1024, 1024), (2, 2048, 1091), (16, 1025, 1028), (17, 1100, 1151), (31, 3072, 1024), (129, 1152, 4160),
+                                   (3, 19000, 1088), (8200, 1024, 1024)])
+def test_float32_products_in_two_16_bit_parts(m, n, k):
+    """The larger matrices' kernel: clusters and whole tiles, tokens split inside and before, ends of tiles, chunks and stretches.
+
+    |error| <= sum |a w| times: 2 * 2^-23 (either operand's parts), 2^-22 (the product of the low parts), 12 * 2^-23 (what twelve
+    instructions cut off a chunk's sum), (chunks of a stretch + 8) * 2^-24 (additions), 2^-23 (what is given back for the cut)."""
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(m + n + k)
+    # chunks of a row, and rows, of very different size: each has its own power of two
+    size = torch.exp2(torch.randint(-20, 20, (m, k // 64 + 1), generator=gen, device=DEV).float()).repeat_interleave(64, 1)[:, :k]
+    a = torch.randn((m, k), generator=gen, device=DEV) * size
+    w = torch.randn((n, k), generator=gen, device=DEV) * torch.exp2(torch.randint(-9, 9, (n, 1), generator=gen, device=DEV).float())
+    w[n // 2] = 0.0
+    got = ops.gemm_generic(a, w)
+    rows = torch.arange(m, device=DEV) if m < 1000 else torch.tensor([0, 1, 127, 128, 8191, 8192, m - 1], device=DEV)
+    chunks = (k + 63) // 64
+    bound = (a[rows].double().abs() @ w.double().abs().T) * (2 * 2.0 ** -23 + 2.0 ** -22 + 13 * 2.0 ** -23 + ((chunks + 7) // 8 + 8) * 2.0 ** -24)
+    assert ((got[rows].double() - a[rows].double() @ w.double().T).abs() <= bound).all()
+    # a row's bits are its own: alone, beside others, off 16-byte boundaries, added to an output
+    for i in (0, m - 1):
+        assert torch.equal(ops.gemm_generic(a[i:i + 1], w)[0], got[i])
+    odd_w, odd_a = torch.empty((n, k + 1), device=DEV), torch.empty((m, k + 3), device=DEV)
+    odd_w[:, :k], odd_a[:, 1:k + 1] = w, a
+    assert torch.equal(ops.gemm_generic(odd_a[:, 1:k + 1], odd_w[:, :k]), got)
+    out = torch.randn((m, n + 5), generator=gen, device=DEV)
+    want = out.clone()
+    want[:, 3:n + 3] += got
+    ops.gemm_generic(a, w, out=out[:, 3:n + 3], accumulate=True)
+    assert torch.equal(out, want)
+    # what is no finite number, or grows to none, comes out as plain multiply-adds give it
+    a[0, 7], w[1, k - 1], w[2, 0], a[m - 1, k - 2], w[3, k - 2] = float("inf"), float("nan"), -float("inf"), 3e38, 3e38
+    odd, part = ops.gemm_generic(a, w)[rows], a[rows].contiguous()
+    ref, lib = torch.empty((len(rows), n), device=DEV), ops._bind()
+    assert lib.gi_gemm_generic(ref.data_ptr(), 0, ops.GEMM_STORE, part.data_ptr(), 0, w.data_ptr(), 0, len(rows), n, k, k, k, n, ops._stream()) == 0
+    assert torch.equal(torch.isnan(odd), torch.isnan(ref)) and torch.equal(odd[ref.isinf()], ref[ref.isinf()])
+    assert ops.gemm_f32_split_status() == 0
+
+
 @pytest.mark.parametrize("vocab", [4099, 8192, 20001, 70000, 128256])
 @pytest.mark.parametrize("temp,top_k,top_p", [(0.0, 0, 1.0), (0.7, 40, 0.9), (1.3, 1, 1.0), (0.9, 300, 0.95), (0.9, 2048, 0.95), (0.8, 2049, 1.0), (1.0, 0, 1.0), (0.5, 0, 0.9)])
 def test_sampler_picks_do_not_depend_on_the_blocks_a_row_gets(vocab, temp, top_k, top_p):
