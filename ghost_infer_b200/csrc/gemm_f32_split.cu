@@ -13,9 +13,17 @@
 // A tile is 128 rows of W (the "M" side of the instruction, split by four warps on the way from shared into tensor memory)
 // times up to 128 tokens (the "N" side, in shared memory).  One thread feeds both rings with TMA, one issues the
 // products, four warps split W, eight drain accumulators; two chunks of W and two accumulators in tensor memory, so that all
-// four overlap.  Up to 16 tokens (FEW) two more warps split the tokens themselves, eight warps split W in turns, and where W
-// has few rows the blocks of a cluster share the stretches of a tile, which meet in distributed shared memory; more tokens
-// are split once by a kernel of their own, into scratch.
+// four overlap.  Up to 32 tokens (FEW, tiles of 16) two more warps split the tokens themselves, eight warps split W in turns, and
+// where there are few tiles the blocks of a cluster share the stretches of a tile, which meet in distributed shared memory;
+// more tokens are split once by a kernel of their own, into scratch.
+//
+// Steps of one token a sequence keep gemm_f32.cu's kernels (ops.one_token_step): they are bound by the bytes of W, and there the
+// chain of a chunk (32 KB: split 0.4 us, twelve products 0.5 us at 16 tokens as at 128, since each reads 128 rows of W out of
+// tensor memory) is longer than the chunk's share of the memory's time: a 1B model's step of four 1.98 ms against 1.72.
+// B200, one launch beside one of gemm_f32.cu: 601 rows 16,384 x 2,048 223 us (181 TFLOP/s) against 960; 2,048 x 8,192 150 against
+// 550; 64 rows 46 against 134 and 112 against 150; 16 rows 51 against 72 and 48 against 48.  What bounds it with many rows is
+// the draining warps (64 columns a thread and chunk), with few the one thread's products.
+// Distance from 64 bits (2-norms): 1.2e-7 against 1.5e-7 (K 2,048), 1.4e-7 against 2.3e-7 (K 8,192), 1.2e-7 against 1.3e-7 (K 1,024).
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <float.h>
@@ -31,7 +39,7 @@ using namespace gi::tc;
 constexpr int ROWS = 128;              // rows of W a tile = lanes of tensor memory
 constexpr int CK = 64;                 // numbers of K a chunk
 constexpr int STRETCHES = 8;
-constexpr int FEW_MAX = 16;            // tokens of the FEW form
+constexpr int FEW_TILE = 16, FEW_MAX = 32;   // tokens a tile of the FEW form, and tokens up to which it is taken
 constexpr int SLAB = 8192;             // tokens split into scratch at a time
 constexpr uint32_t W_STAGE = ROWS * CK * 4;
 
@@ -54,7 +62,7 @@ struct Args {
 
 template <bool FEW, bool CLUSTER>
 struct Shape {
-  static constexpr int NT = FEW ? FEW_MAX : 128;             // tokens a tile at most
+  static constexpr int NT = FEW ? FEW_TILE : 128;             // tokens a tile at most
   static constexpr int W_STAGES = CLUSTER ? 4 : FEW ? 6 : 3, X_STAGES = FEW ? 4 : 3, A_STAGES = FEW ? 4 : 2;
   // Slots of a chunk's powers of two and of its two barriers, from splitting to draining.  W is split at most A_STAGES chunks
   // ahead of the products, tokens X_STAGES, and the products are at most two ahead of the drained ones: six would do.
@@ -303,12 +311,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc = (1u << 4) | ((uint32_t)(a.nt >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);   // float sums of 16-bit floats
-      bool ok = true, ahead = false;
+      bool ok = true;
       int it = 0;
       for (int tile = tile0; tile < a.tiles && ok; tile += tile_step)
         for (int c = c_first; c < c_last && ok; ++c, ++it) {
           const int st = it & 1, as = it % S::A_STAGES, xs = it % S::X_STAGES;
-          ok = ahead || wait_full(it, 2);
+          ok = wait_full(it, 2);
           if (!ok) break;
           tc_fence_after();
           const uint32_t d = tmem + st * S::NT, hi = tmem + S::A_AT + as * 64, lo = hi + 32;
@@ -317,8 +325,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
           for (int k = 0; k < CK / 16; ++k) mma_a_tmem(d, lo + 8 * k, x_hi + 2 * k, idesc, k > 0);
 #pragma unroll
           for (int k = 0; k < CK / 16; ++k) mma_a_tmem(d, hi + 8 * k, x_lo + 2 * k, idesc, 1);
-          // asked while products are queued: a wait at the chunk's end would leave the tensor cores without any
-          ahead = mbar_try_wait(full + 8 * ((it + 1) % S::SLOTS), (uint32_t)(((it + 1) / S::SLOTS) & 1));
 #pragma unroll
           for (int k = 0; k < CK / 16; ++k) mma_a_tmem(d, hi + 8 * k, x_hi + 2 * k, idesc, 1);
           tc_commit(done + 8 * (it % S::SLOTS));
@@ -409,24 +415,27 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const float f = fw[slot * ROWS + row];
         const uint64_t f2 = pack2(f, f);
         const uint32_t d = tmem + lane_base + st * S::NT;
-        // the next group is on its way while this one is added
-        uint32_t r[2][GROUP];
-        if (col_of(0) < nt) tc_ld16(d + col_of(0), r[0]);
+        auto take = [&](int g, const uint32_t (&r)[GROUP]) {
 #pragma unroll
-        for (int g = 0; g < GROUPS; ++g) {
-          const int col = col_of(g);
-          if (col < nt) {
-            ulonglong2 x[GROUP / 4];
+          for (int j = 0; j < GROUP; j += 4) {
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(fx + slot * S::NT + col_of(g) + j);
+            fma2(acc[(g * GROUP + j) / 2], (uint64_t)r[j] | (uint64_t)r[j + 1] << 32, mul2(x.x, f2));
+            fma2(acc[(g * GROUP + j) / 2 + 1], (uint64_t)r[j + 2] | (uint64_t)r[j + 3] << 32, mul2(x.y, f2));
+          }
+        };
+        // (a third of a chunk's time; one group asked for while the one before is added was slower: 253 against 223 us at 601 x 16,384 x 2,048)
 #pragma unroll
-            for (int j = 0; j < GROUP; j += 4) x[j / 4] = *reinterpret_cast<const ulonglong2*>(fx + slot * S::NT + col + j);
-            wait_ld16(r[g & 1]);
-            if (g + 1 < GROUPS && col_of(g + 1) < nt) tc_ld16(d + col_of(g + 1), r[(g + 1) & 1]);
-            const uint32_t (&v)[GROUP] = r[g & 1];
-#pragma unroll
-            for (int j = 0; j < GROUP; j += 4) {
-              fma2(acc[(g * GROUP + j) / 2], (uint64_t)v[j] | (uint64_t)v[j + 1] << 32, mul2(x[j / 4].x, f2));
-              fma2(acc[(g * GROUP + j) / 2 + 1], (uint64_t)v[j + 2] | (uint64_t)v[j + 3] << 32, mul2(x[j / 4].y, f2));
+        for (int g = 0; g < GROUPS; g += 2) {                // (columns past the tile's tokens hold what nobody reads)
+          if (col_of(g) < nt) {
+            uint32_t r[GROUP], r1[GROUP];
+            tc_ld16(d + col_of(g), r);
+            if (g + 1 < GROUPS) {
+              tc_ld16(d + col_of(g + 1), r1);
+              wait_ld16(r1);
             }
+            wait_ld16(r);
+            take(g, r);
+            if (g + 1 < GROUPS) take(g + 1, r1);
           }
         }
         tc_fence_before();
@@ -436,7 +445,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         left = a.per_stretch;                                // a stretch ends
         if constexpr (CLUSTER) {
           // where the cluster reads it
-          float* red = reinterpret_cast<float*>(smem + S::RED_AT) + stretch * FEW_MAX * ROWS;
+          float* red = reinterpret_cast<float*>(smem + S::RED_AT) + stretch * FEW_TILE * ROWS;
 #pragma unroll
           for (int j = 0; j < S::COLS / 2; ++j) {
             red[(2 * j) * ROWS + row] = lo_of(acc[j]);
@@ -513,12 +522,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     // tokens: sixteen lanes a chunk of a token; the two warps take turns, and a chunk's numbers are asked for a turn early
     const int l = lane & 15, sub = lane >> 4, n_chunks = c_last - c_first;
     const int total = tile0 < a.tiles ? ((a.tiles - tile0 + tile_step - 1) / tile_step) * n_chunks : 0;
-    float4 next[FEW_MAX / 2];
+    float4 next[FEW_TILE / 2];
     auto ask = [&](int it) {
-      const int k = (c_first + it % n_chunks) * CK + l * 4;
+      const int k = (c_first + it % n_chunks) * CK + l * 4, m0 = (tile0 + it / n_chunks * tile_step) % a.tiles_m * FEW_TILE;
 #pragma unroll
-      for (int i = 0; i < FEW_MAX / 2; ++i) {
-        const int m = 2 * i + sub;
+      for (int i = 0; i < FEW_TILE / 2; ++i) {
+        const int m = m0 + 2 * i + sub;
         const float* src = a.A + (size_t)m * a.lda + k;
         next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (m < a.M) {
@@ -537,15 +546,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     if (warp - 2 < total) ask(warp - 2);
     for (int it = warp - 2; it < total && ok; it += 2) {
       const int xs = it % S::X_STAGES, slot = it % S::SLOTS;
-      float4 v[FEW_MAX / 2];
+      float4 v[FEW_TILE / 2];
 #pragma unroll
-      for (int i = 0; i < FEW_MAX / 2; ++i) v[i] = next[i];
+      for (int i = 0; i < FEW_TILE / 2; ++i) v[i] = next[i];
       if (it + 2 < total) ask(it + 2);
       ok = wait_done(it - S::X_STAGES, 5);
       if (!ok) break;
 #pragma unroll
-      for (int i = 0; i < FEW_MAX / 2; ++i) {
-        if (2 * i >= a.M) break;
+      for (int i = 0; i < FEW_TILE / 2; ++i) {
+        if (2 * i >= a.M) break;                             // (a later tile's missing tokens: zeros)
         const int m = 2 * i + sub;
         float top = fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));
 #pragma unroll
@@ -570,11 +579,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     cluster_sync();
     const int used = (a.chunks + a.per_stretch - 1) / a.per_stretch;
     const uint32_t red = smem_u32(smem + S::RED_AT);
-    for (int i = rank * S::THREADS + (int)threadIdx.x; i < a.M * ROWS; i += a.cluster * S::THREADS) {
-      const int m = i / ROWS, n = tile0 * ROWS + i % ROWS;
+    const int m0 = tile0 % a.tiles_m * FEW_TILE, n0 = tile0 / a.tiles_m * ROWS;
+    for (int i = rank * S::THREADS + (int)threadIdx.x; i < min(FEW_TILE, a.M - m0) * ROWS; i += a.cluster * S::THREADS) {
+      const int m = m0 + i / ROWS, n = n0 + i % ROWS;
       float parts[STRETCHES];
 #pragma unroll
-      for (int r = 0; r < STRETCHES; ++r) parts[r] = r < used ? ld_remote(red + 4u * (uint32_t)(r % mine * FEW_MAX * ROWS + i), r / mine) : 0.f;
+      for (int r = 0; r < STRETCHES; ++r) parts[r] = r < used ? ld_remote(red + 4u * (uint32_t)(r % mine * FEW_TILE * ROWS + i), r / mine) : 0.f;
       float v = parts[0];
 #pragma unroll
       for (int r = 1; r < STRETCHES; ++r)
@@ -703,11 +713,11 @@ extern "C" int gi_gemm_f32_split(float* out, int mode, const float* A, const flo
   }
   if (M <= FEW_MAX) {
     a.out = out; a.A = A;
-    a.M = M; a.nt = FEW_MAX; a.tiles_m = 1; a.tiles = tiles_n;
-    a.cluster = w_tma ? cluster_of<true>(tiles_n) : cluster_of<false>(tiles_n);
+    a.M = M; a.nt = FEW_TILE; a.tiles_m = (M + FEW_TILE - 1) / FEW_TILE; a.tiles = a.tiles_m * tiles_n;
+    a.cluster = w_tma ? cluster_of<true>(a.tiles) : cluster_of<false>(a.tiles);
     if (a.cluster > 1)
-      return w_tma ? launch_split<true, true, true>(mw, mh, ml, a, tiles_n * a.cluster, s) : launch_split<true, true, false>(mw, mh, ml, a, tiles_n * a.cluster, s);
-    const int blocks = tiles_n < sms ? tiles_n : sms;
+      return w_tma ? launch_split<true, true, true>(mw, mh, ml, a, a.tiles * a.cluster, s) : launch_split<true, true, false>(mw, mh, ml, a, a.tiles * a.cluster, s);
+    const int blocks = a.tiles < sms ? a.tiles : sms;
     return w_tma ? launch_split<true, false, true>(mw, mh, ml, a, blocks, s) : launch_split<true, false, false>(mw, mh, ml, a, blocks, s);
   }
   for (int m0 = 0; m0 < M; m0 += SLAB) {

@@ -229,6 +229,11 @@ class Engine:
         """The model over the tokens of `ctx`: embedding, the scheduled layers, then final norm and head on
         the wanted rows only (src/model.rs:1173-1188)."""
         from ..kernels import ops
+        with ops.one_token_step(ctx.is_decode):
+            return self._forward(ctx)
+
+    def _forward(self, ctx: StepContext) -> Optional[torch.Tensor]:
+        from ..kernels import ops
         model = self.model
         schedule, injection = model.spec.schedule, getattr(model, "injection", None)
         blocks_read = self._first_readers

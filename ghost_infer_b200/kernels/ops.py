@@ -8,6 +8,7 @@ the CPU and nothing falls back to library code.
 from __future__ import annotations
 
 import contextlib
+import contextvars
 import ctypes
 import os
 import weakref
@@ -510,10 +511,26 @@ def silu_mul(gate_up: torch.Tensor, out: Optional[torch.Tensor] = None, interlea
     return out
 
 
+_one_token = contextvars.ContextVar("one_token_step", default=False)
+
+
+@contextlib.contextmanager
+def one_token_step(on: bool):
+    """Around the products of a step that brings one token a sequence.  Such steps keep the plain 32-bit products, which are
+    bound by the bytes of the weights and faster there; all others, whatever their size, take the tensor cores' for larger
+    matrices.  (One-token rows and prompt rows differ by rounding anyway: their attention is summed in another order.)  Held
+    per thread."""
+    token = _one_token.set(bool(on))
+    try:
+        yield
+    finally:
+        _one_token.reset(token)
+
+
 def gemm_generic(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None,
                  out_dtype: Optional[torch.dtype] = None, accumulate: bool = False) -> torch.Tensor:
     """out[M, N] (+)= a[M, K] @ w[N, K]^T with 32-bit accumulation: in float32 the matrices of 1,024 rows and columns or more
-    on tensor cores (every number in two 16-bit parts), the rest on CUDA cores."""
+    on tensor cores (every number in two 16-bit parts; not within `one_token_step`), the rest on CUDA cores."""
     lib = _bind()
     _cuda(a, "activations")
     _cuda(w, "weights")
@@ -530,7 +547,7 @@ def gemm_generic(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor
     if out.shape != (m, n):
         raise KernelError(f"matrix product: output is {tuple(out.shape)}, wanted {(m, n)}")
     mode = GEMM_ACCUM_F32 if accumulate else GEMM_STORE
-    if a.dtype == w.dtype == out.dtype == torch.float32:
+    if a.dtype == w.dtype == out.dtype == torch.float32 and not _one_token.get():
         need = lib.gi_gemm_f32_split_scratch(m, n, k)
         if need >= 0:                        # a larger matrix: on the tensor cores, whatever the rows
             scratch = torch.empty((need,), dtype=torch.uint8, device=a.device) if need > 0 else None
@@ -829,11 +846,13 @@ def gemm_tc_tail_tiles(on: bool) -> None:
 
 
 def gemm_tc_status() -> int:
-    """0 if every wait inside the tensor-core product was met since the last call; synchronises the device."""
+    """0 if every wait inside the tensor-core products was met since the last call (the 32-bit one's codes: 16 and more);
+    synchronises the device."""
     lib = _bind()
     status = ctypes.c_int(0)
     _check(lib, lib.gi_gemm_tc_status(ctypes.byref(status)), 0)
-    return status.value
+    other = gemm_f32_split_status()
+    return status.value or (16 + other if other else 0)
 
 
 def gemm_f32_split_status() -> int:
@@ -850,7 +869,7 @@ def check_status() -> None:
     clears the kernels' status words; synchronises the device."""
     bad = []
     for name, fn in (("prompt product", gemm_tc_status), ("decode product", gemm_stream_status),
-                     ("prompt attention", attn_prefill_t5_status), ("32-bit product", gemm_f32_split_status)):
+                     ("prompt attention", attn_prefill_t5_status)):
         code = fn()
         if code:
             bad.append(f"{name} (wait {code})")

@@ -1138,7 +1138,7 @@ def test_float32_products_share_one_order_of_additions(m, n, k, accumulate):
     assert ((got.double() - exact).abs() <= bound).all()
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 1024, 1024), (2, 2048, 1091), (16, 1025, 1028), (17, 1100, 1151), (31, 3072, 1024), (129, 1152, 4160),
+@pytest.mark.parametrize("m,n,k", [(1, 1024, 1024), (2, 2048, 1091), (16, 1025, 1028), (17, 1100, 1151), (32, 3072, 1024), (33, 1024, 1088), (129, 1152, 4160),
                                    (3, 19000, 1088), (8200, 1024, 1024)])
 def test_float32_products_in_two_16_bit_parts(m, n, k):
     """The larger matrices' kernel: clusters and whole tiles, tokens split inside and before, ends of tiles, chunks and stretches.
