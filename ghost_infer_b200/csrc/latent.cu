@@ -478,73 +478,95 @@ bmm_heads_mma_kernel(__nv_bfloat16* __restrict__ out, long ldo, long ohs, const 
   }
 }
 
-// ---- the same for a step of few rows (one-token steps): bound by the bytes of the heads' matrices ------------------------
+// ---- the same for a step of few rows (one-token steps): bound by the trips to memory and the bytes of the heads' matrices -------
 // grid (column tiles of 16, heads); a block stages up to 8 rows' numbers for its head in shared memory and streams 16 rows of
 // the head's matrix past them, 16 bytes per lane per load, four columns in flight; a warp takes 4 columns, its lanes cut K
-// between them and their sums meet in a fixed order.  bfloat16, K a multiple of 8, rows on 16-byte boundaries.
+// between them and the 32 sums (4 columns, 8 rows) meet in a fixed order, halving what a lane holds at every exchange: 31
+// exchanges, and each lane ends with one sum (32 butterflies of five were 160, the longest part of the kernel).  The matrix is
+// asked for in L2 before the dependency wait (a prefetch reads no values: right whoever wrote it) and its first numbers are
+// loaded beside the rows'.  bfloat16, K a multiple of 8, rows on 16-byte boundaries.
 constexpr int GV_ROWS = 8, GV_COLS = 16;      // a warp takes 4 columns
+
+// One exchange among the lanes: of 2 * HALF sums a lane keeps the half that bit BIT of its number names.
+template <int HALF, int BIT>
+__device__ __forceinline__ void gv_halve(float (&v)[4 * GV_ROWS], int lane) {
+  const bool upper = (lane & BIT) != 0;
+#pragma unroll
+  for (int i = 0; i < HALF; ++i) {
+    const float send = upper ? v[i] : v[i + HALF], keep = upper ? v[i + HALF] : v[i];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, BIT);
+  }
+}
 
 __global__ void __launch_bounds__(128)
 bmm_heads_gemv_kernel(__nv_bfloat16* __restrict__ out, long ldo, long ohs, const __nv_bfloat16* A, long lda, long ahs,
-                      const __nv_bfloat16* __restrict__ W, long whs, long ldw, int M, int N, int K) {
+                      const __nv_bfloat16* W, long whs, long ldw, int M, int N, int K) {
   extern __shared__ __align__(16) unsigned char gv_smem[];
   __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(gv_smem);      // [GV_ROWS][K]
-  gi::pdl_prologue();
+  gi::pdl_launch_dependents();
   const int h = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const __nv_bfloat16* Ah = A + (size_t)h * ahs;
-  const __nv_bfloat16* Wh = W + (size_t)h * whs;
   const int n_base = blockIdx.x * GV_COLS + warp * 4;
+  const __nv_bfloat16* wp[4];
+#pragma unroll
+  for (int jj = 0; jj < 4; ++jj) wp[jj] = W + (size_t)h * whs + (size_t)min(n_base + jj, N - 1) * ldw;     // past the end: repeated, not stored
+  for (int k = lane * 8; k < K; k += 256)
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) asm volatile("prefetch.global.L2 [%0];" ::"l"(wp[jj] + k));
+  gi::pdl_wait();
   for (int r0 = 0; r0 < M; r0 += GV_ROWS) {
     const int rows = min(GV_ROWS, M - r0);
+    uint4 next[4] = {};
+    if (lane * 8 < K) {
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) next[jj] = *reinterpret_cast<const uint4*>(wp[jj] + lane * 8);
+    }
     __syncthreads();
     for (int idx = tid; idx < rows * (K / 8); idx += 128) {
       const int r = idx / (K / 8), ch = idx % (K / 8);
       *reinterpret_cast<uint4*>(As + (size_t)r * K + ch * 8) = *reinterpret_cast<const uint4*>(Ah + (size_t)(r0 + r) * lda + ch * 8);
     }
     __syncthreads();
-    for (int j0 = 0; j0 < 4; j0 += 4) {
-      if (n_base + j0 >= N) break;                      // the same for the whole warp
-      const __nv_bfloat16* wp[4];
+    if (n_base >= N) continue;                          // the same for the whole warp
+    float acc[4 * GV_ROWS];                             // [column][row]
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) wp[jj] = Wh + (size_t)min(n_base + j0 + jj, N - 1) * ldw;     // past the end: repeated, not stored
-      float acc[4][GV_ROWS];
+    for (int i = 0; i < 4 * GV_ROWS; ++i) acc[i] = 0.f;
+    for (int k = lane * 8; k < K; k += 256) {
+      uint4 wv[4];
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj)
+      for (int jj = 0; jj < 4; ++jj) wv[jj] = next[jj];
+      if (k + 256 < K) {
 #pragma unroll
-        for (int r = 0; r < GV_ROWS; ++r) acc[jj][r] = 0.f;
-      for (int k = lane * 8; k < K; k += 256) {
-        uint4 wv[4];
+        for (int jj = 0; jj < 4; ++jj) next[jj] = *reinterpret_cast<const uint4*>(wp[jj] + k + 256);
+      }
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) wv[jj] = *reinterpret_cast<const uint4*>(wp[jj] + k);
+      for (int r = 0; r < GV_ROWS; ++r) {
+        if (r < rows) {
+          const uint4 av = *reinterpret_cast<const uint4*>(As + (size_t)r * K + k);
+          const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
 #pragma unroll
-        for (int r = 0; r < GV_ROWS; ++r) {
-          if (r < rows) {
-            const uint4 av = *reinterpret_cast<const uint4*>(As + (size_t)r * K + k);
-            const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
+          for (int jj = 0; jj < 4; ++jj) {
+            const uint32_t ww[4] = {wv[jj].x, wv[jj].y, wv[jj].z, wv[jj].w};
+            float& sum = acc[jj * GV_ROWS + r];
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-              const uint32_t ww[4] = {wv[jj].x, wv[jj].y, wv[jj].z, wv[jj].w};
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                acc[jj][r] = fmaf(__uint_as_float(aw[i] << 16), __uint_as_float(ww[i] << 16), acc[jj][r]);
-                acc[jj][r] = fmaf(__uint_as_float(aw[i] & 0xffff0000u), __uint_as_float(ww[i] & 0xffff0000u), acc[jj][r]);
-              }
+            for (int i = 0; i < 4; ++i) {
+              sum = fmaf(__uint_as_float(aw[i] << 16), __uint_as_float(ww[i] << 16), sum);
+              sum = fmaf(__uint_as_float(aw[i] & 0xffff0000u), __uint_as_float(ww[i] & 0xffff0000u), sum);
             }
           }
         }
       }
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        const int n = n_base + j0 + jj;
-#pragma unroll
-        for (int r = 0; r < GV_ROWS; ++r) {
-          if (r >= rows) break;
-          const float v = gi::warp_sum(acc[jj][r]);
-          if (lane == 0 && n < N) out[(size_t)(r0 + r) * ldo + (size_t)h * ohs + n] = __float2bfloat16_rn(v);
-        }
-      }
     }
+    __syncwarp();                                       // (K below 256: lanes past its end had nothing to add)
+    gv_halve<16, 16>(acc, lane);
+    gv_halve<8, 8>(acc, lane);
+    gv_halve<4, 4>(acc, lane);
+    gv_halve<2, 2>(acc, lane);
+    gv_halve<1, 1>(acc, lane);
+    // lane l holds column l / 8, row l % 8
+    const int n = n_base + lane / GV_ROWS, r = lane % GV_ROWS;
+    if (r < rows && n < N) out[(size_t)(r0 + r) * ldo + (size_t)h * ohs + n] = __float2bfloat16_rn(acc[0]);
   }
 }
 
