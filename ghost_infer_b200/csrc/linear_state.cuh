@@ -47,15 +47,30 @@ __device__ __forceinline__ float ls_softplus(float v) { return v > 20.f ? v : lo
 
 // One halving step among a column's 8 lanes: of 2 * HALF values a lane keeps the half its bit `BIT` of the lane number
 // names and adds the other lane's partial sums of the same values.
-template <int HALF, int BIT>
-__device__ __forceinline__ void ls_halve(float (&v)[LS_TB], int lane) {
+template <int HALF, int BIT, int C>
+__device__ __forceinline__ void ls_halve(float (&v)[LS_TB * C], int lane) {
   const bool upper = (lane & BIT) != 0;
 #pragma unroll
-  for (int k = 0; k < HALF; ++k) {
-    const float send = upper ? v[k] : v[k + HALF];
-    const float keep = upper ? v[k + HALF] : v[k];
+  for (int k = 0; k < HALF * C; ++k) {
+    const float send = upper ? v[k] : v[k + HALF * C];
+    const float keep = upper ? v[k + HALF * C] : v[k];
     v[k] = keep + __shfl_xor_sync(0xffffffffu, send, BIT);
   }
+}
+
+// two products, two fused multiply-adds in one instruction; each half is rounded as the single one would be
+__device__ __forceinline__ uint64_t ls_pair(float a, float b) { return (uint64_t)__float_as_uint(a) | (uint64_t)__float_as_uint(b) << 32; }
+__device__ __forceinline__ float ls_lo(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float ls_hi(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ uint64_t ls_mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t ls_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
 
 // Sixteen bytes of a row as 32-bit numbers.
@@ -72,6 +87,8 @@ __device__ __forceinline__ void ls_load16(const __nv_bfloat16* p, float (&out)[8
     out[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
   }
 }
+// All of the block's threads, from wherever they are.
+__device__ __forceinline__ void ls_block_barrier() { asm volatile("bar.sync 0;" ::: "memory"); }
 // The preparing threads among themselves (barrier 1; the block's own barrier is 0).
 __device__ __forceinline__ void ls_prep_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(LS_PREP) : "memory"); }
 
@@ -99,17 +116,21 @@ template <int KR> struct LsChunk { static constexpr int value = KR >= 32 ? 8 : 1
 // WALK: the step holds sequences of many tokens, and eight whole tokens run without a test between them; without it (steps
 // of one token a sequence) the kernel is the same but smaller, so that two blocks fit an SM at every tile width.
 // Two blocks an SM for the narrower tiles too: a grid of about as many blocks as SMs times two then runs as one round.
-template <typename T, int KR, int COLS, bool DELTA, bool WALK, bool ROT, bool KEYED>
-__global__ void __launch_bounds__(COLS * LS_LANES + LS_PREP, (COLS <= 16 || !WALK) ? 2 : 1)
+// C: columns a thread holds.  A token's key and query (and decays) leave shared memory once per thread, sixteen bytes a lane, and
+// a walk with one column a thread spends about half its time on that (four wavefronts a load, eight loads a token and warp);
+// without the delta rule a thread therefore holds several columns, two numbers an instruction.
+template <typename T, int KR, int COLS, int C, bool DELTA, bool WALK, bool ROT, bool KEYED>
+__global__ void __launch_bounds__(COLS / C * LS_LANES + LS_PREP, (COLS <= 16 || !WALK || (C > 1 && KR < 32)) ? 2 : 1)
 linear_state_kernel(const LsArgs a) {
   constexpr int Kp = KR * LS_LANES;            // rows with padding
   constexpr int M = KR / 4;                    // groups of four rows per lane; also a preparing lane's share of a row
-  constexpr int NC = COLS * LS_LANES;          // threads that hold S
+  constexpr int NC = COLS / C * LS_LANES;      // threads that hold S
   constexpr int CH = LsChunk<KR>::value;
   constexpr int BUF = 2 * CH * Kp + 2 * CH * COLS + 2 * CH + (KEYED ? CH * Kp : 0);     // the decays come last
   constexpr int KEYS_AT = 2 * CH * Kp + 2 * CH * COLS + 2 * CH;
   static_assert(KEYS_AT % 4 == 0, "the decays start on a 16-byte boundary");
   constexpr int VW = 16 / (int)sizeof(T);      // numbers of a row in sixteen bytes
+  static_assert(COLS % C == 0 && (C == 1 || !DELTA), "whole threads; the delta rule's column is one thread's");
   static_assert(CH % LS_TB == 0 && CH <= LS_PREP && (CH * Kp) % LS_PREP == 0 && COLS % VW == 0 && CH * COLS / VW <= LS_PREP,
                 "whole exchanges; a preparing thread per token, and per group of a chunk's values");
   extern __shared__ __align__(16) float sm[];
@@ -130,34 +151,37 @@ linear_state_kernel(const LsArgs a) {
   const float dc = a.decay_c != nullptr ? a.decay_c[h] : 1.0f;
   const float rate = ap != nullptr ? expf(dc) : 0.f, bias = (ap != nullptr && a.dt_bias != nullptr) ? a.dt_bias[h] : 0.f;
 
-  // a chunk's tokens made ready in buffer `buf` by the 128 preparing threads together.  First every thread loads its share
-  // of the chunk's rows (sixteen bytes at a time where the rows allow it), all loads before anything is computed from them,
-  // so a chunk costs one trip to memory; silu is applied on the way into shared memory.  Then, for unit vectors, one warp
-  // per token sums the squares of its row in shared memory and scales it in place.
-  auto prepare = [&](int c, float* buf) {
-    float* sq = buf; float* sk = sq + CH * Kp; float* sv = sk + CH * Kp; float* sg = sv + CH * COLS; float* sb = sg + CH;
+  // A chunk's tokens are made ready by the 128 preparing threads together, in two parts.  `fetch`: every thread loads its share
+  // of the chunk's rows into registers (sixteen bytes at a time where the rows allow it), a chunk before they are wanted, so
+  // that the trip to memory passes while the chunk before is walked.  `put`: silu on the way into shared memory; then the
+  // turns, and for unit vectors one warp per token sums the squares of its row in shared memory and scales it in place.
+  const bool act = a.in_act != 0;
+  constexpr int RG = (CH * Kp / 2 + LS_PREP - 1) / LS_PREP;          // pairs a thread turns, per operand
+  constexpr int DG = KEYED ? (CH * Kp / 4 + LS_PREP - 1) / LS_PREP : 1;
+  constexpr int QG = (CH * Kp / VW + LS_PREP - 1) / LS_PREP;         // groups of VW numbers a thread moves, per operand
+  constexpr int QS = CH * Kp / LS_PREP, VS = (CH * COLS + LS_PREP - 1) / LS_PREP;
+  constexpr int QN = QG * VW > QS ? QG * VW : QS, VN = VW > VS ? VW : VS;
+  float av, bv, qr[QN], kr[QN], vr[VN];
+  float2 cs[ROT ? RG : 1];
+  float4 dr[DG];                                                     // per-key decays
+  const int pt = tid - NC;
+  const int vpr = COLS / VW, vt = pt / vpr, vc = (pt - vt * vpr) * VW;      // at most CH * COLS / VW <= 128 groups
+  auto fetch = [&](int c) {
     const int n = min(CH, qlen - c * CH);
-    const int pt = tid - NC;
     const size_t tokc = (size_t)tok0 + (size_t)c * CH;
-    const bool act = a.in_act != 0;
     // decay and write strength: one thread per token
-    float av = 0.f, bv = 0.f;
+    av = bv = 0.f;
     if (pt < n) {
       if (ap != nullptr) av = gi::ldf(ap + (tokc + pt) * a.lda + h);
       if (bp != nullptr) bv = gi::ldf(bp + (tokc + pt) * a.ldb + h);
     }
-    constexpr int RG = (CH * Kp / 2 + LS_PREP - 1) / LS_PREP;        // pairs a thread turns, per operand
-    float2 cs[ROT ? RG : 1];
     if (ROT) {
 #pragma unroll
       for (int i = 0; i < RG; ++i) {
         const int g = pt + i * LS_PREP;
-        cs[i] = g < n * a.half ? a.table[(tokc + g / a.half) * a.half + g % a.half] : make_float2(1.f, 0.f);
+        cs[i] = g < n * a.half ? a.table[tokc * a.half + g] : make_float2(1.f, 0.f);
       }
     }
-    // per-key decays: loaded with the rows, stored with them (sixteen bytes a thread where K allows it)
-    constexpr int DG = KEYED ? (CH * Kp / 4 + LS_PREP - 1) / LS_PREP : 1;
-    float4 dr[DG];
     if (KEYED) {
       const int gpr = (K + 3) / 4, total = n * gpr;
       const size_t ldg = (size_t)a.heads * K;
@@ -179,52 +203,20 @@ linear_state_kernel(const LsArgs a) {
         }
       }
     }
-    const float qs = KEYED ? a.q_scale : 1.0f;
     if (a.vec_in) {
-      constexpr int QG = (CH * Kp / VW + LS_PREP - 1) / LS_PREP;     // groups of VW numbers a thread moves, per operand
       const int gpr = K / VW, total = n * gpr;
-      float qr[QG][VW], kr[QG][VW];
 #pragma unroll
       for (int i = 0; i < QG; ++i) {
         const int g = pt + i * LS_PREP;
         if (g < total) {
           const int t = g / gpr, r0 = (g - t * gpr) * VW;
-          ls_load16(qp + (tokc + t) * a.ldq + (size_t)hk * K + r0, qr[i]);
-          ls_load16(kp + (tokc + t) * a.ldk + (size_t)hk * K + r0, kr[i]);
+          ls_load16(qp + (tokc + t) * a.ldq + (size_t)hk * K + r0, *reinterpret_cast<float (*)[VW]>(qr + i * VW));
+          ls_load16(kp + (tokc + t) * a.ldk + (size_t)hk * K + r0, *reinterpret_cast<float (*)[VW]>(kr + i * VW));
         }
       }
-      float vr[VW];
-      const int vpr = COLS / VW, vt = pt / vpr, vc = (pt - vt * vpr) * VW;     // at most CH * COLS / VW <= 128 groups
-      const bool vlive = vt < n && j0 + vc < V;
-      if (vlive) ls_load16(vp + (tokc + vt) * a.ldv + (size_t)h * V + j0 + vc, vr);
-#pragma unroll
-      for (int i = 0; i < QG; ++i) {
-        const int g = pt + i * LS_PREP;
-        if (g < total) {
-          const int t = g / gpr, r0 = (g - t * gpr) * VW;
-#pragma unroll
-          for (int e = 0; e < VW; e += 4) {
-            float4 q4 = make_float4(qr[i][e], qr[i][e + 1], qr[i][e + 2], qr[i][e + 3]);
-            float4 k4 = make_float4(kr[i][e], kr[i][e + 1], kr[i][e + 2], kr[i][e + 3]);
-            if (act) {
-              q4.x = ls_silu(q4.x); q4.y = ls_silu(q4.y); q4.z = ls_silu(q4.z); q4.w = ls_silu(q4.w);
-              k4.x = ls_silu(k4.x); k4.y = ls_silu(k4.y); k4.z = ls_silu(k4.z); k4.w = ls_silu(k4.w);
-            }
-            if (ROT) { k4.x *= a.k_scale; k4.y *= a.k_scale; k4.z *= a.k_scale; k4.w *= a.k_scale; }
-            if (KEYED) { q4.x *= qs; q4.y *= qs; q4.z *= qs; q4.w *= qs; }
-            *reinterpret_cast<float4*>(sq + t * Kp + r0 + e) = q4;
-            *reinterpret_cast<float4*>(sk + t * Kp + r0 + e) = k4;
-          }
-        }
-      }
-      if (vlive) {
-#pragma unroll
-        for (int e = 0; e < VW; ++e) sv[vt * COLS + vc + e] = act ? ls_silu(vr[e]) : vr[e];     // V is a multiple of VW here
-      }
+      if (vt < n && j0 + vc < V) ls_load16(vp + (tokc + vt) * a.ldv + (size_t)h * V + j0 + vc, *reinterpret_cast<float (*)[VW]>(vr));
     } else {
-      constexpr int QS = CH * Kp / LS_PREP, VS = (CH * COLS + LS_PREP - 1) / LS_PREP;
       const int total = n * K;
-      float qr[QS], kr[QS], vr[VS];
 #pragma unroll
       for (int i = 0; i < QS; ++i) {
         const int e = pt + i * LS_PREP;
@@ -239,6 +231,41 @@ linear_state_kernel(const LsArgs a) {
         const int e = pt + i * LS_PREP, t = e / COLS, cc = e % COLS;
         vr[i] = (t < n && j0 + cc < V) ? gi::ldf(vp + (tokc + t) * a.ldv + (size_t)h * V + j0 + cc) : 0.f;
       }
+    }
+  };
+  auto put = [&](int c, float* buf) {
+    float* sq = buf; float* sk = sq + CH * Kp; float* sv = sk + CH * Kp; float* sg = sv + CH * COLS; float* sb = sg + CH;
+    const int n = min(CH, qlen - c * CH);
+    const size_t tokc = (size_t)tok0 + (size_t)c * CH;
+    const float qs = KEYED ? a.q_scale : 1.0f;
+    if (a.vec_in) {
+      const int gpr = K / VW, total = n * gpr;
+#pragma unroll
+      for (int i = 0; i < QG; ++i) {
+        const int g = pt + i * LS_PREP;
+        if (g < total) {
+          const int t = g / gpr, r0 = (g - t * gpr) * VW;
+#pragma unroll
+          for (int e = 0; e < VW; e += 4) {
+            float4 q4 = make_float4(qr[i * VW + e], qr[i * VW + e + 1], qr[i * VW + e + 2], qr[i * VW + e + 3]);
+            float4 k4 = make_float4(kr[i * VW + e], kr[i * VW + e + 1], kr[i * VW + e + 2], kr[i * VW + e + 3]);
+            if (act) {
+              q4.x = ls_silu(q4.x); q4.y = ls_silu(q4.y); q4.z = ls_silu(q4.z); q4.w = ls_silu(q4.w);
+              k4.x = ls_silu(k4.x); k4.y = ls_silu(k4.y); k4.z = ls_silu(k4.z); k4.w = ls_silu(k4.w);
+            }
+            if (ROT) { k4.x *= a.k_scale; k4.y *= a.k_scale; k4.z *= a.k_scale; k4.w *= a.k_scale; }
+            if (KEYED) { q4.x *= qs; q4.y *= qs; q4.z *= qs; q4.w *= qs; }
+            *reinterpret_cast<float4*>(sq + t * Kp + r0 + e) = q4;
+            *reinterpret_cast<float4*>(sk + t * Kp + r0 + e) = k4;
+          }
+        }
+      }
+      if (vt < n && j0 + vc < V) {
+#pragma unroll
+        for (int e = 0; e < VW; ++e) sv[vt * COLS + vc + e] = act ? ls_silu(vr[e]) : vr[e];     // V is a multiple of VW here
+      }
+    } else {
+      const int total = n * K;
 #pragma unroll
       for (int i = 0; i < QS; ++i) {
         const int e = pt + i * LS_PREP;
@@ -322,9 +349,8 @@ linear_state_kernel(const LsArgs a) {
     }
   };
 
-  const int col = tid / LS_LANES, lane = tid % LS_LANES;    // of the threads that hold S
-  const int j = j0 + col;
-  float S[KR];
+  const int col = tid / LS_LANES * C, lane = tid % LS_LANES;    // of the threads that hold S: the first of their columns
+  uint64_t S[C][KR / 2];                                        // two rows side by side
   if (prep) {
     if (K < Kp) {                  // rows past K stay zero in both buffers: nothing writes them again
       for (int e = tid - NC; e < 2 * CH * Kp; e += LS_PREP) {
@@ -337,111 +363,246 @@ linear_state_kernel(const LsArgs a) {
       }
       ls_prep_barrier();
     }
-    prepare(0, sm);
+    fetch(0);
+    put(0, sm);
+    if (n_chunks > 1) fetch(1);
+    // (the two kinds of threads have loops of their own, which keeps either's registers out of the other's)
+    for (int c = 0; c < n_chunks; ++c) {
+      ls_block_barrier();
+      if (c > 0) write_out(c - 1, sm + ((c - 1) & 1) * BUF, NC, LS_PREP);
+      if (c + 1 < n_chunks) put(c + 1, sm + ((c + 1) & 1) * BUF);
+      if (c + 2 < n_chunks) fetch(c + 2);
+    }
   } else {
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const int i = 4 * (lane + LS_LANES * m);
-      if (a.vec_state && j < V && i < K) {
-        const float4 s4 = *reinterpret_cast<const float4*>(S_row + (size_t)j * K + i);
-        S[4 * m] = s4.x; S[4 * m + 1] = s4.y; S[4 * m + 2] = s4.z; S[4 * m + 3] = s4.w;
-      } else {
+    for (int cc = 0; cc < C; ++cc)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[4 * m + e] = (j < V && i + e < K) ? S_row[(size_t)j * K + i + e] : 0.f;
+      for (int m = 0; m < M; ++m) {
+        const int i = 4 * (lane + LS_LANES * m), j = j0 + col + cc;
+        float s4[4] = {0.f, 0.f, 0.f, 0.f};
+        if (a.vec_state && j < V && i < K) {
+          const float4 v = *reinterpret_cast<const float4*>(S_row + (size_t)j * K + i);
+          s4[0] = v.x; s4[1] = v.y; s4[2] = v.z; s4[3] = v.w;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s4[e] = (j < V && i + e < K) ? S_row[(size_t)j * K + i + e] : 0.f;
+        }
+        S[cc][2 * m] = ls_pair(s4[0], s4[1]);
+        S[cc][2 * m + 1] = ls_pair(s4[2], s4[3]);
       }
-    }
-  }
   for (int c = 0; c < n_chunks; ++c) {
-    __syncthreads();             // chunk c is ready in buffer c & 1; the other buffer's tokens and this one's read-outs are used up
+    ls_block_barrier();          // chunk c is ready in buffer c & 1; the other buffer's tokens and this one's read-outs are used up
     float* buf = sm + (c & 1) * BUF;
-    if (prep) {
-      if (c > 0) write_out(c - 1, sm + ((c - 1) & 1) * BUF, NC, LS_PREP);
-      if (c + 1 < n_chunks) prepare(c + 1, sm + ((c + 1) & 1) * BUF);
-      continue;
-    }
     const float* sq = buf; const float* sk = sq + CH * Kp; const float* sv = sk + CH * Kp;
     const float* sg = sv + CH * COLS; const float* sb = sg + CH;
     float* so = buf + 2 * CH * Kp + CH * COLS + 2 * CH;
     const int n = min(CH, qlen - c * CH);
-    // one token: the state's columns walk on, `out` takes this lane's share of the read-out
-    auto token = [&](int t, float& out) {
+    // one token: the state's columns walk on, `out` takes this lane's share of the read-outs
+    auto token = [&](int t, float* out) {
       const float g = KEYED ? 1.0f : sg[t];
-      float kk[KR], qq[KR];
       const float* sd = buf + KEYS_AT;
+      ulonglong2 kk[M], qq[M];
 #pragma unroll
       for (int m = 0; m < M; ++m) {
-        const float4 k4 = *reinterpret_cast<const float4*>(sk + t * Kp + 4 * (lane + LS_LANES * m));
-        const float4 q4 = *reinterpret_cast<const float4*>(sq + t * Kp + 4 * (lane + LS_LANES * m));
-        kk[4 * m] = k4.x; kk[4 * m + 1] = k4.y; kk[4 * m + 2] = k4.z; kk[4 * m + 3] = k4.w;
-        qq[4 * m] = q4.x; qq[4 * m + 1] = q4.y; qq[4 * m + 2] = q4.z; qq[4 * m + 3] = q4.w;
+        kk[m] = *reinterpret_cast<const ulonglong2*>(sk + t * Kp + 4 * (lane + LS_LANES * m));
+        qq[m] = *reinterpret_cast<const ulonglong2*>(sq + t * Kp + 4 * (lane + LS_LANES * m));
       }
-      float u = sv[t * COLS + col];
+      float u[C];
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc) u[cc] = sv[t * COLS + col + cc];
       if (DELTA) {
-        float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;     // four chains, then a tree: the order is fixed by K alone
+        uint64_t d01 = 0, d23 = 0;                        // four chains, then a tree: the order is fixed by K alone
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-          d0 = fmaf(S[4 * m], kk[4 * m], d0);
-          d1 = fmaf(S[4 * m + 1], kk[4 * m + 1], d1);
-          d2 = fmaf(S[4 * m + 2], kk[4 * m + 2], d2);
-          d3 = fmaf(S[4 * m + 3], kk[4 * m + 3], d3);
+          d01 = ls_fma2(S[0][2 * m], kk[m].x, d01);
+          d23 = ls_fma2(S[0][2 * m + 1], kk[m].y, d23);
         }
-        float d = (d0 + d1) + (d2 + d3);
+        float d = (ls_lo(d01) + ls_hi(d01)) + (ls_lo(d23) + ls_hi(d23));
         d += __shfl_xor_sync(0xffffffffu, d, 1);
         d += __shfl_xor_sync(0xffffffffu, d, 2);
         d += __shfl_xor_sync(0xffffffffu, d, 4);
-        u = sb[t] * (u - g * d);
+        u[0] = sb[t] * (u[0] - g * d);
       } else if (a.u_direct != nullptr) {
-        u *= sb[t];
+#pragma unroll
+        for (int cc = 0; cc < C; ++cc) u[cc] *= sb[t];
       }
-      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+      uint64_t a01[C], a23[C];
+      const uint64_t g2 = ls_pair(g, g);
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc) a01[cc] = a23[cc] = 0;
 #pragma unroll
       for (int m = 0; m < M; ++m) {
-        if (KEYED) {
-          const float4 d4 = *reinterpret_cast<const float4*>(sd + t * Kp + 4 * (lane + LS_LANES * m));
-          S[4 * m] *= d4.x; S[4 * m + 1] *= d4.y; S[4 * m + 2] *= d4.z; S[4 * m + 3] *= d4.w;
+        ulonglong2 d2;
+        if (KEYED) d2 = *reinterpret_cast<const ulonglong2*>(sd + t * Kp + 4 * (lane + LS_LANES * m));
+        else d2.x = d2.y = g2;
+#pragma unroll
+        for (int cc = 0; cc < C; ++cc) {
+          const uint64_t u2 = ls_pair(u[cc], u[cc]);
+          uint64_t &lo = S[cc][2 * m], &hi = S[cc][2 * m + 1];
+          lo = ls_fma2(kk[m].x, u2, ls_mul2(d2.x, lo));
+          hi = ls_fma2(kk[m].y, u2, ls_mul2(d2.y, hi));
+          a01[cc] = ls_fma2(lo, qq[m].x, a01[cc]);
+          a23[cc] = ls_fma2(hi, qq[m].y, a23[cc]);
         }
-        S[4 * m] = fmaf(kk[4 * m], u, g * S[4 * m]);
-        S[4 * m + 1] = fmaf(kk[4 * m + 1], u, g * S[4 * m + 1]);
-        S[4 * m + 2] = fmaf(kk[4 * m + 2], u, g * S[4 * m + 2]);
-        S[4 * m + 3] = fmaf(kk[4 * m + 3], u, g * S[4 * m + 3]);
-        a0 = fmaf(S[4 * m], qq[4 * m], a0);
-        a1 = fmaf(S[4 * m + 1], qq[4 * m + 1], a1);
-        a2 = fmaf(S[4 * m + 2], qq[4 * m + 2], a2);
-        a3 = fmaf(S[4 * m + 3], qq[4 * m + 3], a3);
       }
-      out = (a0 + a1) + (a2 + a3);
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc) out[cc] = (ls_lo(a01[cc]) + ls_hi(a01[cc])) + (ls_lo(a23[cc]) + ls_hi(a23[cc]));
     };
     for (int t0 = 0; t0 < n; t0 += LS_TB) {
-      float acc[LS_TB];
+      float acc[LS_TB * C];                              // [token][column]
       if (WALK && t0 + LS_TB <= n) {     // eight whole tokens: nothing to test between them, so the next one's loads start early
 #pragma unroll
-        for (int tl = 0; tl < LS_TB; ++tl) token(t0 + tl, acc[tl]);
+        for (int tl = 0; tl < LS_TB; ++tl) token(t0 + tl, acc + tl * C);
       } else {
 #pragma unroll
         for (int tl = 0; tl < LS_TB; ++tl) {
-          acc[tl] = 0.f;
-          if (t0 + tl < n) token(t0 + tl, acc[tl]);      // the same for the whole block
+#pragma unroll
+          for (int cc = 0; cc < C; ++cc) acc[tl * C + cc] = 0.f;
+          if (t0 + tl < n) token(t0 + tl, acc + tl * C);      // the same for the whole block
         }
       }
-      ls_halve<4, 4>(acc, lane);
-      ls_halve<2, 2>(acc, lane);
-      ls_halve<1, 1>(acc, lane);
+      ls_halve<4, 4, C>(acc, lane);
+      ls_halve<2, 2, C>(acc, lane);
+      ls_halve<1, 1, C>(acc, lane);
       // lane l of a column now holds token t0 + l
-      if (t0 + lane < n) so[(t0 + lane) * COLS + col] = acc[0];
+      if (t0 + lane < n) {
+#pragma unroll
+        for (int cc = 0; cc < C; ++cc) so[(t0 + lane) * COLS + col + cc] = acc[cc];
+      }
     }
+  }
   }
   __syncthreads();
   write_out(n_chunks - 1, sm + ((n_chunks - 1) & 1) * BUF, 0, NC + LS_PREP);
-  if (!prep && j < V) {
+  if (!prep) {
+#pragma unroll
+    for (int cc = 0; cc < C; ++cc)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int i = 4 * (lane + LS_LANES * m), j = j0 + col + cc;
+        const float s4[4] = {ls_lo(S[cc][2 * m]), ls_hi(S[cc][2 * m]), ls_lo(S[cc][2 * m + 1]), ls_hi(S[cc][2 * m + 1])};
+        if (j >= V) continue;
+        if (a.vec_state && i < K) {
+          *reinterpret_cast<float4*>(S_row + (size_t)j * K + i) = make_float4(s4[0], s4[1], s4[2], s4[3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (i + e < K) S_row[(size_t)j * K + i + e] = s4[e];
+        }
+      }
+  }
+}
+
+// The same walk for a step of about one token a sequence, without the delta rule, unit vectors or ready-made gates: bound by the
+// bytes of S and the trips to memory, of which the kernel above makes three one after the other (rows, the barrier behind their
+// preparation, S beside it) with a third of its threads waiting.  Here the threads that hold S prepare the token themselves;
+// S is asked for in L2 before the dependency wait (a prefetch reads no values) and loaded beside the rows.  64 registers and
+// 256 threads: four blocks an SM, where the other has two.  Every sum has the other's order, so the bits are the same.
+template <typename T, int KR, int COLS, bool ROT, bool KEYED>
+__global__ void __launch_bounds__(COLS * LS_LANES, 1024 / (COLS * LS_LANES))
+linear_state_step_kernel(const __grid_constant__ LsArgs a) {
+  constexpr int Kp = KR * LS_LANES, M = KR / 4, NC = COLS * LS_LANES;
+  __shared__ __align__(16) float sq[Kp], sk[Kp], sd[KEYED ? Kp : 1], sv[COLS];
+  const int h = blockIdx.x, b = blockIdx.y, j0 = blockIdx.z * COLS, tid = threadIdx.x;
+  const int K = a.K, V = a.V;
+  const int col = tid / LS_LANES, lane = tid % LS_LANES, j = j0 + col;
+  gi::pdl_launch_dependents();
+  const int slot = gi::ld_step(a.seq_slots + b);
+  float* S_col = a.state + (size_t)(slot >= 0 ? slot : a.state_rows - 1) * a.state_ld + ((size_t)h * V + j) * K;
+  if (j < V) {
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int i = 4 * (lane + LS_LANES * m);
+      if (i < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(S_col + i));
+    }
+  }
+  gi::pdl_wait();
+  const int tok0 = a.cu_seqlens[b], qlen = a.cu_seqlens[b + 1] - tok0;
+  if (qlen <= 0) return;
+  const float dc = KEYED ? 1.0f : a.decay_c[h];
+  const int hk = h / (a.heads / a.qk_heads);
+  float S[KR];
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const int i = 4 * (lane + LS_LANES * m);
+    float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (j < V && i < K) {
+      if (a.vec_state) {
+        s4 = *reinterpret_cast<const float4*>(S_col + i);
+      } else {
+        s4.x = S_col[i];
+        if (i + 1 < K) s4.y = S_col[i + 1];
+        if (i + 2 < K) s4.z = S_col[i + 2];
+        if (i + 3 < K) s4.w = S_col[i + 3];
+      }
+    }
+    S[4 * m] = s4.x; S[4 * m + 1] = s4.y; S[4 * m + 2] = s4.z; S[4 * m + 3] = s4.w;
+  }
+  const bool act = a.in_act != 0;
+  const float qs = KEYED ? a.q_scale : 1.0f, ks = ROT ? a.k_scale : 1.0f;
+  for (int t = 0; t < qlen; ++t) {
+    const size_t tok = (size_t)tok0 + t;
+    const T *q = (const T*)a.q + tok * a.ldq + (size_t)hk * K, *k = (const T*)a.k + tok * a.ldk + (size_t)hk * K;
+    if (t > 0) __syncthreads();                        // the token before is used up
+    // a pair that turns is loaded, turned and stored by one thread; the numbers past the pairs one a thread
+    auto query = [&](int i) { const float v = gi::ldf(q + i); return (act ? ls_silu(v) : v) * qs; };
+    auto key = [&](int i) { const float v = gi::ldf(k + i); return (act ? ls_silu(v) : v) * ks; };
+    const int half = ROT ? a.half : 0;
+    for (int i = tid; i < Kp - half; i += NC) {
+      if (i < half) {
+        const int ia = a.adjacent ? 2 * i : i, ib = a.adjacent ? ia + 1 : ia + half;
+        const float2 cs = a.table[tok * half + i];
+        const float qa = query(ia), qb = query(ib), ka = key(ia), kb = key(ib);
+        gi::rotate_pair(qa, qb, cs, &sq[ia], &sq[ib]);
+        gi::rotate_pair(ka, kb, cs, &sk[ia], &sk[ib]);
+      } else {
+        const int at = i + half;
+        sq[at] = at < K ? query(at) : 0.f;
+        sk[at] = at < K ? key(at) : 0.f;
+      }
+    }
+    if (KEYED)
+      for (int i = tid; i < Kp; i += NC) sd[i] = i < K ? a.g_key[tok * (size_t)a.heads * K + (size_t)h * K + i] : 0.f;
+    if (tid < COLS && j0 + tid < V) {
+      const float v = gi::ldf((const T*)a.v + tok * a.ldv + (size_t)h * V + j0 + tid);
+      sv[tid] = act ? ls_silu(v) : v;
+    }
+    __syncthreads();
+    const float u = j < V ? sv[col] : 0.f;
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int i = 4 * (lane + LS_LANES * m);
+      const float4 k4 = *reinterpret_cast<const float4*>(sk + i), q4 = *reinterpret_cast<const float4*>(sq + i);
+      if (KEYED) {
+        const float4 d4 = *reinterpret_cast<const float4*>(sd + i);
+        S[4 * m] *= d4.x; S[4 * m + 1] *= d4.y; S[4 * m + 2] *= d4.z; S[4 * m + 3] *= d4.w;
+      }
+      S[4 * m] = fmaf(k4.x, u, dc * S[4 * m]);
+      S[4 * m + 1] = fmaf(k4.y, u, dc * S[4 * m + 1]);
+      S[4 * m + 2] = fmaf(k4.z, u, dc * S[4 * m + 2]);
+      S[4 * m + 3] = fmaf(k4.w, u, dc * S[4 * m + 3]);
+      a0 = fmaf(S[4 * m], q4.x, a0);
+      a1 = fmaf(S[4 * m + 1], q4.y, a1);
+      a2 = fmaf(S[4 * m + 2], q4.z, a2);
+      a3 = fmaf(S[4 * m + 3], q4.w, a3);
+    }
+    float o = (a0 + a1) + (a2 + a3);
+    o += __shfl_xor_sync(0xffffffffu, o, 4);
+    o += __shfl_xor_sync(0xffffffffu, o, 2);
+    o += __shfl_xor_sync(0xffffffffu, o, 1);
+    if (lane == 0 && j < V) a.o[tok * (size_t)a.heads * V + (size_t)h * V + j] = o;
+  }
+  if (j < V) {
 #pragma unroll
     for (int m = 0; m < M; ++m) {
       const int i = 4 * (lane + LS_LANES * m);
       if (a.vec_state && i < K) {
-        *reinterpret_cast<float4*>(S_row + (size_t)j * K + i) = make_float4(S[4 * m], S[4 * m + 1], S[4 * m + 2], S[4 * m + 3]);
+        *reinterpret_cast<float4*>(S_col + i) = make_float4(S[4 * m], S[4 * m + 1], S[4 * m + 2], S[4 * m + 3]);
       } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (i + e < K) S_row[(size_t)j * K + i + e] = S[4 * m + e];
+          if (i + e < K) S_col[i + e] = S[4 * m + e];
       }
     }
   }
@@ -458,10 +619,12 @@ int ls_sm_count() {
 template <typename T, int KR, int COLS, bool ROT, bool KEYED>
 cudaError_t ls_launch(const LsArgs& a, int n_seqs, bool delta, bool walk, cudaStream_t stream) {
   constexpr int CH = LsChunk<KR>::value;
+  // columns a thread: wide tiles come with many blocks, narrow ones with few, whose warps' own length counts more
+  constexpr int C = KR < 32 && COLS >= 32 ? 4 : 2;
   const size_t smem = 2 * (size_t)((KEYED ? 3 : 2) * CH * KR * LS_LANES + 2 * CH * COLS + 2 * CH) * sizeof(float);
-  const dim3 grid(a.heads, n_seqs, (a.V + COLS - 1) / COLS), block(COLS * LS_LANES + LS_PREP);
+  const dim3 grid(a.heads, n_seqs, (a.V + COLS - 1) / COLS), block((delta ? COLS : COLS / C) * LS_LANES + LS_PREP);
   if constexpr (KEYED) {
-    auto kern = walk ? linear_state_kernel<T, KR, COLS, false, true, false, true> : linear_state_kernel<T, KR, COLS, false, false, false, true>;
+    auto kern = walk ? linear_state_kernel<T, KR, COLS, C, false, true, false, true> : linear_state_kernel<T, KR, COLS, C, false, false, false, true>;
     if (smem > 48 * 1024) {
       static bool configured[2][gi::MAX_DEVICES_SEEN] = {};
       int dev;
@@ -473,19 +636,31 @@ cudaError_t ls_launch(const LsArgs& a, int n_seqs, bool delta, bool walk, cudaSt
     }
     return gi::launch(kern, grid, block, smem, stream, a);
   } else if constexpr (ROT) {
-    return walk ? gi::launch(linear_state_kernel<T, KR, COLS, false, true, true, false>, grid, block, smem, stream, a)
-                : gi::launch(linear_state_kernel<T, KR, COLS, false, false, true, false>, grid, block, smem, stream, a);
+    return walk ? gi::launch(linear_state_kernel<T, KR, COLS, C, false, true, true, false>, grid, block, smem, stream, a)
+                : gi::launch(linear_state_kernel<T, KR, COLS, C, false, false, true, false>, grid, block, smem, stream, a);
   } else {
     if (walk)
-      return delta ? gi::launch(linear_state_kernel<T, KR, COLS, true, true, false, false>, grid, block, smem, stream, a)
-                   : gi::launch(linear_state_kernel<T, KR, COLS, false, true, false, false>, grid, block, smem, stream, a);
-    return delta ? gi::launch(linear_state_kernel<T, KR, COLS, true, false, false, false>, grid, block, smem, stream, a)
-                 : gi::launch(linear_state_kernel<T, KR, COLS, false, false, false, false>, grid, block, smem, stream, a);
+      return delta ? gi::launch(linear_state_kernel<T, KR, COLS, 1, true, true, false, false>, grid, block, smem, stream, a)
+                   : gi::launch(linear_state_kernel<T, KR, COLS, C, false, true, false, false>, grid, block, smem, stream, a);
+    return delta ? gi::launch(linear_state_kernel<T, KR, COLS, 1, true, false, false, false>, grid, block, smem, stream, a)
+                 : gi::launch(linear_state_kernel<T, KR, COLS, C, false, false, false, false>, grid, block, smem, stream, a);
   }
 }
 
 template <typename T, int KR, bool ROT, bool KEYED>
+cudaError_t ls_launch_step(const LsArgs& a, int n_seqs, cudaStream_t stream) {
+  const long per = (long)a.heads * n_seqs, sms = ls_sm_count();
+  const auto grid = [&](int cols) { return dim3(a.heads, n_seqs, (a.V + cols - 1) / cols); };
+  if (per * ((a.V + 31) / 32) >= sms || a.V <= 8) return gi::launch(linear_state_step_kernel<T, KR, 32, ROT, KEYED>, grid(32), dim3(32 * LS_LANES), 0, stream, a);
+  if (per * ((a.V + 15) / 16) >= sms) return gi::launch(linear_state_step_kernel<T, KR, 16, ROT, KEYED>, grid(16), dim3(16 * LS_LANES), 0, stream, a);
+  return gi::launch(linear_state_step_kernel<T, KR, 8, ROT, KEYED>, grid(8), dim3(8 * LS_LANES), 0, stream, a);
+}
+
+template <typename T, int KR, bool ROT, bool KEYED>
 cudaError_t ls_pick_tile(const LsArgs& a, int n_seqs, bool delta, bool walk, cudaStream_t stream) {
+  if constexpr (KR < 32) {
+    if (!walk && !delta && !a.unit_norm && !a.a_in && !a.b_in && !a.g_direct && !a.u_direct) return ls_launch_step<T, KR, ROT, KEYED>(a, n_seqs, stream);
+  }
   // the widest tile that still gives every SM a block: with fewer blocks than SMs the token-by-token walk, whose length a
   // block cannot shorten, runs on a part of the device only
   const long per = (long)a.heads * n_seqs, sms = ls_sm_count();

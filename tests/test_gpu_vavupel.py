@@ -379,6 +379,46 @@ def test_the_rotated_recurrence(dtype, heads, dim, vdim, rot, adjacent):
         assert float(state[0].abs().max()) == 0.0 and float(state[2].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("keyed", [False, True])
+@pytest.mark.parametrize("dim,vdim", [(20, 40), (64, 9), (96, 64), (128, 130), (200, 33)])
+def test_recurrences_give_the_same_bits_in_every_tile(dtype, keyed, dim, vdim):
+    """A step of many sequences takes wide tiles of the state, several columns a thread; few sequences narrow ones; one token each a
+    kernel of its own.  Outputs and state have the same bits."""
+    from ghost_infer_b200.kernels import ops
+    heads, seqs, n = 16, 24, 19
+    g = torch.Generator(device="cuda:0").manual_seed(dim + vdim)
+    rnd = lambda *s: torch.randn(s, device="cuda:0", generator=g)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda:0")
+    q, k, v = rnd(seqs, n, heads * dim).to(dtype), rnd(seqs, n, heads * dim).to(dtype), rnd(seqs, n, heads * vdim).to(dtype)
+    key_decay = torch.rand((seqs, n, heads * dim), device="cuda:0", generator=g) ** 0.1
+    decay, inv = torch.rand(heads, device="cuda:0", generator=g) ** 0.1, 100.0 ** (-torch.arange(dim // 4, device="cuda:0") * 4.0 / dim)
+    first = rnd(seqs + 1, heads * dim * vdim)
+
+    def run(parts):
+        """parts: (sequences, first token, past the last) of every step."""
+        state, out = first.clone(), torch.zeros((seqs, n, heads * vdim), device="cuda:0")
+        for who, a, b in parts:
+            step = type("S", (), {})()
+            step.cu_seqlens, step.seq_slots, step.n_seqs = i32([i * (b - a) for i in range(len(who) + 1)]), i32(who), len(who)
+            rows = [t[who, a:b].reshape(len(who) * (b - a), -1).contiguous() for t in (q, k, v, key_decay)]
+            if keyed:
+                o = ops.linear_state_keyed(*rows, state, step, heads, dim, vdim, 0.5)
+            else:
+                table = ops.rope_table(torch.arange(a, b, dtype=torch.int32, device="cuda:0").repeat(len(who)), inv)
+                o = ops.linear_state_rot(*rows[:3], state, step, heads, dim, vdim, decay, table, dim // 4 * 2, False, 0.3)
+            out[who, a:b] = o.view(len(who), b - a, -1)
+        return out, state
+
+    every = list(range(seqs))
+    want, want_state = run([(every, 0, n)])
+    assert bool(torch.isfinite(want).all())
+    for parts in ([([i], 0, n) for i in every], [(every[:5], 0, n), (every[5:], 0, n)], [(every, 0, 17), (every, 17, 18), (every, 18, n)],
+                  [([i], 0, 16) for i in every] + [([i], t, t + 1) for t in (16, 17, 18) for i in every]):
+        got, state = run(parts)
+        assert torch.equal(got, want) and torch.equal(state, want_state)
+
+
 @pytest.mark.parametrize("rows", [1, 5, 64, 65, 300])
 @pytest.mark.parametrize("ff,width", [(48, 64), (320, 256), (7, 54), (4096, 512)])
 def test_squared_relu_in_the_products(rows, ff, width):
