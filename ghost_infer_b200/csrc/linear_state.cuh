@@ -166,6 +166,16 @@ linear_state_kernel(const LsArgs a) {
   float4 dr[DG];                                                     // per-key decays
   const int pt = tid - NC;
   const int vpr = COLS / VW, vt = pt / vpr, vc = (pt - vt * vpr) * VW;      // at most CH * COLS / VW <= 128 groups
+  // A thread's places in a chunk (token << 16 | number) are the same in every chunk: their divisions are made once (they were half
+  // of what the preparing warps did, and those are the longer part of a narrow tile's chunk).
+  int q_at[QG], d_at[DG], r_at[ROT ? RG : 1];
+  auto place = [](int g, int per) { return per > 0 ? g / per << 16 | g % per : 0x7fff0000; };
+#pragma unroll
+  for (int i = 0; i < QG; ++i) q_at[i] = place(pt + i * LS_PREP, K / VW);
+#pragma unroll
+  for (int i = 0; i < DG; ++i) d_at[i] = place(pt + i * LS_PREP, (K + 3) / 4);
+#pragma unroll
+  for (int i = 0; i < (ROT ? RG : 1); ++i) r_at[i] = place(pt + i * LS_PREP, a.half);
   auto fetch = [&](int c) {
     const int n = min(CH, qlen - c * CH);
     const size_t tokc = (size_t)tok0 + (size_t)c * CH;
@@ -178,19 +188,16 @@ linear_state_kernel(const LsArgs a) {
     if (ROT) {
 #pragma unroll
       for (int i = 0; i < RG; ++i) {
-        const int g = pt + i * LS_PREP;
-        cs[i] = g < n * a.half ? a.table[tokc * a.half + g] : make_float2(1.f, 0.f);
+        cs[i] = (r_at[i] >> 16) < n ? a.table[tokc * a.half + pt + i * LS_PREP] : make_float2(1.f, 0.f);
       }
     }
     if (KEYED) {
-      const int gpr = (K + 3) / 4, total = n * gpr;
       const size_t ldg = (size_t)a.heads * K;
 #pragma unroll
       for (int i = 0; i < DG; ++i) {
-        const int g = pt + i * LS_PREP;
+        const int t = d_at[i] >> 16, r0 = (d_at[i] & 0xffff) * 4;
         dr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (g < total) {
-          const int t = g / gpr, r0 = (g - t * gpr) * 4;
+        if (t < n) {
           const float* p = a.g_key + (tokc + t) * ldg + (size_t)h * K + r0;
           if (K % 4 == 0) {
             dr[i] = *reinterpret_cast<const float4*>(p);
@@ -204,12 +211,10 @@ linear_state_kernel(const LsArgs a) {
       }
     }
     if (a.vec_in) {
-      const int gpr = K / VW, total = n * gpr;
 #pragma unroll
       for (int i = 0; i < QG; ++i) {
-        const int g = pt + i * LS_PREP;
-        if (g < total) {
-          const int t = g / gpr, r0 = (g - t * gpr) * VW;
+        const int t = q_at[i] >> 16, r0 = (q_at[i] & 0xffff) * VW;
+        if (t < n) {
           ls_load16(qp + (tokc + t) * a.ldq + (size_t)hk * K + r0, *reinterpret_cast<float (*)[VW]>(qr + i * VW));
           ls_load16(kp + (tokc + t) * a.ldk + (size_t)hk * K + r0, *reinterpret_cast<float (*)[VW]>(kr + i * VW));
         }
@@ -239,12 +244,10 @@ linear_state_kernel(const LsArgs a) {
     const size_t tokc = (size_t)tok0 + (size_t)c * CH;
     const float qs = KEYED ? a.q_scale : 1.0f;
     if (a.vec_in) {
-      const int gpr = K / VW, total = n * gpr;
 #pragma unroll
       for (int i = 0; i < QG; ++i) {
-        const int g = pt + i * LS_PREP;
-        if (g < total) {
-          const int t = g / gpr, r0 = (g - t * gpr) * VW;
+        const int t = q_at[i] >> 16, r0 = (q_at[i] & 0xffff) * VW;
+        if (t < n) {
 #pragma unroll
           for (int e = 0; e < VW; e += 4) {
             float4 q4 = make_float4(qr[i * VW + e], qr[i * VW + e + 1], qr[i * VW + e + 2], qr[i * VW + e + 3]);
@@ -283,13 +286,11 @@ linear_state_kernel(const LsArgs a) {
     }
     if (KEYED) {
       float* sd = buf + KEYS_AT;
-      const int gpr = (K + 3) / 4, total = n * gpr;
 #pragma unroll
       for (int i = 0; i < DG; ++i) {
-        const int g = pt + i * LS_PREP;
-        if (g < total) {
-          const int t = g / gpr;
-          *reinterpret_cast<float4*>(sd + t * Kp + (g - t * gpr) * 4) = dr[i];       // numbers past K: zeros, inside the padding
+        const int t = d_at[i] >> 16;
+        if (t < n) {
+          *reinterpret_cast<float4*>(sd + t * Kp + (d_at[i] & 0xffff) * 4) = dr[i];       // numbers past K: zeros, inside the padding
         }
       }
     }
@@ -303,9 +304,8 @@ linear_state_kernel(const LsArgs a) {
       ls_prep_barrier();             // the chunk's rows are in shared memory
 #pragma unroll
       for (int i = 0; i < RG; ++i) {
-        const int g = pt + i * LS_PREP;
-        if (g < n * a.half) {
-          const int t = g / a.half, p = g - t * a.half;
+        const int t = r_at[i] >> 16, p = r_at[i] & 0xffff;
+        if (t < n) {
           const int ia = t * Kp + (a.adjacent ? 2 * p : p), ib = a.adjacent ? ia + 1 : ia + a.half;
           float x, y;
           gi::rotate_pair(sq[ia], sq[ib], cs[i], &x, &y);
