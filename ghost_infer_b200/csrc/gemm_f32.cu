@@ -1,5 +1,6 @@
 // The products of the true 32-bit path where rows are 16-byte aligned: out[M,N] (op)= A[M,K] * W[N,K]^T, all float, FFMA
-// only.  gi_gemm_generic sends such operands here and keeps its own kernel for the rest.
+// only.  gi_gemm_generic sends such operands here and keeps its own kernel for the rest.  (Prompt steps' products of larger matrices go to
+// gemm_f32_split.cu; steps of one token a sequence and smaller matrices come here.)
 //
 // One order of additions serves every kernel of the 32-bit path, so that a token's bits do not depend on which of them
 // ran: K is cut into SUM_SEGMENTS stretches of gi::sum_segment(K) numbers (it follows from K alone); in a stretch the

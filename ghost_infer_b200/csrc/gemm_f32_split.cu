@@ -1,6 +1,7 @@
 // The true 32-bit path's larger products on tcgen05 tensor cores: out[M,N] (op)= A[M,K] * W[N,K]^T, all float, for the matrices
-// that gi_gemm_f32_split_scratch takes.  The matrix alone decides (N and K), never the rows: one order of additions serves
-// every number of rows, so a token's bits do not depend on its step.
+// that gi_gemm_f32_split_scratch takes (1,024 rows and columns or more: with fewer columns its distance from 64 bits is not below
+// the multiply-adds').  The matrix alone decides (N and K), never the rows: one order of additions serves every number of rows,
+// so a prompt token's bits do not depend on its step.
 //
 // A number becomes two 16-bit floats: 64 neighbours of a row (a chunk) share a power of two that brings their largest to
 // [2^14, 2^15); hi is the scaled number rounded to 11 bits, lo what is left rounded to 11 bits: 23 bits of each number or

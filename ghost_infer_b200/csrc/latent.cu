@@ -484,7 +484,8 @@ bmm_heads_mma_kernel(__nv_bfloat16* __restrict__ out, long ldo, long ohs, const 
 // between them and the 32 sums (4 columns, 8 rows) meet in a fixed order, halving what a lane holds at every exchange: 31
 // exchanges, and each lane ends with one sum (32 butterflies of five were 160, the longest part of the kernel).  The matrix is
 // asked for in L2 before the dependency wait (a prefetch reads no values: right whoever wrote it) and its first numbers are
-// loaded beside the rows'.  bfloat16, K a multiple of 8, rows on 16-byte boundaries.
+// loaded beside the rows'.  B200, 8 rows, 16 heads of 512 x 128 and of 128 x 512: 5.1 us of a step's time, 9.8 before.
+// bfloat16, K a multiple of 8, rows on 16-byte boundaries.
 constexpr int GV_ROWS = 8, GV_COLS = 16;      // a warp takes 4 columns
 
 // One exchange among the lanes: of 2 * HALF sums a lane keeps the half that bit BIT of its number names.
