@@ -1,32 +1,42 @@
 // The true 32-bit path's larger products on tcgen05 tensor cores: out[M,N] (op)= A[M,K] * W[N,K]^T, all float, for the matrices
-// that gi_gemm_f32_split_scratch takes (1,024 rows and columns or more: with fewer columns its distance from 64 bits is not below
-// the multiply-adds').  The matrix alone decides (N and K), never the rows: one order of additions serves every number of rows,
-// so a prompt token's bits do not depend on its step.
+// that gi_gemm_f32_split_scratch takes (1,024 rows and columns or more).  Between this kernel and the multiply-adds of gemm_f32.cu the
+// matrix (N and K) and the kind of step decide, never the number of rows: a prompt token's bits do not depend on its step.
 //
-// A number becomes two 16-bit floats: 64 neighbours of a row (a chunk) share a power of two that brings their largest to
-// [2^14, 2^15); hi is the scaled number rounded to 11 bits, lo what is left rounded to 11 bits: 23 bits of each number or
-// 2^-39 of its chunk's largest, whichever is more.  A chunk's sum is lo hi' + hi lo' + hi hi', twelve instructions of 16 numbers
-// into a fresh accumulator (products are exact, the tensor cores cut off what does not fit into a sum they add to
-// themselves, hence no longer chains); it leaves tensor memory, gets both powers of two back and is added with one rounding
-// to its stretch's sum, and the at most eight stretches (they follow from K alone) are added in their order.
-// A result that is no finite number is worked out again in plain multiply-adds (a split infinity is none any more).
+// A number becomes three bfloat16 (the splitting of Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial Intelligence
+// Datatype For Higher-Precision Computations", 2019): hi is the number rounded to 8 bits, mid what is left rounded to 8 bits, lo what
+// is left then, which has 8 bits at most.  They have a float's exponent, so the three sum up to the number itself whatever its
+// neighbours are; it is multiplied by 2^24 first, so that this holds down to the smallest floats.  Numbers from 2^103 on and sums from
+// 2^79 on become no finite numbers, and such results are worked out again in plain multiply-adds, as those that really are none.
+// Of the nine products six are made; mid lo', lo mid' and lo lo' are 2^-24 of |a w| together at most, random in sign.
+//
+// The tensor cores cut off what does not fit into a sum that they add to themselves, so no long chain is left to them: hi hi'
+// of 32 numbers of K (two instructions, products of 16 bits) goes into a fresh accumulator, which leaves tensor memory and is
+// added with one rounding to its stretch's sum; a chunk of K is 64 numbers.  The five small products (2^-8 of the whole) have an
+// accumulator of their own, which is read at the end of a stretch.  The at most eight stretches (they follow from K alone) are added in
+// their order.  (With 64 numbers an accumulator, sums of one sign were further from 64 bits than the multiply-adds'.)
 //
 // A tile is 128 rows of W (the "M" side of the instruction, split by four warps on the way from shared into tensor memory)
-// times up to 128 tokens (the "N" side, in shared memory).  One thread feeds both rings with TMA, one issues the
-// products, four warps split W, eight drain accumulators; two chunks of W and two accumulators in tensor memory, so that all
-// four overlap.  Up to 32 tokens (FEW, tiles of 16) two more warps split the tokens themselves, eight warps split W in turns, and
-// where there are few tiles the blocks of a cluster share the stretches of a tile, which meet in distributed shared memory;
-// more tokens are split once by a kernel of their own, into scratch.
+// times up to 96 tokens (the "N" side, in shared memory; 96, since a chunk's two accumulators of hi hi', one of the small products and
+// two chunks of W's parts are 480 of tensor memory's 512 columns).  A chunk's hi hi' is made first and drained while its small
+// products are.  One thread feeds both rings with TMA, one issues the products, four warps
+// split W, twelve drain accumulators.  Up to 32 tokens (FEW, tiles of 16) two more warps split the tokens themselves, eight warps
+// split W in turns, and where there are few tiles the blocks of a cluster share the stretches of a tile, which meet in distributed
+// shared memory; more tokens are split once by a kernel of their own, into scratch (6 bytes a number, 8,192 tokens at a time).
 //
-// Steps of one token a sequence keep gemm_f32.cu's kernels (ops.one_token_step): they are bound by the bytes of W, and there the
-// chain of a chunk (32 KB: split 0.4 us, twelve products 0.5 us at 16 tokens as at 128, since each reads 128 rows of W out of
-// tensor memory) is longer than the chunk's share of the memory's time: a 1B model's step of four 1.98 ms against 1.72.
-// B200, one launch beside one of gemm_f32.cu: 601 rows 16,384 x 2,048 223 us (181 TFLOP/s) against 960; 2,048 x 8,192 150 against
-// 550; 64 rows 46 against 134 and 112 against 150; 16 rows 51 against 72 and 48 against 48.  What bounds it with many rows is
-// the draining warps (64 columns a thread and chunk), with few the one thread's products.
-// Distance from 64 bits (2-norms): 1.2e-7 against 1.5e-7 (K 2,048), 1.4e-7 against 2.3e-7 (K 8,192), 1.2e-7 against 1.3e-7 (K 1,024).
+// An instruction takes 17 + 0.45 clocks a token when a warp issues it together and one lane is elected, and 96 or more when one thread
+// does so in a branch of its own (its operands then have to be brought together first).
+//
+// Steps of one token a sequence keep gemm_f32.cu's kernels (ops.one_token_step), which are bound by the bytes of W there; the
+// smaller matrices do as well, since a launch here has 10 us of set-up and pipeline to fill, longer than what they take there
+// (1,024 x 1,024: 12 us here for 16 rows, 12 there; 24 against 16 for 33).
+// B200, cold L2, one launch beside one of gemm_f32.cu (us): 601 rows 16,384 x 2,048 234 (172 TFLOP/s) against 960; 2,048 x 8,192 136 against
+// 548; 64 rows 46 against 133 and 115 against 151; 16 rows 43 against 72 and 38 against 47; 4 rows 39 against 45 and 32 against 27.
+// What bounds it with many rows is a chunk's trips through shared memory (W in and out, tokens in and out: 170 KB, 1,330 clocks at 128
+// bytes a clock) beside its 24 instructions (1,400 clocks in tiles of 96), of 2,100 measured; with few rows the bytes of W.
+// Distance from 64 bits (2-norms, random numbers): 0.84e-7 against 1.32e-7 (K 1,024), 0.92e-7 against 1.51e-7 (K 2,048), 1.3e-7
+// against 2.3e-7 (K 8,192); of one sign 0.64e-7 against 0.90e-7.
 #include <cuda.h>
-#include <cuda_fp16.h>
+#include <cuda_bf16.h>
 #include <float.h>
 
 #include "api.h"
@@ -56,34 +66,34 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int who
 
 struct Args {
   float* out;
-  const float *A, *W, *fx;             // fx: [chunk][ldf] what brings a token's chunk back to size (not FEW)
+  const float *A, *W;
   long lda, ldw, ldo;
-  int M, N, K, ldf, nt, tiles_m, tiles, chunks, per_stretch, seg, cluster, a_vec, accumulate;
+  int M, N, K, nt, tiles_m, tiles, chunks, per_stretch, seg, cluster, a_vec, accumulate;
 };
 
 template <bool FEW, bool CLUSTER>
 struct Shape {
-  static constexpr int NT = FEW ? FEW_TILE : 128;             // tokens a tile at most
+  static constexpr int NT = FEW ? FEW_TILE : 96;              // tokens a tile at most
   static constexpr int W_STAGES = CLUSTER ? 4 : FEW ? 6 : 3, X_STAGES = FEW ? 4 : 3, A_STAGES = FEW ? 4 : 2;
-  // Slots of a chunk's powers of two and of its two barriers, from splitting to draining.  W is split at most A_STAGES chunks
-  // ahead of the products, tokens X_STAGES, and the products are at most two ahead of the drained ones: six would do.
+  // Slots of a chunk's barriers.  W is split at most A_STAGES chunks ahead of the products, tokens X_STAGES, and the products are
+  // at most one ahead of the drained ones: six would do.
   static constexpr int SLOTS = 8;
-  static constexpr uint32_t X_HALF = NT * 128, X_STAGE = 2 * X_HALF;     // hi rows, then lo rows, 128 bytes each, swizzled
-  static constexpr uint32_t X_AT = W_STAGES * W_STAGE, FW_AT = X_AT + X_STAGES * X_STAGE, FX_AT = FW_AT + SLOTS * ROWS * 4,
-                            RED_AT = FX_AT + SLOTS * NT * 4, BAR_AT = RED_AT + (CLUSTER ? STRETCHES / 2 * NT * ROWS * 4 : 0);
-  static constexpr int N_BARS = 2 * W_STAGES + 2 * SLOTS;
+  static constexpr uint32_t X_PART = NT * 128, X_STAGE = 3 * X_PART;     // hi rows, mid rows, lo rows, 128 bytes each, swizzled
+  static constexpr uint32_t X_AT = W_STAGES * W_STAGE, RED_AT = X_AT + X_STAGES * X_STAGE,
+                            BAR_AT = RED_AT + (CLUSTER ? STRETCHES / 2 * NT * ROWS * 4 : 0);
+  static constexpr int N_BARS = 2 * W_STAGES + 3 * SLOTS + 1;
   static constexpr size_t SMEM = BAR_AT + N_BARS * 8 + 16 + 1024;
   // warp 0 loads, 1 issues products, FEW: 2-3 split tokens, in turns; then the warps that split W, in SETS of four that take
   // turns, and those that drain, in PARTS of four that share a tile's columns, 16 at a time
-  static constexpr int SETS = FEW ? 2 : 1, PARTS = FEW ? 1 : 2;
+  static constexpr int SETS = FEW ? 2 : 1, PARTS = FEW ? 1 : 3;
   static constexpr int SPLIT_WARP = FEW ? 4 : 2, DRAIN_WARP = SPLIT_WARP + 4 * SETS, THREADS = 32 * (DRAIN_WARP + 4 * PARTS);
   static constexpr int COLS = NT / PARTS;                    // columns a draining thread holds
-  // columns of tensor memory: two accumulators, the chunks of W (hi 32, lo 32), and the stretches' sum where registers have no room
-  static constexpr int A_AT = 2 * NT, SUM_AT = A_AT + 64 * A_STAGES, TMEM = 512;
+  // columns of tensor memory: a chunk's two accumulators of hi hi', one of the small products, the chunks of W (hi, mid, lo: 32 each)
+  static constexpr int SMALL_AT = 2 * NT, A_AT = (3 * NT + 31) / 32 * 32, A_COLS = 96, TMEM = 512;
   // A wait names a phase by its parity: whoever takes turns must see every phase of the stages that it waits for.  (With five
   // stages of W a set met a stage every second time round, and its wait was over while the phase before was still open.)
   static_assert(W_STAGES % SETS == 0, "a stage of W belongs to one set");
-  static_assert(SUM_AT + (FEW ? 0 : NT) <= TMEM && SMEM <= 227 * 1024 && SPLIT_WARP % 2 == 0, "what a block has");
+  static_assert(A_AT + A_COLS * A_STAGES <= TMEM && SMEM <= 227 * 1024 && COLS % 16 == 0 && COLS <= 32, "what a block has");
 };
 
 __device__ __forceinline__ uint64_t pack2(float a, float b) { return (uint64_t)__float_as_uint(a) | (uint64_t)__float_as_uint(b) << 32; }
@@ -103,26 +113,30 @@ __device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-// The tensor cores cut off: a chunk's sum comes out small by 8.8e-8 of itself on average (measured, random numbers; 7e-8 with
-// numbers of one sign), so the whole does, and gets that back here.
-__device__ __forceinline__ float whole(float v) { return fmaf(v, 8.5e-8f, v); }
+constexpr float SCALE = 16777216.f, BACK = 1.f / (SCALE * SCALE);      // what both operands are multiplied by, and the result's way back
 
-// the power of two that brings `top` to [2^14, 2^15) (a chunk of zeros or of the smallest numbers: 2^126), and its inverse
-__device__ __forceinline__ float scale_of(float top, float* back) {
-  const int s = min(141 - (int)(__float_as_uint(top) >> 23), 126);
-  *back = __uint_as_float((uint32_t)(127 - s) << 23);
-  return __uint_as_float((uint32_t)(127 + s) << 23);
-}
-// two neighbours as 16-bit pairs
-__device__ __forceinline__ void split2(float a, float b, float scale, uint32_t* hi, uint32_t* lo) {
-  const uint64_t y = mul2(pack2(a, b), pack2(scale, scale));
-  const __half2 h = __floats2half2_rn(lo_of(y), hi_of(y));
-  const float2 f = __half22float2(h);
-  const __half2 l = __floats2half2_rn(lo_of(y) - f.x, hi_of(y) - f.y);
-  *hi = *reinterpret_cast<const uint32_t*>(&h);
-  *lo = *reinterpret_cast<const uint32_t*>(&l);
+// two neighbours as pairs of bfloat16 whose sums they are, times SCALE (lo has 8 bits: the rest's upper half as it is)
+__device__ __forceinline__ void split2(float a, float b, uint32_t* hi, uint32_t* mid, uint32_t* lo) {
+  const uint64_t minus1 = pack2(-1.f, -1.f);
+  uint64_t rest = mul2(pack2(a, b), pack2(SCALE, SCALE));
+  auto part = [&](uint32_t* to) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo_of(rest), hi_of(rest));
+    *to = *reinterpret_cast<const uint32_t*>(&h);
+  };
+  auto subtract = [&](uint32_t v) { fma2(rest, (uint64_t)(v << 16) | (uint64_t)(v & 0xffff0000u) << 32, minus1); };     // exact
+  part(hi);
+  subtract(*hi);
+  part(mid);
+  subtract(*mid);
+  *lo = __byte_perm((uint32_t)rest, (uint32_t)(rest >> 32), 0x7632);
 }
 
+// One lane of a warp that is together, the same at every call.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void mma_a_tmem(uint32_t d, uint32_t a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -133,12 +147,6 @@ __device__ __forceinline__ void mma_a_tmem(uint32_t d, uint32_t a, uint64_t desc
 __device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -182,62 +190,49 @@ __device__ __noinline__ void plain_result(const Args& args, int m, int n) {
   *o = args.accumulate ? *o + sum : sum;
 }
 
-// Splits `rows` rows of A into two 16-bit planes [rows][chunks * 64] (zeros past K) and fx.  Sixteen lanes take a chunk.
+// Splits `rows` rows of A into three planes [rows][chunks * 64] of 16-bit parts (zeros past K), four numbers a thread.
 __global__ void __launch_bounds__(256)
-split_rows_kernel(uint2* __restrict__ hi, uint2* __restrict__ lo, float* __restrict__ fx, const float* A, long lda, int rows, int K, int chunks,
-                  int ldf, int a_vec) {
+split_rows_kernel(uint2* __restrict__ planes, const float* A, long lda, int rows, int K, int chunks, int a_vec) {
   gi::pdl_prologue();
-  const long i = (long)blockIdx.x * 16 + (threadIdx.x >> 4);
-  const int l = threadIdx.x & 15;
-  const bool live = i < (long)rows * chunks;
-  const int m = live ? (int)(i / chunks) : 0, c = live ? (int)(i % chunks) : 0, k = c * CK + l * 4;
+  const long quads = (long)chunks * (CK / 4), i = (long)blockIdx.x * 256 + threadIdx.x, plane = rows * quads;
+  if (i >= plane) return;
+  const int m = (int)(i / quads), k = (int)(i % quads) * 4;
   float v[4] = {0.f, 0.f, 0.f, 0.f};
-  if (live) {
-    const float* src = A + (size_t)m * lda + k;
-    if (a_vec && k + 4 <= K) {
-      const float4 f = *reinterpret_cast<const float4*>(src);
-      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-    } else {
+  const float* src = A + (size_t)m * lda + k;
+  if (a_vec && k + 4 <= K) {
+    const float4 f = *reinterpret_cast<const float4*>(src);
+    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+  } else {
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (k + e < K) v[e] = src[e];
-    }
+    for (int e = 0; e < 4; ++e)
+      if (k + e < K) v[e] = src[e];
   }
-  float top = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  float back;
-  const float scale = scale_of(top, &back);
-  uint2 h, w;
-  split2(v[0], v[1], scale, &h.x, &w.x);
-  split2(v[2], v[3], scale, &h.y, &w.y);
-  if (live) {
-    hi[i * 16 + l] = h;
-    lo[i * 16 + l] = w;
-    if (l == 0) fx[(size_t)c * ldf + m] = back;
-  }
+  uint2 hi, mid, lo;
+  split2(v[0], v[1], &hi.x, &mid.x, &lo.x);
+  split2(v[2], v[3], &hi.y, &mid.y, &lo.y);
+  planes[i] = hi;
+  planes[plane + i] = mid;
+  planes[2 * plane + i] = lo;
 }
 
 // CLUSTER: `a.cluster` blocks share a tile's stretches (FEW only).  W_TMA: rows of W start on 16-byte boundaries; else its
 // warps load their rows themselves.
 template <bool FEW, bool CLUSTER, bool W_TMA>
 __global__ void __launch_bounds__(Shape<FEW, CLUSTER>::THREADS, 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
-                  const __grid_constant__ Args a) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ Args a) {
   using S = Shape<FEW, CLUSTER>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  float* fw = reinterpret_cast<float*>(smem + S::FW_AT);     // [SLOTS][ROWS]
-  float* fx = reinterpret_cast<float*>(smem + S::FX_AT);     // [SLOTS][NT]
   const uint32_t bars = smem_u32(smem + S::BAR_AT);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + S::BAR_AT + S::N_BARS * 8);
-  // Two barriers a chunk, so that the one thread that issues products waits once and signals once: `full` - its rows of W are
-  // split (4 warps), its tokens are there (1) and its accumulator is drained (the chunk before the last one's; 4 warps a part);
-  // `done` - its products are: its operands' places are free and its accumulator is ready.
-  const uint32_t w_full = bars, w_empty = w_full + 8 * S::W_STAGES, full = w_empty + 8 * S::W_STAGES, done = full + 8 * S::SLOTS;
+  // Barriers of a chunk: `full` - its rows of W are split (4 warps), its tokens are there (1) and its accumulators are drained (of the
+  // chunk before; 4 warps a part); `large` - its hi hi' are made; `done` - all its products are, its operands' places are free.
+  // `small` - a stretch's small products are read.
+  const uint32_t w_full = bars, w_empty = w_full + 8 * S::W_STAGES, full = w_empty + 8 * S::W_STAGES, done = full + 8 * S::SLOTS,
+                 large = done + 8 * S::SLOTS, small = large + 8 * S::SLOTS;
   auto wait_full = [&](int it, int who) { return mbar_wait(full + 8 * (it % S::SLOTS), (uint32_t)((it / S::SLOTS) & 1), who); };
   auto wait_done = [&](int it, int who) { return it < 0 || mbar_wait(done + 8 * (it % S::SLOTS), (uint32_t)((it / S::SLOTS) & 1), who); };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S::W_STAGES; ++i) {
@@ -247,7 +242,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     for (int i = 0; i < S::SLOTS; ++i) {
       mbar_init(full + 8 * i, 5 + 4 * S::PARTS);
       mbar_init(done + 8 * i, 1);
+      mbar_init(large + 8 * i, 1);
     }
+    mbar_init(small, 4 * S::PARTS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -271,7 +268,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   gi::pdl_launch_dependents();
   gi::pdl_wait();
 
@@ -296,11 +293,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             ok = wait_done(it - S::X_STAGES, 1);
             if (!ok) break;
             const uint32_t dst = smem_u32(smem + S::X_AT + st * S::X_STAGE), bar = full + 8 * slot;
-            mbar_expect_tx(bar, (uint32_t)a.nt * 260u);
-            tma_load_2d(dst, &map_hi, c * CK, m0, bar);
-            tma_load_2d(dst + S::X_HALF, &map_lo, c * CK, m0, bar);
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(smem_u32(fx + slot * S::NT)), "l"(a.fx + (size_t)c * a.ldf + m0), "r"((uint32_t)a.nt * 4u), "r"(bar) : "memory");
+            mbar_expect_tx(bar, (uint32_t)a.nt * 384u);
+            for (int p = 0; p < 3; ++p) tma_load_2d(dst + p * S::X_PART, &map_x, c * CK, p * a.M + m0, bar);
           }
           ++loaded;
         }
@@ -310,28 +304,47 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       for (int i = max(0, loaded - S::X_STAGES); !FEW && i < loaded; ++i) wait_full(i, 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(a.nt >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);   // float sums of 16-bit floats
-      bool ok = true;
-      int it = 0;
-      for (int tile = tile0; tile < a.tiles && ok; tile += tile_step)
-        for (int c = c_first; c < c_last && ok; ++c, ++it) {
-          const int st = it & 1, as = it % S::A_STAGES, xs = it % S::X_STAGES;
-          ok = wait_full(it, 2);
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.nt >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);   // float sums of bfloat16
+    const uint32_t x_at = __shfl_sync(0xffffffffu, smem_u32(smem + S::X_AT), 0);
+    bool ok = true;
+    int it = 0, stretches = 0;
+    for (int tile = tile0; tile < a.tiles && ok; tile += tile_step) {
+      int left = 0;
+      for (int c = c_first; c < c_last && ok; ++c, ++it) {
+        const int as = it % S::A_STAGES, xs = it % S::X_STAGES;
+        const bool fresh = left == 0;                        // a stretch begins
+        left = (fresh ? a.per_stretch : left) - 1;
+        ok = __all_sync(0xffffffffu, wait_full(it, 2));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t s = tmem + S::SMALL_AT, hi = tmem + S::A_AT + as * S::A_COLS, mid = hi + 32, lo = hi + 64;
+        const uint64_t x_hi = smem_desc(x_at + xs * S::X_STAGE), x_mid = x_hi + (S::X_PART >> 4), x_lo = x_hi + (2 * S::X_PART >> 4);
+        auto product = [&](uint32_t w, uint64_t x, bool first) {
+#pragma unroll
+          for (int k = 0; k < CK / 16; ++k) mma_a_tmem(s, w + 8 * k, x + 2 * k, idesc, !(first && k == 0));
+        };
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < CK / 16; ++k) mma_a_tmem(tmem + k / 2 * S::NT, hi + 8 * k, x_hi + 2 * k, idesc, k & 1);
+          tc_commit(large + 8 * (it % S::SLOTS));
+        }
+        if (fresh && stretches++ > 0) {
+          ok = __all_sync(0xffffffffu, mbar_wait(small, (uint32_t)(stretches & 1), 2));
           if (!ok) break;
           tc_fence_after();
-          const uint32_t d = tmem + st * S::NT, hi = tmem + S::A_AT + as * 64, lo = hi + 32;
-          const uint64_t x_hi = smem_desc(smem_u32(smem + S::X_AT + xs * S::X_STAGE)), x_lo = x_hi + (S::X_HALF >> 4);
-#pragma unroll
-          for (int k = 0; k < CK / 16; ++k) mma_a_tmem(d, lo + 8 * k, x_hi + 2 * k, idesc, k > 0);
-#pragma unroll
-          for (int k = 0; k < CK / 16; ++k) mma_a_tmem(d, hi + 8 * k, x_lo + 2 * k, idesc, 1);
-#pragma unroll
-          for (int k = 0; k < CK / 16; ++k) mma_a_tmem(d, hi + 8 * k, x_hi + 2 * k, idesc, 1);
+        }
+        if (elect_one()) {
+          product(mid, x_hi, fresh);
+          product(hi, x_mid, false);
+          product(mid, x_mid, false);
+          product(lo, x_hi, false);
+          product(hi, x_lo, false);
           tc_commit(done + 8 * (it % S::SLOTS));
         }
-      wait_done(it - 1, 2);                                  // its products, as the loads above
+        __syncwarp();
+      }
     }
+    wait_done(it - 1, 2);                                    // its products, as the loads above
   } else if (warp >= S::SPLIT_WARP && warp < S::DRAIN_WARP) {
     // a row of W a thread
     const int set = (warp - S::SPLIT_WARP) / 4;
@@ -353,38 +366,30 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         };
         if (W_TMA) ok = mbar_wait(w_full + 8 * ws, (uint32_t)((it / S::W_STAGES) & 1), 3);
         if (!ok) break;
-        float4 v[CK / 4];
-        float top = 0.f, top1 = 0.f;
+        ok = wait_done(it - S::A_STAGES, 3);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t dst = tmem + lane_base + S::A_AT + as * S::A_COLS;
 #pragma unroll
-        for (int p = 0; p < CK / 4; ++p) v[p] = piece(p);
+        for (int q = 0; q < CK / 16; ++q) {
+          uint32_t hi[8], mid[8], lo[8];
+          float4 v[4];
+#pragma unroll
+          for (int p = 0; p < 4; ++p) v[p] = piece(4 * q + p);
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            const float4 f = v[p];
+            split2(f.x, f.y, &hi[2 * p], &mid[2 * p], &lo[2 * p]);
+            split2(f.z, f.w, &hi[2 * p + 1], &mid[2 * p + 1], &lo[2 * p + 1]);
+          }
+          tc_st8(dst + 8 * q, hi);
+          tc_st8(dst + 32 + 8 * q, mid);
+          tc_st8(dst + 64 + 8 * q, lo);
+        }
         if (W_TMA) {
           __syncwarp();
           if (lane == 0) mbar_arrive(w_empty + 8 * ws);
         }
-#pragma unroll
-        for (int p = 0; p < CK / 4; ++p) {
-          top = fmaxf(top, fmaxf(fabsf(v[p].x), fabsf(v[p].y)));
-          top1 = fmaxf(top1, fmaxf(fabsf(v[p].z), fabsf(v[p].w)));
-        }
-        float back;
-        const float scale = scale_of(fmaxf(top, top1), &back);
-        ok = wait_done(it - S::A_STAGES, 3);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t dst = tmem + lane_base + S::A_AT + as * 64;
-#pragma unroll
-        for (int q = 0; q < CK / 16; ++q) {
-          uint32_t hi[8], lo[8];
-#pragma unroll
-          for (int p = 0; p < 4; ++p) {
-            const float4 f = v[4 * q + p];
-            split2(f.x, f.y, scale, &hi[2 * p], &lo[2 * p]);
-            split2(f.z, f.w, scale, &hi[2 * p + 1], &lo[2 * p + 1]);
-          }
-          tc_st8(dst + 8 * q, hi);
-          tc_st8(dst + 32 + 8 * q, lo);
-        }
-        fw[it % S::SLOTS * ROWS + row] = back;
         wait_st();
         tc_fence_before();
         __syncwarp();
@@ -398,52 +403,49 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     auto col_of = [&](int g) { return (g * S::PARTS + part) * GROUP; };
     bool ok = true;
     int it = 0;
-    if (lane == 0) {                                         // nothing to drain before the first two chunks
-      mbar_arrive(full);
-      mbar_arrive(full + 8);
-    }
+    if (lane == 0) mbar_arrive(full);                        // nothing to drain before the first chunk
     for (int tile = tile0; tile < a.tiles && ok; tile += tile_step) {
       const int m0 = tile % a.tiles_m * a.nt, n = tile / a.tiles_m * ROWS + row, nt = a.nt;
-      uint64_t acc[S::COLS / 2], sum[FEW ? S::COLS / 2 : 1];
+      uint64_t acc[S::COLS / 2], sum[S::COLS / 2];
 #pragma unroll
-      for (int j = 0; j < S::COLS / 2; ++j) acc[j] = 0;
+      for (int j = 0; j < S::COLS / 2; ++j) acc[j] = sum[j] = 0;
+      // an accumulator's columns of this part, added (columns past the tile's tokens hold what nobody reads)
+      auto take = [&](uint32_t d) {
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g)
+          if (col_of(g) < nt) {
+            uint32_t r[GROUP];
+            tc_ld16(d + col_of(g), r);
+            wait_ld16(r);
+#pragma unroll
+            for (int j = 0; j < GROUP; j += 2) {
+              uint64_t& v = acc[(g * GROUP + j) / 2];
+              v = add2(v, (uint64_t)r[j] | (uint64_t)r[j + 1] << 32);
+            }
+          }
+      };
       int left = a.per_stretch, stretch = 0;
       for (int c = c_first; c < c_last && ok; ++c, ++it) {
-        const int st = it & 1, slot = it % S::SLOTS;
-        ok = wait_full(it, 4) && wait_done(it, 4);
+        ok = mbar_wait(large + 8 * (it % S::SLOTS), (uint32_t)((it / S::SLOTS) & 1), 4);
         if (!ok) break;
         tc_fence_after();
-        const float f = fw[slot * ROWS + row];
-        const uint64_t f2 = pack2(f, f);
-        const uint32_t d = tmem + lane_base + st * S::NT;
-        auto take = [&](int g, const uint32_t (&r)[GROUP]) {
-#pragma unroll
-          for (int j = 0; j < GROUP; j += 4) {
-            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(fx + slot * S::NT + col_of(g) + j);
-            fma2(acc[(g * GROUP + j) / 2], (uint64_t)r[j] | (uint64_t)r[j + 1] << 32, mul2(x.x, f2));
-            fma2(acc[(g * GROUP + j) / 2 + 1], (uint64_t)r[j + 2] | (uint64_t)r[j + 3] << 32, mul2(x.y, f2));
-          }
-        };
-        // (a third of a chunk's time; one group asked for while the one before is added was slower: 253 against 223 us at 601 x 16,384 x 2,048)
-#pragma unroll
-        for (int g = 0; g < GROUPS; g += 2) {                // (columns past the tile's tokens hold what nobody reads)
-          if (col_of(g) < nt) {
-            uint32_t r[GROUP], r1[GROUP];
-            tc_ld16(d + col_of(g), r);
-            if (g + 1 < GROUPS) {
-              tc_ld16(d + col_of(g + 1), r1);
-              wait_ld16(r1);
-            }
-            wait_ld16(r);
-            take(g, r);
-            if (g + 1 < GROUPS) take(g + 1, r1);
-          }
-        }
+        take(tmem + lane_base);
+        take(tmem + lane_base + S::NT);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(full + 8 * ((it + 2) % S::SLOTS));
-        if (--left > 0 && c + 1 < c_last) continue;
-        left = a.per_stretch;                                // a stretch ends
+        if (lane == 0) mbar_arrive(full + 8 * ((it + 1) % S::SLOTS));
+        const bool ends = --left == 0 || c + 1 == c_last;    // a stretch ends
+        if (ends) {
+          ok = wait_done(it, 4);
+          if (!ok) break;
+          tc_fence_after();
+          take(tmem + lane_base + S::SMALL_AT);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(small);
+        }
+        if (!ends) continue;
+        left = a.per_stretch;
         if constexpr (CLUSTER) {
           // where the cluster reads it
           float* red = reinterpret_cast<float*>(smem + S::RED_AT) + stretch * FEW_TILE * ROWS;
@@ -451,72 +453,40 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
           for (int j = 0; j < S::COLS / 2; ++j) {
             red[(2 * j) * ROWS + row] = lo_of(acc[j]);
             red[(2 * j + 1) * ROWS + row] = hi_of(acc[j]);
-            acc[j] = 0;
-          }
-        } else if constexpr (FEW) {
-#pragma unroll
-          for (int j = 0; j < S::COLS / 2; ++j) {
-            sum[j] = stretch == 0 ? acc[j] : add2(sum[j], acc[j]);
-            acc[j] = 0;
           }
         } else {
-          const uint32_t t = tmem + lane_base + S::SUM_AT;
-          const bool last = c + 1 == c_last;
 #pragma unroll
-          for (int g = 0; g < GROUPS; ++g) {
-            const int col = col_of(g);
-            if (col < nt) {
-              uint32_t s[GROUP];
-              if (stretch > 0) {
-                tc_ld16(t + col, s);
-                wait_ld16(s);
-#pragma unroll
-                for (int j = 0; j < GROUP; j += 2) {
-                  uint64_t& v = acc[(g * GROUP + j) / 2];
-                  v = add2((uint64_t)s[j] | (uint64_t)s[j + 1] << 32, v);
-                }
-              }
-              if (!last) {
-#pragma unroll
-                for (int j = 0; j < GROUP; j += 2) {
-                  uint64_t& v = acc[(g * GROUP + j) / 2];
-                  s[j] = (uint32_t)v;
-                  s[j + 1] = (uint32_t)(v >> 32);
-                  v = 0;
-                }
-                tc_st16(t + col, s);
-              }
-            }
-          }
-          if (!last) wait_st();
+          for (int j = 0; j < S::COLS / 2; ++j) sum[j] = stretch == 0 ? acc[j] : add2(sum[j], acc[j]);
         }
+#pragma unroll
+        for (int j = 0; j < S::COLS / 2; ++j) acc[j] = 0;
         ++stretch;
       }
       if (!ok) break;
-      if (!CLUSTER && n < a.N) {
-        const int live = min(nt, a.M - m0);
+      if constexpr (!CLUSTER) {
+        const int live = n < a.N ? min(nt, a.M - m0) : 0;
         const long ldo = a.ldo;
         const bool add = a.accumulate != 0;
         float* o = a.out + (size_t)m0 * ldo + n;
-        uint32_t odd[(S::NT + 31) / 32] = {};                // results that are no finite numbers: after the others
+        uint32_t odd = 0;                                    // results that are no finite numbers: after the others
 #pragma unroll
         for (int g = 0; g < GROUPS; ++g) {
           const int col = col_of(g);
 #pragma unroll
           for (int j = 0; j < GROUP; ++j) {
-            const uint64_t both = FEW ? sum[FEW ? (g * GROUP + j) / 2 : 0] : acc[(g * GROUP + j) / 2];
-            const float v = whole((j & 1) ? hi_of(both) : lo_of(both));
-            const bool fine = fabsf(v) <= FLT_MAX;
+            const uint64_t both = sum[(g * GROUP + j) / 2];
+            const float v = ((j & 1) ? hi_of(both) : lo_of(both)) * BACK;
             float* at = o + (size_t)(col + j) * ldo;
             if (col + j < live) {
-              if (fine) *at = add ? *at + v : v;
-              else odd[g * S::PARTS * GROUP / 32] |= 1u << (g * S::PARTS * GROUP % 32 + j);
+              if (fabsf(v) <= FLT_MAX) *at = add ? *at + v : v;
+              else odd |= 1u << (g * GROUP + j);
             }
           }
         }
-#pragma unroll
-        for (int i = 0; i < (S::NT + 31) / 32; ++i)
-          for (uint32_t rest = odd[i]; rest; rest &= rest - 1) plain_result(a, m0 + 32 * i + part * GROUP + __ffs((int)rest) - 1, n);
+        for (; odd; odd &= odd - 1) {
+          const int i = __ffs((int)odd) - 1;
+          plain_result(a, m0 + col_of(i / GROUP) + i % GROUP, n);
+        }
       }
     }
   } else if constexpr (FEW) {
@@ -557,18 +527,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       for (int i = 0; i < FEW_TILE / 2; ++i) {
         if (2 * i >= a.M) break;                             // (a later tile's missing tokens: zeros)
         const int m = 2 * i + sub;
-        float top = fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        float back;
-        const float scale = scale_of(top, &back);
-        uint2 h, w;
-        split2(v[i].x, v[i].y, scale, &h.x, &w.x);
-        split2(v[i].z, v[i].w, scale, &h.y, &w.y);
+        uint2 hi, mid, lo;
+        split2(v[i].x, v[i].y, &hi.x, &mid.x, &lo.x);
+        split2(v[i].z, v[i].w, &hi.y, &mid.y, &lo.y);
         unsigned char* dst = smem + S::X_AT + xs * S::X_STAGE + m * 128 + ((l >> 1) ^ (m & 7)) * 16 + (l & 1) * 8;
-        *reinterpret_cast<uint2*>(dst) = h;
-        *reinterpret_cast<uint2*>(dst + S::X_HALF) = w;
-        if (l == 0) fx[slot * S::NT + m] = back;
+        *reinterpret_cast<uint2*>(dst) = hi;
+        *reinterpret_cast<uint2*>(dst + S::X_PART) = mid;
+        *reinterpret_cast<uint2*>(dst + 2 * S::X_PART) = lo;
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
@@ -590,7 +555,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
       for (int r = 1; r < STRETCHES; ++r)
         if (r < used) v += parts[r];
-      v = whole(v);
+      v *= BACK;
       if (n < a.N) {
         float* o = a.out + (size_t)m * a.ldo + n;
         if (fabsf(v) <= FLT_MAX) *o = a.accumulate ? *o + v : v;
@@ -648,7 +613,7 @@ int cluster_of(int tiles) {
 }
 
 template <bool FEW, bool CLUSTER, bool W_TMA>
-int launch_split(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap& ml, const Args& a, int blocks, cudaStream_t s) {
+int launch_split(const CUtensorMap& mw, const CUtensorMap& mx, const Args& a, int blocks, cudaStream_t s) {
   const int rc = allow_smem<FEW, CLUSTER, W_TMA>();
   if (rc != GI_OK) return rc;
   cudaLaunchConfig_t cfg = {};
@@ -671,11 +636,10 @@ int launch_split(const CUtensorMap& mw, const CUtensorMap& mh, const CUtensorMap
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
-  return gi::check(cudaLaunchKernelEx(&cfg, gemm_split_kernel<FEW, CLUSTER, W_TMA>, mw, mh, ml, a), "gemm_f32_split");
+  return gi::check(cudaLaunchKernelEx(&cfg, gemm_split_kernel<FEW, CLUSTER, W_TMA>, mw, mx, a), "gemm_f32_split");
 }
 
-int pad16(int m) { return (m + 15) / 16 * 16; }
-long plane_bytes(long rows, int chunks) { return rows * chunks * CK * 2; }
+long planes_bytes(long rows, int chunks) { return 3 * rows * chunks * CK * 2; }
 
 }  // namespace
 
@@ -684,7 +648,7 @@ extern "C" long gi_gemm_f32_split_scratch(int M, int N, int K) {
   if (M <= 0 || N < 1024 || K < 1024) return -1;
   if (M <= FEW_MAX) return 0;
   const int rows = M < SLAB ? M : SLAB, chunks = (K + CK - 1) / CK;
-  return 2 * plane_bytes(rows, chunks) + (long)chunks * (pad16(rows) + 128) * 4;
+  return planes_bytes(rows, chunks);
 }
 
 extern "C" int gi_gemm_f32_split(float* out, int mode, const float* A, const float* W, int M, int N, int K, long lda, long ldw, long ldo,
@@ -707,7 +671,7 @@ extern "C" int gi_gemm_f32_split(float* out, int mode, const float* A, const flo
   a.a_vec = (lda % 4 == 0 && ((uintptr_t)A & 15) == 0) ? 1 : 0;
   a.accumulate = mode == GI_GEMM_ACCUM_F32 ? 1 : 0;
   const bool w_tma = ldw % 4 == 0 && ((uintptr_t)W & 15) == 0 && K % 4 == 0;
-  CUtensorMap mw = {}, mh = {}, ml = {};
+  CUtensorMap mw = {}, mx = {};
   if (w_tma) {
     const int rc = gi::tensor_map_2d_ex(&mw, W, N, K, ldw, GI_F32, 32, ROWS);
     if (rc != GI_OK) return rc;
@@ -717,36 +681,32 @@ extern "C" int gi_gemm_f32_split(float* out, int mode, const float* A, const flo
     a.M = M; a.nt = FEW_TILE; a.tiles_m = (M + FEW_TILE - 1) / FEW_TILE; a.tiles = a.tiles_m * tiles_n;
     a.cluster = w_tma ? cluster_of<true>(a.tiles) : cluster_of<false>(a.tiles);
     if (a.cluster > 1)
-      return w_tma ? launch_split<true, true, true>(mw, mh, ml, a, a.tiles * a.cluster, s) : launch_split<true, true, false>(mw, mh, ml, a, a.tiles * a.cluster, s);
+      return w_tma ? launch_split<true, true, true>(mw, mx, a, a.tiles * a.cluster, s) : launch_split<true, true, false>(mw, mx, a, a.tiles * a.cluster, s);
     const int blocks = a.tiles < sms ? a.tiles : sms;
-    return w_tma ? launch_split<true, false, true>(mw, mh, ml, a, blocks, s) : launch_split<true, false, false>(mw, mh, ml, a, blocks, s);
+    return w_tma ? launch_split<true, false, true>(mw, mx, a, blocks, s) : launch_split<true, false, false>(mw, mx, a, blocks, s);
   }
   for (int m0 = 0; m0 < M; m0 += SLAB) {
     const int rows = M - m0 < SLAB ? M - m0 : SLAB;
-    unsigned char* hi = (unsigned char*)scratch;
-    unsigned char* lo = hi + plane_bytes(rows, a.chunks);
-    float* fx = reinterpret_cast<float*>(lo + plane_bytes(rows, a.chunks));
     a.out = out + (size_t)m0 * ldo;
     a.A = A + (size_t)m0 * lda;
     a.M = rows;
-    a.ldf = pad16(rows) + 128;
-    a.fx = fx;
-    int rc = gi::check(gi::launch(split_rows_kernel, dim3((unsigned)(((long)rows * a.chunks + 15) / 16)), dim3(256), 0, s, (uint2*)hi, (uint2*)lo, fx, a.A, lda,
-                                  rows, K, a.chunks, a.ldf, a.a_vec), "gemm_f32_split: tokens");
+    const long quads = (long)rows * a.chunks * (CK / 4);
+    int rc = gi::check(gi::launch(split_rows_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, s, (uint2*)scratch, a.A, lda, rows, K,
+                                  a.chunks, a.a_vec), "gemm_f32_split: tokens");
     if (rc != GI_OK) return rc;
-    // tokens a tile: a chunk takes a block about 512 + 5 tokens clocks (shared memory's and tensor memory's reads), a launch as
-    // many rounds of tiles as the fullest SM has
+    // tokens a tile: a chunk takes a block about 1,100 + 11 tokens clocks (2,048 x 8,192: 1,640 in tiles of 48, 2,000 in tiles of 80), a
+    // launch as many rounds of tiles as the fullest SM has
     long best = 0;
-    for (int nt = 16; nt <= 128; nt += 16) {
-      const long tiles = (long)((rows + nt - 1) / nt) * tiles_n, cost = (tiles + sms - 1) / sms * (512 + 5 * nt);
+    for (int nt = 16; nt <= Shape<false, false>::NT; nt += 16) {
+      const long tiles = (long)((rows + nt - 1) / nt) * tiles_n, cost = (tiles + sms - 1) / sms * (1100 + 11 * nt);
       if (best == 0 || cost <= best) best = cost, a.nt = nt, a.tiles_m = (rows + nt - 1) / nt;
     }
     a.tiles = a.tiles_m * tiles_n;
-    rc = gi::tensor_map_2d_ex(&mh, hi, rows, (long)a.chunks * CK, (long)a.chunks * CK, GI_BF16, 64, a.nt);
-    if (rc == GI_OK) rc = gi::tensor_map_2d_ex(&ml, lo, rows, (long)a.chunks * CK, (long)a.chunks * CK, GI_BF16, 64, a.nt);
+    // one map over the three planes (a tile's rows past the last token are the next plane's: nobody reads their results)
+    rc = gi::tensor_map_2d_ex(&mx, scratch, 3L * rows, (long)a.chunks * CK, (long)a.chunks * CK, GI_BF16, 64, a.nt);
     if (rc != GI_OK) return rc;
     const int blocks = a.tiles < sms ? a.tiles : sms;
-    rc = w_tma ? launch_split<false, false, true>(mw, mh, ml, a, blocks, s) : launch_split<false, false, false>(mw, mh, ml, a, blocks, s);
+    rc = w_tma ? launch_split<false, false, true>(mw, mx, a, blocks, s) : launch_split<false, false, false>(mw, mx, a, blocks, s);
     if (rc != GI_OK) return rc;
   }
   return GI_OK;

@@ -530,7 +530,7 @@ def one_token_step(on: bool):
 def gemm_generic(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None,
                  out_dtype: Optional[torch.dtype] = None, accumulate: bool = False) -> torch.Tensor:
     """out[M, N] (+)= a[M, K] @ w[N, K]^T with 32-bit accumulation: in float32 the matrices of 1,024 rows and columns or more
-    on tensor cores (every number in two 16-bit parts; not within `one_token_step`), the rest on CUDA cores."""
+    on tensor cores (every number as the sum of three 16-bit parts; not within `one_token_step`), the rest on CUDA cores."""
     lib = _bind()
     _cuda(a, "activations")
     _cuda(w, "weights")
