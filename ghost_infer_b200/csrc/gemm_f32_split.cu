@@ -56,19 +56,15 @@ constexpr uint32_t W_STAGE = ROWS * CK * 4;
 
 __device__ int g_split_status = 0;
 
-// A wait of this kernel is over in microseconds (its inputs are complete when it starts); it gives up after a second or so.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int who) {
-  for (uint32_t i = 0; i < (1u << 20); ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  atomicCAS(&g_split_status, 0, who);
-  return false;
-}
+// No wait depends on what the numbers are but for the time that a tile full of results that are no finite numbers takes (a few
+// milliseconds); all end after WAIT_LIMIT tries.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int who) { return gi::tc::mbar_wait(bar, parity, who, &g_split_status); }
 
 struct Args {
   float* out;
   const float *A, *W;
   long lda, ldw, ldo;
-  int M, N, K, nt, tiles_m, tiles, chunks, per_stretch, seg, cluster, a_vec, accumulate;
+  int M, N, K, nt, tiles_m, tiles, chunks, per_stretch, seg, cluster, a_vec, w_vec, accumulate;
 };
 
 template <bool FEW, bool CLUSTER>
@@ -176,11 +172,18 @@ __device__ __forceinline__ void cluster_sync() {
 // one result by plain multiply-adds, in the order of gemm_f32.cu
 __device__ __noinline__ void plain_result(const Args& args, int m, int n) {
   const float *a = args.A + (size_t)m * args.lda, *w = args.W + (size_t)n * args.ldw;
+  const bool vec = args.a_vec && args.w_vec;
   float sum = 0.f;
   for (int s = 0; s < args.K; s += args.seg) {
     float even = 0.f, odd = 0.f;
     const int end = min(args.K, s + args.seg);
-    for (int k = s; k < end; k += 2) {
+    int k = s;
+    for (; vec && k + 4 <= end; k += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
+      even = fmaf(x.z, y.z, fmaf(x.x, y.x, even));
+      odd = fmaf(x.w, y.w, fmaf(x.y, y.y, odd));
+    }
+    for (; k < end; k += 2) {
       even = fmaf(a[k], w[k], even);
       if (k + 1 < end) odd = fmaf(a[k + 1], w[k + 1], odd);
     }
@@ -188,6 +191,18 @@ __device__ __noinline__ void plain_result(const Args& args, int m, int n) {
   }
   float* o = args.out + (size_t)m * args.ldo + n;
   *o = args.accumulate ? *o + sum : sum;
+}
+// A warp's results of token m that are no finite numbers (`mine`: this lane's is none).  A token that holds a NaN has no other results,
+// and reading it is all that takes: a sequence that has diverged does not hold up the others of its step.
+__device__ __noinline__ void again(const Args& args, int m, int n, bool mine) {
+  const float* a = args.A + (size_t)m * args.lda;
+  bool nan = false;
+  for (int k = threadIdx.x & 31; k < args.K; k += 32) nan |= a[k] != a[k];
+  if (__any_sync(0xffffffffu, nan)) {
+    if (mine) args.out[(size_t)m * args.ldo + n] = __int_as_float(0x7fffffff);
+  } else if (mine) {
+    plain_result(args, m, n);
+  }
 }
 
 // Splits `rows` rows of A into three planes [rows][chunks * 64] of 16-bit parts (zeros past K), four numbers a thread.
@@ -483,9 +498,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
           }
         }
-        for (; odd; odd &= odd - 1) {
-          const int i = __ffs((int)odd) - 1;
-          plain_result(a, m0 + col_of(i / GROUP) + i % GROUP, n);
+        for (uint32_t rest = __reduce_or_sync(0xffffffffu, odd); rest; rest &= rest - 1) {
+          const int i = __ffs((int)rest) - 1;
+          again(a, m0 + col_of(i / GROUP) + i % GROUP, n, (odd >> i & 1) != 0);
         }
       }
     }
@@ -546,7 +561,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const int used = (a.chunks + a.per_stretch - 1) / a.per_stretch;
     const uint32_t red = smem_u32(smem + S::RED_AT);
     const int m0 = tile0 % a.tiles_m * FEW_TILE, n0 = tile0 / a.tiles_m * ROWS;
-    for (int i = rank * S::THREADS + (int)threadIdx.x; i < min(FEW_TILE, a.M - m0) * ROWS; i += a.cluster * S::THREADS) {
+    for (int i = rank * S::THREADS + (int)threadIdx.x; i < min(FEW_TILE, a.M - m0) * ROWS; i += a.cluster * S::THREADS) {     // whole warps
       const int m = m0 + i / ROWS, n = n0 + i % ROWS;
       float parts[STRETCHES];
 #pragma unroll
@@ -556,11 +571,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       for (int r = 1; r < STRETCHES; ++r)
         if (r < used) v += parts[r];
       v *= BACK;
-      if (n < a.N) {
+      const bool fine = fabsf(v) <= FLT_MAX;
+      if (n < a.N && fine) {
         float* o = a.out + (size_t)m * a.ldo + n;
-        if (fabsf(v) <= FLT_MAX) *o = a.accumulate ? *o + v : v;
-        else plain_result(a, m, n);
+        *o = a.accumulate ? *o + v : v;
       }
+      const bool odd = n < a.N && !fine;
+      if (__any_sync(0xffffffffu, odd)) again(a, m, n, odd);
     }
     cluster_sync();                                          // nobody leaves while its sums are read
   }
@@ -669,8 +686,9 @@ extern "C" int gi_gemm_f32_split(float* out, int mode, const float* A, const flo
   a.per_stretch = (a.chunks + STRETCHES - 1) / STRETCHES;
   a.seg = gi::sum_segment(K);
   a.a_vec = (lda % 4 == 0 && ((uintptr_t)A & 15) == 0) ? 1 : 0;
+  a.w_vec = (ldw % 4 == 0 && ((uintptr_t)W & 15) == 0) ? 1 : 0;
   a.accumulate = mode == GI_GEMM_ACCUM_F32 ? 1 : 0;
-  const bool w_tma = ldw % 4 == 0 && ((uintptr_t)W & 15) == 0 && K % 4 == 0;
+  const bool w_tma = a.w_vec && K % 4 == 0;
   CUtensorMap mw = {}, mx = {};
   if (w_tma) {
     const int rc = gi::tensor_map_2d_ex(&mw, W, N, K, ldw, GI_F32, 32, ROWS);
