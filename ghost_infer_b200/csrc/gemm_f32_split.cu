@@ -290,7 +290,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   if (warp == 0) {
     if (lane == 0 && (W_TMA || !FEW)) {
       bool ok = true;
-      int it = 0, loaded = 0;
+      int it = 0, w_loaded = 0, x_loaded = 0;
       for (int tile = tile0; tile < a.tiles && ok; tile += tile_step) {
         const int m0 = tile % a.tiles_m * a.nt, n0 = tile / a.tiles_m * ROWS;
         for (int c = c_first; c < c_last && ok; ++c, ++it) {
@@ -302,6 +302,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             const uint32_t dst = smem_u32(smem + st * W_STAGE);
             tma_load_2d(dst, &map_w, c * CK, n0, w_full + 8 * st);
             tma_load_2d(dst + W_STAGE / 2, &map_w, c * CK + 32, n0, w_full + 8 * st);
+            ++w_loaded;
           }
           if (!FEW) {
             const int st = it % S::X_STAGES, slot = it % S::SLOTS;
@@ -310,13 +311,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             const uint32_t dst = smem_u32(smem + S::X_AT + st * S::X_STAGE), bar = full + 8 * slot;
             mbar_expect_tx(bar, (uint32_t)a.nt * 384u);
             for (int p = 0; p < 3; ++p) tma_load_2d(dst + p * S::X_PART, &map_x, c * CK, p * a.M + m0, bar);
+            ++x_loaded;
           }
-          ++loaded;
         }
       }
       // the block does not leave before its copies have landed, also where somebody gave up
-      for (int i = max(0, loaded - S::W_STAGES); W_TMA && i < loaded; ++i) mbar_wait(w_full + 8 * (i % S::W_STAGES), (uint32_t)((i / S::W_STAGES) & 1), 1);
-      for (int i = max(0, loaded - S::X_STAGES); !FEW && i < loaded; ++i) wait_full(i, 1);
+      for (int i = max(0, w_loaded - S::W_STAGES); i < w_loaded; ++i) mbar_wait(w_full + 8 * (i % S::W_STAGES), (uint32_t)((i / S::W_STAGES) & 1), 1);
+      for (int i = max(0, x_loaded - S::X_STAGES); i < x_loaded; ++i) wait_full(i, 1);
     }
   } else if (warp == 1) {
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.nt >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);   // float sums of bfloat16

@@ -232,6 +232,34 @@ def test_no_order_of_events_shows_stale_data(few, cluster, w_tma, tiles, chunks)
         walk(seed, k, few, cluster, w_tma, tiles, chunks)
 
 
+@pytest.mark.parametrize("few,cluster", [(True, False), (False, False)])
+def test_a_thread_that_gives_up_waits_for_all_its_copies(few, cluster):
+    """The loading thread may give up between a chunk's rows of W, which it has asked for by then, and its tokens."""
+    text, k = source(), kernel(few, cluster)
+    counts = {}
+    for kind, stages in (("w", "w_stages"), ("x", "x_stages")):
+        # counted behind its own copies, and as many of the last ones waited for as are under way
+        assert re.search(rf"tma_load_2d\([^;]*&map_{kind}[^;]*;(?: }})? \+\+{kind}_loaded;", text), kind
+        assert re.search(rf"for \(int i = max\(0, {kind}_loaded - S::{kind.upper()}_STAGES\); i < {kind}_loaded; \+\+i\)", text), kind
+        counts[kind] = k[stages]
+    for given_up_at in range(2 * 12):
+        issued, loaded, place = set(), {"w": 0, "x": 0}, 0
+        for it in range(12):
+            for kind in "wx":
+                if kind == "x" and few:
+                    continue
+                if place == given_up_at:
+                    break
+                place += 1
+                issued = {c for c in issued if c[0] != kind or c[1] > it - counts[kind]} | {(kind, it)}     # the one before in its place has landed
+                loaded[kind] += 1
+            else:
+                continue
+            break
+        waited = {(kind, i) for kind in "wx" for i in range(max(0, loaded[kind] - counts[kind]), loaded[kind])}
+        assert issued <= waited
+
+
 @pytest.mark.parametrize("change", [dict(w_stages=3), dict(count_small=4), dict(drained_for=2), dict(behind_a=5)])
 def test_a_barrier_that_does_not_fit_is_found_out(change):
     """A ring that two sets share unevenly, a barrier that some of its warps do not count for, an accumulator drained for the wrong
