@@ -551,8 +551,10 @@ def gemm_generic(a: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor
         need = lib.gi_gemm_f32_split_scratch(m, n, k)
         if need >= 0:                        # a larger matrix: on the tensor cores, whatever the rows
             scratch = torch.empty((need,), dtype=torch.uint8, device=a.device) if need > 0 else None
+            # few tokens: one launch; more: two for every 8,192 of them
             _check(lib, lib.gi_gemm_f32_split(out.data_ptr(), mode, a.data_ptr(), w.data_ptr(), m, n, k, lda, ldw, ldo,
-                                              scratch.data_ptr() if scratch is not None else None, need, _stream()), 2 if need > 0 else 1)
+                                              scratch.data_ptr() if scratch is not None else None, need, _stream()),
+                   2 * ((m + 8191) // 8192) if need > 0 else 1)
             return out
     _check(lib, lib.gi_gemm_generic(out.data_ptr(), _dt(out, "output"), mode, a.data_ptr(), _dt(a, "activations"),
                                     w.data_ptr(), _dt(w, "weights"), m, n, k, lda, ldw, ldo, _stream()))

@@ -171,6 +171,18 @@ def test_the_kind_of_step_decides_between_the_kernels(m):
     assert torch.equal(ops.gemm_generic(a, small), plain(a, small))
 
 
+@pytest.mark.parametrize("m,launches", [(32, 1), (33, 2), (8192, 2), (8193, 4)])
+def test_launches_are_counted(m, launches):
+    a, w = torch.zeros((m, 1024), device=DEV), torch.zeros((1024, 1024), device=DEV)
+    ops.gemm_generic(a, w)
+    before = ops.launches
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ops.gemm_generic(a, w)
+        torch.cuda.synchronize()
+    ours = [e for e in prof.events() if "split" in e.name and e.device_type == torch.autograd.DeviceType.CUDA]
+    assert ops.launches - before == launches == len(ours)
+
+
 @pytest.fixture(scope="module")
 def wide_engine(tmp_path_factory):
     """Widths from which the prompts' products run on tensor cores."""
