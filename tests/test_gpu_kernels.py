@@ -1112,7 +1112,12 @@ def test_prompt_attention_with_one_row_warp_far_behind_the_others(hd, slow_warp)
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_float32_products_share_one_order_of_additions(m, n, k, accumulate):
     """The kernels of few and of many rows and the general one (which takes rows that start off a 16-byte boundary) give
-    the same bits; |error| <= (terms in a chain + chains + 2) * 2^-24 * sum |a w|, the bound of any summation."""
+    the same bits; |error| <= (terms in a chain + chains + 2) * 2^-24 * sum |a w|, the bound of any summation.  (As in a step of
+    one token a sequence: in others the larger matrices are the tensor cores'.)"""
+    def times(a, w, **kw):
+        with ops.one_token_step(True):
+            return ops.gemm_generic(a, w, **kw)
+
     gen = torch.Generator(device=DEV)
     gen.manual_seed(m * 7 + n + k)
     a = torch.randn((m, k), generator=gen, device=DEV)
@@ -1121,16 +1126,16 @@ def test_float32_products_share_one_order_of_additions(m, n, k, accumulate):
 
     def product(a, w):
         if not accumulate:
-            return ops.gemm_generic(a, w)
+            return times(a, w)
         out = start.clone()
-        return ops.gemm_generic(a, w, out=out, accumulate=True)
+        return times(a, w, out=out, accumulate=True)
 
     got = product(a, w)
     odd = torch.empty((n, k + 1), device=DEV)
     odd[:, :k] = w
     assert torch.equal(got, product(a, odd[:, :k]))                      # general kernel
-    assert torch.equal(got[:1], ops.gemm_generic(a[:1], w, out=start[:1].clone(), accumulate=True) if accumulate else ops.gemm_generic(a[:1], w))
-    many = ops.gemm_generic(a.repeat((600 + m - 1) // m, 1), w)          # enough rows for the tiled kernel
+    assert torch.equal(got[:1], times(a[:1], w, out=start[:1].clone(), accumulate=True) if accumulate else times(a[:1], w))
+    many = times(a.repeat((600 + m - 1) // m, 1), w)          # enough rows for the tiled kernel
     assert accumulate or torch.equal(got, many[:m])
     chain = ((k + 31) // 32 + 31) // 32 * 16
     exact = a.double() @ w.double().T + (start.double() if accumulate else 0)
