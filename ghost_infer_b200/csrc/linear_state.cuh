@@ -113,16 +113,18 @@ struct LsArgs {
 // tokens per chunk: two buffers of it stay under 48 KB of shared memory
 template <int KR> struct LsChunk { static constexpr int value = KR >= 32 ? 8 : 16; };
 
-// WALK: the step holds sequences of many tokens, and eight whole tokens run without a test between them; without it (steps
-// of one token a sequence) the kernel is the same but smaller, so that two blocks fit an SM at every tile width.
-// Two blocks an SM for the narrower tiles too: a grid of about as many blocks as SMs times two then runs as one round.
+// For steps in which some sequence brings several tokens; the others (about one token a sequence) take linear_state_step_kernel.
+// Two blocks an SM for the narrower tiles: a grid of about as many blocks as SMs times two then runs as one round.
 // C: columns a thread holds.  A token's key and query (and decays) leave shared memory once per thread, sixteen bytes a lane, and
 // a walk with one column a thread spends about half its time on that (four wavefronts a load, eight loads a token and warp);
-// without the delta rule a thread therefore holds several columns, two numbers an instruction.  B200: turned queries and keys,
-// 8 prompts of 150 to 410 tokens, 16 heads of 128 x 128: 248 us a launch, 407 with one column; decays per key, prompts of 1,203,
-// 501 and 852 tokens, 12 heads of 96 x 64 (tiles of 8 columns): 148 us, 207 with the divisions in every chunk, 225 before.
-template <typename T, int KR, int COLS, int C, bool DELTA, bool WALK, bool ROT, bool KEYED>
-__global__ void __launch_bounds__(COLS / C * LS_LANES + LS_PREP, (COLS <= 16 || !WALK || (C > 1 && KR < 32)) ? 2 : 1)
+// without the delta rule a thread therefore holds several columns, two numbers an instruction.  B200, us a launch with several and with
+// one column: 8 prompts of 150 to 410 tokens, 16 heads of 128 x 128 (tiles of 32, four columns): turned 191 and 306, keyed 175 and 310,
+// constant decays 256 and 365, ready-made gates 154 and 224; 8 heads of 256 x 256 (two columns): 416 and 586, 365 and 586, 646 and 670, 277
+// and 412.  One prompt of 2,048 tokens in tiles of 8 (two columns): 16 heads of 128 x 128 308 and 367, 263 and 314, 517 and 494, 222 and
+// 250; where the grid is no more than a block an SM a warp's own length is all there is, and one column would be faster with
+// gates and decays per key (12 heads of 96 x 64: 236 and 256, 213 and 191, 449 and 439, 197 and 158).
+template <typename T, int KR, int COLS, int C, bool DELTA, bool ROT, bool KEYED>
+__global__ void __launch_bounds__(COLS / C * LS_LANES + LS_PREP, (COLS <= 16 || (C > 1 && KR < 32)) ? 2 : 1)
 linear_state_kernel(const LsArgs a) {
   constexpr int Kp = KR * LS_LANES;            // rows with padding
   constexpr int M = KR / 4;                    // groups of four rows per lane; also a preparing lane's share of a row
@@ -452,7 +454,7 @@ linear_state_kernel(const LsArgs a) {
     };
     for (int t0 = 0; t0 < n; t0 += LS_TB) {
       float acc[LS_TB * C];                              // [token][column]
-      if (WALK && t0 + LS_TB <= n) {     // eight whole tokens: nothing to test between them, so the next one's loads start early
+      if (t0 + LS_TB <= n) {     // eight whole tokens: nothing to test between them, so the next one's loads start early
 #pragma unroll
         for (int tl = 0; tl < LS_TB; ++tl) token(t0 + tl, acc + tl * C);
       } else {
@@ -495,14 +497,16 @@ linear_state_kernel(const LsArgs a) {
   }
 }
 
-// The same walk for a step of about one token a sequence, without the delta rule, unit vectors or ready-made gates: bound by the
-// bytes of S and the trips to memory, of which the kernel above makes three one after the other (rows, the barrier behind their
-// preparation, S beside it) with a third of its threads waiting.  Here the threads that hold S prepare the token themselves;
-// S is asked for in L2 before the dependency wait (a prefetch reads no values) and loaded beside the rows.  64 registers and
-// 256 threads: four blocks an SM, where the other has two.  Every sum has the other's order, so the bits are the same.  B200, in a
-// step of 8 sequences (16 heads of 128 x 128, 17 MB of state read and written): 5.3 us of the step's time, 16.7 before.
-template <typename T, int KR, int COLS, bool ROT, bool KEYED>
-__global__ void __launch_bounds__(COLS * LS_LANES, 1024 / (COLS * LS_LANES))
+// The same walk for a step of about one token a sequence: bound by the bytes of S and the trips to memory, of which the kernel
+// above would make three one after the other (rows, the barrier behind their preparation, S beside it) with a third of its threads
+// waiting.  Here the threads that hold S prepare the token themselves; S is asked for in L2 before the dependency wait (a prefetch
+// reads no values) and loaded beside the rows.  64 registers and 256 threads: four blocks an SM, where the other has two (keys of more
+// than 128 numbers: 128 registers, two).  Every sum has the other's order, so the bits are the same.  B200, in a step of 8
+// sequences (16 heads of 128 x 128, 17 MB of state read and written): 5.3 us of the step's time, 16.7 in the kernel above.  One launch
+// of 64 sequences, us, here and there: the same heads turned 31 and 66, constant decays 37 and 72, ready-made gates 35 and 50 (64 with
+// several columns a thread), delta rule 35 and 82; 8 heads of 256 x 256 66 and 84, delta rule 74 and 111.
+template <typename T, int KR, int COLS, bool DELTA, bool ROT, bool KEYED>
+__global__ void __launch_bounds__(COLS * LS_LANES, (KR < 32 ? 1024 : 512) / (COLS * LS_LANES))
 linear_state_step_kernel(const __grid_constant__ LsArgs a) {
   constexpr int Kp = KR * LS_LANES, M = KR / 4, NC = COLS * LS_LANES;
   __shared__ __align__(16) float sq[Kp], sk[Kp], sd[KEYED ? Kp : 1], sv[COLS];
@@ -522,7 +526,9 @@ linear_state_step_kernel(const __grid_constant__ LsArgs a) {
   gi::pdl_wait();
   const int tok0 = a.cu_seqlens[b], qlen = a.cu_seqlens[b + 1] - tok0;
   if (qlen <= 0) return;
-  const float dc = KEYED ? 1.0f : a.decay_c[h];
+  constexpr bool GATES = !ROT && !KEYED;               // projected or ready made, and unit vectors
+  const float dc = KEYED || a.decay_c == nullptr ? 1.0f : a.decay_c[h];
+  const float rate = GATES && a.a_in != nullptr ? expf(dc) : 0.f, bias = GATES && a.a_in != nullptr && a.dt_bias != nullptr ? a.dt_bias[h] : 0.f;
   const int hk = h / (a.heads / a.qk_heads);
   float S[KR];
 #pragma unroll
@@ -547,6 +553,13 @@ linear_state_step_kernel(const __grid_constant__ LsArgs a) {
     const size_t tok = (size_t)tok0 + t;
     const T *q = (const T*)a.q + tok * a.ldq + (size_t)hk * K, *k = (const T*)a.k + tok * a.ldk + (size_t)hk * K;
     if (t > 0) __syncthreads();                        // the token before is used up
+    float g = dc, strength = 1.f;
+    if (GATES) {
+      if (a.a_in != nullptr) g = expf(-rate * ls_softplus(gi::ldf((const T*)a.a_in + tok * a.lda + h) + bias));
+      if (DELTA) strength = 1.0f / (1.0f + expf(-gi::ldf((const T*)a.b_in + tok * a.ldb + h)));
+      if (a.g_direct != nullptr) g = a.g_direct[tok * a.heads + h];
+      if (!DELTA && a.u_direct != nullptr) strength = a.u_direct[tok * a.heads + h];
+    }
     // a pair that turns is loaded, turned and stored by one thread; the numbers past the pairs one a thread
     auto query = [&](int i) { const float v = gi::ldf(q + i); return (act ? ls_silu(v) : v) * qs; };
     auto key = [&](int i) { const float v = gi::ldf(k + i); return (act ? ls_silu(v) : v) * ks; };
@@ -571,7 +584,46 @@ linear_state_step_kernel(const __grid_constant__ LsArgs a) {
       sv[tid] = act ? ls_silu(v) : v;
     }
     __syncthreads();
-    const float u = j < V ? sv[col] : 0.f;
+    if (GATES && a.unit_norm) {
+      if (tid < 32) {
+        float qv[M], kv[M], s1 = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+          qv[i] = sq[tid + 32 * i];
+          kv[i] = sk[tid + 32 * i];
+          s1 = fmaf(qv[i], qv[i], s1);
+          s2 = fmaf(kv[i], kv[i], s2);
+        }
+        s1 = gi::warp_sum(s1);
+        s2 = gi::warp_sum(s2);
+        const float fq = a.q_scale / sqrtf(s1 + a.norm_eps), fk = 1.0f / sqrtf(s2 + a.norm_eps);
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+          sq[tid + 32 * i] = qv[i] * fq;
+          sk[tid + 32 * i] = kv[i] * fk;
+        }
+      }
+      __syncthreads();
+    }
+    float u = j < V ? sv[col] : 0.f;
+    if (DELTA) {
+      float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const float4 k4 = *reinterpret_cast<const float4*>(sk + 4 * (lane + LS_LANES * m));
+        d0 = fmaf(S[4 * m], k4.x, d0);
+        d1 = fmaf(S[4 * m + 1], k4.y, d1);
+        d2 = fmaf(S[4 * m + 2], k4.z, d2);
+        d3 = fmaf(S[4 * m + 3], k4.w, d3);
+      }
+      float d = (d0 + d1) + (d2 + d3);
+      d += __shfl_xor_sync(0xffffffffu, d, 1);
+      d += __shfl_xor_sync(0xffffffffu, d, 2);
+      d += __shfl_xor_sync(0xffffffffu, d, 4);
+      u = strength * (u - g * d);
+    } else if (GATES && a.u_direct != nullptr) {
+      u *= strength;
+    }
     float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
 #pragma unroll
     for (int m = 0; m < M; ++m) {
@@ -581,10 +633,10 @@ linear_state_step_kernel(const __grid_constant__ LsArgs a) {
         const float4 d4 = *reinterpret_cast<const float4*>(sd + i);
         S[4 * m] *= d4.x; S[4 * m + 1] *= d4.y; S[4 * m + 2] *= d4.z; S[4 * m + 3] *= d4.w;
       }
-      S[4 * m] = fmaf(k4.x, u, dc * S[4 * m]);
-      S[4 * m + 1] = fmaf(k4.y, u, dc * S[4 * m + 1]);
-      S[4 * m + 2] = fmaf(k4.z, u, dc * S[4 * m + 2]);
-      S[4 * m + 3] = fmaf(k4.w, u, dc * S[4 * m + 3]);
+      S[4 * m] = fmaf(k4.x, u, g * S[4 * m]);
+      S[4 * m + 1] = fmaf(k4.y, u, g * S[4 * m + 1]);
+      S[4 * m + 2] = fmaf(k4.z, u, g * S[4 * m + 2]);
+      S[4 * m + 3] = fmaf(k4.w, u, g * S[4 * m + 3]);
       a0 = fmaf(S[4 * m], q4.x, a0);
       a1 = fmaf(S[4 * m + 1], q4.y, a1);
       a2 = fmaf(S[4 * m + 2], q4.z, a2);
@@ -620,56 +672,51 @@ int ls_sm_count() {
 }
 
 template <typename T, int KR, int COLS, bool ROT, bool KEYED>
-cudaError_t ls_launch(const LsArgs& a, int n_seqs, bool delta, bool walk, cudaStream_t stream) {
+cudaError_t ls_launch(const LsArgs& a, int n_seqs, bool delta, cudaStream_t stream) {
   constexpr int CH = LsChunk<KR>::value;
   // columns a thread: wide tiles come with many blocks, narrow ones with few, whose warps' own length counts more
   constexpr int C = KR < 32 && COLS >= 32 ? 4 : 2;
   const size_t smem = 2 * (size_t)((KEYED ? 3 : 2) * CH * KR * LS_LANES + 2 * CH * COLS + 2 * CH) * sizeof(float);
   const dim3 grid(a.heads, n_seqs, (a.V + COLS - 1) / COLS), block((delta ? COLS : COLS / C) * LS_LANES + LS_PREP);
   if constexpr (KEYED) {
-    auto kern = walk ? linear_state_kernel<T, KR, COLS, C, false, true, false, true> : linear_state_kernel<T, KR, COLS, C, false, false, false, true>;
+    auto kern = linear_state_kernel<T, KR, COLS, C, false, false, true>;
     if (smem > 48 * 1024) {
-      static bool configured[2][gi::MAX_DEVICES_SEEN] = {};
+      static bool configured[gi::MAX_DEVICES_SEEN] = {};
       int dev;
-      if (gi::unconfigured_here(configured[walk ? 1 : 0], &dev)) {
+      if (gi::unconfigured_here(configured, &dev)) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        if (dev >= 0) configured[walk ? 1 : 0][dev] = true;
+        if (dev >= 0) configured[dev] = true;
       }
     }
     return gi::launch(kern, grid, block, smem, stream, a);
   } else if constexpr (ROT) {
-    return walk ? gi::launch(linear_state_kernel<T, KR, COLS, C, false, true, true, false>, grid, block, smem, stream, a)
-                : gi::launch(linear_state_kernel<T, KR, COLS, C, false, false, true, false>, grid, block, smem, stream, a);
+    return gi::launch(linear_state_kernel<T, KR, COLS, C, false, true, false>, grid, block, smem, stream, a);
   } else {
-    if (walk)
-      return delta ? gi::launch(linear_state_kernel<T, KR, COLS, 1, true, true, false, false>, grid, block, smem, stream, a)
-                   : gi::launch(linear_state_kernel<T, KR, COLS, C, false, true, false, false>, grid, block, smem, stream, a);
-    return delta ? gi::launch(linear_state_kernel<T, KR, COLS, 1, true, false, false, false>, grid, block, smem, stream, a)
-                 : gi::launch(linear_state_kernel<T, KR, COLS, C, false, false, false, false>, grid, block, smem, stream, a);
+    return delta ? gi::launch(linear_state_kernel<T, KR, COLS, 1, true, false, false>, grid, block, smem, stream, a)
+                 : gi::launch(linear_state_kernel<T, KR, COLS, C, false, false, false>, grid, block, smem, stream, a);
   }
 }
 
-template <typename T, int KR, bool ROT, bool KEYED>
-cudaError_t ls_launch_step(const LsArgs& a, int n_seqs, cudaStream_t stream) {
-  const long per = (long)a.heads * n_seqs, sms = ls_sm_count();
-  const auto grid = [&](int cols) { return dim3(a.heads, n_seqs, (a.V + cols - 1) / cols); };
-  if (per * ((a.V + 31) / 32) >= sms || a.V <= 8) return gi::launch(linear_state_step_kernel<T, KR, 32, ROT, KEYED>, grid(32), dim3(32 * LS_LANES), 0, stream, a);
-  if (per * ((a.V + 15) / 16) >= sms) return gi::launch(linear_state_step_kernel<T, KR, 16, ROT, KEYED>, grid(16), dim3(16 * LS_LANES), 0, stream, a);
-  return gi::launch(linear_state_step_kernel<T, KR, 8, ROT, KEYED>, grid(8), dim3(8 * LS_LANES), 0, stream, a);
+template <typename T, int KR, int COLS, bool ROT, bool KEYED>
+cudaError_t ls_launch_step(const LsArgs& a, int n_seqs, bool delta, cudaStream_t stream) {
+  const dim3 grid(a.heads, n_seqs, (a.V + COLS - 1) / COLS), block(COLS * LS_LANES);
+  if constexpr (!ROT && !KEYED) {
+    if (delta) return gi::launch(linear_state_step_kernel<T, KR, COLS, true, false, false>, grid, block, 0, stream, a);
+  }
+  return gi::launch(linear_state_step_kernel<T, KR, COLS, false, ROT, KEYED>, grid, block, 0, stream, a);
 }
 
 template <typename T, int KR, bool ROT, bool KEYED>
 cudaError_t ls_pick_tile(const LsArgs& a, int n_seqs, bool delta, bool walk, cudaStream_t stream) {
-  if constexpr (KR < 32) {
-    if (!walk && !delta && !a.unit_norm && !a.a_in && !a.b_in && !a.g_direct && !a.u_direct) return ls_launch_step<T, KR, ROT, KEYED>(a, n_seqs, stream);
-  }
   // the widest tile that still gives every SM a block: with fewer blocks than SMs the token-by-token walk, whose length a
   // block cannot shorten, runs on a part of the device only
   const long per = (long)a.heads * n_seqs, sms = ls_sm_count();
-  if (per * ((a.V + 31) / 32) >= sms || a.V <= 8) return ls_launch<T, KR, 32, ROT, KEYED>(a, n_seqs, delta, walk, stream);
-  if (per * ((a.V + 15) / 16) >= sms) return ls_launch<T, KR, 16, ROT, KEYED>(a, n_seqs, delta, walk, stream);
-  return ls_launch<T, KR, 8, ROT, KEYED>(a, n_seqs, delta, walk, stream);
+  if (per * ((a.V + 31) / 32) >= sms || a.V <= 8)
+    return walk ? ls_launch<T, KR, 32, ROT, KEYED>(a, n_seqs, delta, stream) : ls_launch_step<T, KR, 32, ROT, KEYED>(a, n_seqs, delta, stream);
+  if (per * ((a.V + 15) / 16) >= sms)
+    return walk ? ls_launch<T, KR, 16, ROT, KEYED>(a, n_seqs, delta, stream) : ls_launch_step<T, KR, 16, ROT, KEYED>(a, n_seqs, delta, stream);
+  return walk ? ls_launch<T, KR, 8, ROT, KEYED>(a, n_seqs, delta, stream) : ls_launch_step<T, KR, 8, ROT, KEYED>(a, n_seqs, delta, stream);
 }
 
 // What every entry point checks and fills in alike (the pointers and sizes are set).

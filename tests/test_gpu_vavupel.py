@@ -419,6 +419,57 @@ def test_recurrences_give_the_same_bits_in_every_tile(dtype, keyed, dim, vdim):
         assert torch.equal(got, want) and torch.equal(state, want_state)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["constant", "silu", "gates", "delta"])
+@pytest.mark.parametrize("dim,vdim", [(20, 40), (96, 64), (200, 33), (256, 64)])
+def test_plain_recurrences_give_the_same_bits_in_every_tile(dtype, kind, dim, vdim):
+    """As above, for constant decays (also with silu on the way in), ready-made gates and the delta rule."""
+    from ghost_infer_b200.kernels import ops
+    heads, seqs, n = 8, 24, 18
+    g = torch.Generator(device="cuda:0").manual_seed(dim + vdim)
+    rnd = lambda *s: torch.randn(s, device="cuda:0", generator=g)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda:0")
+    q, k, v = rnd(seqs, n, heads * dim).to(dtype), (rnd(seqs, n, heads * dim) * dim ** -0.5).to(dtype), rnd(seqs, n, heads * vdim).to(dtype)
+    decay, beta = torch.rand(heads, device="cuda:0", generator=g) ** 0.1, rnd(seqs, n, heads).to(dtype)
+    keep, put = torch.rand((seqs, n, heads), device="cuda:0", generator=g), torch.rand((seqs, n, heads), device="cuda:0", generator=g)
+    first = rnd(seqs + 1, heads * dim * vdim)
+
+    def run(parts):
+        state, out = first.clone(), torch.zeros((seqs, n, heads * vdim), device="cuda:0")
+        for who, a, b in parts:
+            step = type("S", (), {})()
+            step.cu_seqlens, step.seq_slots, step.n_seqs = i32([i * (b - a) for i in range(len(who) + 1)]), i32(who), len(who)
+            qq, kk, vv, bb, ke, pu = (t[who, a:b].reshape(len(who) * (b - a), -1).contiguous() for t in (q, k, v, beta, keep, put))
+            if kind == "gates":
+                o = ops.linear_state_gated(qq, kk, vv, state, step, heads, dim, vdim, ke, pu)
+            elif kind == "delta":
+                o = ops.linear_state(qq, kk, vv, state, step, heads, heads, dim, vdim, decay, decay_in=bb, dt_bias=decay, beta_in=bb, unit_norm=True, delta=True)
+            else:
+                o = ops.linear_state(qq, kk, vv, state, step, heads, heads, dim, vdim, decay, in_act=kind == "silu")
+            out[who, a:b] = o.view(len(who), b - a, -1)
+        return out, state
+
+    every = list(range(seqs))
+    want, want_state = run([(every, 0, n)])
+    assert bool(torch.isfinite(want).all())
+    if kind in ("constant", "gates"):                    # in 64 bits: S <- g S + k (u v)^T, o = S^T q
+        s, exact, size = first[:seqs].double().view(seqs, heads, vdim, dim), [], []
+        big = s.abs()
+        for t in range(n):
+            kt, qt, vt = (x[:, t].double().view(seqs, heads, -1) for x in (k, q, v))
+            f, u = (keep[:, t], put[:, t]) if kind == "gates" else (decay.expand(seqs, heads), torch.ones((seqs, heads), device="cuda:0"))
+            f, w = f.double()[..., None, None], (vt * u.double()[..., None])[..., None] * kt[:, :, None]
+            s, big = f * s + w, f * big + w.abs()
+            exact.append((s * qt[:, :, None]).sum(-1).view(seqs, -1))
+            size.append((big * qt[:, :, None].abs()).sum(-1).view(seqs, -1))
+        # three roundings a token, and at most dim / 8 + 8 additions a sum
+        assert ((want.double() - torch.stack(exact, 1)).abs() <= torch.stack(size, 1) * (3 * n + dim / 8 + 8) * 2.0 ** -24).all()
+    for parts in ([([i], 0, n) for i in every], [(every[:5], 0, n), (every[5:], 0, n)], [(every, 0, 16), (every, 16, 17), (every, 17, n)],
+                  [([i], 0, 16) for i in every] + [([i], t, t + 1) for t in (16, 17) for i in every]):
+        got, state = run(parts)
+        assert torch.equal(got, want) and torch.equal(state, want_state)
+
+
 @pytest.mark.parametrize("rows", [1, 5, 64, 65, 300])
 @pytest.mark.parametrize("ff,width", [(48, 64), (320, 256), (7, 54), (4096, 512)])
 def test_squared_relu_in_the_products(rows, ff, width):
