@@ -51,7 +51,7 @@ class WeightSpec(NamedTuple):
 @dataclass
 class Runtime:
     """Where and in which precision a model runs.  `dtype` is the dtype of activations and of the
-    cache: torch.bfloat16 (the serving path) or torch.float32 (everything in true 32-bit)."""
+    cache: torch.bfloat16 (the serving path) or torch.float32 (everything held and summed in 32 bits)."""
     device: torch.device
     dtype: torch.dtype
     shared: Dict[str, torch.Tensor] = field(default_factory=dict)     # tensors several parts read: one device copy each
