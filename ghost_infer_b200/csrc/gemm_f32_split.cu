@@ -26,15 +26,18 @@
 // An instruction takes 17 + 0.45 clocks a token when a warp issues it together and one lane is elected, and 96 or more when one thread
 // does so in a branch of its own (its operands then have to be brought together first).
 //
-// Steps of one token a sequence keep gemm_f32.cu's kernels (ops.one_token_step), which are bound by the bytes of W there; the
-// smaller matrices do as well, since a launch here has 10 us of set-up and pipeline to fill, longer than what they take there
-// (1,024 x 1,024: 12 us here for 16 rows, 12 there; 24 against 16 for 33).
+// Steps of one token a sequence keep gemm_f32.cu's kernels (ops.one_token_step): a layer of a 1B model takes 105 us here and 102
+// there with one to four sequences, the common case (119 and 164 with 16; the number of sequences must not decide, or a
+// token's bits would depend on it).  The smaller matrices do as well, since a launch here has 10 us of set-up and pipeline
+// to fill, longer than what they take there (1,024 x 1,024: 12 us here for 16 rows, 12 there; 24 against 16 for 33).
 // B200, cold L2, one launch beside one of gemm_f32.cu (us): 601 rows 16,384 x 2,048 234 (172 TFLOP/s) against 960; 2,048 x 8,192 136 against
 // 548; 64 rows 46 against 133 and 115 against 151; 16 rows 43 against 72 and 38 against 47; 4 rows 39 against 45 and 32 against 27.
-// What bounds it with many rows is a chunk's trips through shared memory (W in and out, tokens in and out: 170 KB, 1,330 clocks at 128
-// bytes a clock) beside its 24 instructions (1,400 clocks in tiles of 96), of 2,100 measured; with few rows the bytes of W.
+// What bounds it with many rows: tensor cores busy 57 % of the time, issue slots 55 % (splitting and draining warps), shared memory's
+// 128 bytes a clock about 60 % (W, tokens and their parts: 170 KB a chunk), one waiting for another; eight splitting warps in the
+// place of four were slower (601 rows 269 us), as was a first half split before its place is free (241).  With few rows: the bytes of W.
 // Distance from 64 bits (2-norms, random numbers): 0.84e-7 against 1.32e-7 (K 1,024), 0.92e-7 against 1.51e-7 (K 2,048), 1.3e-7
-// against 2.3e-7 (K 8,192); of one sign 0.64e-7 against 0.90e-7.
+// against 2.3e-7 (K 8,192); of one sign 0.64e-7 against 0.90e-7; rows of W with eight numbers 5.3e-8 against 5.9e-8, with one (where the
+// multiply-adds round once) 2.6e-8 against 2.5e-8.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <float.h>
