@@ -517,8 +517,8 @@ _one_token = contextvars.ContextVar("one_token_step", default=False)
 @contextlib.contextmanager
 def one_token_step(on: bool):
     """Around the products of a step that brings one token a sequence.  Such steps keep the plain 32-bit products,
-    bound by the bytes of the weights; all others, whatever their size, take the tensor cores' for larger matrices.  (One-token rows and prompt rows differ by rounding anyway: their attention is summed in another order.)  Held
-    per thread."""
+    bound by the bytes of the weights; all others, whatever their size, take the tensor cores' for larger matrices.  (One-token
+    rows and prompt rows differ by rounding anyway: their attention is summed in another order.)  Held per thread."""
     token = _one_token.set(bool(on))
     try:
         yield
